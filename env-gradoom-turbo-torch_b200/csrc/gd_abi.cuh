@@ -12,18 +12,14 @@
 #define GD_HOST_CHUNKS 4
 
 struct gd_renderer {
-  GdScene sc;
   int32_t header[GD_HDR_WORDS];
   const void *blobDev;
   int device;
   int maxThings;
   int ctas;
-  size_t smemBytes;          /* dynamic shared memory and staged tables with the whole 240-row frame on chip ... */
-  int stageMask;
-  size_t smemBytesView;      /* ... and with the 208 view rows only (calls that draw no status bar and want no full
-                                frame): the 10 KB go to more staged tables */
-  int stageMaskView;
-  int secWallsN, vtxWallsN, V;
+  size_t smemBytes;          /* dynamic shared memory per CTA */
+  bool chip;                 /* the walk's tables are in it */
+  GdParams base;             /* scene, table pointers and shared-memory offsets of every launch */
   /* gd_render_step_host overlaps the device->host copy of one lane chunk with
    * the drawing of the next on this side stream */
   cudaStream_t copyStream;
@@ -33,8 +29,52 @@ struct gd_renderer {
   int decalSlots;
   uint8_t *decalScratch;
   size_t decalScratchBytes;
+  GdSide *sides;             /* 2 W crossing records, the line of every fragment */
+  int *fragLine;
   GdWall *fragScratch;       /* ctas x F records, allocated with the renderer when the scene has split lines */
+  GdRow *fragRows;
 };
+
+/* Crossing records of the scene, once per renderer.  Texture indices are passed on as they are (the checked build
+ * tests them where they are drawn); sectors out of range count as absent. */
+__global__ void gd_side_setup_kernel(GdScene sc, GdSide *sides, int *fragLine) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= sc.W * 2) return;
+  const int w = i >> 1, side = i & 1;
+  if (side == 0 && sc.F > 0)
+    for (int f = sc.fragOff[w]; f < sc.fragOff[w + 1] && f < sc.F; ++f)
+      if (f >= 0) fragLine[f] = w;
+  int here = sc.wsec[i], there = sc.wsec[i ^ 1];
+  if (here < 0 || here >= sc.S) here = 0;
+  if (there < -1 || there >= sc.S) there = -1;
+  const bool oneSided = there < 0;
+  const int other = oneSided ? 0 : there;
+  const float vf = sc.secF[here * 2], vc = sc.secF[here * 2 + 1], of = sc.secF[other * 2], oc = sc.secF[other * 2 + 1];
+  const int4 ri = *reinterpret_cast<const int4 *>(&sc.secI[here * 4]), oi = *reinterpret_cast<const int4 *>(&sc.secI[other * 4]);
+  const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
+  const bool horizontal = fabsf(wl.w - wl.y) < 1e-6f, vertical = fabsf(wl.z - wl.x) < 1e-6f;
+  GdSide o;
+  for (int k = 0; k < 3; ++k) o.tex[k] = sc.sideTex[i * 3 + k];
+  o.contrast = vertical ? 16 : (horizontal ? -16 : 0);
+  o.tox = gd_rint(sc.sideOff[i * 2] * 65536.0f);
+  o.yoff = sc.sideOff[i * 2 + 1];
+  o.repeat = gd_rint(sc.wlen[w] * 65536.0f);
+  o.pad = 0;
+  unsigned f = GD_C_RASTER | GD_C_VALID;
+  const bool lightDiff = ri.x != oi.x;
+  if (oneSided || vc != oc || ri.z != oi.z || lightDiff) f |= GD_C_MARK_CEIL;
+  if (oneSided || vf != of || ri.y != oi.y || lightDiff) f |= GD_C_MARK_FLOOR;
+  if (oneSided) {
+    f |= GD_C_ONE_SIDED | (o.tex[0] >= 0 ? GD_C_TIER0 : 0u);
+  } else {
+    if (vf < of) f |= GD_C_LOWER | (o.tex[1] >= 0 ? GD_C_TIER1 : 0u);
+    if (vc > oc) f |= GD_C_UPPER | (o.tex[2] >= 0 ? GD_C_TIER2 : 0u);
+    if (vf > of) f |= GD_C_FLOOR_ABOVE;
+    if (vc < oc) f |= GD_C_CEIL_BELOW;
+  }
+  o.flags = f;
+  sides[i] = o;
+}
 
 static const void *gd_section(const uint8_t *dev, const int32_t *h, int s) { return dev + h[GD_HDR_SECTION0 + s]; }
 
@@ -60,20 +100,50 @@ extern "C" const char *gd_error_string(int code) {
  * kernel's static shared memory, so renderers of different scenes can live side
  * by side.  Returns that limit, or -1. */
 typedef void (*gd_kernel_fn)(const GdParams);
-/* the instantiation that draws a scene: with or without the code for split lines */
-static gd_kernel_fn gd_kernel_for(const GdScene &sc) { return sc.F > 0 ? gd_render_kernel<true> : gd_render_kernel<false>; }
+/* the instantiation that draws a scene: with or without the code for split lines, tables on chip or in scratch */
+static gd_kernel_fn gd_kernel_for(const gd_renderer *r) {
+  if (r->base.sc.F > 0) return r->chip ? gd_render_kernel<true, true> : gd_render_kernel<true, false>;
+  return r->chip ? gd_render_kernel<false, true> : gd_render_kernel<false, false>;
+}
 
 static int gd_raise_shared_limit(int maxOptin) {
   int limit = maxOptin;
-  const gd_kernel_fn kernels[2] = {gd_render_kernel<false>, gd_render_kernel<true>};
-  for (int k = 0; k < 2; ++k) {
+  const gd_kernel_fn kernels[4] = {gd_render_kernel<false, false>, gd_render_kernel<true, false>, gd_render_kernel<false, true>,
+                                   gd_render_kernel<true, true>};
+  for (int k = 0; k < 4; ++k) {
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, kernels[k]) != cudaSuccess) return -1;
     if (maxOptin - (int)fa.sharedSizeBytes < limit) limit = maxOptin - (int)fa.sharedSizeBytes;
   }
-  for (int k = 0; k < 2; ++k)
+  for (int k = 0; k < 4; ++k)
     if (cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) return -1;
   return limit;
+}
+
+/* Shared-memory offsets of a scene (r->base), with the walk's tables on chip or not; returns the total. */
+static size_t gd_layout(gd_renderer *r, int secWallsN, bool chip) {
+  GdParams &b = r->base;
+  const int W = b.sc.W, S = b.sc.S, F = b.sc.F;
+  size_t o = GD_OFF_HOT + (size_t)W * sizeof(GdHot);
+  auto take = [&o](size_t bytes) { const size_t at = o; o += gd_align16(bytes); return (int)at; };
+  b.offSectors = take((size_t)S * 16);
+  b.offSecOff = take(((size_t)S + 1) * 2);
+  b.offSecWalls = take((size_t)secWallsN * 2);
+  b.offVtx = take((size_t)W * 8);
+  b.offFrags = take((size_t)F * 4);
+  b.offActors = take((size_t)(r->maxThings > 0 ? r->maxThings : 1) * sizeof(GdActor));
+  if (chip) {
+    b.offRows = take(((size_t)W + F) * 4 * sizeof(GdRow));
+    b.offPrep = take((size_t)W * 16);
+    b.offPlanes = take((size_t)S * 2 * GD_PLANE_BYTES);
+    b.offSides = take((size_t)W * 2 * sizeof(GdSide));
+  } else {
+    b.offRows = 0;
+    b.offPrep = W * 4 * (int)sizeof(GdRow);
+    b.offPlanes = b.offPrep + W * 16;
+    b.offSides = 0;
+  }
+  return o;
 }
 
 extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob_dev, size_t blob_bytes, int device,
@@ -93,14 +163,15 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
   r->copyStream = nullptr;
   r->copiesDone = nullptr;
   r->decalScratch = nullptr;
-  r->fragScratch = nullptr;
+  r->fragScratch = nullptr; r->fragRows = nullptr; r->sides = nullptr; r->fragLine = nullptr;
   for (int c = 0; c < GD_HOST_CHUNKS; ++c) r->chunkDone[c] = nullptr;
   memcpy(r->header, h, sizeof r->header);
   r->device = device;
   r->blobDev = blob_dev;
   r->maxThings = max_things;
   const uint8_t *d = (const uint8_t *)blob_dev;
-  GdScene &sc = r->sc;
+  memset(&r->base, 0, sizeof r->base);
+  GdScene &sc = r->base.sc;
   sc.W = h[GD_H_WALLS]; sc.S = h[GD_H_SECTORS]; sc.T = h[GD_H_TEXTURES];
   sc.texH = h[GD_H_TEX_H]; sc.texW = h[GD_H_TEX_W];
   sc.P = h[GD_H_SPRITES]; sc.sprH = h[GD_H_SPR_H]; sc.sprW = h[GD_H_SPR_W];
@@ -144,42 +215,57 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
   sc.decalBlack = SECP(uint8_t, GD_S_DECAL_BLACK);
   sc.F = h[GD_H_FRAGMENTS]; sc.fragOff = SECP(int32_t, GD_S_FRAG_OFF); sc.fragFixed = SECP(int32_t, GD_S_FRAG_FIXED);
   r->decals = nullptr; r->decalSlots = 0; r->decalScratch = nullptr; r->decalScratchBytes = 0;
-  r->fragScratch = nullptr;
 #undef SECP
-  r->smemBytes = gd_shared_bytes(sc.W, max_things, GD_SCREEN_H);
-  r->smemBytesView = gd_shared_bytes(sc.W, max_things, GD_VH);
-  r->secWallsN = h[GD_H_SEC_WALLS_N]; r->vtxWallsN = h[GD_H_VTX_WALLS_N]; r->V = h[GD_H_VERTICES];
-  r->stageMask = r->stageMaskView = 0;
+  const int secWallsN = h[GD_H_SEC_WALLS_N];
+  if (secWallsN < 0 || secWallsN > 65535) { delete r; return GD_ERR_SIZE; }
   int prev = 0;
   if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) { delete r; return GD_ERR_CUDA; }
-  int maxOptin = 0, sms = 0;
+  int maxOptin = 0, perSmBytes = 0, reserved = 0, sms = 0;
   cudaDeviceGetAttribute(&maxOptin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  cudaDeviceGetAttribute(&perSmBytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+  cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   int rc = GD_OK;
   const int limit = gd_raise_shared_limit(maxOptin);
+  /* what one of two CTAs on an SM may take beside the kernel's static shared memory */
+  const size_t half = (size_t)(perSmBytes / 2 - reserved - (maxOptin - limit));
+  r->smemBytes = gd_layout(r, secWallsN, true);
+  r->chip = r->smemBytes <= half;
+  if (!r->chip) r->smemBytes = gd_layout(r, secWallsN, false);
   if (limit < 0) {
     rc = GD_ERR_CUDA;
-  } else if ((size_t)limit < r->smemBytes) {
+  } else if ((size_t)limit < r->smemBytes || (size_t)sc.W * 2 > GD_AUX_BYTES) {
     rc = GD_ERR_SHARED;
   } else {
-    /* stage as many topology tables as the SM's shared memory still holds */
-    for (int bit = 1; bit <= GD_STAGE_ROWPROJ; bit <<= 1) {
-      size_t extra = gd_stage_bytes(bit, sc.W, sc.S, r->V, r->secWallsN, r->vtxWallsN);
-      if (r->smemBytes + extra <= (size_t)limit) { r->smemBytes += extra; r->stageMask |= bit; }
-      if (r->smemBytesView + extra <= (size_t)limit) { r->smemBytesView += extra; r->stageMaskView |= bit; }
-    }
     int perSm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, gd_kernel_for(sc), GD_THREADS, r->smemBytes) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, gd_kernel_for(r), GD_THREADS, r->smemBytes) != cudaSuccess ||
         perSm < 1)
       rc = GD_ERR_CUDA;
     else
       r->ctas = sms * perSm;  /* one persistent CTA per resident slot */
   }
-  if (rc == GD_OK && sc.F > 0) {
-    void *mem = nullptr;
-    if (cudaMalloc(&mem, (size_t)r->ctas * sc.F * sizeof(GdWall)) != cudaSuccess) rc = GD_ERR_CUDA;
-    r->fragScratch = (GdWall *)mem;
+  if (rc == GD_OK) {
+    void *sides = nullptr, *mem = nullptr, *rows = nullptr;
+    const size_t sideBytes = (size_t)sc.W * 2 * sizeof(GdSide);
+    if (cudaMalloc(&sides, sideBytes + (size_t)sc.F * 4) != cudaSuccess) rc = GD_ERR_CUDA;
+    r->sides = (GdSide *)sides;
+    r->fragLine = (int *)((uint8_t *)sides + sideBytes);
+    if (rc == GD_OK && sc.F > 0) {
+      if (cudaMalloc(&mem, (size_t)r->ctas * sc.F * sizeof(GdWall)) != cudaSuccess) rc = GD_ERR_CUDA;
+      r->fragScratch = (GdWall *)mem;
+      if (!r->chip && cudaMalloc(&rows, (size_t)r->ctas * sc.F * 4 * sizeof(GdRow)) != cudaSuccess) rc = GD_ERR_CUDA;
+      r->fragRows = (GdRow *)rows;
+    }
+    if (rc == GD_OK) {
+      gd_side_setup_kernel<<<(sc.W * 2 + 127) / 128, 128>>>(sc, r->sides, r->fragLine);
+      if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) rc = GD_ERR_CUDA;
+    }
   }
+  r->base.maxThings = max_things;
+  r->base.sides = r->sides; r->base.fragLine = r->fragLine; r->base.fragScratch = r->fragScratch; r->base.fragRows = r->fragRows;
+  r->base.secWallsN = secWallsN;
+  r->base.perCta = gd_scratch_per_cta(sc.W, sc.S);
+  r->base.queueOffset = (size_t)r->ctas * r->base.perCta;
   r->copyStream = nullptr;
   r->copiesDone = nullptr;
   for (int c = 0; c < GD_HOST_CHUNKS; ++c) r->chunkDone[c] = nullptr;
@@ -206,6 +292,8 @@ extern "C" void gd_renderer_destroy(gd_renderer *r) {
   if (r->copyStream) cudaStreamDestroy(r->copyStream);
   if (r->decalScratch) cudaFree(r->decalScratch);
   if (r->fragScratch) cudaFree(r->fragScratch);
+  if (r->fragRows) cudaFree(r->fragRows);
+  if (r->sides) cudaFree(r->sides);
   if (switched) cudaSetDevice(prev);
   delete r;
 }
@@ -232,12 +320,12 @@ extern "C" int gd_renderer_bind_decals(gd_renderer *r, const void *decals, int s
 }
 
 extern "C" size_t gd_renderer_scratch_bytes(const gd_renderer *r) {
-  return r ? (size_t)r->ctas * gd_scratch_per_cta(r->sc.W, r->sc.S) + 16 : 0;
+  return r ? (size_t)r->ctas * r->base.perCta + 16 : 0;
 }
 
 extern "C" int gd_renderer_ctas(const gd_renderer *r) { return r ? r->ctas : 0; }
 extern "C" size_t gd_renderer_shared_bytes(const gd_renderer *r) { return r ? r->smemBytes : 0; }
-extern "C" size_t gd_renderer_shared_bytes_view(const gd_renderer *r) { return r ? r->smemBytesView : 0; }
+extern "C" size_t gd_renderer_shared_bytes_view(const gd_renderer *r) { return r ? r->smemBytes : 0; }
 
 static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing *things, int n, int flags,
                      uint8_t *stack, const uint8_t *reset_mask, uint8_t *obs_out, uint8_t *indexed_out,
@@ -254,21 +342,13 @@ static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing 
   uintptr_t align = (uintptr_t)lanes | (uintptr_t)things | (uintptr_t)stack | (uintptr_t)obs_out |
                     (uintptr_t)indexed_out | (uintptr_t)rgb_out | (uintptr_t)scratch;
   if (align & 15) return GD_ERR_ALIGN;
-  GdParams p;
-  p.sc = r->sc;
-  p.lanes = lanes; p.things = things; p.maxThings = r->maxThings; p.n = n; p.flags = flags;
+  GdParams p = r->base;
+  p.lanes = lanes; p.things = things; p.n = n; p.flags = flags;
   p.stack = stack; p.ringHead = ring_head; p.resetMask = reset_mask; p.obsOut = obs_out; p.indexedOut = indexed_out; p.rgbOut = rgb_out;
   p.scratch = (uint8_t *)scratch; p.status = status;
-  p.queueOffset = (size_t)r->ctas * gd_scratch_per_cta(r->sc.W, r->sc.S);
-  /* the status-bar rows of the frame stay off chip when nothing of this call shows them */
-  const bool viewOnly = (flags & GD_F_MASK_HUD) && !(flags & GD_F_DRAW_HUD) && !indexed_out && !rgb_out;
-  p.frameRows = viewOnly ? GD_VH : GD_SCREEN_H;
-  p.stageMask = viewOnly ? r->stageMaskView : r->stageMask;
-  p.secWallsN = r->secWallsN; p.vtxWallsN = r->vtxWallsN; p.V = r->V;
   p.decals = r->decals; p.decalSlots = r->decalSlots; p.decalScratch = r->decalScratch;
-  p.fragScratch = r->fragScratch;
   int grid = n < r->ctas ? n : r->ctas;
-  gd_kernel_for(r->sc)<<<grid, GD_THREADS, viewOnly ? r->smemBytesView : r->smemBytes, (cudaStream_t)stream>>>(p);
+  gd_kernel_for(r)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
 
@@ -421,8 +501,8 @@ extern "C" int gd_render_step_host(const gd_renderer *r, const int32_t *lanes_ho
 #define GD_STATIC_MAX_CTAS 32
 #define GD_STATIC_MAX_WALLS 256
 /* a scene of W walls has fewer than W sectors (three walls bound a sector, a wall bounds two) */
-#define GD_STATIC_PER_CTA ((GD_SCRATCH_FIXED + GD_STATIC_MAX_WALLS * 2 * GD_PLANE_ENTRY_BYTES + \
-                            GD_STATIC_MAX_WALLS * 4 * sizeof(GdRowProj) + 31) & ~(size_t)15)
+#define GD_STATIC_PER_CTA ((GD_SCRATCH_FIXED + GD_STATIC_MAX_WALLS * (2 * GD_PLANE_ENTRY_BYTES + 2 * GD_PLANE_BYTES + \
+                            sizeof(GdWall) + 4 * sizeof(GdRowProj) + 4 * sizeof(GdRow) + 16) + 127) & ~(size_t)63)
 #define GD_STATIC_SCRATCH_BYTES (GD_STATIC_MAX_CTAS * GD_STATIC_PER_CTA + 16)
 #define GD_STATIC_MAX_DEVICES 64
 
@@ -440,7 +520,7 @@ extern "C" int gd_render_step_static(const gd_renderer *r, const int32_t *lanes,
   if (!r || !lanes || !stack || !status) return GD_ERR_NULL;
   if (r->maxThings > 0 && !things) return GD_ERR_NULL;
   if (n < 0) return GD_ERR_SIZE;
-  if (r->sc.W > GD_STATIC_MAX_WALLS || r->sc.S > GD_STATIC_MAX_WALLS) return GD_ERR_STATIC_LIMIT;
+  if (r->base.sc.W > GD_STATIC_MAX_WALLS || r->base.sc.S > GD_STATIC_MAX_WALLS) return GD_ERR_STATIC_LIMIT;
   if (r->device < 0 || r->device >= GD_STATIC_MAX_DEVICES) return GD_ERR_STATIC_LIMIT;
   if (n == 0) return GD_OK;
   uintptr_t align = (uintptr_t)lanes | (uintptr_t)things | (uintptr_t)stack;
@@ -460,22 +540,18 @@ extern "C" int gd_render_step_static(const gd_renderer *r, const int32_t *lanes,
     scratch = (unsigned char *)address;
     gd_static_scratch_ptr[current] = scratch;
   }
-  GdParams p;
-  p.sc = r->sc;
-  p.lanes = lanes; p.things = (const gd_thing *)things; p.maxThings = r->maxThings; p.n = n;
+  GdParams p = r->base;
+  p.lanes = lanes; p.things = (const gd_thing *)things; p.n = n;
   p.flags = GD_F_STACK_ROLL | (mask_hud ? GD_F_MASK_HUD : GD_F_DRAW_HUD);
   p.stack = stack; p.ringHead = 0; p.resetMask = nullptr; p.obsOut = nullptr; p.indexedOut = nullptr; p.rgbOut = nullptr;
   p.scratch = scratch; p.status = status;
   /* lane queue: the last 16 bytes of the array; zero when the library is
    * loaded and left at zero by every launch */
   p.queueOffset = (size_t)GD_STATIC_MAX_CTAS * GD_STATIC_PER_CTA;
-  p.frameRows = GD_SCREEN_H; p.stageMask = r->stageMask;
-  p.secWallsN = r->secWallsN; p.vtxWallsN = r->vtxWallsN; p.V = r->V;
   p.decals = r->decals; p.decalSlots = r->decalSlots; p.decalScratch = r->decalScratch;
-  p.fragScratch = r->fragScratch;
   int grid = n < r->ctas ? n : r->ctas;
   if (grid > GD_STATIC_MAX_CTAS) grid = GD_STATIC_MAX_CTAS;
-  gd_kernel_for(r->sc)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
+  gd_kernel_for(r)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
 

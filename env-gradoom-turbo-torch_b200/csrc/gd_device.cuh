@@ -180,15 +180,62 @@ struct GdView {
   int flashLight;
 };
 
-/* Per-wall record kept in shared memory for the lane being drawn. */
+/* Per-wall record of the lane being drawn, in the CTA's scratch: what the slow path of the walk, the sprites and
+ * the middle textures read. */
 struct __align__(8) GdWall {
   i64 visL[2], visStep[2], visSl[2];  /* wallscan light per side */
   i64 sl, sr;                         /* projected half-open span (unbounded when rejected) */
   i64 dl, dr;                         /* clipped endpoint depths, 20.12 */
   int tx[2], ty[2];                   /* view coordinates in stored endpoint order */
-  short isl, isr;                     /* span owned by the column-ray test */
-  unsigned char hasColumns, frontF, oneSided, pad;
+  unsigned char frontF, oneSided;
 };
+
+/* What the column walk reads of a wall of the lane being drawn, kept in shared memory: the ray test's
+ * lane-dependent operands, the owned columns and the sectors on its two sides.  A wall outside the
+ * frustum has dn = 0 and an empty span, so no column ray ever meets it. */
+struct __align__(16) GdHot {
+  float segx, segy, offx, offy;   /* extent of the wall, and its start as seen from the viewer */
+  float dn;                       /* offx * segy - offy * segx: the column-independent numerator of the ray distance */
+  unsigned span;                  /* columns [span & 0xFFFF, span >> 16) owned by the column-ray test; 0xFFFF, 0: none */
+  int secs;                       /* front sector (low 16 bits), back sector (high 16 bits, -1: none) */
+  unsigned bits;                  /* GD_HOT_* and the projected span [sl, sr) clamped to -1 .. 321, stored + 1 */
+};
+#define GD_HOT_SL(b) ((int)((b) & 1023u) - 1)
+#define GD_HOT_SR(b) ((int)(((b) >> 10) & 1023u) - 1)
+#define GD_HOT_ONESIDED (1u << 20)
+#define GD_HOT_FRONT (1u << 21)
+#define GD_HOT_SPLIT (1u << 22)
+#define GD_HOT_NEIGHBOUR (1u << 23)   /* another line between the same two sectors shares an endpoint */
+#define GD_HOT_BRIDGE0 (1u << 24)     /* one-sided lines that may own the columns past its start, past its end */
+#define GD_HOT_BRIDGE1 (1u << 25)
+#define GD_HOT_STATIC (GD_HOT_SPLIT | GD_HOT_NEIGHBOUR | GD_HOT_BRIDGE0 | GD_HOT_BRIDGE1)
+
+/* Everything of a crossing that depends on the wall and the side it is seen from alone; built once per
+ * scene.  The flags assume that the sectors of the crossing are the wall's own two. */
+struct __align__(16) GdSide {
+  int tex[3];                     /* middle, lower, upper texture, -1: none */
+  int contrast;                   /* fake contrast: +16 vertical, -16 horizontal */
+  float yoff;
+  unsigned flags;                 /* GD_C_ONE_SIDED .. GD_C_CEIL_BELOW, static part */
+  i64 tox;                        /* texture x offset, 16.16 */
+  i64 repeat;                     /* wall length, 16.16 */
+  i64 pad;
+};
+
+/* flags of one crossing of a column */
+#define GD_C_RASTER 1u            /* draws, marks and clips */
+#define GD_C_ONE_SIDED 2u
+#define GD_C_MARK_CEIL 4u
+#define GD_C_MARK_FLOOR 8u
+#define GD_C_LOWER 16u            /* view floor below the other sector's */
+#define GD_C_UPPER 32u            /* view ceiling above the other sector's */
+#define GD_C_TIER0 64u            /* the tier has rows to draw: middle, lower, upper */
+#define GD_C_TIER1 128u
+#define GD_C_TIER2 256u
+#define GD_C_FLOOR_ABOVE 512u     /* view floor above the other sector's */
+#define GD_C_CEIL_BELOW 1024u     /* view ceiling below the other sector's */
+#define GD_C_PORTAL 2048u         /* a portal behind a projected solid contributes its clips */
+#define GD_C_VALID 4096u
 
 /* One clip event of a column: what a drawn seg contributes to sprite clipping
  * and to visplane ownership. Rows are 0..208 and fit a byte. */
@@ -203,6 +250,19 @@ struct __align__(4) GdEvent {
 };
 
 #define GD_MAX_EVENTS 48
+
+/* Row projection of one (wall or fragment, plane height) pair, the form the walk reads: the row is
+ * (a + x * step) >> 16 clamped to the view, with forced rows left of column `la` and from column `lb` on. */
+struct __align__(16) GdRow {
+  int a, step;
+  unsigned lim;                   /* la | lb << 10 | GD_ROW_* */
+  int vis;                        /* wallscan light of a side: origin in the side's floor row, step in its ceiling row */
+};
+#define GD_ROW_LEFT_TOP (1u << 20)    /* the rows forced on the left are row 0, else the bottom row */
+#define GD_ROW_RIGHT_TOP (1u << 21)
+#define GD_ROW_WIDE (1u << 22)        /* does not fit this form: take the full record */
+#define GD_ROW_LIGHT_WIDE (1u << 23)  /* the same of the light of the side */
+#define GD_ROW_PLAIN (1023u << 10)    /* no column is forced */
 
 /* Row projection of one (wall, plane height) pair: everything of the OWallMost
  * replay that does not depend on the screen column. */

@@ -230,7 +230,7 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int count = min(sh.misc[1], GD_FALLBACK_MAX);
   int *queue = (int *)sh.hitD;
-  unsigned *anchors = (unsigned *)sh.hitA;           /* [row][GD_WARPS] column bits */
+  unsigned *anchors = sh.anchors;                    /* [row][GD_WARPS] column bits */
   unsigned *owned = sh.masks + 7 * GD_SW;            /* drawn pixels are marked owned */
   if (tid == 0) { sh.misc[2] = GD_VH; sh.misc[3] = -1; sh.misc[11] = 0; }
   if (warp == 0) gd_flat_bounds_setup(sc, v, sh.misc);
@@ -243,7 +243,7 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
     if (!own.unresolved) {
       GdPlaneSpan p;
       gd_plane_setup(sc, sh.planeTab, own.sector, own.isFloor, px, p);
-      sh.frame[py * GD_SW + px] = (uint8_t)gd_plane_pixel<false>(p, v.center, gd_shared_addr(sh.yslope), gd_shared_addr(sh.colormap), py);
+      sh.frame[py * GD_SW + px] = (uint8_t)gd_plane_pixel(sc, p, v.center, py);
       atomicOr(&owned[(py >> 5) * GD_SW + px], 1u << (py & 31));
       queue[i] = -1;
     } else {
@@ -324,7 +324,7 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
     const bool isFloor = ((float)py - gd_flat_ray(sc, v, px).center) > 0;
     GdPlaneSpan p;
     gd_plane_setup(sc, sh.planeTab, sector, isFloor, px, p);
-    sh.frame[py * GD_SW + px] = (uint8_t)gd_plane_pixel<false>(p, v.center, gd_shared_addr(sh.yslope), gd_shared_addr(sh.colormap), py);
+    sh.frame[py * GD_SW + px] = (uint8_t)gd_plane_pixel(sc, p, v.center, py);
     atomicOr(&owned[(py >> 5) * GD_SW + px], 1u << (py & 31));
   }
   __syncthreads();

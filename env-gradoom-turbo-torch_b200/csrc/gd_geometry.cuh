@@ -101,17 +101,23 @@ __device__ __noinline__ void gd_project_fixed(const GdView &v, const i64 fx[2], 
 }
 
 /* Project wall w of the map for this lane (engine.py:10747-10869, 11207-11302,
- * 11359-11427).  The ray-owned span is completed by gd_wall_span below. */
-__device__ __forceinline__ void gd_project_wall(const GdScene &sc, const GdView &v, int w, GdWall &out) {
-  const float *wl = &sc.walls[w * 4];
-  const i64 fx[2] = {gd_rint(wl[0] * 65536.0f), gd_rint(wl[2] * 65536.0f)};
-  const i64 fy[2] = {gd_rint(wl[1] * 65536.0f), gd_rint(wl[3] * 65536.0f)};
+ * 11359-11427), and the lane-dependent operands of its column-ray test.  The
+ * ray-owned span is completed by gd_wall_spans below. */
+__device__ __forceinline__ void gd_project_wall(const GdScene &sc, const GdView &v, int w, GdWall &out, GdHot &hot) {
+  const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
+  const i64 fx[2] = {gd_rint(wl.x * 65536.0f), gd_rint(wl.z * 65536.0f)};
+  const i64 fy[2] = {gd_rint(wl.y * 65536.0f), gd_rint(wl.w * 65536.0f)};
   gd_project_fixed(v, fx, fy, out);
-  out.oneSided = gd_wsec(sc, w * 2 + 1) < 0;
-  float sx = wl[0], sy = wl[1];
-  float segx = wl[2] - sx, segy = wl[3] - sy;
-  float vfsx = v.x - sx, vfsy = v.y - sy;
-  out.frontF = (segx * vfsy - segy * vfsx) < 0;
+  const bool oneSided = gd_wsec(sc, w * 2 + 1) < 0;
+  const float segx = wl.z - wl.x, segy = wl.w - wl.y;
+  const float vfsx = v.x - wl.x, vfsy = v.y - wl.y;
+  const bool front = (segx * vfsy - segy * vfsx) < 0;
+  out.oneSided = oneSided; out.frontF = front;
+  hot.segx = segx; hot.segy = segy;
+  hot.offx = wl.x - v.x; hot.offy = wl.y - v.y;
+  hot.dn = hot.offx * segy - hot.offy * segx;
+  const unsigned sl = (unsigned)(gd_clamp(out.sl, -1, GD_SW + 1) + 1), sr = (unsigned)(gd_clamp(out.sr, -1, GD_SW + 1) + 1);
+  hot.bits = sl | (sr << 10) | (oneSided ? GD_HOT_ONESIDED : 0u) | (front ? GD_HOT_FRONT : 0u) | (hot.bits & GD_HOT_STATIC);
 }
 
 /* One piece of a line a node builder split (engine.py:11478-11500): projected like a line, from its
@@ -120,43 +126,28 @@ __device__ __forceinline__ void gd_project_fragment(const GdScene &sc, const GdV
   const int4 q = *reinterpret_cast<const int4 *>(&sc.fragFixed[f * 4]);
   const i64 fx[2] = {q.x, q.z}, fy[2] = {q.y, q.w};
   gd_project_fixed(v, fx, fy, out);
-  out.oneSided = 0; out.frontF = 0; out.hasColumns = 0; out.isl = 0; out.isr = 0; out.pad = 0;
+  out.oneSided = 0; out.frontF = 0;
 }
 
-/* Column-ray test of wall w at column x (engine.py:11317-11331).  Returns the
- * raw distance / along and the geometric-hit flag; span validity is applied by
- * gd_hit. */
-__device__ __forceinline__ void gd_ray_test(const GdScene &sc, const GdView &v, int w, float rx, float ry,
-                                            float &distance, float &along, bool &geo, bool &positive) {
-  const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
-  float sx = wl.x, sy = wl.y;
-  float segx = wl.z - sx, segy = wl.w - sy;
-  float offx = sx - v.x, offy = sy - v.y;
-  float den = rx * segy - ry * segx;
-  bool small = fabsf(den) < 1e-6f;
-  float safe = small ? 1.0f : den;
-  distance = (offx * segy - offy * segx) / safe;
-  along = (offx * ry - offy * rx) / safe;
-  positive = !small && distance > 0;
-  geo = positive && along >= 0 && along <= 1;
+/* Does the column ray (rx, ry) cross the wall (engine.py:11317-11331)?  The
+ * comparisons of the rounded quotients dn / den and an / den with 0 and 1 depend
+ * only on signs and magnitudes: both numerators are differences of products of
+ * map-scale numbers, so a nonzero one is far too large for its quotient to
+ * underflow, and a quotient of two floats rounds to at most 1 only when the
+ * numerator is not larger. */
+__device__ __forceinline__ bool gd_ray_geo(const GdHot &h, float rx, float ry) {
+  const float den = rx * h.segy - ry * h.segx;
+  const float safe = fabsf(den) < 1e-6f ? 1.0f : den;
+  const float an = h.offx * ry - h.offy * rx;
+  const bool positive = (h.dn != 0.0f) && ((h.dn < 0) == (safe < 0));
+  const bool alongOk = (an == 0.0f) || (((an < 0) == (safe < 0)) && fabsf(an) <= fabsf(safe));
+  return !(fabsf(den) < 1e-6f) && positive && alongOk;
 }
 
-/* Same test without the divisions, for the span sweep: the comparisons of the
- * rounded quotients with 0 and 1 depend only on signs and magnitudes. */
-__device__ __forceinline__ bool gd_ray_geo(const float4 wl, const GdView &v, float rx, float ry) {
-  float sx = wl.x, sy = wl.y;
-  float segx = wl.z - sx, segy = wl.w - sy;
-  float offx = sx - v.x, offy = sy - v.y;
-  float den = rx * segy - ry * segx;
-  bool small = fabsf(den) < 1e-6f;
-  float safe = small ? 1.0f : den;
-  float dn = offx * segy - offy * segx;
-  float an = offx * ry - offy * rx;
-  /* dn / safe > 0: both are differences of products of map-scale numbers, so a
-   * nonzero dn is far too large for the quotient to underflow to zero */
-  bool positive = (dn != 0.0f) && ((dn < 0) == (safe < 0));
-  bool alongOk = (an == 0.0f) || (((an < 0) == (safe < 0)) && fabsf(an) <= fabsf(safe));
-  return !small && positive && alongOk;
+/* Does the ray meet the wall's line in front of the viewer (the `positive` of engine.py:11317-11331)? */
+__device__ __forceinline__ bool gd_ray_meets_line(const GdHot &h, float rx, float ry) {
+  const float den = rx * h.segy - ry * h.segx;
+  return !(fabsf(den) < 1e-6f) && h.dn != 0.0f && ((h.dn < 0) == (den < 0));
 }
 
 /* ---- per (column, wall) hit -------------------------------------------- */
@@ -166,18 +157,21 @@ struct GdHit {
   bool geo, proj, left;
 };
 
-/* engine.py:11440-11459 */
-__device__ __forceinline__ GdHit gd_hit(const GdScene &sc, const GdView &v, const GdWall *walls, int w, int x,
-                                        float rx, float ry) {
+/* engine.py:11317-11331, 11440-11459 */
+__device__ __forceinline__ GdHit gd_hit(const GdScene &sc, int w, int x, float rx, float ry) {
   GdHit h;
-  float distance, along;
-  bool geo, positive;
   w = GD_CHECK_INDEX(w, sc.W);
-  gd_ray_test(sc, v, w, rx, ry, distance, along, geo, positive);
-  const GdWall &wv = walls[w];
-  bool screenValid = wv.hasColumns && x >= wv.isl && x < wv.isr;
-  bool pv = positive && screenValid;
-  bool valid = wv.oneSided ? (pv && wv.frontF) : (geo || pv);
+  const GdHot hot = gd_hot(w);
+  const float den = rx * hot.segy - ry * hot.segx;
+  const bool small = fabsf(den) < 1e-6f;
+  const float safe = small ? 1.0f : den;
+  const float distance = hot.dn / safe;
+  const float along = (hot.offx * ry - hot.offy * rx) / safe;
+  const bool positive = !small && distance > 0;
+  const int isl = (short)(hot.span & 0xFFFFu), isr = (int)(hot.span >> 16);
+  const bool geo = positive && along >= 0 && along <= 1;
+  const bool pv = positive && x >= isl && x < isr;
+  const bool valid = (hot.bits & GD_HOT_ONESIDED) ? (pv && (hot.bits & GD_HOT_FRONT)) : (geo || pv);
   h.d = valid ? distance : GD_INF;
   float ac = along;
   if (!(ac >= 0.0f)) ac = (ac != ac) ? ac : 0.0f;
@@ -185,28 +179,34 @@ __device__ __forceinline__ GdHit gd_hit(const GdScene &sc, const GdView &v, cons
   h.along = ac;
   h.geo = geo;
   h.proj = pv;
-  h.left = (x == wv.isl);
+  h.left = (x == isl);
   return h;
 }
 
-__device__ __noinline__ GdHit gd_hit_slow(const GdScene &sc_, const GdView &v_, const GdWall *walls, int w, int x,
-                                          float rx, float ry) {
+/* the same out of line, as three words */
+__device__ __noinline__ uint3 gd_hit_words(const GdScene &sc_, int w, int x, float rx, float ry) {
   const GdScene &sc = *gd_as_shared(&sc_);
-  const GdView &v = *gd_as_shared(&v_);
-  return gd_hit(sc, v, walls, w, x, rx, ry);
+  const GdHit h = gd_hit(sc, w, x, rx, ry);
+  return make_uint3(__float_as_uint(h.d), __float_as_uint(h.along), (h.geo ? 1u : 0u) | (h.proj ? 2u : 0u) | (h.left ? 4u : 0u));
+}
+__device__ __forceinline__ GdHit gd_hit_slow(const GdScene &sc, int w, int x, float rx, float ry) {
+  const uint3 q = gd_hit_words(sc, w, x, rx, ry);
+  GdHit h;
+  h.d = __uint_as_float(q.x); h.along = __uint_as_float(q.y);
+  h.geo = q.z & 1u; h.proj = (q.z & 2u) != 0; h.left = (q.z & 4u) != 0;
+  return h;
 }
 
 __device__ __forceinline__ float gd_tol(float d) { return fmaxf(fabsf(d) / 128.0f, 4.0f); }
 
 /* Endpoint owner of wall w at column x (engine.py:11589-11730). */
-__device__ __noinline__ void gd_endpoint_owner(const GdScene &sc_, const GdView &v_, const GdWall *walls, int w, int x, float rx,
-                                  float ry, const GdHit &hw, int &ownerIdx, float &ownerDist) {
+__device__ __noinline__ void gd_endpoint_owner(const GdScene &sc_, const GdWall *walls, int w, int x, float rx, float ry,
+                                               const GdHit &hw, int &ownerIdx, float &ownerDist) {
   const GdScene &sc = *gd_as_shared(&sc_);
-  const GdView &v = *gd_as_shared(&v_);
   const GdWall &wv = walls[w];
   float d = hw.d;
   float tol = gd_tol(d);
-  bool subpixel = (wv.sr - wv.sl <= 1) && !wv.oneSided;
+  bool subpixel = (wv.sr - wv.sl <= 1) && !(gd_hot(w).bits & GD_HOT_ONESIDED);
   bool usesStart = hw.along <= 0.5f;
   int oi = w;
   float od = d;
@@ -219,8 +219,8 @@ __device__ __noinline__ void gd_endpoint_owner(const GdScene &sc_, const GdView 
     bool rHas = usesStart ? hasS : hasE;
     int oIdx = usesStart ? eIdx : sIdx, oSlot = usesStart ? nd[3] : nd[2];
     bool oHas = usesStart ? hasE : hasS;
-    GdHit hr = (rIdx == w) ? hw : gd_hit(sc, v, walls, rIdx, x, rx, ry);
-    GdHit ho = (oIdx == w) ? hw : gd_hit(sc, v, walls, oIdx, x, rx, ry);
+    GdHit hr = (rIdx == w) ? hw : gd_hit_slow(sc, rIdx, x, rx, ry);
+    GdHit ho = (oIdx == w) ? hw : gd_hit_slow(sc, oIdx, x, rx, ry);
     bool rOwns = rHas && hr.proj && hr.left;
     bool oOwns = subpixel && oHas && ho.proj && ho.left && (fabsf(ho.d - d) <= tol);
     bool useO = oOwns && (!rOwns || ho.d < hr.d || (ho.d == hr.d && oSlot < rSlot));
@@ -234,7 +234,7 @@ __device__ __noinline__ void gd_endpoint_owner(const GdScene &sc_, const GdView 
 #pragma unroll 1
     for (int k = n0; k < n1; ++k) {
       int nb = GD_CHECK_INDEX(sc.nbIdx[k], sc.W), fl = sc.nbFlags[k];
-      GdHit hn = gd_hit(sc, v, walls, nb, x, rx, ry);
+      GdHit hn = gd_hit_slow(sc, nb, x, rx, ry);
       bool rayNb = usesStart ? (fl & 1) : ((fl >> 1) & 1);
       bool sel = rayNb || (subpixel && (fabsf(hn.d - d) <= tol));
       float cand = (hn.proj && hn.left && sel) ? hn.d : GD_INF;
@@ -249,26 +249,27 @@ __device__ __noinline__ void gd_endpoint_owner(const GdScene &sc_, const GdView 
   ownerDist = has ? od : d;
 }
 
-/* PrepWall for one (column, wall) (engine.py:10672-10739). */
-__device__ __noinline__ void gd_prep_wall(const GdScene &sc_, const GdWall &wv, int w, int x, i64 &hoff, i64 &vstep) {
-  const GdScene &sc = *gd_as_shared(&sc_);
-  i64 tx1 = wv.tx[0], tx2 = wv.tx[1], ty1 = wv.ty[0], ty2 = wv.ty[1];
-  double uozOrigin = (double)((float)tx1 * 160.0f);
-  double uozStep = (double)(-(float)ty1);
-  double invzOrigin = (double)((float)(tx1 - tx2) * 160.0f);
-  float invzStepF = (float)(ty2 - ty1);
-  double invzStep = (double)invzStepF;
-  double col = (double)x - 160.0;
-  double top = uozOrigin + uozStep * col;
-  double bottom = invzOrigin + invzStep * col;
-  double safeBottom = bottom == 0 ? 1.0 : bottom;
-  double fraction = top / safeBottom;
-  i64 repeat = gd_rint(sc.wlen[w] * 65536.0f);
+/* PrepWall (engine.py:10672-10739): the operands that depend on the wall alone, and the evaluation at
+ * one column.  `repeat`: the wall's length in 16.16. */
+__device__ __forceinline__ float4 gd_prep_setup(const GdWall &wv) {
+  const i64 tx1 = wv.tx[0], tx2 = wv.tx[1], ty1 = wv.ty[0], ty2 = wv.ty[1];
+  return make_float4((float)tx1 * 160.0f, (float)ty1, (float)(tx1 - tx2) * 160.0f, (float)(ty2 - ty1));
+}
+__device__ __forceinline__ void gd_prep_eval(const float4 q, i64 repeat, int x, i64 &hoff, i64 &vstep) {
+  const double col = (double)x - 160.0;
+  const double top = (double)q.x + (double)(-q.y) * col;
+  const double bottom = (double)q.z + (double)q.w * col;
+  const double safeBottom = bottom == 0 ? 1.0 : bottom;
+  const double fraction = top / safeBottom;
   hoff = (i64)floor(fraction * (double)repeat + 0.5);
   const double wms = (320 * 200.0 / 320.0 / 240) * 64.0 / (320 / 2.0);
-  double depthScale = (double)(invzStepF * (float)wms);
-  double depthOrigin = (double)((-(float)uozStep) * (float)wms);
+  const double depthScale = (double)(q.w * (float)wms);
+  const double depthOrigin = (double)(q.y * (float)wms);
   vstep = (i64)floor(fraction * depthScale + depthOrigin + 0.5);
+}
+__device__ __noinline__ void gd_prep_wall(const GdScene &sc_, const GdWall &wv, int w, int x, i64 &hoff, i64 &vstep) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  gd_prep_eval(gd_prep_setup(wv), gd_rint(sc.wlen[w] * 65536.0f), x, hoff, vstep);
 }
 
 /* OWallMost row projection (engine.py:12294-12605), one fragment per wall. */
@@ -366,8 +367,9 @@ __device__ __forceinline__ i64 gd_line_vis(const GdScene &sc, const GdWall *wall
   return q->visL[side] + ((i64)x - q->visSl[side]) * q->visStep[side];
 }
 
-/* Column-independent part of gd_project_rows for one (wall, height). */
-__device__ __noinline__ void gd_rowproj_setup(const GdView &v_, const GdWall &wv, float worldZ, GdRowProj &o) {
+/* Column-independent part of gd_project_rows for one (wall, height): the full record, and the form
+ * the walk reads (its `vis` word is the caller's). */
+__device__ __noinline__ void gd_rowproj_setup(const GdView &v_, const GdWall &wv, float worldZ, GdRowProj &o, GdRow &row) {
   const GdView &v = *gd_as_shared(&v_);
   i64 wsl = wv.sl, wsr = wv.sr;
   i64 wdl = gd_max(wv.dl, 1), wdr = gd_max(wv.dr, 1);
@@ -415,9 +417,53 @@ __device__ __noinline__ void gd_rowproj_setup(const GdView &v_, const GdWall &wv
   o.botA = (short)gd_clamp(botA, -1, GD_SW + 1); o.botB = (short)gd_clamp(botB, -1, GD_SW + 1);
   i64 pl = gd_div(num, gd_max(cdl, 1)), pr = gd_div(num, gd_max(cdr, 1));
   o.pl = pl;
-  o.pstep = gd_div(pr - pl, gd_max(cr - cl, 1));
+  const i64 pstep = gd_div(pr - pl, gd_max(cr - cl, 1));
+  o.pstep = pstep;
   o.cl = cl;
   o.pad = 0;
+  /* The walk's form computes center + pl + (x - cl) * pstep modulo 2^32, which is exact where the result fits: the
+   * row is linear, so it is enough to look at the first and last owned column that is not forced. */
+  unsigned lim = GD_ROW_PLAIN;
+  bool wide = false;
+  i64 a = v.center + pl - gd_wmul(cl, pstep), step = pstep;
+  if (entAbove || entBelow) {
+    lim = 1023u | (1023u << 10) | (entAbove ? GD_ROW_LEFT_TOP : 0u);
+    a = 0; step = 0;
+  } else {
+    int la = 0, lb = 1023;
+    const bool top = topA < topB, bottom = botA < botB;
+    if (bottom && belowL) la = o.botB;
+    if (bottom && belowR) lb = o.botA;
+    if (top && aboveL) { la = o.topB; lim |= GD_ROW_LEFT_TOP; }
+    if (top && aboveR) { lb = o.topA; lim |= GD_ROW_RIGHT_TOP; }
+    la = max(la, 0); lb = max(lb, 0);
+    if (la > lb) { if (lim & GD_ROW_LEFT_TOP) lb = la; else la = lb; }    /* where both reach a column, the top wins */
+    /* the one column exempt from both: next to the forced columns as a rule, where it moves their bound */
+    const int cx = o.collapsedX;
+    if (cx >= 0 && (cx < la || cx >= lb)) {
+      if (cx == la - 1) la = cx;
+      else if (cx == lb) lb = cx + 1;
+      else wide = true;
+    }
+    lim = (lim & ~GD_ROW_PLAIN) | (unsigned)la | ((unsigned)lb << 10);
+    const i64 x0 = gd_max(gd_max(wsl, 0), la), x1 = gd_min(gd_min(wsr, GD_SW), lb) - 1;
+    if (x0 <= x1) {
+      const i64 r0 = v.center + pl + gd_wmul(x0 - cl, pstep), r1 = v.center + pl + gd_wmul(x1 - cl, pstep);
+      wide = wide || r0 != (i64)(int)r0 || r1 != (i64)(int)r1;
+    }
+    wide = wide || (aboveL && belowL) || (aboveR && belowR);
+  }
+  if (wide) lim |= GD_ROW_WIDE;
+  row.a = (int)a; row.step = (int)step; row.lim = lim;
+}
+
+__device__ __forceinline__ int gd_row_eval(const GdRow &r, int x) {
+  int y = min(max((int)((unsigned)r.a + (unsigned)x * (unsigned)r.step) >> 16, 0), GD_VH);
+  if ((r.lim & 0xFFFFFu) != GD_ROW_PLAIN) {
+    if (x < (int)(r.lim & 1023u)) y = (r.lim & GD_ROW_LEFT_TOP) ? 0 : GD_VH;
+    if (x >= (int)((r.lim >> 10) & 1023u)) y = (r.lim & GD_ROW_RIGHT_TOP) ? 0 : GD_VH;
+  }
+  return y;
 }
 
 __device__ __forceinline__ int gd_rowproj_eval(const GdView &v, const GdWall &wv, const GdRowProj &o, int x) {
@@ -444,17 +490,17 @@ __device__ __forceinline__ int4 gd_sec_info(const GdScene &sc, int s) {
 }
 
 __device__ __forceinline__ bool gd_same_pair(const GdScene &sc, int a, int b) {
-  int a0 = gd_wsec(sc, a * 2), a1 = gd_wsec(sc, a * 2 + 1), b0 = gd_wsec(sc, b * 2), b1 = gd_wsec(sc, b * 2 + 1);
+  int a0 = gd_hot_front(a), a1 = gd_hot_back(a), b0 = gd_hot_front(b), b1 = gd_hot_back(b);
   return (a0 == b0 && a1 == b1) || (a0 == b1 && a1 == b0);
 }
 __device__ __forceinline__ bool gd_shares_endpoint(const GdScene &sc, int a, int b) {
-  int a0 = sc.wvtx[a * 2], a1 = sc.wvtx[a * 2 + 1], b0 = sc.wvtx[b * 2], b1 = sc.wvtx[b * 2 + 1];
+  int a0 = gd_vertex(sc, a, 0), a1 = gd_vertex(sc, a, 1), b0 = gd_vertex(sc, b, 0), b1 = gd_vertex(sc, b, 1);
   return a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1;
 }
 __device__ __noinline__ bool gd_opposing_pair(const GdScene &sc_, int a, int b) {
   const GdScene &sc = *gd_as_shared(&sc_);
   if (!gd_same_pair(sc, a, b)) return false;
-  if (gd_wsec(sc, a * 2 + 1) < 0 || gd_wsec(sc, b * 2 + 1) < 0) return false;
+  if (gd_hot_back(a) < 0 || gd_hot_back(b) < 0) return false;
   if (gd_shares_endpoint(sc, a, b)) return false;
   const float *A = &sc.walls[a * 4], *B = &sc.walls[b * 4];
   float adx = A[2] - A[0], ady = A[3] - A[1], bdx = B[2] - B[0], bdy = B[3] - B[1];
@@ -463,10 +509,10 @@ __device__ __noinline__ bool gd_opposing_pair(const GdScene &sc_, int a, int b) 
   return dot < 0 && fabsf(cross) < 1e-6f;
 }
 __device__ __forceinline__ bool gd_two_distinct(const GdScene &sc, int w) {
-  return gd_wsec(sc, w * 2 + 1) >= 0 && gd_wsec(sc, w * 2) != gd_wsec(sc, w * 2 + 1);
+  return gd_hot_back(w) >= 0 && gd_hot_front(w) != gd_hot_back(w);
 }
 __device__ bool gd_bridge_pair_of(const GdScene &sc, int a, int b, int &p0, int &p1) {
-  int a0 = gd_wsec(sc, a * 2), a1 = gd_wsec(sc, a * 2 + 1), b0 = gd_wsec(sc, b * 2), b1 = gd_wsec(sc, b * 2 + 1);
+  int a0 = gd_hot_front(a), a1 = gd_hot_back(a), b0 = gd_hot_front(b), b1 = gd_hot_back(b);
   int shared = 0, sv = -2;
   if (a0 == b0 || a0 == b1) { shared++; sv = a0; }
   if (a1 == b0 || a1 == b1) { shared++; sv = a1; }
@@ -476,7 +522,7 @@ __device__ bool gd_bridge_pair_of(const GdScene &sc, int a, int b, int &p0, int 
   return true;
 }
 __device__ __forceinline__ bool gd_set_equals(const GdScene &sc, int w, int p0, int p1) {
-  int s0 = gd_wsec(sc, w * 2), s1 = gd_wsec(sc, w * 2 + 1);
+  int s0 = gd_hot_front(w), s1 = gd_hot_back(w);
   if (p0 == p1) return s0 == p0 && s1 == p0;
   return (s0 == p0 && s1 == p1) || (s0 == p1 && s1 == p0);
 }
@@ -495,8 +541,8 @@ __device__ __noinline__ bool gd_portal_bridge(const GdScene &sc_, int slot, int 
   const GdScene &sc = *gd_as_shared(&sc_);
   index = 0;
   if (!gd_two_distinct(sc, path) || owner == path) return false;
-  int v = sc.wvtx[path * 2 + slot];
-  if (sc.wvtx[owner * 2] != v && sc.wvtx[owner * 2 + 1] != v) return false;
+  int v = gd_vertex(sc, path, slot);
+  if (gd_vertex(sc, owner, 0) != v && gd_vertex(sc, owner, 1) != v) return false;
   if (!gd_two_distinct(sc, owner)) return false;
   int p0, p1;
   if (!gd_bridge_pair_of(sc, path, owner, p0, p1)) return false;
@@ -508,7 +554,7 @@ __device__ __noinline__ bool gd_sector_bridge(const GdScene &sc_, int slot, int 
   if (!gd_two_distinct(sc, pending) || path == pending || !gd_two_distinct(sc, path)) return false;
   int p0, p1;
   if (!gd_bridge_pair_of(sc, pending, path, p0, p1)) return false;
-  return gd_unique_at_vertex(sc, sc.wvtx[pending * 2 + slot], pending, path, p0, p1, index);
+  return gd_unique_at_vertex(sc, gd_vertex(sc, pending, slot), pending, path, p0, p1, index);
 }
 
 /* ---- phase: ray-owned spans (engine.py:11333-11438) --------------------- */
@@ -528,48 +574,63 @@ __device__ __forceinline__ bool gd_wall_in_frustum(const float4 wl, const GdView
   return true;
 }
 
+/* Lists the walls that a column ray may cross, and with them wall 0 and the first blocking wall, which the
+ * rules fall back to; projects them; finds their ray-owned spans.  Every other wall gets the record no ray
+ * meets.  The list stays in aux until the walk begins. */
 __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShared &sh_) {
   const GdScene &sc = *gd_as_shared(&sc_);
   const GdView &v = *gd_as_shared(&v_);
   const GdShared &sh = *gd_as_shared(&sh_);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   GdWall *walls = sh.walls;
-  short *list = (short *)sh.hitD;           /* walls that need the sweep */
-  if (threadIdx.x == 0) sh.misc[2] = 0;
+  short *list = (short *)(gd_smem + GD_OFF_AUX);
+  int *listed = (int *)(gd_smem + GD_OFF_MISC) + 2;
+  if (threadIdx.x == 0) *listed = 0;
   __syncthreads();
+  const int block0 = GD_CHECK_INDEX(sc.blocking[0], sc.W);
   for (int w = threadIdx.x; w < sc.W; w += GD_THREADS) {
     const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
-    walls[w].isl = -1;
-    walls[w].isr = -1;
-    if (gd_wall_in_frustum(wl, v)) list[atomicAdd(&sh.misc[2], 1)] = (short)w;
+    if (gd_wall_in_frustum(wl, v) || w == 0 || w == block0) {
+      list[atomicAdd(listed, 1)] = (short)w;
+    } else {
+      gd_hot(w).dn = 0.0f;
+      gd_hot(w).span = 0xFFFFu;
+    }
   }
   __syncthreads();
-  const int n = sh.misc[2];
+  const int n = *listed;
+  for (int i = threadIdx.x; i < n; i += GD_THREADS) {
+    const int w = list[i];
+    gd_project_wall(sc, v, w, walls[w], gd_hot(w));
+  }
+  __syncthreads();
   float rxs[GD_SW / 32], rys[GD_SW / 32];
 #pragma unroll
   for (int chunk = 0; chunk < GD_SW / 32; ++chunk) gd_ray(v, chunk * 32 + lane, rxs[chunk], rys[chunk]);
-  /* first and last column whose ray crosses the wall, kept in isl / isr */
+  /* first and last column whose ray crosses the wall */
   for (int i = warp; i < n; i += GD_WARPS) {
     const int w = list[i];
-    const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
+    const GdHot h = gd_hot(w);
     int first = -1, last = -1;
 #pragma unroll
     for (int chunk = 0; chunk < GD_SW / 32; ++chunk) {
-      unsigned m = __ballot_sync(0xffffffffu, gd_ray_geo(wl, v, rxs[chunk], rys[chunk]));
+      unsigned m = __ballot_sync(0xffffffffu, gd_ray_geo(h, rxs[chunk], rys[chunk]));
       if (m) {
         if (first < 0) first = chunk * 32 + __ffs(m) - 1;
         last = chunk * 32 + 31 - __clz(m);
       }
     }
-    if (lane == 0) { walls[w].isl = (short)first; walls[w].isr = (short)last; }
+    if (lane == 0) gd_hot(w).span = ((unsigned)first & 0xFFFFu) | ((unsigned)(last + 1) << 16);
   }
   __syncthreads();
-  for (int w = threadIdx.x; w < sc.W; w += GD_THREADS) {
-    GdWall &wv = walls[w];
-    const int first = wv.isl, last = wv.isr;
+  for (int i = threadIdx.x; i < n; i += GD_THREADS) {
+    const int w = list[i];
+    const GdWall &wv = walls[w];
+    GdHot &hot = gd_hot(w);
+    const int first = (short)(hot.span & 0xFFFFu), end = (int)(hot.span >> 16);
     bool hasColumns = first >= 0;
     i64 isl = hasColumns ? first : 0;
-    i64 isr = hasColumns ? last + 1 : GD_SW;
+    i64 isr = hasColumns ? end : GD_SW;
     const i64 cf = 160 * GD_FU;
     i64 ecol[2];
     bool evis[2];
@@ -581,7 +642,7 @@ __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShar
       ecol[e] = (pf >> 16) + (tx >= 0);
       evis[e] = ty > 0 && tx >= -ty && tx <= ty && ecol[e] >= 0 && ecol[e] <= GD_SW;
     }
-    bool fff = wv.frontF;
+    bool fff = (hot.bits & GD_HOT_FRONT) != 0;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       bool visible = evis[e] && hasColumns;
@@ -595,9 +656,7 @@ __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShar
       hasColumns = isr > isl;
     }
     hasColumns = hasColumns && (wv.sr > wv.sl);
-    wv.isl = (short)isl;
-    wv.isr = (short)isr;
-    wv.hasColumns = hasColumns;
+    hot.span = ((unsigned)isl & 0xFFFFu) | (hasColumns ? (unsigned)isr << 16 : 0u);
   }
 }
 
@@ -606,23 +665,17 @@ __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShar
  * lowest wall index, as the reference's first-minimum over its ascending
  * blocking list.  Only walls that passed the frustum test can be crossed, and
  * the division is spent only on walls the sign test says are crossed. */
-__device__ void gd_blocking_raycast(const GdScene &sc_, const GdView &v_, const GdShared &sh_, const short *list, int listed,
-                                    float rx, float ry, float &wallDistance, int &blockingWall) {
+__device__ void gd_blocking_raycast(const GdScene &sc_, const short *list, int listed, float rx, float ry, float &wallDistance,
+                                    int &blockingWall) {
   const GdScene &sc = *gd_as_shared(&sc_);
-  const GdView &v = *gd_as_shared(&v_);
-  const GdShared &sh = *gd_as_shared(&sh_);
   float best = GD_INF;
   int bestWall = GD_CHECK_INDEX(sc.blocking[0], sc.W);
 #pragma unroll 1
   for (int i = 0; i < listed; ++i) {
     const int w = list[i];
-    if (!sh.walls[w].oneSided) continue;
-    const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
-    if (!gd_ray_geo(wl, v, rx, ry)) continue;
-    float distance, along;
-    bool geo, positive;
-    gd_ray_test(sc, v, w, rx, ry, distance, along, geo, positive);
-    float d = geo ? distance : GD_INF;
+    const GdHot h = gd_hot(w);
+    if (!(h.bits & GD_HOT_ONESIDED) || !gd_ray_geo(h, rx, ry)) continue;
+    const float d = h.dn / (rx * h.segy - ry * h.segx);
     if (d < best || (d == best && w < bestWall && isfinite(d))) { best = d; bestWall = w; }
   }
   blockingWall = bestWall;

@@ -459,7 +459,7 @@ extern "C" int gd_player_tics(const gd_renderer *r, int32_t *players, const uint
   if (cudaGetDevice(&current) != cudaSuccess) return GD_ERR_CUDA;
   if (current != r->device) return GD_ERR_DEVICE;
   GdMoveParams q;
-  const GdScene &sc = r->sc;
+  const GdScene &sc = r->base.sc;
   q.map.W = sc.W; q.map.S = sc.S; q.map.nStarts = r->header[GD_H_STARTS];
   q.map.walls = sc.walls; q.map.wsec = sc.wsec; q.map.edgeOff = sc.edgeOff; q.map.edgeWalls = sc.edgeWalls;
   q.map.fineSine = sc.fineSine; q.map.secF = sc.secF;

@@ -1,24 +1,35 @@
 /*
  * Fused render-to-observation kernel for sm_100a.
  *
- * One persistent CTA of 320 threads draws one environment lane at a time:
- *   1. every wall of the map is projected once per lane into shared memory
- *      (threads over walls), and its ray-owned column span is found by a warp
- *      sweeping the 320 column rays with ballots;
+ * One persistent CTA of 320 threads draws one environment lane at a time, two
+ * CTAs to an SM:
+ *   1. the walls that a column ray may cross are listed and projected once per
+ *      lane, and their ray-owned column spans are found by warps sweeping the
+ *      320 column rays with ballots;
  *   2. thread x then walks column x front to back through the sector portals,
  *      keeping the ceiling / floor clip pair in registers, drawing wall tiers
  *      and the visplane rows they uncover straight into the palette-indexed
- *      frame held in shared memory (aligned groups of four columns exchange
- *      their tier bounds with warp shuffles);
- *   3. thread x draws the depth-sorted sprites of column x against the clip
- *      events its walk recorded;
+ *      frame (aligned groups of four columns exchange their tier bounds with
+ *      warp shuffles);
+ *   3. the depth-sorted sprites are drawn against the clip events the walk
+ *      recorded for the columns they may cover;
  *   4. the weapon and, on request, the status bar are composited;
  *   5. the 320x240 frame is reduced to the 84x84 grayscale observation with the
  *      exact integer area weights and written, 16 bytes per store, into the
  *      four-frame stack; the RGB24 frame is written only when asked for.
- * Only the lane record, the thing records and the stack slot touch HBM; the
- * indexed frame never leaves the SM.  Tensor cores are unused: nothing here is
- * a contraction.
+ * Only the lane record, the thing records and the stack slots have to cross
+ * HBM; the indexed frame, the clip events and the CTA's tables stay in L2.
+ * Tensor cores are unused: nothing here is a contraction.
+ *
+ * What bounds it is the supply of instructions: the whole kernel is far larger
+ * than the instruction caches, so a phase costs what its code costs to fetch
+ * and its chains to wait for.  Measured with one 10-warp CTA per SM (frame in
+ * shared memory, every rule of the walk in its loop): 5.17 ms per 4096 lanes of
+ * the 64-sector map, 32.0 ms per 8192 lanes of the 256-sector map; two such
+ * CTAs per SM were slower (5.95 ms: warps waiting for instructions went from
+ * 0.9 to 5.0 per issue).  With the plain crossings decided apart from the full
+ * set of rules and the walk's tables in 16-byte records, two CTAs per SM take
+ * 3.99 and 20.2 ms.
  *
  * The arithmetic restates src/gradoom/engine.py (file:line beside each
  * function) and must stay bit-identical to it; compile with -fmad=false.
@@ -52,26 +63,42 @@ struct GdParams {
   uint8_t *indexedOut;       /* n x 240 x 320, optional */
   uint8_t *rgbOut;           /* n x 240 x 320 x 3, optional */
   uint8_t *scratch;          /* ctas x gd_scratch_per_cta(W), then the lane queue (2 words, zero between launches) */
-  size_t queueOffset;
-  int stageMask;             /* which scene tables each CTA copies into shared memory */
-  int frameRows;             /* rows of the frame kept in shared memory: GD_VIEW_H when neither the status bar
-                                nor a full frame is wanted (the 32 rows make room for more tables), else GD_SCREEN_H */
-  int secWallsN, vtxWallsN, V;
+  size_t queueOffset, perCta;
+  const GdSide *sides;       /* 2 W crossing records (built with the renderer) */
+  const int *fragLine;       /* F: the line of each projection fragment */
+  /* byte offsets in shared memory; those of the last four are offsets into the CTA's scratch tables when
+   * they do not fit on chip (kChip false) */
+  int offSectors, offSecOff, offSecWalls, offVtx, offFrags, offActors;
+  int offRows, offPrep, offPlanes, offSides;
+  int secWallsN;
   int *status;
   const gd_decal *decals;    /* n x decalSlots rings of bullet chips, or null */
   int decalSlots;
   uint8_t *decalScratch;     /* ctas x gd_decal_scratch_per_cta(decalSlots) */
   GdWall *fragScratch;       /* ctas x F fragment records, when the scene has split lines */
+  GdRow *fragRows;           /* ctas x F x 4 row projections of the fragments, when they are not on chip */
 };
 
 #define GD_SCRATCH_EVENTS_BYTES (GD_MAX_EVENTS * GD_SW * (int)sizeof(GdEvent))
 #define GD_SCRATCH_VSEC_BYTES (GD_VH * GD_SW * 2)   /* flat fallback: vertically repaired sector per pixel */
-#define GD_SCRATCH_FIXED (GD_SCRATCH_EVENTS_BYTES + GD_SW * 4 + GD_SCRATCH_VSEC_BYTES)
+#define GD_SCRATCH_ANCHOR_BYTES (GD_VH * GD_WARPS * 4)
+#define GD_SCRATCH_VSEC (GD_SCRATCH_EVENTS_BYTES + GD_SW * 4)
+#define GD_SCRATCH_ANCHORS (GD_SCRATCH_VSEC + GD_SCRATCH_VSEC_BYTES)
+#define GD_SCRATCH_FRAME (GD_SCRATCH_ANCHORS + GD_SCRATCH_ANCHOR_BYTES)
+#define GD_SCRATCH_FIXED (GD_SCRATCH_FRAME + GD_SCREEN_H * GD_SW)
 #define GD_PLANE_ENTRY_BYTES 88          /* sizeof(GdPlaneEntry), checked below */
-__host__ __device__ inline size_t gd_scratch_plane_bytes(int S) { return ((size_t)S * 2 * GD_PLANE_ENTRY_BYTES + 15) & ~(size_t)15; }
-__host__ __device__ inline size_t gd_scratch_per_cta(int W, int S) {
-  return (GD_SCRATCH_FIXED + gd_scratch_plane_bytes(S) + (size_t)W * 4 * sizeof(GdRowProj) + 15) & ~(size_t)15;
+#define GD_PLANE_BYTES 48                /* sizeof(GdPlane), checked below */
+/* After the fixed part: the full wall records, the full row projections, the full span setups, and the tables of
+ * the walk, which live here when they do not fit in shared memory: row projections, column operands, span setups. */
+__host__ __device__ inline size_t gd_align16(size_t v) { return (v + 15) & ~(size_t)15; }
+__host__ __device__ inline size_t gd_scratch_walls(int, int) { return gd_align16(GD_SCRATCH_FIXED); }
+__host__ __device__ inline size_t gd_scratch_rowproj(int W, int) { return gd_scratch_walls(0, 0) + gd_align16((size_t)W * sizeof(GdWall)); }
+__host__ __device__ inline size_t gd_scratch_planes(int W, int S) { return gd_scratch_rowproj(W, S) + gd_align16((size_t)W * 4 * sizeof(GdRowProj)); }
+__host__ __device__ inline size_t gd_scratch_tables(int W, int S) { return gd_scratch_planes(W, S) + gd_align16((size_t)S * 2 * GD_PLANE_ENTRY_BYTES); }
+__host__ __device__ inline size_t gd_table_bytes(int W, int S) {
+  return (size_t)W * 4 * sizeof(GdRow) + (size_t)W * 16 + (size_t)S * 2 * GD_PLANE_BYTES;
 }
+__host__ __device__ inline size_t gd_scratch_per_cta(int W, int S) { return gd_scratch_tables(W, S) + gd_table_bytes(W, S); }
 
 struct GdActor {
   float x, y, depth;
@@ -83,80 +110,61 @@ struct GdActor {
   unsigned char alive;
 };
 
-/* ---- shared memory carve-up -------------------------------------------- */
+/* ---- shared memory ------------------------------------------------------- */
+/* The CTA's shared memory begins with these fixed areas; the walls' records follow, then the tables whose
+ * sizes depend on the scene (offsets in GdParams).  The palette-indexed frame itself lives in the CTA's
+ * scratch, which stays in L2: its pixels are stored once each, a warp's 32 columns of a row in one sector,
+ * and the 77 KB that leaves free on chip let two lanes share an SM. */
+#define GD_OFF_COLORMAP 0                                  /* 32 x 256 */
+#define GD_OFF_PAL64 (GD_OFF_COLORMAP + 32 * 256)          /* 256: R | G<<20 | B<<40 */
+#define GD_OFF_PAL32 (GD_OFF_PAL64 + 256 * 8)              /* 256: r | g << 8 | b << 16, for the RGB24 output */
+#define GD_OFF_YSLOPE (GD_OFF_PAL32 + 256 * 4)             /* 208 */
+#define GD_OFF_LANE (GD_OFF_YSLOPE + GD_VIEW_H * 4)        /* 32 */
+#define GD_OFF_OWNER (GD_OFF_LANE + GD_LANE_WORDS * 4)     /* 10 words of column bits: boundary_has_projected_owner; words 16..25: the
+                                                              walk may go on after leaving the map; words 32..41: some wall's
+                                                              projected span starts here */
+#define GD_OWNER_WORDS 48
+#define GD_OFF_MISC (GD_OFF_OWNER + GD_OWNER_WORDS * 4)                   /* 16 ints: start sector, fallback queue length, its unresolved
+                                                              rows' range, GdFlatBounds */
+#define GD_OFF_MASKS (GD_OFF_MISC + 64)                    /* 14 x 320: per-column filled / plane-owned row bitmasks */
+#define GD_OFF_MASKED_DIST (GD_OFF_MASKS + 14 * 320 * 4)   /* 320: nearest masked drawseg of the column ... */
+#define GD_OFF_MASKED_INFO (GD_OFF_MASKED_DIST + 320 * 4)  /* ... its wall << 16 | ceiling clip << 8 | floor clip; 0xFFFF0000 | .. = none */
+#define GD_OFF_CAND (GD_OFF_MASKED_INFO + 320 * 4)         /* 320 x 64 bits: things that may show in the column */
+#define GD_OFF_AUX (GD_OFF_CAND + 320 * 8)                 /* 10,240 bytes for one phase at a time: listed walls, fallback queue,
+                                                              chip ranks, status-bar list, 84 x 84 result */
+#define GD_AUX_BYTES (8 * 320 * 4)
+#define GD_OFF_AUX2 (GD_OFF_AUX + GD_AUX_BYTES)            /* 4,096: sectors of points, sprite columns, chip spans */
+#define GD_OFF_HOT (GD_OFF_AUX2 + 4096)                    /* W wall records */
+static_assert(GD_OFF_HOT % 16 == 0 && GD_OFF_AUX % 16 == 0, "vector loads");
+
 struct GdPlaneEntry;
 
 struct GdShared {
   GdPlaneEntry *planeTab; /* scratch: per (sector, floor/ceiling) span setup of the lane being drawn */
-  uint8_t *frame;       /* 240 x 320 */
-  uint8_t *colormap;    /* 32 x 256 */
-  uint8_t *playpal;     /* 768 */
-  unsigned *yslope;     /* 208 */
-  int32_t *lane;        /* 32 */
-  float *wallDistance;  /* 320 */
-  short *blockingWall;  /* 320 */
-  unsigned *ownerMask;  /* 10 words: boundary_has_projected_owner; words 16..25: columns whose walk goes on after leaving the map */
-  GdWall *walls;        /* W */
+  uint8_t *frame;       /* scratch: 240 x 320 */
+  uint8_t *colormap;
+  int32_t *lane;
+  unsigned *ownerMask;
+  GdWall *walls;        /* scratch: W, the listed ones filled */
   GdWall *frags;        /* scratch: F projection fragments of split lines (only their spans, depths and light) */
+  unsigned *anchors;    /* scratch: flat fallback */
   GdActor *actors;      /* maxThings */
-  unsigned long long *pal64;  /* 256: R | G<<20 | B<<40 */
-  uint8_t *obs;         /* 84 x 84; shares the memory of hitD, which is free once the sprites are drawn */
-  int *misc;            /* 16 ints: start sector, fallback queue length, its unresolved rows' range, GdFlatBounds */
-  unsigned *masks;      /* 14 x 320: per-column filled / plane-owned row bitmasks */
-  unsigned *pal32;      /* 256: the lane's palette as r | g << 8 | b << 16, for the RGB24 output */
-  float *maskedDist;    /* 320: nearest masked drawseg of the column ... */
-  unsigned *maskedInfo; /* ... its wall << 16 | ceiling clip << 8 | floor clip; 0xFFFF0000 | .. = none */
-  float *hitD, *hitA;   /* 8 x 320 each: per-column cache of this iteration's wall hits */
-  uint8_t *hitF;        /* 8 x 320 */
+  unsigned long long *pal64;
+  uint8_t *obs;         /* 84 x 84; aux */
+  int *misc;
+  unsigned *masks;
+  unsigned *pal32;
+  float *maskedDist;
+  unsigned *maskedInfo;
+  float *hitD, *hitA;   /* the two aux areas */
+  const unsigned short *secOff, *secWalls;   /* incident walls of every sector */
 };
 
-__host__ __device__ inline size_t gd_align16(size_t v) { return (v + 15) & ~(size_t)15; }
-
-__host__ __device__ inline size_t gd_shared_bytes(int W, int maxThings, int frameRows) {
-  size_t b = 0;
-  b += gd_align16((size_t)frameRows * GD_SW);
-  b += gd_align16(32 * 256);
-  b += gd_align16(768);
-  b += gd_align16(GD_VH * 4);
-  b += gd_align16(GD_LANE_WORDS * 4);
-  b += gd_align16(GD_SW * 4);
-  b += gd_align16(GD_SW * 2);
-  b += gd_align16(32 * 4);
-  b += gd_align16(256 * 8);
-  b += gd_align16(64);
-  b += gd_align16(14 * GD_SW * 4);
-  b += 2 * gd_align16(GD_SW * 4);
-  b += gd_align16(256 * 4);
-  b += 2 * gd_align16(8 * GD_SW * 4) + gd_align16(8 * GD_SW);
-  b += gd_align16((size_t)W * sizeof(GdWall));
-  b += gd_align16((size_t)(maxThings > 0 ? maxThings : 1) * sizeof(GdActor));
-  return b;
-}
-
-__device__ inline void gd_carve(uint8_t *base, int W, int maxThings, int frameRows, GdShared &s) {
-  size_t o = 0;
-  s.frame = base + o; o += gd_align16((size_t)frameRows * GD_SW);
-  s.colormap = base + o; o += gd_align16(32 * 256);
-  s.playpal = base + o; o += gd_align16(768);
-  s.yslope = (unsigned *)(base + o); o += gd_align16(GD_VH * 4);
-  s.lane = (int32_t *)(base + o); o += gd_align16(GD_LANE_WORDS * 4);
-  s.wallDistance = (float *)(base + o); o += gd_align16(GD_SW * 4);
-  s.blockingWall = (short *)(base + o); o += gd_align16(GD_SW * 2);
-  s.ownerMask = (unsigned *)(base + o); o += gd_align16(32 * 4);
-  s.pal64 = (unsigned long long *)(base + o); o += gd_align16(256 * 8);
-  s.misc = (int *)(base + o); o += gd_align16(64);
-  s.masks = (unsigned *)(base + o); o += gd_align16(14 * GD_SW * 4);
-  s.maskedDist = (float *)(base + o); o += gd_align16(GD_SW * 4);
-  s.maskedInfo = (unsigned *)(base + o); o += gd_align16(GD_SW * 4);
-  s.pal32 = (unsigned *)(base + o); o += gd_align16(256 * 4);
-  s.hitD = (float *)(base + o); o += gd_align16(8 * GD_SW * 4);
-  s.hitA = (float *)(base + o); o += gd_align16(8 * GD_SW * 4);
-  s.hitF = base + o; o += gd_align16(8 * GD_SW);
-  s.obs = (uint8_t *)s.hitD;
-  static_assert(8 * GD_SW * 4 >= GD_OBS * GD_OBS && 8 * GD_SW * 4 >= (GD_HUD_MAX_PATCHES + 1) * 16, "obs aliases hitD");
-  s.walls = (GdWall *)(base + o); o += gd_align16((size_t)W * sizeof(GdWall));
-  s.actors = (GdActor *)(base + o);
-}
+__device__ __forceinline__ GdHot &gd_hot(int w) { return reinterpret_cast<GdHot *>(gd_smem + GD_OFF_HOT)[w]; }
+__device__ __forceinline__ int gd_hot_front(int w) { return (int)(short)(gd_hot(w).secs & 0xFFFF); }
+__device__ __forceinline__ int gd_hot_back(int w) { return gd_hot(w).secs >> 16; }
+/* endpoint vertex of a wall: the scene's `wvtx` holds 32-bit ids in global memory, this copy is on chip */
+__device__ __forceinline__ int gd_vertex(const GdScene &sc, int w, int slot) { return gd_as_shared(sc.wvtx)[w * 2 + slot]; }
 
 #include "gd_geometry.cuh"
 #include "gd_walk.cuh"
@@ -167,65 +175,83 @@ __device__ inline void gd_carve(uint8_t *base, int W, int maxThings, int frameRo
 
 /* ---- the kernel ----------------------------------------------------------- */
 
-/* Two instantiations: kSplit = the scene carries projection fragments of split lines. */
-template <bool kSplit>
-__global__ void __launch_bounds__(GD_THREADS, 1) gd_render_kernel(const GdParams p) {
+/* kSplit: the scene carries projection fragments of split lines.  kChip: the walk's tables fit in shared memory
+ * beside a second CTA. */
+template <bool kSplit, bool kChip>
+__global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_constant__ GdParams p) {
   /* The scene descriptor, the shared-memory map and the lane's view are read by
-   * every helper through references; keeping them in shared memory (one copy
+   * the phases around the walk through references; keeping them in shared memory (one copy
    * per CTA) keeps those reads off the per-thread stack. */
   __shared__ GdScene sScene;
   __shared__ GdShared sShared;
   __shared__ GdView sView;
   const int tid = threadIdx.x;
-  GdRowProj *stagedRowproj = nullptr;
-  {
+  uint8_t *myScratch = p.scratch + (size_t)blockIdx.x * p.perCta;
+  uint8_t *tables = myScratch + gd_scratch_tables(p.sc.W, p.sc.S);
+  uint8_t *frame = myScratch + GD_SCRATCH_FRAME;
+  if (tid == 0) {
     GdScene sc = p.sc;
     GdShared sh;
-    gd_carve(gd_smem, sc.W, p.maxThings, p.frameRows, sh);
-    uint8_t *cursor = gd_smem + gd_shared_bytes(sc.W, p.maxThings, p.frameRows);
-    const int m = p.stageMask;
-    if (m & GD_STAGE_WALLS) sc.walls = (const float *)gd_stage_copy(cursor, sc.walls, (size_t)sc.W * 16);
-    if (m & GD_STAGE_WSEC) sc.wsec = (const int32_t *)gd_stage_copy(cursor, sc.wsec, (size_t)sc.W * 8);
-    if (m & GD_STAGE_SECLIST) {
-      sc.secOff = (const int32_t *)gd_stage_copy(cursor, sc.secOff, (size_t)(sc.S + 1) * 4);
-      sc.secWalls = (const int32_t *)gd_stage_copy(cursor, sc.secWalls, (size_t)(p.secWallsN > 0 ? p.secWallsN : 1) * 4);
-    }
-    if (m & GD_STAGE_SECTORS) {
-      sc.secF = (const float *)gd_stage_copy(cursor, sc.secF, (size_t)sc.S * 8);
-      sc.secI = (const int32_t *)gd_stage_copy(cursor, sc.secI, (size_t)sc.S * 16);
-    }
-    if (m & GD_STAGE_WVTX) sc.wvtx = (const int32_t *)gd_stage_copy(cursor, sc.wvtx, (size_t)sc.W * 8);
-    if (m & GD_STAGE_WLEN) sc.wlen = (const float *)gd_stage_copy(cursor, sc.wlen, (size_t)sc.W * 4);
-    if (m & GD_STAGE_SIDETEX) sc.sideTex = (const int32_t *)gd_stage_copy(cursor, sc.sideTex, (size_t)sc.W * 24);
-    if (m & GD_STAGE_SIDEOFF) sc.sideOff = (const float *)gd_stage_copy(cursor, sc.sideOff, (size_t)sc.W * 16);
-    if (m & GD_STAGE_VTXLIST) {
-      sc.vtxOff = (const int32_t *)gd_stage_copy(cursor, sc.vtxOff, (size_t)(p.V + 1) * 4);
-      sc.vtxWalls = (const int32_t *)gd_stage_copy(cursor, sc.vtxWalls, (size_t)(p.vtxWallsN > 0 ? p.vtxWallsN : 1) * 4);
-    }
-    if (m & GD_STAGE_ROWPROJ) { stagedRowproj = (GdRowProj *)cursor; cursor += gd_align16((size_t)sc.W * 4 * sizeof(GdRowProj)); }
-    sh.planeTab = (GdPlaneEntry *)(p.scratch + (size_t)blockIdx.x * gd_scratch_per_cta(sc.W, sc.S) + GD_SCRATCH_FIXED);
+    sh.planeTab = (GdPlaneEntry *)(myScratch + gd_scratch_planes(sc.W, sc.S));
+    sh.frame = frame;
+    sh.colormap = gd_smem + GD_OFF_COLORMAP;
+    sh.lane = (int32_t *)(gd_smem + GD_OFF_LANE);
+    sh.ownerMask = (unsigned *)(gd_smem + GD_OFF_OWNER);
+    sh.walls = (GdWall *)(myScratch + gd_scratch_walls(sc.W, sc.S));
     sh.frags = p.fragScratch ? p.fragScratch + (size_t)blockIdx.x * sc.F : nullptr;
     if (!sh.frags) sc.F = 0;
-    if (tid == 0) { sScene = sc; sShared = sh; }
+    sh.anchors = (unsigned *)(myScratch + GD_SCRATCH_ANCHORS);
+    sh.actors = (GdActor *)(gd_smem + p.offActors);
+    sh.pal64 = (unsigned long long *)(gd_smem + GD_OFF_PAL64);
+    sh.obs = gd_smem + GD_OFF_AUX;
+    sh.misc = (int *)(gd_smem + GD_OFF_MISC);
+    sh.masks = (unsigned *)(gd_smem + GD_OFF_MASKS);
+    sh.pal32 = (unsigned *)(gd_smem + GD_OFF_PAL32);
+    sh.maskedDist = (float *)(gd_smem + GD_OFF_MASKED_DIST);
+    sh.maskedInfo = (unsigned *)(gd_smem + GD_OFF_MASKED_INFO);
+    sh.secOff = (const unsigned short *)(gd_smem + p.offSecOff);
+    sh.secWalls = (const unsigned short *)(gd_smem + p.offSecWalls);
+    sh.hitD = (float *)(gd_smem + GD_OFF_AUX);
+    sh.hitA = (float *)(gd_smem + GD_OFF_AUX2);
+    sc.wvtx = (const int32_t *)(gd_smem + p.offVtx);
+    sScene = sc; sShared = sh;
+#ifdef GD_CHECKED
+    gdCheckedStatus = p.status;
+#endif
   }
   __syncthreads();
   const GdScene &sc = sScene;
   const GdShared &sh = sShared;
-#ifdef GD_CHECKED
-  if (tid == 0) gdCheckedStatus = p.status;
-  __syncthreads();
-#endif
   /* tables shared by every lane this CTA draws */
   for (int i = tid; i < 32 * 256 / 4; i += GD_THREADS)
-    ((unsigned *)sh.colormap)[i] = ((const unsigned *)sc.colormap)[i];
+    ((unsigned *)(gd_smem + GD_OFF_COLORMAP))[i] = ((const unsigned *)sc.colormap)[i];
   gd_lane_palette(sc, sh, 0);
+  for (int w = tid; w < sc.W; w += GD_THREADS) {
+    const int front = gd_wsec(sc, w * 2), back = gd_wsec(sc, w * 2 + 1);
+    gd_hot(w).secs = (front & 0xFFFF) | (back << 16);
+    const bool neighbour = sc.nbDirect ? sc.nbDirectTab[w * 4] >= 0 || sc.nbDirectTab[w * 4 + 1] >= 0 : sc.nbOff[w + 1] > sc.nbOff[w];
+    gd_hot(w).bits = (back < 0 ? GD_HOT_ONESIDED : 0u) | (kSplit && sc.fragOff[w + 1] > sc.fragOff[w] ? GD_HOT_SPLIT : 0u) |
+                     (neighbour ? GD_HOT_NEIGHBOUR : 0u) | (sc.sbStartOff[w + 1] > sc.sbStartOff[w] ? GD_HOT_BRIDGE0 : 0u) |
+                     (sc.sbEndOff[w + 1] > sc.sbEndOff[w] ? GD_HOT_BRIDGE1 : 0u);
+    ((int2 *)(gd_smem + p.offVtx))[w] = ((const int2 *)p.sc.wvtx)[w];
+  }
+  for (int s = tid; s < sc.S; s += GD_THREADS)
+    ((float4 *)(gd_smem + p.offSectors))[s] = make_float4(sc.secF[s * 2], sc.secF[s * 2 + 1], __int_as_float(sc.secI[s * 4]), 0.0f);
+  for (int s = tid; s <= sc.S; s += GD_THREADS) ((unsigned short *)(gd_smem + p.offSecOff))[s] = (unsigned short)sc.secOff[s];
+  for (int i = tid; i < p.secWallsN; i += GD_THREADS)
+    ((unsigned short *)(gd_smem + p.offSecWalls))[i] = (unsigned short)GD_CHECK_INDEX(sc.secWalls[i], sc.W);
+  if (kChip)
+    for (int i = tid; i < sc.W * 2 * (int)(sizeof(GdSide) / 16); i += GD_THREADS)
+      ((uint4 *)(gd_smem + p.offSides))[i] = ((const uint4 *)p.sides)[i];
   bool paletteBlended = false;    /* CTA-uniform: the shared palette holds a lane's screen-flash blend */
-  uint8_t *myScratch = p.scratch + (size_t)blockIdx.x * gd_scratch_per_cta(sc.W, sc.S);
   GdEvent *events = (GdEvent *)myScratch;
   int *eventCount = (int *)(myScratch + GD_SCRATCH_EVENTS_BYTES);
-  unsigned short *vsec = (unsigned short *)(myScratch + GD_SCRATCH_EVENTS_BYTES + GD_SW * 4);
-  GdRowProj *rowproj = stagedRowproj ? stagedRowproj
-                                     : (GdRowProj *)(myScratch + GD_SCRATCH_FIXED + gd_scratch_plane_bytes(sc.S));
+  unsigned short *vsec = (unsigned short *)(myScratch + GD_SCRATCH_VSEC);
+  GdRowProj *rowproj = (GdRowProj *)(myScratch + gd_scratch_rowproj(sc.W, sc.S));
+  GdRow *rows = (GdRow *)(kChip ? gd_smem + p.offRows : tables + p.offRows);
+  GdRow *fragRows = kChip ? rows + sc.W * 4 : p.fragRows + (size_t)blockIdx.x * sc.F * 4;
+  float4 *prep = (float4 *)(kChip ? gd_smem + p.offPrep : tables + p.offPrep);
+  GdPlane *planes = (GdPlane *)(kChip ? gd_smem + p.offPlanes : tables + p.offPlanes);
 
   /* Lanes differ a lot in cost (a long corridor crosses many sectors), so the
    * persistent CTAs take lanes from a shared counter instead of a fixed stride.
@@ -243,7 +269,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gd_render_kernel(const GdParams
       if (p.resetMask && !p.resetMask[l]) continue;  /* uniform across the CTA */
     }
     if (tid < GD_LANE_WORDS) sh.lane[tid] = p.lanes[(size_t)l * GD_LANE_WORDS + tid];
-    if (tid < 10) { sh.ownerMask[tid] = 0; sh.ownerMask[16 + tid] = 0; }
+    if (tid < GD_OWNER_WORDS) sh.ownerMask[tid] = 0;
     if (tid == 0) sh.misc[1] = 0;
     /* sector of every thing and of the player (slot 64): lowest index that
      * contains the point (engine.py:9598-9617), found by all threads together
@@ -309,51 +335,73 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gd_render_kernel(const GdParams
       den = gd_max(den, 1);
       i64 ys = gd_div(GD_FOCAL_Y << 16, den);
       if (den <= (GD_FOCAL_Y >> 15)) ys = (1LL << 31) - 1;
-      sh.yslope[tid] = (unsigned)ys;
+      ((unsigned *)(gd_smem + GD_OFF_YSLOPE))[tid] = (unsigned)ys;
     }
-    for (int w = tid; w < sc.W; w += GD_THREADS) gd_project_wall(sc, v, w, sh.walls[w]);
     if (kSplit)
-      for (int f = tid; f < sc.F; f += GD_THREADS) gd_project_fragment(sc, v, f, sh.frags[f]);
-    for (int idx = GD_THREADS - 1 - tid; idx < sc.S * 2; idx += GD_THREADS)   /* the threads the walls leave idle */
-      gd_plane_entry_setup(sc, v, idx >> 1, (idx & 1) != 0, sh.planeTab[idx]);
+      for (int f = tid; f < sc.F; f += GD_THREADS) {
+        GdWall &q = sh.frags[f];
+        gd_project_fragment(sc, v, f, q);
+        const unsigned sl = (unsigned)gd_clamp(q.sl, 0, GD_SW), sr = (unsigned)gd_clamp(q.sr, 0, GD_SW);
+        ((unsigned *)(gd_smem + p.offFrags))[f] = q.sr > q.sl ? sl | (sr << 16) : 0u;
+      }
+    for (int idx = GD_THREADS - 1 - tid; idx < sc.S * 2; idx += GD_THREADS)   /* the threads the things leave idle */
+      gd_plane_entry_setup(sc, v, idx >> 1, (idx & 1) != 0, sh.planeTab[idx], planes[idx]);
     for (int a = tid; a < nThings; a += GD_THREADS) {
       int sector = pointSector[a] == 0x7fffffff ? 0 : pointSector[a];
       gd_actor_setup(sc, v, p.things[(size_t)l * p.maxThings + a], sector, sh.actors[a]);
     }
     if (tid == GD_THREADS - 1) sh.misc[0] = pointSector[64] == 0x7fffffff ? 0 : pointSector[64];
-    __syncthreads();
     gd_wall_spans(sc, v, sh);
-    /* row projection tables, for the walls that passed the frustum test (the
-     * walk selects no other wall) */
-    for (int idx = tid; idx < sh.misc[2] * 4; idx += GD_THREADS) {
-      int w = ((const short *)sh.hitD)[idx >> 2], slot = idx & 3;
-      int sector = gd_wsec(sc, w * 2 + (slot >> 1));
-      if (sector >= 0) gd_rowproj_setup(v, sh.walls[w], sc.secF[sector * 2 + (slot & 1)], rowproj[w * 4 + slot]);
-    }
-    __syncthreads();
-    const short *frustumList = (const short *)sh.hitD;
+    const short *frustumList = (const short *)(gd_smem + GD_OFF_AUX);
     const int frustumListed = sh.misc[2];
+    __syncthreads();
+    /* row projections, light and column operands of the listed walls (the walk selects no other wall) and of the
+     * fragments in view */
+    const int fragTasks = kSplit ? sc.F * 4 : 0;
+    for (int idx = tid; idx < frustumListed * 4 + fragTasks; idx += GD_THREADS) {
+      const bool piece = kSplit && idx >= frustumListed * 4;
+      const int f = piece ? (idx - frustumListed * 4) >> 2 : 0, slot = idx & 3;
+      if (piece && ((const unsigned *)(gd_smem + p.offFrags))[f] == 0u) continue;
+      const int w = piece ? p.fragLine[f] : frustumList[idx >> 2];
+      const GdWall &q = piece ? sh.frags[f] : sh.walls[w];
+      const int sector = gd_wsec(sc, w * 2 + (slot >> 1)), sd = slot >> 1;
+      GdRow row;
+      row.a = row.step = 0; row.lim = GD_ROW_WIDE; row.vis = 0;
+      if (sector >= 0) {
+        GdRowProj unused;
+        gd_rowproj_setup(v, q, sc.secF[sector * 2 + (slot & 1)], piece ? unused : rowproj[w * 4 + slot], row);
+        /* the light of the side, modulo 2^32 as well: exact while the owned columns' values fit */
+        const i64 step = q.visStep[sd], origin = q.visL[sd] - gd_wmul(q.visSl[sd], step);
+        const i64 l0 = origin + gd_wmul(gd_max(q.sl, 0), step), l1 = origin + gd_wmul(gd_min(q.sr, GD_SW) - 1, step);
+        if (l0 != (i64)(int)l0 || l1 != (i64)(int)l1) row.lim |= GD_ROW_LIGHT_WIDE;
+        row.vis = (int)((slot & 1) ? step : origin);
+      }
+      (piece ? fragRows + f * 4 : rows + w * 4)[slot] = row;
+    }
     for (int i = tid; i < frustumListed; i += GD_THREADS) {   /* walls outside the frustum own no column */
       const int w = frustumList[i];
-      int xl = sh.walls[w].isl;
+      prep[w] = gd_prep_setup(sh.walls[w]);
+      const int xl = (int)(short)(gd_hot(w).span & 0xFFFFu);
       if (xl >= 0 && xl < GD_SW) {
         float rx, ry;
         gd_ray(v, xl, rx, ry);
-        GdHit h = gd_hit(sc, v, sh.walls, w, xl, rx, ry);
+        GdHit h = gd_hit_slow(sc, w, xl, rx, ry);
         if (isfinite(h.d)) atomicOr(&sh.ownerMask[xl >> 5], 1u << (xl & 31));
+        if (h.proj) atomicOr(&sh.ownerMask[32 + (xl >> 5)], 1u << (xl & 31));
       }
     }
     gd_mark_afterlife_columns(sc, sh);
     {
-      float rx, ry, wd;
-      int bw;
-      gd_ray(v, tid, rx, ry);
-      gd_blocking_raycast(sc, v, sh, frustumList, frustumListed, rx, ry, wd, bw);
-      sh.wallDistance[tid] = wd;
-      sh.blockingWall[tid] = (short)bw;
+      float rx, ry, wd = 0.0f;
+      int bw = 0;
+      if (nThings > 0) {
+        gd_ray(v, tid, rx, ry);
+        gd_blocking_raycast(sc, frustumList, frustumListed, rx, ry, wd, bw);
+      }
+      ((unsigned long long *)(gd_smem + GD_OFF_CAND))[tid] = gd_sprite_candidates(sc, sh, nThings, wd, bw);
     }
     __syncthreads();
-    gd_walk<kSplit>(sc, v, sh, events, eventCount, rowproj, p.status, sh.misc[0]);
+    gd_walk<kSplit, kChip>(p, sc, v, sh, frame, tables, events, eventCount, rowproj, sh.misc[0]);
     __syncthreads();
     /* Rows no seg ever claimed show the per-pixel flat fallback.  They are
      * queued (the hit cache is free once every column has finished its walk)

@@ -62,8 +62,29 @@ __device__ __forceinline__ bool gd_behind(const GdScene &sc, const GdWall &wv, i
   return (nearD > ac.depthFixed) || ((farD > ac.depthFixed) && (side <= 0));
 }
 
+/* The things that may show in column x = threadIdx.x (engine.py:14684-14720): in front of the viewer, across the
+ * column, and not behind the nearest one-sided wall of the column's ray (at `wd`, wall `bw`). */
+__device__ __noinline__ unsigned long long gd_sprite_candidates(const GdScene &sc_, const GdShared &sh_, int nThings, float wd, int bw) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  const GdShared &sh = *gd_as_shared(&sh_);
+  const int x0 = threadIdx.x;
+  unsigned long long cand = 0;
+#pragma unroll 1
+  for (int a = 0; a < nThings; ++a) {
+    const GdActor &ac = *gd_as_shared(&sh.actors[a]);
+    if (!(ac.alive && x0 >= ac.left && x0 < ac.right && ac.depth > 0)) continue;
+    bool rayVisible = ac.depth < wd;
+    if (!rayVisible) {
+      const GdWall &bwv = sh.walls[bw];
+      rayVisible = !(x0 >= bwv.sl && x0 < bwv.sr) || gd_behind(sc, bwv, bw, ac);
+    }
+    if (rayVisible) cand |= 1ull << a;
+  }
+  return cand;
+}
+
 /* Sprites cluster in a few screen columns, so the drawing is spread by rows:
- * every column thread first lists its visible candidates; then the warps take
+ * the columns with candidates are listed; then the warps take
  * the listed columns from a counter and draw each candidate's rows 32 at a
  * time, far to near. */
 __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared &sh_, const GdEvent *events,
@@ -73,27 +94,12 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
   const GdShared &sh = *gd_as_shared(&sh_);
   const int x0 = threadIdx.x, lane = threadIdx.x & 31;
   if (nThings <= 0) return;                          /* block-uniform */
-  unsigned long long *candOf = (unsigned long long *)sh.hitD;       /* per column */
+  const unsigned long long *candOf = (const unsigned long long *)(gd_smem + GD_OFF_CAND);
   short *list = (short *)sh.hitA;
   int *counters = &sh.misc[2];                       /* [0] listed columns, [1] next to draw */
   if (x0 == 0) { counters[0] = 0; counters[1] = 0; }
   __syncthreads();
-  {
-    unsigned long long cand = 0;
-    int bw = sh.blockingWall[x0];
-    const GdWall &bwv = sh.walls[bw];
-    bool bowns = x0 >= bwv.sl && x0 < bwv.sr;
-    float wd = sh.wallDistance[x0];
-    for (int a = 0; a < nThings; ++a) {
-      const GdActor &ac = sh.actors[a];
-      if (!(ac.alive && x0 >= ac.left && x0 < ac.right && ac.depth > 0)) continue;
-      bool rayVisible = ac.depth < wd;
-      rayVisible = rayVisible || !bowns || gd_behind(sc, bwv, bw, ac);
-      if (rayVisible) cand |= 1ull << a;
-    }
-    candOf[x0] = cand;
-    if (cand) list[atomicAdd(&counters[0], 1)] = (short)x0;
-  }
+  if (candOf[x0]) list[atomicAdd(&counters[0], 1)] = (short)x0;
   __syncthreads();
   const int listed = counters[0];
   for (;;) {
@@ -186,7 +192,6 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
 
 /* ---- phase: weapon (engine.py:14994-15121) ------------------------------ */
 __device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, uint8_t *frame, int id, i64 hoff, i64 voff) {
-  frame = gd_as_shared(frame);
   const GdScene &sc = *gd_as_shared(&sc_);
 #ifdef GD_CHECKED
   if (id >= sc.Q || id < -1) { if (threadIdx.x == 0) atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX); }

@@ -6,56 +6,69 @@
 /* ---- visplane rows (engine.py:10879-10954, 10588-10616, 13372-13405) ---- */
 struct GdPlaneSpan {
   i64 basex, basey, pviewx, pviewy, phf, gv, shadeBase;
-  const uint8_t *tex;
+  unsigned tex;
   int wbits, hbits, texW;
-  bool narrow;   /* the row's light term fits 32-bit arithmetic (see gd_plane_pixel) */
 };
 
 /* Column-independent part of a span setup, one entry per (sector, floor or
  * ceiling), rebuilt for every lane: the three divisions of R_DrawSpan's setup
- * leave the per-crossing path. */
+ * leave the per-crossing path.  GdPlane is the form the walk reads: it holds when every
+ * operand fits 32 bits (`flags` says so), which leaves the pixel with 32 x 32 -> 64 multiplies. */
 struct GdPlaneEntry {
   i64 phf, gv, shadeBase, xstep, ystep, bx0, by0, pviewx, pviewy;
-  const uint8_t *tex;
-  int wbits, hbits;
+  unsigned tex;
+  int wbits, hbits, pad;
 };
+struct __align__(16) GdPlane {
+  int phf, gv, shadeBase;
+  unsigned flags;                 /* 32 - wbits | 32 - hbits << 8 | GD_PLANE_NARROW */
+  int bx0, xstep, by0, ystep;
+  unsigned pviewx, pviewy, tex;
+  int pad;
+};
+#define GD_PLANE_NARROW 65536u
 
-static_assert(sizeof(GdPlaneEntry) == GD_PLANE_ENTRY_BYTES, "scratch layout");
+static_assert(sizeof(GdPlaneEntry) == GD_PLANE_ENTRY_BYTES && sizeof(GdPlane) == GD_PLANE_BYTES, "scratch layout");
 
 __device__ __noinline__ void gd_plane_entry_setup(const GdScene &sc_, const GdView &v_, int sector, bool isFloor,
-                                                  GdPlaneEntry &e) {
+                                                  GdPlaneEntry &e, GdPlane &n) {
   const GdScene &sc = *gd_as_shared(&sc_);
   const GdView &v = *gd_as_shared(&v_);
   float ph = isFloor ? (v.viewZ - gd_sec_floor(sc, sector)) : (gd_sec_ceil(sc, sector) - v.viewZ);
   int4 si = gd_sec_info(sc, sector);
   int tex = GD_CHECK_INDEX(isFloor ? si.y : si.z, sc.T);
   const int4 ti = *reinterpret_cast<const int4 *>(&sc.texInfo[tex * 4]);
-  e.wbits = ti.z; e.hbits = ti.w;
-  e.tex = sc.texAtlas + (size_t)tex * sc.texH * sc.texW;
-  i64 xscale = 1LL << (32 - e.wbits), yscale = 1LL << (32 - e.hbits);
+  const int wbits = ti.z, hbits = ti.w;
+  const unsigned texel0 = (unsigned)tex * (unsigned)(sc.texH * sc.texW);
+  i64 xscale = 1LL << (32 - wbits), yscale = 1LL << (32 - hbits);
   i64 fs = v.vsin, fc = v.vcos;
-  e.xstep = gd_div(xscale * fs, GD_FOCAL_X);
-  e.ystep = gd_div(yscale * fc, GD_FOCAL_X);
-  e.bx0 = (xscale * fc) >> 16;
-  e.by0 = (yscale * -fs) >> 16;
-  e.pviewx = gd_wmul(xscale, v.vx) >> 16;
-  e.pviewy = gd_wmul(yscale, -v.vy) >> 16;
-  e.phf = gd_rint(ph * 65536.0f);
-  e.gv = gd_min(gd_div(GD_FLOOR_VIS << 16, gd_max(e.phf, 1)), (1LL << 31) - 1);
+  const i64 xstep = gd_div(xscale * fs, GD_FOCAL_X), ystep = gd_div(yscale * fc, GD_FOCAL_X);
+  const i64 bx0 = (xscale * fc) >> 16, by0 = (yscale * -fs) >> 16;
+  const i64 pviewx = gd_wmul(xscale, v.vx) >> 16, pviewy = gd_wmul(yscale, -v.vy) >> 16;
+  const i64 phf = gd_rint(ph * 65536.0f);
+  const i64 gv = gd_min(gd_div(GD_FLOOR_VIS << 16, gd_max(phf, 1)), (1LL << 31) - 1);
   i64 light = si.x + v.flashLight * 16;
-  e.shadeBase = 64 * GD_FU - (light + 12) * (GD_FU / 4);
-  /* gv lies in [0, 2^31) by construction; with the screen centre within +-2^30 (any pitch short of
-   * +-89.5 degrees) and a shade base that fits an int, the light term of a pixel needs one 32 x 32 -> 64
-   * multiply; the flag travels in the spare bits of hbits */
-  const bool narrow = v.center > -(1LL << 30) && v.center < (1LL << 30) && e.shadeBase > -(1LL << 31) && e.shadeBase < (1LL << 31);
-  e.hbits |= narrow ? 256 : 0;
+  const i64 shadeBase = 64 * GD_FU - (light + 12) * (GD_FU / 4);
+  e.wbits = wbits; e.hbits = hbits; e.tex = texel0; e.pad = 0;
+  e.xstep = xstep; e.ystep = ystep; e.bx0 = bx0; e.by0 = by0;
+  e.pviewx = pviewx; e.pviewy = pviewy; e.phf = phf; e.gv = gv; e.shadeBase = shadeBase;
+  /* gv lies in [0, 2^31) by construction; columns run from -159 to 160; the screen centre is within
+   * +-2^30 for any pitch short of +-89.5 degrees */
+  const i64 big = 1LL << 30;
+  const bool narrow = phf >= 0 && phf < 2 * big && shadeBase > -big && shadeBase < big && v.center > -big && v.center < big &&
+                      gd_max(bx0, -bx0) + 160 * gd_max(xstep, -xstep) < 2 * big &&
+                      gd_max(by0, -by0) + 160 * gd_max(ystep, -ystep) < 2 * big && wbits > 0 && hbits > 0;
+  n.phf = (int)phf; n.gv = (int)gv; n.shadeBase = (int)shadeBase;
+  n.flags = (unsigned)(32 - wbits) | ((unsigned)(32 - hbits) << 8) | (narrow ? GD_PLANE_NARROW : 0u);
+  n.bx0 = (int)bx0; n.xstep = (int)xstep; n.by0 = (int)by0; n.ystep = (int)ystep;
+  n.pviewx = (unsigned)pviewx; n.pviewy = (unsigned)pviewy; n.tex = texel0; n.pad = 0;
 }
 
 __device__ __forceinline__ void gd_plane_setup(const GdScene &sc, const GdPlaneEntry *table, int sector, bool isFloor,
                                                int x, GdPlaneSpan &p) {
   const GdPlaneEntry &e = table[gd_secidx(sc, sector) * 2 + (isFloor ? 1 : 0)];
   i64 col = (i64)x - 159;
-  p.wbits = e.wbits; p.hbits = e.hbits & 255; p.narrow = (e.hbits & 256) != 0; p.texW = sc.texW;
+  p.wbits = e.wbits; p.hbits = e.hbits; p.texW = sc.texW;
   p.tex = e.tex;
   p.basex = e.bx0 + col * e.xstep;
   p.basey = e.by0 + col * e.ystep;
@@ -66,29 +79,36 @@ __device__ __forceinline__ void gd_plane_setup(const GdScene &sc, const GdPlaneE
   p.shadeBase = e.shadeBase;
 }
 
-/* One visplane pixel (R_DrawSpan, engine.py:10879-10954).  kNarrow: the span's `narrow` flag holds, so
- * |center - y * 65536| < 2^31 and the light term is exact in 32-bit arithmetic: vis = min(gv * rowDist >> 16,
- * 24 * 65536) is 24 * 65536 exactly when the 64-bit product is at least 0x18 << 32. */
-template <bool kNarrow>
-__device__ __forceinline__ unsigned gd_plane_pixel(const GdPlaneSpan &p, i64 center, unsigned yslope, unsigned colormap, int y) {
-  i64 distance = gd_wmul(p.phf, (i64)gd_lds32(yslope + y * 4)) >> 16;
+/* One visplane pixel (R_DrawSpan, engine.py:10879-10954), any operands. */
+__device__ __noinline__ unsigned gd_plane_pixel(const GdScene &sc_, const GdPlaneSpan &p, i64 center, int y) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  const unsigned yslope = ((const unsigned *)(gd_smem + GD_OFF_YSLOPE))[y];
+  i64 distance = gd_wmul(p.phf, (i64)yslope) >> 16;
   i64 xfrac = ((gd_wmul(distance, p.basex) >> 16) + p.pviewx) & GD_U32MASK;
   i64 yfrac = ((gd_wmul(distance, p.basey) >> 16) + p.pviewy) & GD_U32MASK;
   int u = (int)(xfrac >> (32 - p.wbits)), tv = (int)(yfrac >> (32 - p.hbits));
-  uint8_t texel = p.tex[tv * p.texW + u];
-  int shade;
-  if (kNarrow) {
-    const int rowDist = abs((int)center - (y << 16));
-    const i64 vis64 = (i64)(int)p.gv * (i64)rowDist;
-    const int vis = (unsigned)(vis64 >> 32) >= 0x18u ? 24 * 65536 : (int)(unsigned)(vis64 >> 16);
-    shade = min(max(((int)p.shadeBase - vis) >> 16, 0), 31);
-  } else {
-    i64 rowDist = center - (i64)y * GD_FU;
-    if (rowDist < 0) rowDist = -rowDist;
-    i64 vis = gd_min(gd_wmul(p.gv, rowDist) >> 16, 24 * GD_FU);
-    shade = (int)gd_clamp((p.shadeBase - vis) >> 16, 0, 31);
-  }
-  return gd_lds8(colormap + shade * 256 + texel);
+  uint8_t texel = sc.texAtlas[p.tex + (unsigned)(tv * p.texW + u)];
+  i64 rowDist = center - (i64)y * GD_FU;
+  if (rowDist < 0) rowDist = -rowDist;
+  i64 vis = gd_min(gd_wmul(p.gv, rowDist) >> 16, 24 * GD_FU);
+  int shade = (int)gd_clamp((p.shadeBase - vis) >> 16, 0, 31);
+  return gd_smem[GD_OFF_COLORMAP + shade * 256 + texel];
+}
+
+/* The same in 32-bit arithmetic: the span is narrow and |distance| < 2^31 for its rows (see
+ * gd_walk).  vis = min(gv * rowDist >> 16, 24 * 65536) is 24 * 65536 exactly when the 64-bit product is
+ * at least 0x18 << 32. */
+struct GdNarrowSpan { unsigned phf, pviewx, pviewy, tex; int basex, basey, gv, shadeBase, xshift, yshift; };
+__device__ __forceinline__ unsigned gd_plane_pixel_narrow(const GdNarrowSpan &p, const uint8_t *atlas, int texW, int center, int y) {
+  const unsigned yslope = ((const unsigned *)(gd_smem + GD_OFF_YSLOPE))[y];
+  const int distance = (int)(((unsigned long long)p.phf * yslope) >> 16);
+  const unsigned xfrac = (unsigned)(((i64)distance * p.basex) >> 16) + p.pviewx;
+  const unsigned yfrac = (unsigned)(((i64)distance * p.basey) >> 16) + p.pviewy;
+  const unsigned texel = atlas[p.tex + (yfrac >> p.yshift) * (unsigned)texW + (xfrac >> p.xshift)];
+  const i64 vis64 = (i64)p.gv * (i64)abs(center - (y << 16));
+  const int vis = (unsigned)(vis64 >> 32) >= 0x18u ? 24 * 65536 : (int)(unsigned)(vis64 >> 16);
+  const int shade = min(max((p.shadeBase - vis) >> 16, 0), 31);
+  return gd_smem[GD_OFF_COLORMAP + shade * 256 + texel];
 }
 
 /* The 208-row column masks live in shared memory, one word column per screen
@@ -134,7 +154,7 @@ __device__ __forceinline__ bool gd_state_equal(const GdColState &a, const GdColS
 struct GdIter {
   int wall, side;
   bool rasterValid, valid, oneSided;
-  int renderCurrent, otherSector;
+  int renderCurrent, renderOther, otherSector;
   float distance;
   i64 vis;
   int ctop, cbot, cupbot, clowtop;
@@ -154,72 +174,39 @@ struct GdIter {
 
 /* kSplit: the scene has lines a node builder split; the other instantiation carries none of that code */
 template <bool kSplit>
-__device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdWall *walls, const GdWall *frags,
-                                 const unsigned *ownerMask, const GdRowProj *rowproj, float *hitD, float *hitA, uint8_t *hitF, int x, float rx,
-                                 float ry, const GdColState &c, GdIter &it) {
-  const GdScene &sc = *gd_as_shared(&sc_);
-  const GdView &v = *gd_as_shared(&v_);
-  walls = gd_as_shared(walls); ownerMask = gd_as_shared(ownerMask);
-  hitD = gd_as_shared(hitD); hitA = gd_as_shared(hitA); hitF = gd_as_shared(hitF);
+__device__ __forceinline__ void gd_column_decide(const GdScene &sc, const GdView &v, const GdShared &sh, const GdWall *walls, const GdWall *frags,
+                                                 const GdRowProj *rowproj, int x, float rx, float ry, const GdColState &c, GdIter &it) {
+  const unsigned *ownerMask = (const unsigned *)(gd_smem + GD_OFF_OWNER);
   const int curSector = c.cur;
   const int current = GD_CHECK_SECTOR(curSector < 0 ? 0 : curSector, sc.S);
   const float prev = c.prev;
-  const int i0 = sc.secOff[current], i1 = sc.secOff[current + 1];
-  /* every rule below looks at the walls of the current sector: test each once
-   * and keep the results in this column's slice of shared memory */
-  constexpr int kCache = 8;
-  const int nCache = min(i1 - i0, kCache);
-#pragma unroll 1
-  for (int k = 0; k < nCache; ++k) {
-    GdHit h = gd_hit(sc, v, walls, GD_CHECK_INDEX(sc.secWalls[i0 + k], sc.W), x, rx, ry);
-    hitD[k * GD_SW + x] = h.d;
-    hitA[k * GD_SW + x] = h.along;
-    hitF[k * GD_SW + x] = (uint8_t)((h.geo ? 1 : 0) | (h.proj ? 2 : 0) | (h.left ? 4 : 0));
-  }
-  auto loadHit = [&](int k) -> GdHit {
-    GdHit h;
-    h.d = hitD[k * GD_SW + x];
-    h.along = hitA[k * GD_SW + x];
-    uint8_t f = hitF[k * GD_SW + x];
-    h.geo = f & 1; h.proj = (f & 2) != 0; h.left = (f & 4) != 0;
-    return h;
-  };
-  /* one out-of-line copy of the uncached test serves every rule below */
-  auto cachedHit = [&](int w) -> GdHit {
-#pragma unroll 1
-    for (int k = 0; k < nCache; ++k)
-      if (sc.secWalls[i0 + k] == w) return loadHit(k);
-    return gd_hit_slow(sc, v, walls, w, x, rx, ry);
-  };
-#define HIT(w) cachedHit(w)
-#define HITK(k) (((k) - i0) < nCache ? loadHit((k) - i0) : gd_hit_slow(sc, v, walls, GD_CHECK_INDEX(sc.secWalls[k], sc.W), x, rx, ry))
+  const unsigned short *secOff = sh.secOff, *secWalls = sh.secWalls;
+  const int i0 = secOff[current], i1 = secOff[current + 1];
+#define ONE_SIDED(w) ((gd_hot(w).bits & GD_HOT_ONESIDED) != 0)
+#define HIT(w) gd_hit_slow(sc, w, x, rx, ry)
+#define HITK(k) HIT(secWalls[k])
   float distance = GD_INF;
   int wallIndex = 0;
   if (curSector >= 0) {
-#pragma unroll 1
-    for (int k = i0; k < i1; ++k) {
-      int w = GD_CHECK_INDEX(sc.secWalls[k], sc.W);
-      GdHit h = HITK(k);
-      if (h.d > prev && h.d < distance) { distance = h.d; wallIndex = w; }
-    }
+    /* nearest wall, and the nearest one-sided one, which goes first when it is within 1e-3 */
     float sd = GD_INF;
     int sw = 0;
 #pragma unroll 1
     for (int k = i0; k < i1; ++k) {
-      int w = GD_CHECK_INDEX(sc.secWalls[k], sc.W);
-      if (!walls[w].oneSided) continue;
-      GdHit h = HITK(k);
-      if (!(h.d > prev) || !isfinite(h.d)) continue;
-      if (fabsf(h.d - distance) <= 1e-3f && h.d < sd) { sd = h.d; sw = w; }
+      const int w = secWalls[k];
+      const GdHit h = HIT(w);
+      if (!(h.d > prev)) continue;
+      if (h.d < distance) { distance = h.d; wallIndex = w; }
+      if (h.d < sd && ONE_SIDED(w)) { sd = h.d; sw = w; }
     }
-    if (isfinite(sd)) { distance = sd; wallIndex = sw; }
+    if (fabsf(sd - distance) <= 1e-3f) { distance = sd; wallIndex = sw; }
   }
   GdHit hSel = HIT(wallIndex);
   const float *selWall = &sc.walls[wallIndex * 4];
   bool selUsesStart = hSel.along <= 0.5f;
   float selEpX = selUsesStart ? selWall[0] : selWall[2], selEpY = selUsesStart ? selWall[1] : selWall[3];
-  int selVtx = sc.wvtx[wallIndex * 2 + (selUsesStart ? 0 : 1)];
-#define SHARES_SEL(w) (sc.wvtx[(w) * 2] == selVtx || sc.wvtx[(w) * 2 + 1] == selVtx)
+  int selVtx = gd_vertex(sc, wallIndex, selUsesStart ? 0 : 1);
+#define SHARES_SEL(w) (gd_vertex(sc, w, 0) == selVtx || gd_vertex(sc, w, 1) == selVtx)
   bool continuesOwner = c.pendOwnerBoundary && selEpX == c.pendOwnerEpX && selEpY == c.pendOwnerEpY;
   bool continuesEp = c.pendEpBoundary && selEpX == c.pendEpEpX && selEpY == c.pendEpEpY;
   int selSlot = hSel.along > 0.5f;
@@ -239,8 +226,8 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   if (!selIsProjected) {
 #pragma unroll 1
     for (int k = i0; k < i1; ++k) {
-      int w = GD_CHECK_INDEX(sc.secWalls[k], sc.W);
-      if (!walls[w].oneSided || !SHARES_SEL(w)) continue;
+      int w = secWalls[k];
+      if (!ONE_SIDED(w) || !SHARES_SEL(w)) continue;
       GdHit h = HITK(k);
       if (h.proj && h.left && (h.d > prev + 1e-3f) && h.d < psd) { psd = h.d; psi = w; }
     }
@@ -252,8 +239,8 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
 #pragma unroll 1
       for (int k = off[wallIndex]; k < off[wallIndex + 1]; ++k) {
         int b = GD_CHECK_INDEX(idx[k], sc.W);
-        bool inc = gd_wsec(sc, b * 2) == current || gd_wsec(sc, b * 2 + 1) == current;
-        if (!inc || !walls[b].oneSided) continue;
+        bool inc = gd_hot_front(b) == current || gd_hot_back(b) == current;
+        if (!inc || !ONE_SIDED(b)) continue;
         GdHit h = HIT(b);
         if (h.proj && h.left && (h.d > prev + 1e-3f) && h.d < sbd) { sbd = h.d; sbi = b; }
       }
@@ -265,15 +252,15 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   GdHit hW = (wallIndex == psPathIndex) ? hSel : HIT(wallIndex);
   int seo = wallIndex;
   float sed = hW.d;
-  if (!hW.proj) gd_endpoint_owner(sc, v, walls, wallIndex, x, rx, ry, hW, seo, sed);
+  if (!hW.proj) gd_endpoint_owner(sc, walls, wallIndex, x, rx, ry, hW, seo, sed);
   bool eoPathIsGeo = hW.geo;
   bool replaceEo = (seo != wallIndex) && (sed > prev + 1e-3f);
   if (replaceEo) { distance = sed; wallIndex = seo; hW = HIT(wallIndex); }
   int nopIndex = wallIndex;
   float nopDist = distance;
   bool nopIsGeo = replaceEo ? eoPathIsGeo : hW.geo;
-  bool nopFromFront = curSector == gd_wsec(sc, nopIndex * 2);
-  int nopOther = nopFromFront ? gd_wsec(sc, nopIndex * 2 + 1) : gd_wsec(sc, nopIndex * 2);
+  bool nopFromFront = curSector == gd_hot_front(nopIndex);
+  int nopOther = nopFromFront ? gd_hot_back(nopIndex) : gd_hot_front(nopIndex);
   bool selOwnerIsProjected = hW.proj;
   bool selOwnerExclRight = walls[wallIndex].sr == x;
   i64 selOwnerSpan = walls[wallIndex].sr - walls[wallIndex].sl;
@@ -283,8 +270,8 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   if (!selOwnerIsProjected) {
 #pragma unroll 1
     for (int k = i0; k < i1; ++k) {
-      int w = GD_CHECK_INDEX(sc.secWalls[k], sc.W);
-      if (walls[w].oneSided) continue;
+      int w = secWalls[k];
+      if (ONE_SIDED(w)) continue;
       GdHit h = HITK(k);
       if (!h.proj || !(h.d > prev + 1e-3f)) continue;
       bool topological = false;
@@ -300,17 +287,17 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   }
   /* projected sector bridge (engine.py:12073-12164) */
   const int pew = c.pendEpWall;
-  bool peFromCur = curSector == gd_wsec(sc, pew * 2);
-  int peOther = peFromCur ? gd_wsec(sc, pew * 2 + 1) : gd_wsec(sc, pew * 2);
+  bool peFromCur = curSector == gd_hot_front(pew);
+  int peOther = peFromCur ? gd_hot_back(pew) : gd_hot_front(pew);
   bool usePsb = false;
   if (c.pendEpBoundary && !selOwnerIsProjected && selOwnerExclRight && nopIsGeo) {
-    bool peIncident = peFromCur || curSector == gd_wsec(sc, pew * 2 + 1);
+    bool peIncident = peFromCur || curSector == gd_hot_back(pew);
     const float *peWall = &sc.walls[pew * 4];
     int peSlot = (c.pendEpEpX == peWall[2] && c.pendEpEpY == peWall[3]) ? 1 : 0;
     int psbIndex;
     bool psbExists = gd_sector_bridge(sc, peSlot, pew, nopIndex, psbIndex);
     if (psbExists && peIncident && peOther >= 0 && nopOther >= 0 && (walls[pew].sr - walls[pew].sl <= 1)) {
-      int b0 = gd_wsec(sc, psbIndex * 2), b1 = gd_wsec(sc, psbIndex * 2 + 1);
+      int b0 = gd_hot_front(psbIndex), b1 = gd_hot_back(psbIndex);
       bool matches = (b0 == peOther && b1 == nopOther) || (b1 == peOther && b0 == nopOther);
       GdHit hb = HIT(psbIndex);
       GdHit hp = HIT(pew);
@@ -331,7 +318,7 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
                      !((pendEpHasFwd || completesPendEpBridge) && !selIsProjected && selExclRight && !replaceNp);
   bool geometric = replaceNp ? nopIsGeo : (replaceEo ? eoPathIsGeo : hW.geo);
   bool nokpp = replaceNp && nopIsGeo && nopOther >= 0;
-  int front = gd_wsec(sc, wallIndex * 2), back = gd_wsec(sc, wallIndex * 2 + 1);
+  int front = gd_hot_front(wallIndex), back = gd_hot_back(wallIndex);
   bool fromFront = curSector == front;
   int otherSector = fromFront ? back : front;
   int renderCurrent = usePsb ? peOther : (completesOpposing ? otherSector : current);
@@ -342,8 +329,8 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   const bool splitLine = kSplit && gd_line_is_split(sc, wallIndex);      /* a node builder cut this line: the slow way */
   i64 vis = splitLine ? gd_line_vis(sc, walls, frags, wallIndex, side, x)
                       : wv.visL[side] + ((i64)x - wv.visSl[side]) * wv.visStep[side];
-  bool psFromFront = curSector == gd_wsec(sc, psPathIndex * 2);
-  int psOther = psFromFront ? gd_wsec(sc, psPathIndex * 2 + 1) : gd_wsec(sc, psPathIndex * 2);
+  bool psFromFront = curSector == gd_hot_front(psPathIndex);
+  int psOther = psFromFront ? gd_hot_back(psPathIndex) : gd_hot_front(psPathIndex);
   bool pskpp = hasProjectedSolidOwner && hSel.geo && psOther >= 0;
   int safeOther = renderOther < 0 ? 0 : renderOther;
   float viewFloor = gd_sec_floor(sc, renderCurrent), viewCeil = gd_sec_ceil(sc, renderCurrent);
@@ -390,7 +377,7 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   it.markCeil = oneSided || viewCeil != otherCeil || ri.z != oi.z || lightDiff;
   it.markFloor = oneSided || viewFloor != otherFloor || ri.y != oi.y || lightDiff;
   it.wall = wallIndex; it.side = side; it.rasterValid = rasterValid; it.valid = valid;
-  it.oneSided = oneSided; it.renderCurrent = renderCurrent; it.otherSector = otherSector;
+  it.oneSided = oneSided; it.renderCurrent = renderCurrent; it.renderOther = renderOther; it.otherSector = otherSector;
   it.distance = distance; it.vis = vis;
   it.ctop = ctop; it.cbot = cbot; it.cupbot = cupbot; it.clowtop = clowtop;
   it.viewFloor = viewFloor; it.viewCeil = viewCeil; it.otherFloor = otherFloor; it.otherCeil = otherCeil;
@@ -407,9 +394,9 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   if (endpointOnly) {
 #pragma unroll 1
     for (int k = i0; k < i1; ++k) {
-      int w = GD_CHECK_INDEX(sc.secWalls[k], sc.W);
+      int w = secWalls[k];
       GdHit h = HITK(k);
-      bool os = walls[w].oneSided;
+      bool os = ONE_SIDED(w);
       bool fut = (h.geo || (os && isfinite(h.d))) && (h.d > distance + 1e-3f);
       if (fut && h.d < cnd) { cnd = h.d; cni = w; }
       bool sharesEp = gd_shares_endpoint(sc, w, wallIndex);
@@ -421,10 +408,10 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
     }
     /* endpointOnly implies otherSector >= 0 */
 #pragma unroll 1
-    for (int k = sc.secOff[otherSector]; k < sc.secOff[otherSector + 1]; ++k) {
-      int w = GD_CHECK_INDEX(sc.secWalls[k], sc.W);
+    for (int k = secOff[otherSector]; k < secOff[otherSector + 1]; ++k) {
+      int w = secWalls[k];
       GdHit h = HIT(w);
-      bool os = walls[w].oneSided;
+      bool os = ONE_SIDED(w);
       bool fut = (h.geo || (os && isfinite(h.d))) && (h.d > distance + 1e-3f);
       if (fut && h.d < ond) { ond = h.d; oni = w; }
       bool sharesEp = gd_shares_endpoint(sc, w, wallIndex);
@@ -436,8 +423,8 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   bool tied = endpointOnly && isfinite(cnd) && cni == oni && gd_opposing_pair(sc, wallIndex, cni);
   bool entersOther = endpointOnly && otherSector >= 0 && ((ond < cnd) || tied);
   bool entersShared = endpointOnly && otherSector >= 0 && (osd < csd);
-  bool gpFromFront = curSector == gd_wsec(sc, gpi * 2);
-  int gpOther = gpFromFront ? gd_wsec(sc, gpi * 2 + 1) : gd_wsec(sc, gpi * 2);
+  bool gpFromFront = curSector == gd_hot_front(gpi);
+  int gpOther = gpFromFront ? gd_hot_back(gpi) : gd_hot_front(gpi);
   bool usesGeo = endpointOnly && isfinite(gpd) && gpOther >= 0;
   int ppbIdx = 0;
   bool epb = false;
@@ -465,117 +452,166 @@ __device__ void gd_column_decide(const GdScene &sc_, const GdView &v_, const GdW
   it.epFwdIdx = epFwdIdx; it.ppbIdx = ppbIdx; it.psPathIndex = psPathIndex; it.psFromFront = psFromFront;
 #undef HIT
 #undef HITK
+#undef ONE_SIDED
 #undef SHARES_SEL
 }
 
-/* Draw rows [ya,yb) of one wall tier in column x, skipping rows [ea,eb)
- * (the overlapping lower tier, which has priority) and rows already filled.
- * engine.py:12762-12884. */
-struct GdTierCtx {
-  i64 hoff, tox, vstepBase, light;
-  float yoff;
-  int tailBottom;   /* rows >= tailBottom use the group's first-column light; 255+ = never */
+/* What one iteration of a column hands to the drawing code, whichever path decided it. */
+struct GdCross {
+  int wall, side;
+  unsigned flags;                 /* GD_C_* */
+  unsigned tops, bots;            /* clamped rows: ctop | clowtop << 16, (255 - cbot) | (255 - cupbot) << 16 */
+  int vis;                        /* wallscan light, saturated (see gd_vis_clamp) */
+  int rc, ro;                     /* sector this side, sector beyond (0 when there is none) */
+  float dist;
+  int cur;                        /* next sector and distance */
+  float prev;
+  bool pend, pendEnd, settled;
+  bool portalFront;               /* GD_C_PORTAL: the crossed portal behind the projected solid */
+  int portalWall, portalOther;
+  float portalDist;
 };
 
-__device__ __noinline__ void gd_draw_tier(const GdScene &sc_, const GdView &v_, const GdShared &sh_, int x, int ya, int yb, int ea,
-                             int eb, int texId, float originZ, const GdTierCtx &t, i64 vis, i64 firstVis,
-                             bool tailValid, int tailBottom, int oa, int ob, bool oTailValid, int oTailBottom,
-                             unsigned *filled) {
+/* The light term is min(vis, 24 * 65536) taken from a base of magnitude below 2^30 and clamped to 31 shades:
+ * anything below -2^30 is shade 31 either way. */
+__device__ __forceinline__ int gd_vis_clamp(i64 vis) { return (int)gd_clamp(vis, -(1LL << 30), 24 * GD_FU); }
+__device__ __forceinline__ int gd_shade_base(int light) { return 64 * (int)GD_FU - (light + 12) * (int)(GD_FU / 4); }
+__device__ __forceinline__ int gd_shade(int base, int vis) { return min(max((base - vis) >> 16, 0), 31); }
+
+/* One iteration of a column by the full set of rules, with its traversal update (engine.py:13242-13371).  About
+ * one column in eighty needs it: next to a wall's end the projected span and the ray test disagree, or a rule
+ * carried something over from the crossing before. */
+template <bool kSplit>
+__device__ __noinline__ void gd_slow_step(const GdScene &sc_, const GdView &v_, const GdShared &sh_, const GdRowProj *rowproj, int x, float rx, float ry, bool stopsOutside, GdColState &c,
+                                          GdCross &o) {
   const GdScene &sc = *gd_as_shared(&sc_);
   const GdView &v = *gd_as_shared(&v_);
   const GdShared &sh = *gd_as_shared(&sh_);
-  if (texId < 0 || ya >= yb) return;
-#ifdef GD_CHECKED
-  if (texId >= sc.T) { atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX); return; }   /* the tier stays undrawn */
-#endif
-  filled = gd_as_shared(filled);
-  const int4 ti = *reinterpret_cast<const int4 *>(&sc.texInfo[texId * 4]);
-  int tw = ti.x, hbits = ti.w;
-  int u = gd_pymod_width((t.hoff + t.tox) >> 16, tw);
-  i64 vstep = t.vstepBase * (1LL << (14 - hbits));
-  i64 texMid = gd_rint((originZ - v.viewZ) * 65536.0f + t.yoff * 65536.0f);
-  /* frac(y) = (texMid << (16-bits)) + ((vstep * (y*FU - center + FU)) >> 16); the
-   * y term is a multiple of 2^16 inside the shift, so it steps by vstep exactly. */
-  unsigned base = (unsigned)(gd_shl(texMid, 16 - hbits) + (gd_wmul(vstep, GD_FU - v.center) >> 16));
-  unsigned step = (unsigned)vstep;
-  const uint8_t *col = sc.texAtlasCol + ((size_t)texId * sc.texW + u) * sc.texH;
-  int shadeN = gd_wall_shade(t.light, vis), shadeT = gd_wall_shade(t.light, firstVis);
-  const unsigned cmN = gd_shared_addr(sh.colormap + shadeN * 256), cmT = gd_shared_addr(sh.colormap + shadeT * 256);
-  /* rows lit with the group's first-column light */
-  const int tailA = tailValid ? tailBottom : GD_VH, oTailA = oTailValid ? max(oa, oTailBottom) : 0,
-            oTailB = oTailValid ? ob : 0;
-  const int shift = 32 - hbits;
-  const unsigned dst = gd_shared_addr(sh.frame + x);
-#pragma unroll 1
-  for (int k = ya >> 5; k <= (yb - 1) >> 5; ++k) {
-    unsigned have = filled[k * GD_SW];
-    unsigned m = gd_range_word(k, ya, yb) & ~gd_range_word(k, ea, eb) & ~have;
-    if (!m) continue;
-    filled[k * GD_SW] = have | m;
-    const unsigned tailM = gd_range_word(k, tailA, GD_VH) | gd_range_word(k, oTailA, oTailB);
-    const int y0 = k << 5;
-    /* two rows per trip; an odd last row is simply drawn twice */
-#pragma unroll 1
-    while (m) {
-      int b0 = __ffs(m) - 1;
-      m &= m - 1;
-      int b1 = m ? __ffs(m) - 1 : b0;
-      m &= m - 1;
-      unsigned f0 = base + (unsigned)(y0 + b0) * step, f1 = base + (unsigned)(y0 + b1) * step;
-      const unsigned t0 = col[f0 >> shift], t1 = col[f1 >> shift];
-      const unsigned p0 = gd_lds8(((tailM >> b0) & 1u ? cmT : cmN) + t0), p1 = gd_lds8(((tailM >> b1) & 1u ? cmT : cmN) + t1);
-      gd_sts8(dst + (y0 + b0) * GD_SW, p0);
-      gd_sts8(dst + (y0 + b1) * GD_SW, p1);
-    }
+  const GdColState before = c;
+  GdIter it;
+  gd_column_decide<kSplit>(sc, v, sh, sh.walls, sh.frags, rowproj, x, rx, ry, c, it);
+  o.wall = it.wall; o.side = it.side; o.rc = gd_secidx(sc, it.renderCurrent); o.dist = it.distance;
+  o.ro = it.renderOther < 0 ? 0 : it.renderOther;
+  o.tops = (unsigned)it.ctop | ((unsigned)it.clowtop << 16);
+  o.bots = (unsigned)(255 - it.cbot) | ((unsigned)(255 - it.cupbot) << 16);
+  o.vis = gd_vis_clamp(it.vis);
+  o.flags = (it.rasterValid ? GD_C_RASTER : 0u) | (it.valid ? GD_C_VALID : 0u) | (it.oneSided ? GD_C_ONE_SIDED : 0u) |
+            (it.markCeil ? GD_C_MARK_CEIL : 0u) | (it.markFloor ? GD_C_MARK_FLOOR : 0u) |
+            (it.viewFloor < it.otherFloor ? GD_C_LOWER : 0u) | (it.viewCeil > it.otherCeil ? GD_C_UPPER : 0u) |
+            (it.tier[0] ? GD_C_TIER0 : 0u) | (it.tier[1] ? GD_C_TIER1 : 0u) | (it.tier[2] ? GD_C_TIER2 : 0u) |
+            (it.viewFloor > it.otherFloor ? GD_C_FLOOR_ABOVE : 0u) | (it.viewCeil < it.otherCeil ? GD_C_CEIL_BELOW : 0u) |
+            (it.pskpp ? GD_C_PORTAL : 0u);
+  o.portalWall = it.psPathIndex; o.portalOther = it.psOther; o.portalFront = it.psFromFront; o.portalDist = it.psDist;
+  /* traversal update */
+  float prior = c.prev;
+  float np = prior;
+  if (it.valid) {
+    if (it.nokpp) np = it.nopDist;
+    else if (it.pskpp) np = it.psDist;
+    else if (it.entersShared && (it.osd < it.distance)) np = prior;
+    else if (it.usesGeo) np = it.gpDist;
+    else np = it.distance;
   }
+  if (it.valid && it.epb) np = prior;
+  if (it.valid && it.cppb) np = fmaxf(it.distance, c.pendPortalBridgeExit);
+  c.prev = np;
+  if (it.startsOwner) { c.pendOwnerEpX = it.selEpX; c.pendOwnerEpY = it.selEpY; }
+  c.pendOwnerBoundary = it.startsOwner || (c.pendOwnerBoundary && it.continuesOwner);
+  if (it.endpointOnly) { c.pendEpEpX = it.epEpX; c.pendEpEpY = it.epEpY; c.pendEpWall = it.wall; }
+  c.pendEpBoundary = it.endpointOnly;
+  if (it.pendEpHasFwd) c.pendEpBridgeIndex = it.epFwdIdx;
+  c.pendEpBridgeBoundary = it.pendEpHasFwd;
+  int next;
+  if (it.nokpp) next = it.nopOther;
+  else if (it.pskpp) next = it.psOther;
+  else if (it.usesGeo) next = it.gpOther;
+  else if (it.valid && !it.oneSided && (it.geometric || it.entersOther || it.entersShared)) next = it.otherSector;
+  else if (it.endpointOnly) next = c.cur;
+  else next = -1;
+  if (it.epb) next = it.otherSector;
+  if (it.cppb) next = c.pendPortalBridgeSector;
+  if (it.epb) {
+    c.pendPortalBridgeIndex = it.ppbIdx;
+    c.pendPortalBridgeSector = it.gpOther;
+    c.pendPortalBridgeExit = it.gpDist;
+  }
+  c.pendPortalBridge = it.epb;
+  c.cur = next;
+  o.cur = next; o.prev = np;
+  o.pendEnd = c.pendEpBoundary && !(c.pendOwnerBoundary || c.pendEpBridgeBoundary || c.pendPortalBridge);
+  o.pend = c.pendOwnerBoundary || c.pendEpBoundary || c.pendEpBridgeBoundary || c.pendPortalBridge;
+  /* A column that has left the map repeats the same decision on the same state forever; once an iteration
+   * changes nothing and draws nothing it can stop. */
+  o.settled = (before.cur < 0 && !it.rasterValid && !it.pskpp && gd_state_equal(before, c)) || (next < 0 && stopsOutside);
+}
+
+__device__ __forceinline__ void gd_put_event(GdEvent *events, int &nEvents, int x, float dist, int wall, int sector, unsigned tiers,
+                                             unsigned sil, unsigned floor) {
+  if (nEvents < GD_MAX_EVENTS) {
+    unsigned *e = (unsigned *)&events[nEvents * GD_SW + x];
+    e[0] = (unsigned)__float_as_int(dist);
+    e[1] = ((unsigned)wall & 0xFFFFu) | ((unsigned)sector << 16);
+    e[2] = tiers; e[3] = sil; e[4] = floor;
+  }
+  nEvents++;
+}
+static_assert(sizeof(GdEvent) == 20, "written as five words");
+
+/* Clips contributed by the portal crossed behind a projected solid (engine.py:12965-13069). */
+template <bool kSplit>
+__device__ __noinline__ int2 gd_portal_clips(const GdScene &sc_, const GdView &v_, const GdShared &sh_, int x, const GdCross &o, int clips,
+                                             GdEvent *events, int nEvents) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  const GdView &v = *gd_as_shared(&v_);
+  const GdShared &sh = *gd_as_shared(&sh_);
+  int ceilClip = clips & 255, floorClip = clips >> 8;
+  const int pIdx = o.portalWall;
+  const int pSafeOther = o.portalOther < 0 ? 0 : o.portalOther;
+  const float viewFloor = gd_sec_floor(sc, o.rc), viewCeil = gd_sec_ceil(sc, o.rc);
+  const float pOtherFloor = gd_sec_floor(sc, pSafeOther), pOtherCeil = gd_sec_ceil(sc, pSafeOther);
+  const int pSide = o.portalFront ? 0 : 1;
+  const int32_t *ptex = &sc.sideTex[(pIdx * 2 + pSide) * 3];
+  int pTop = gd_rows<kSplit>(sc, v, sh, pIdx, viewCeil, x), pBottom = gd_rows<kSplit>(sc, v, sh, pIdx, viewFloor, x);
+  int pLowerTop = gd_rows<kSplit>(sc, v, sh, pIdx, pOtherFloor, x);
+  int pUpperBottom = gd_rows<kSplit>(sc, v, sh, pIdx, pOtherCeil, x);
+  int pct = max(pTop, ceilClip), pcb = min(pBottom, floorClip);
+  int pcub = max(min(pUpperBottom, floorClip), pct);
+  int pclt = min(max(pLowerTop, ceilClip), pcb);
+  int4 ri = gd_sec_info(sc, o.rc), oi = gd_sec_info(sc, pSafeOther);
+  bool ld = ri.x != oi.x;
+  bool pDrawsUpper = (viewCeil > pOtherCeil) && ptex[2] >= 0;
+  bool pMarksCeil = (viewCeil != pOtherCeil) || ri.z != oi.z || ld;
+  if (pDrawsUpper || pMarksCeil) ceilClip = pDrawsUpper ? pcub : pct;
+  bool pDrawsLower = (viewFloor < pOtherFloor) && ptex[1] >= 0;
+  bool pMarksFloor = (viewFloor != pOtherFloor) || ri.y != oi.y || ld;
+  if (pDrawsLower || pMarksFloor) floorClip = pDrawsLower ? pclt : pcb;
+  bool pMasked = ptex[0] >= 0;
+  bool pBottomSil = (viewFloor > pOtherFloor) || (v.viewZ < pOtherFloor) || pMasked;
+  bool pTopSil = (viewCeil < pOtherCeil) || (v.viewZ > pOtherCeil) || pMasked;
+  if ((pBottomSil || pTopSil) && events)
+    gd_put_event(events, nEvents, x, o.portalDist, pIdx, -1, 0u,
+                 (pTopSil ? (unsigned)ceilClip : 0u) | ((pBottomSil ? (unsigned)floorClip : 255u) << 8), 0u);
+  return make_int2(ceilClip | (floorClip << 8), nEvents);
 }
 
 /* Rows [ya,yb) of column x that no plane owns yet become the span's; those no wall tier filled are drawn.
- * The pointers and the centre are taken into registers first: the byte stores into the frame would make the
- * compiler read them again from the shared structures on every trip. */
-template <bool kNarrow>
-__device__ __forceinline__ void gd_plane_rows(const GdPlaneSpan &p, i64 center, const GdShared &sh, int x, int ya, int yb,
-                                              unsigned *owned, const unsigned *filled) {
-  const unsigned dst = gd_shared_addr(sh.frame + x);
-  const unsigned yslope = gd_shared_addr(sh.yslope), colormap = gd_shared_addr(sh.colormap);
-  owned = gd_as_shared(owned); filled = gd_as_shared(filled);
-#pragma unroll 1
-  for (int k = ya >> 5; k <= (yb - 1) >> 5; ++k) {
-    unsigned have = owned[k * GD_SW];
-    unsigned fresh = gd_range_word(k, ya, yb) & ~have;
-    if (!fresh) continue;
-    owned[k * GD_SW] = have | fresh;
-    unsigned m = fresh & ~filled[k * GD_SW];
-    const int y0 = k << 5;
-#pragma unroll 1
-    while (m) {
-      int b0 = __ffs(m) - 1;
-      m &= m - 1;
-      int b1 = m ? __ffs(m) - 1 : b0;
-      m &= m - 1;
-      const unsigned p0 = gd_plane_pixel<kNarrow>(p, center, yslope, colormap, y0 + b0);
-      const unsigned p1 = gd_plane_pixel<kNarrow>(p, center, yslope, colormap, y0 + b1);
-      gd_sts8(dst + (y0 + b0) * GD_SW, p0);
-      gd_sts8(dst + (y0 + b1) * GD_SW, p1);
-    }
-  }
-}
-
-__device__ __noinline__ void gd_mark_plane(const GdScene &sc_, const GdView &v_, const GdShared &sh_, int x, int ya, int yb,
-                              int sector, bool isFloor, unsigned *owned, const unsigned *filled) {
+ * This is the form for spans whose operands need 64 bits. */
+__device__ __noinline__ void gd_plane_rows_wide(const GdScene &sc_, const GdView &v_, const GdShared &sh_, int x, int ya, int yb,
+                                                int sector, bool isFloor) {
   const GdScene &sc = *gd_as_shared(&sc_);
   const GdView &v = *gd_as_shared(&v_);
   const GdShared &sh = *gd_as_shared(&sh_);
-  if (ya >= yb) return;
-  const int k0 = ya >> 5, k1 = (yb - 1) >> 5;
-  unsigned any = 0;
-#pragma unroll 1
-  for (int k = k0; k <= k1; ++k) any |= gd_range_word(k, ya, yb) & ~owned[k * GD_SW];
-  if (!any) return;
   GdPlaneSpan p;
   gd_plane_setup(sc, sh.planeTab, sector, isFloor, x, p);
-  if (p.narrow) gd_plane_rows<true>(p, v.center, sh, x, ya, yb, owned, filled);
-  else gd_plane_rows<false>(p, v.center, sh, x, ya, yb, owned, filled);
+  unsigned *filled = (unsigned *)(gd_smem + GD_OFF_MASKS) + x, *owned = filled + 7 * GD_SW;
+#pragma unroll 1
+  for (int y = ya; y < yb; ++y) {
+    const unsigned bit = 1u << (y & 31);
+    const int k = (y >> 5) * GD_SW;
+    if (owned[k] & bit) continue;
+    owned[k] |= bit;
+    if (!(filled[k] & bit)) sh.frame[y * GD_SW + x] = (uint8_t)gd_plane_pixel(sc, p, v.center, y);
+  }
 }
 
 /* ---- two-sided middle textures (engine.py:13424-13745) -----------------------
@@ -603,13 +639,13 @@ __device__ __noinline__ void gd_masked_pass(const GdScene &sc_, const GdView &v_
 #pragma unroll 1
   for (int i = 0; i < sc.M; ++i) {
     const int k = GD_CHECK_INDEX(sc.maskedWalls[i], sc.W);
-    const int sd = sh.walls[k].frontF ? 0 : 1;
+    const int sd = (gd_hot(k).bits & GD_HOT_FRONT) ? 0 : 1;
     const int t = sc.sideTex[(k * 2 + sd) * 3];
     if (t < 0) continue;
 #ifdef GD_CHECKED
     if (t >= sc.T) { atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX); continue; }
 #endif
-    GdHit h = gd_hit_slow(sc, v, sh.walls, k, x, rx, ry);
+    GdHit h = gd_hit_slow(sc, k, x, rx, ry);
     if (h.proj && h.d < best) { best = h.d; w = k; side = sd; texId = t; leftEdge = h.left; }
   }
   /* what this column drew, for the decal layer's depth test: the crossing's distance in
@@ -684,7 +720,8 @@ __device__ __noinline__ void gd_masked_pass(const GdScene &sc_, const GdView &v_
  * column (engine.py:11589-11730, 11905-11990, 12005-12072), or through the rules that need
  * wall 0's projected span to end at this column (engine.py:11930-11962, 12073-12164).  Every
  * other column draws nothing, records nothing and changes nothing the frame depends on once
- * it is outside, so its walk can stop there.  This marks the columns that must go on. */
+ * it is outside, so its walk can stop there.  This marks the columns that may have to go on; all these rules
+ * ask for some wall whose projected span starts at the column, which the walk tests as well. */
 __device__ void gd_mark_afterlife_columns(const GdScene &sc, const GdShared &sh) {
   unsigned *busy = sh.ownerMask + 16;
   const int n0 = sc.secOff[1] - sc.secOff[0];
@@ -700,245 +737,419 @@ __device__ void gd_mark_afterlife_columns(const GdScene &sc, const GdShared &sh)
                      : (sc.nbDirect ? sc.nbDirectTab[i - n0] : sc.nbIdx[nb0 + (i - n0)]);
       if (w < 0) continue;                            /* no neighbour at that endpoint */
       w = GD_CHECK_INDEX(w, sc.W);
-      xl = sh.walls[w].isl;
+      xl = (int)(short)(gd_hot(w).span & 0xFFFFu);
     }
     if (xl >= 0 && xl < GD_SW) atomicOr(&busy[xl >> 5], 1u << (xl & 31));
   }
 }
 
-template <bool kSplit>
-__device__ void gd_walk(const GdScene &sc_, const GdView &v_, const GdShared &sh_, GdEvent *events, int *eventCount,
-                        const GdRowProj *rowproj, int *status, int startSector) {
+/* ---- phase: per-column portal walk (engine.py:11561-13371) -------------- */
+/* Thread x walks column x front to back.  Nearly every crossing is plain: nothing is carried over from the one
+ * before, and the nearest wall of the current sector is both crossed by the column's ray and owned by its
+ * projected span.  None of the ownership rules can then change the outcome: the owner rules ask for a selected
+ * wall that is not projected here (engine.py:11589-11730, 11905-12164), the endpoint rules for one that is not
+ * crossed (13070-13241), the bridges for something pending.  Such a crossing is decided below in one pass over
+ * the sector's walls; every other one takes gd_slow_step.  What bounds the walk is instruction fetch and issue:
+ * the loop is kept small enough for the instruction cache, and its operands are shared-memory tables at offsets
+ * that are launch constants. */
+/* Does the ray cross `wall` nearer to the endpoint (ex, ey) than to its other one (engine.py:11650-11668)? */
+__device__ __noinline__ bool gd_meets_end(int wall, float rx, float ry, const float *walls, float ex, float ey) {
+  const GdHot &h = gd_hot(wall);
+  const bool usesStart = (h.offx * ry - h.offy * rx) / (rx * h.segy - ry * h.segx) <= 0.5f;
+  const float2 e = *reinterpret_cast<const float2 *>(&walls[wall * 4 + (usesStart ? 0 : 2)]);
+  return e.x == ex && e.y == ey;
+}
+
+/* The ray of column x crosses wall `sel`, the nearest of the sector, but its projected span does not own the column, and
+ * nothing is pending.  True when no rule can hand the crossing to another wall (a superset of their conditions, without
+ * the distances): no one-sided wall of the sector at the same vertex, and none that may own the columns past the wall's
+ * end, starts its span here (engine.py:11905-11962), no line between the same two sectors touches it (11589-11730), no
+ * wall that owns the column is between the same sectors or takes over past a short line's right end (12005-12072), and
+ * the line is not itself too narrow to draw. */
+__device__ __noinline__ bool gd_quiet_crossing(const GdScene &sc_, const unsigned short *secWalls, int k0, int k1, int sel, int x,
+                                               float rx, float ry, bool spanStarts) {
   const GdScene &sc = *gd_as_shared(&sc_);
+  const GdHot s = gd_hot(sel);
+  const bool endsHere = GD_HOT_SR(s.bits) == x;
+  /* the clamped span is never wider than the real one */
+  if (endsHere && GD_HOT_SR(s.bits) - GD_HOT_SL(s.bits) <= 2) return false;
+  int vertex = -1;
+  if (spanStarts) {
+    if (s.bits & GD_HOT_NEIGHBOUR) return false;
+    if (endsHere && sc.wlen[sel] <= 32.0f) return false;
+    const bool usesStart = (s.offx * ry - s.offy * rx) / (rx * s.segy - ry * s.segx) <= 0.5f;
+    vertex = gd_vertex(sc, sel, usesStart ? 0 : 1);
+    if (endsHere && (s.bits & (usesStart ? GD_HOT_BRIDGE0 : GD_HOT_BRIDGE1))) {
+      const int32_t *off = usesStart ? sc.sbStartOff : sc.sbEndOff, *idx = usesStart ? sc.sbStartIdx : sc.sbEndIdx;
+#pragma unroll 1
+      for (int k = off[sel]; k < off[sel + 1]; ++k) {
+        const GdHot &h = gd_hot(GD_CHECK_INDEX(idx[k], sc.W));
+        if ((h.bits & GD_HOT_ONESIDED) && x == (int)(short)(h.span & 0xFFFFu) && x < (int)(h.span >> 16) && gd_ray_meets_line(h, rx, ry)) return false;
+      }
+    }
+  }
+  const int swapped = (int)(((unsigned)s.secs << 16) | ((unsigned)s.secs >> 16));
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    const int w = secWalls[k];
+    const GdHot &h = gd_hot(w);
+    const int isl = (int)(short)(h.span & 0xFFFFu);
+    if (w == sel || x < isl || x >= (int)(h.span >> 16) || !gd_ray_meets_line(h, rx, ry)) continue;
+    if (h.bits & GD_HOT_ONESIDED) {
+      if (x == isl && (gd_vertex(sc, w, 0) == vertex || gd_vertex(sc, w, 1) == vertex)) return false;
+    } else if (h.secs == s.secs || h.secs == swapped) {
+      return false;
+    }
+  }
+  return true;
+}
+
+__device__ __noinline__ int gd_light_wide(const GdWall &wv, int side, int x) {
+  return gd_vis_clamp(wv.visL[side] + gd_wmul((i64)x - wv.visSl[side], wv.visStep[side]));
+}
+
+/* Row bounds of a column outside the wall's projected span: the whole-wall projection (engine.py:12393-12410).
+ * Returns floor | ceiling << 8 of this side and of the side beyond, and the light. */
+__device__ __noinline__ uint3 gd_rows_outside(const GdView &v_, const GdWall &wv, const GdRowProj *rp, int side, bool beyond, int x) {
   const GdView &v = *gd_as_shared(&v_);
-  const GdShared &sh = *gd_as_shared(&sh_);
+  const i64 column = (i64)x - wv.sl;
+  unsigned r[2] = {0u, 0u};
+#pragma unroll 1
+  for (int k = 0; k < (beyond ? 4 : 2); ++k) {
+    const GdRowProj &q = rp[((k >> 1) ^ side) * 2 + (k & 1)];
+    r[k >> 1] |= (unsigned)gd_clamp((v.center + q.opl + gd_wmul(column, q.ostep)) >> 16, 0, GD_VH) << (8 * (k & 1));
+  }
+  return make_uint3(r[0], r[1], (unsigned)gd_light_wide(wv, side, x));
+}
+
+template <bool kSplit, bool kChip>
+__device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, const GdView &v, const GdShared &sh, uint8_t *frame,
+                                        uint8_t *tables, GdEvent *events, int *eventCount, const GdRowProj *rowproj, int startSector) {
   const int x = threadIdx.x;
-  const int lane = x & 31;
-  const unsigned quadBase = lane & ~3u;
+  const int quadBase = x & 28;
+  const unsigned quad = 15u << quadBase;
   float rx, ry;
   gd_ray(v, x, rx, ry);
-  unsigned *filled = gd_as_shared(sh.masks) + x, *owned = filled + 7 * GD_SW;
+  const GdRow *rows = (const GdRow *)(kChip ? gd_smem + p.offRows : tables + p.offRows);
+  const GdRow *fragRows = kChip ? rows + p.sc.W * 4 : p.fragRows + (size_t)blockIdx.x * p.sc.F * 4;
+  const float4 *prep = (const float4 *)(kChip ? gd_smem + p.offPrep : tables + p.offPrep);
+  const GdPlane *planes = (const GdPlane *)(kChip ? gd_smem + p.offPlanes : tables + p.offPlanes);
+  const GdSide *sides = kChip ? (const GdSide *)(gd_smem + p.offSides) : p.sides;
+  const float4 *sectors = (const float4 *)(gd_smem + p.offSectors);
+  const unsigned short *secOff = (const unsigned short *)(gd_smem + p.offSecOff), *secWalls = (const unsigned short *)(gd_smem + p.offSecWalls);
+  const unsigned *yslope = (const unsigned *)(gd_smem + GD_OFF_YSLOPE);
+  unsigned *filled = (unsigned *)(gd_smem + GD_OFF_MASKS) + x, *owned = filled + 7 * GD_SW;
 #pragma unroll
-  for (int k = 0; k < 7; ++k) { filled[k * GD_SW] = 0; owned[k * GD_SW] = 0; }
-  if (sc.M > 0) { sh.maskedDist[x] = GD_INF; sh.maskedInfo[x] = 0xFFFF0000u | GD_VH; }
-  GdColState c;
-  c.cur = startSector; c.ceilClip = 0; c.floorClip = GD_VH; c.prev = 0.0f;
+  for (int k = 0; k < 14; ++k) filled[k * GD_SW] = 0;
+  float *maskedDist = (float *)(gd_smem + GD_OFF_MASKED_DIST) + x;
+  unsigned *maskedInfo = (unsigned *)(gd_smem + GD_OFF_MASKED_INFO) + x;
+  if (p.sc.M > 0) { *maskedDist = GD_INF; *maskedInfo = 0xFFFF0000u | GD_VH; }
+  GdColState c;                     /* read and written by the slow path only */
   c.pendOwnerBoundary = c.pendEpBoundary = c.pendEpBridgeBoundary = c.pendPortalBridge = false;
   c.pendOwnerEpX = c.pendOwnerEpY = c.pendEpEpX = c.pendEpEpY = 0.0f;
   c.pendEpWall = c.pendEpBridgeIndex = c.pendPortalBridgeIndex = 0;
   c.pendPortalBridgeSector = -1;
   c.pendPortalBridgeExit = 0.0f;
-  bool settled = false;
-  const bool stopsOutside = !((sh.ownerMask[16 + (x >> 5)] >> (x & 31)) & 1u);
+  GdCross o;
+  int cur = startSector, ceilClip = 0, floorClip = GD_VH;
+  float prev = 0.0f;
+  bool pend = false, settled = false;
+  bool pendEnd = false;             /* all that is pending is that the last crossing met a wall's end only */
+  const unsigned *columns = (const unsigned *)(gd_smem + GD_OFF_OWNER) + (x >> 5);
+  const bool spanStarts = (columns[32] >> (x & 31)) & 1u;         /* some wall's projected span starts here */
+  const bool stopsOutside = !(spanStarts && ((columns[16] >> (x & 31)) & 1u));
+  /* clip events are read where sprites or chips may cover the column */
+  const bool wantEvents = p.decals != nullptr || ((const unsigned long long *)(gd_smem + GD_OFF_CAND))[x] != 0;
   int nEvents = 0;
-  bool overflow = false;
 
-  for (int iter = 0; iter < sc.S; ++iter) {
+#pragma unroll 1
+  for (int iter = 0; iter < p.sc.S; ++iter) {
     if (__all_sync(0xffffffffu, settled)) break;
-    GdIter it;
-    if (!settled) {
-      gd_column_decide<kSplit>(sc, v, sh.walls, sh.frags, sh.ownerMask, rowproj, sh.hitD, sh.hitA, sh.hitF, x, rx, ry, c, it);
-    } else {
-      it.wall = -1 - x; it.side = 0; it.tier[0] = it.tier[1] = it.tier[2] = false;
-      it.ctop = it.clowtop = 0; it.cbot = it.cupbot = 0; it.vis = 0;
-      it.rasterValid = false; it.valid = false; it.pskpp = false;
-    }
-    /* aligned four-column wallscan groups (engine.py:12694-12761) */
-    bool same = true;
-    bool groupValid[3];
-    int groupBottom[3];
-    {
-      int w0 = __shfl_sync(0xffffffffu, it.wall, quadBase), s0 = __shfl_sync(0xffffffffu, it.side, quadBase);
-#pragma unroll
-      for (int k = 1; k < 4; ++k) {
-        int wk = __shfl_sync(0xffffffffu, it.wall, quadBase + k), sk = __shfl_sync(0xffffffffu, it.side, quadBase + k);
-        same = same && (wk == w0) && (sk == s0);
-      }
-#pragma unroll
-      for (int tier = 0; tier < 3; ++tier) {
-        int top = tier == 1 ? it.clowtop : it.ctop;
-        int bot = tier == 2 ? it.cupbot : it.cbot;
-        int topMax = -1, botMin = 1 << 20;
-        bool all = true;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          topMax = max(topMax, __shfl_sync(0xffffffffu, top, quadBase + k));
-          botMin = min(botMin, __shfl_sync(0xffffffffu, bot, quadBase + k));
-          int tk = __shfl_sync(0xffffffffu, (int)it.tier[tier], quadBase + k);  /* never short-circuit a shuffle */
-          all = all && (tk != 0);
+    const bool active = !settled;
+    int wall = -1 - x, side = 0, vis = 0, rc = 0, ro = 0, next = -1;
+    unsigned flags = 0, tops = 0, bots = 0;
+    float dist = 0.0f, nextPrev = 0.0f;
+    if (active) {
+      bool slow = (pend && !pendEnd) || cur < 0;
+      if (!slow) {
+        /* nearest wall beyond prev; a one-sided one within 1e-3 of it goes first (engine.py:11589-11640) */
+        float best = GD_INF, solid = GD_INF;
+        unsigned bestTag = 0, solidTag = 0;           /* wall | 1 << 31: crossed by the ray | 1 << 30: owned by the projected span */
+        const int k1 = secOff[cur + 1];
+#pragma unroll 1
+        for (int k = secOff[cur]; k < k1; ++k) {
+          const int w = secWalls[k];
+          const float4 g = *reinterpret_cast<const float4 *>(&gd_hot(w));
+          const int4 h = *(reinterpret_cast<const int4 *>(&gd_hot(w)) + 1);
+          const float dn = __int_as_float(h.x);
+          const float den = rx * g.y - ry * g.x;
+          if (fabsf(den) < 1e-6f || dn == 0.0f || (dn < 0) != (den < 0)) continue;
+          const float an = g.z * ry - g.w * rx;
+          const bool geo = an == 0.0f || ((an < 0) == (den < 0) && fabsf(an) <= fabsf(den));
+          const bool proj = x >= (int)(short)(h.y & 0xFFFF) && x < (int)((unsigned)h.y >> 16);
+          const bool oneSided = ((unsigned)h.w & GD_HOT_ONESIDED) != 0;
+          if (!(oneSided ? (proj && ((unsigned)h.w & GD_HOT_FRONT)) : (geo || proj))) continue;
+          const float d = dn / den;
+          if (!(d > prev)) continue;
+          const unsigned tag = (unsigned)w | (geo ? 0x80000000u : 0u) | (proj ? 0x40000000u : 0u);
+          if (d < best) { best = d; bestTag = tag; }
+          if (oneSided && d < solid) { solid = d; solidTag = tag; }
         }
-        groupValid[tier] = same && all && topMax < botMin;
-        groupBottom[tier] = botMin;
-      }
-    }
-    i64 firstVis = __shfl_sync(0xffffffffu, it.vis, quadBase);
-    if (settled) continue;
-
-    const GdColState before = c;
-    const int wallIndex = it.wall, side = it.side;
-    const GdWall &wv = sh.walls[wallIndex];
-    GdEvent ev;
-    ev.dist = it.distance; ev.wall = (short)wallIndex; ev.sector = -1;
-    ev.t0a = ev.t0b = ev.t1a = ev.t1b = 0; ev.silTop = 0; ev.silBot = 255;
-    ev.ceilA = ev.ceilB = ev.floorA = ev.floorB = 0; ev.pad0 = 0; ev.pad1 = 0;
-    if (it.rasterValid) {
-      /* visplane rows uncovered by this seg (engine.py:12637-12655) */
-      int cpb = min(it.ctop, c.floorClip), fpt = max(it.cbot, c.ceilClip);
-      ev.sector = (short)it.renderCurrent;
-      if (it.markFloor && fpt < c.floorClip) {
-        ev.floorA = (unsigned char)fpt; ev.floorB = (unsigned char)c.floorClip;
-        gd_mark_plane(sc, v, sh, x, fpt, c.floorClip, it.renderCurrent, true, owned, filled);
-      }
-      if (it.markCeil && c.ceilClip < cpb) {
-        ev.ceilA = (unsigned char)c.ceilClip; ev.ceilB = (unsigned char)cpb;
-        gd_mark_plane(sc, v, sh, x, c.ceilClip, cpb, it.renderCurrent, false, owned, filled);
-      }
-      /* wall tiers */
-      GdTierCtx t;
-      gd_prep_wall(sc, wv, wallIndex, x, t.hoff, t.vstepBase);
-      i64 repeat = gd_rint(sc.wlen[wallIndex] * 65536.0f);
-      if (side != 0) t.hoff = repeat - t.hoff;
-      if (wv.sl > 0 && t.hoff < 0) t.hoff = 0;
-      if (t.hoff >= repeat) t.hoff = repeat - 1;
-      const float *soff = &sc.sideOff[(wallIndex * 2 + side) * 2];
-      t.tox = gd_rint(soff[0] * 65536.0f);
-      t.yoff = soff[1];
-      const float *wl = &sc.walls[wallIndex * 4];
-      bool horizontal = fabsf(wl[3] - wl[1]) < 1e-6f, vertical = fabsf(wl[2] - wl[0]) < 1e-6f;
-      t.light = gd_sec_info(sc, it.renderCurrent).x + v.flashLight * 16 + (vertical ? 16 : (horizontal ? -16 : 0));
-      t.tailBottom = 0;
-      if (it.oneSided) {
-        if (it.ctop < it.cbot) {
-          ev.t0a = (unsigned char)it.ctop; ev.t0b = (unsigned char)it.cbot;
-          if (it.tex[0] >= 0) ev.pad0 |= 1;
-          gd_draw_tier(sc, v, sh, x, it.ctop, it.cbot, 0, 0, it.tex[0], it.viewCeil, t, it.vis, firstVis,
-                       groupValid[0], groupBottom[0], 0, 0, false, 0, filled);
+        if (fabsf(solid - best) <= 1e-3f) { best = solid; bestTag = solidTag; }
+        wall = (int)(bestTag & 0x3FFFFFFFu);
+        const unsigned kind = bestTag >> 30;          /* 3: crossed and owned, 2: crossed, 1: owned, 0: nothing beyond prev */
+        if (kind == 3u) slow = pendEnd && gd_meets_end(wall, rx, ry, p.sc.walls, c.pendEpEpX, c.pendEpEpY);
+        else if (pendEnd) slow = true;
+        else if (kind == 2u) slow = !gd_quiet_crossing(sc, secWalls, secOff[cur], k1, wall, x, rx, ry, spanStarts);
+        else if (kind == 1u) slow = !(gd_hot(wall).bits & GD_HOT_ONESIDED);     /* a one-sided end of the column either way */
+        else slow = spanStarts;
+        if (!slow && kind == 0u) {
+          /* no wall is left and no span starts here: no rule finds another one, the column leaves the map */
+          wall = -1 - x;
+        } else
+        if (!slow) {
+          const int secs = gd_hot(wall).secs;
+          const unsigned bits = gd_hot(wall).bits;
+          const int front = (int)(short)(secs & 0xFFFF), back = secs >> 16;
+          side = cur == front ? 0 : 1;
+          const int other = side ? front : back;
+          const GdRow *unit = rows + wall * 4;
+          if (kSplit && (bits & GD_HOT_SPLIT)) {
+            /* the first fragment whose half-open span holds the column (engine.py:12310-12376) */
+            const unsigned *spans = (const unsigned *)(gd_smem + p.offFrags);
+            const int f1 = p.sc.fragOff[wall + 1];
+            int f = p.sc.fragOff[wall];
+#pragma unroll 1
+            for (; f < f1; ++f)
+              if (x >= (int)(spans[f] & 0xFFFFu) && x < (int)(spans[f] >> 16)) break;
+            unit = f < f1 ? fragRows + f * 4 : nullptr;      /* none: the whole line's projection */
+          } else {
+            if (x < GD_HOT_SL(bits) || x >= GD_HOT_SR(bits)) unit = nullptr;
+          }
+          slow = side && cur != back;
+          if (!slow) {
+            unsigned wide = 0u;
+            int bottom, top, beyondBottom = 0, beyondTop = 0;
+            if (unit) {
+              const GdRow rf = unit[side * 2], rt = unit[side * 2 + 1];
+              wide = rf.lim | rt.lim;
+              bottom = gd_row_eval(rf, x); top = gd_row_eval(rt, x);
+              vis = min((int)((unsigned)rf.vis + (unsigned)x * (unsigned)rt.vis), 24 * (int)GD_FU);
+              if (rf.lim & GD_ROW_LIGHT_WIDE)
+                vis = gd_light_wide(kSplit && (bits & GD_HOT_SPLIT) ? sh.frags[(unit - fragRows) >> 2] : sh.walls[wall], side, x);
+              if (other >= 0) {
+                const GdRow ol = unit[(side ^ 1) * 2], ou = unit[(side ^ 1) * 2 + 1];
+                wide |= ol.lim | ou.lim;
+                beyondBottom = gd_row_eval(ol, x); beyondTop = gd_row_eval(ou, x);
+              }
+            } else {
+              const uint3 r = gd_rows_outside(v, sh.walls[wall], rowproj + wall * 4, side, other >= 0, x);
+              bottom = r.x & 255u; top = (r.x >> 8) & 255u;
+              beyondBottom = r.y & 255u; beyondTop = (r.y >> 8) & 255u;
+              vis = (int)r.z;
+            }
+            const GdSide &sd = sides[wall * 2 + side];
+            flags = sd.flags;
+            const int ctop = max(top, ceilClip), cbot = min(bottom, floorClip);
+            int cupbot = ctop, clowtop = cbot;
+            if (other >= 0) {
+              clowtop = min(max(beyondBottom, ceilClip), cbot);
+              cupbot = max(min(beyondTop, floorClip), ctop);
+            }
+            slow = (wide & GD_ROW_WIDE) != 0;
+            tops = (unsigned)ctop | ((unsigned)clowtop << 16);
+            bots = (unsigned)(255 - cbot) | ((unsigned)(255 - cupbot) << 16);
+            /* the static flags name the tiers that have a texture; they need rows as well */
+            if (ctop >= cbot) flags &= ~GD_C_TIER0;
+            if (clowtop >= cbot) flags &= ~GD_C_TIER1;
+            if (ctop >= cupbot) flags &= ~GD_C_TIER2;
+            rc = cur; ro = other < 0 ? 0 : other;
+            dist = best;
+            next = other; nextPrev = best;
+          }
         }
+      }
+      if (slow) {
+        c.cur = cur; c.prev = prev; c.ceilClip = ceilClip; c.floorClip = floorClip;
+        gd_slow_step<kSplit>(sc, v, sh, rowproj, x, rx, ry, stopsOutside, c, o);
+        wall = o.wall; side = o.side; flags = o.flags; tops = o.tops; bots = o.bots; vis = o.vis; rc = o.rc; ro = o.ro;
+        dist = o.dist; next = o.cur; nextPrev = o.prev; pend = o.pend; pendEnd = o.pendEnd; settled = o.settled;
       } else {
-        bool lowerCond = it.viewFloor < it.otherFloor, upperCond = it.viewCeil > it.otherCeil;
-        int la = 0, lb = 0;
-        if (lowerCond && it.clowtop < it.cbot) {
-          la = it.clowtop; lb = it.cbot;
-          ev.t1a = (unsigned char)la; ev.t1b = (unsigned char)lb;
-          if (it.tex[1] >= 0) ev.pad0 |= 2;
-          bool upperOn = upperCond && it.ctop < it.cupbot;
-          gd_draw_tier(sc, v, sh, x, la, lb, 0, 0, it.tex[1], it.otherFloor, t, it.vis, firstVis, groupValid[1],
-                       groupBottom[1], it.ctop, it.cupbot, upperOn && groupValid[2], groupBottom[2], filled);
+        settled = next < 0 && stopsOutside;
+        if (pend) { pend = pendEnd = false; c.pendEpBoundary = false; }
+      }
+    }
+    /* aligned four-column wallscan groups (engine.py:12694-12761): tops and bottoms travel as byte maxima */
+    const int key = wall * 2 + side;
+    const bool same = (__ballot_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, quadBase)) & quad) == quad;
+    const bool all0 = (__ballot_sync(0xffffffffu, (flags & GD_C_TIER0) != 0) & quad) == quad;
+    const bool all1 = (__ballot_sync(0xffffffffu, (flags & GD_C_TIER1) != 0) & quad) == quad;
+    const bool all2 = (__ballot_sync(0xffffffffu, (flags & GD_C_TIER2) != 0) & quad) == quad;
+    unsigned topMax = __vmaxu2(tops, __shfl_xor_sync(0xffffffffu, tops, 1)), botMax = __vmaxu2(bots, __shfl_xor_sync(0xffffffffu, bots, 1));
+    topMax = __vmaxu2(topMax, __shfl_xor_sync(0xffffffffu, topMax, 2));
+    botMax = __vmaxu2(botMax, __shfl_xor_sync(0xffffffffu, botMax, 2));
+    const int firstVis = __shfl_sync(0xffffffffu, vis, quadBase);
+    if (!active) continue;
+
+    if (flags & GD_C_RASTER) {
+      const int ctop = (int)(tops & 0xFFFFu), clowtop = (int)(tops >> 16), cbot = 255 - (int)(bots & 0xFFFFu), cupbot = 255 - (int)(bots >> 16);
+      const int oldCeil = ceilClip, oldFloor = floorClip;
+      const float4 here = sectors[rc], there = sectors[ro];    /* floor, ceiling, light */
+      const int centerRow = (int)(v.center >> 16);
+      /* visplane rows uncovered by this seg (engine.py:12637-12655) */
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+        const bool isFloor = q == 0;
+        const int ya = isFloor ? max(cbot, ceilClip) : ceilClip, yb = isFloor ? floorClip : min(ctop, floorClip);
+        if (!(flags & (isFloor ? GD_C_MARK_FLOOR : GD_C_MARK_CEIL)) || ya >= yb) continue;
+        const int k1 = (yb - 1) >> 5;
+        unsigned any = 0;
+#pragma unroll 1
+        for (int k = ya >> 5; k <= k1; ++k) any |= gd_range_word(k, ya, yb) & ~owned[k * GD_SW];
+        if (!any) continue;
+        const int4 *e = reinterpret_cast<const int4 *>(&planes[rc * 2 + (isFloor ? 1 : 0)]);
+        const int4 e0 = e[0];
+        /* rows lie farther from the viewer towards the horizon: the row that bounds the span's distance */
+        const unsigned far = ya > centerRow ? yslope[ya] : (yb <= centerRow ? yslope[yb - 1] : 0xffffffffu);
+        if (!((unsigned)e0.w & GD_PLANE_NARROW) || ((unsigned long long)(unsigned)e0.x * far) >> 47) {
+          gd_plane_rows_wide(sc, v, sh, x, ya, yb, rc, isFloor);
+          continue;
         }
-        if (upperCond && it.ctop < it.cupbot) {
-          ev.t0a = (unsigned char)it.ctop; ev.t0b = (unsigned char)it.cupbot;
-          if (it.tex[2] >= 0) ev.pad0 |= 1;
-          gd_draw_tier(sc, v, sh, x, it.ctop, it.cupbot, la, lb, it.tex[2], it.otherCeil, t, it.vis, firstVis,
-                       groupValid[2], groupBottom[2], 0, 0, false, 0, filled);
+        const int4 e1 = e[1], e2 = e[2];
+        GdNarrowSpan s;
+        s.phf = (unsigned)e0.x; s.gv = e0.y; s.shadeBase = e0.z;
+        s.xshift = e0.w & 63; s.yshift = (e0.w >> 8) & 63;
+        s.basex = e1.x + (x - 159) * e1.y; s.basey = e1.z + (x - 159) * e1.w;
+        s.pviewx = (unsigned)e2.x; s.pviewy = (unsigned)e2.y; s.tex = (unsigned)e2.z;
+        const int center = (int)v.center;
+#pragma unroll 1
+        for (int k = ya >> 5; k <= k1; ++k) {
+          const unsigned have = owned[k * GD_SW];
+          const unsigned fresh = gd_range_word(k, ya, yb) & ~have;
+          if (!fresh) continue;
+          owned[k * GD_SW] = have | fresh;
+          unsigned m = fresh & ~filled[k * GD_SW];
+          const int y0 = k << 5;
+          /* two rows per trip; an odd last row is simply drawn twice */
+#pragma unroll 1
+          while (m) {
+            const int b0 = __ffs(m) - 1;
+            m &= m - 1;
+            const int b1 = m ? __ffs(m) - 1 : b0;
+            m &= m - 1;
+            const unsigned p0 = gd_plane_pixel_narrow(s, p.sc.texAtlas, p.sc.texW, center, y0 + b0);
+            const unsigned p1 = gd_plane_pixel_narrow(s, p.sc.texAtlas, p.sc.texW, center, y0 + b1);
+            frame[(unsigned)((y0 + b0) * GD_SW + x)] = (uint8_t)p0;
+            frame[(unsigned)((y0 + b1) * GD_SW + x)] = (uint8_t)p1;
+          }
+        }
+      }
+      /* wall tiers: middle or lower first, then upper; the lower one has priority where they overlap
+       * (engine.py:12762-12884) */
+      const GdSide &sd = sides[wall * 2 + side];
+      const bool oneSided = (flags & GD_C_ONE_SIDED) != 0;
+      const bool lowRange = !oneSided && (flags & GD_C_LOWER) && clowtop < cbot, upRange = !oneSided && (flags & GD_C_UPPER) && ctop < cupbot;
+      if (flags & (GD_C_TIER0 | GD_C_TIER1 | GD_C_TIER2)) {
+        const i64 repeat = sd.repeat;
+        i64 hoff, vstepBase;
+        gd_prep_eval(prep[wall], repeat, x, hoff, vstepBase);
+        if (side != 0) hoff = repeat - hoff;
+        if (GD_HOT_SL(gd_hot(wall).bits) > 0 && hoff < 0) hoff = 0;
+        if (hoff >= repeat) hoff = repeat - 1;
+        const i64 column = (hoff + sd.tox) >> 16;
+        const int base = gd_shade_base(__float_as_int(here.z) + v.flashLight * 16 + sd.contrast);
+        const unsigned cmN = (unsigned)gd_shade(base, vis) * 256u, cmT = (unsigned)gd_shade(base, firstVis) * 256u;
+#pragma unroll 1
+        for (int q = 0; q < 2; ++q) {
+          const bool upper = q == 1;
+          if (!(flags & (upper ? GD_C_TIER2 : (oneSided ? GD_C_TIER0 : GD_C_TIER1)))) continue;
+          const int texId = sd.tex[upper ? 2 : (oneSided ? 0 : 1)];
+#ifdef GD_CHECKED
+          if (texId >= sc.T) { atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX); continue; }   /* the tier stays undrawn */
+#endif
+          const int ya = upper || oneSided ? ctop : clowtop, yb = upper ? cupbot : cbot;
+          const float originZ = upper ? there.y : (oneSided ? here.y : there.x);
+          const int ea = upper && lowRange ? clowtop : 0, eb = upper && lowRange ? cbot : 0;
+          /* rows lit with the group's first-column light: below the group's highest bottom */
+          const int gb0 = 255 - (int)(botMax & 0xFFFFu), gb2 = 255 - (int)(botMax >> 16);
+          const bool group2 = same && all2 && (int)(topMax & 0xFFFFu) < gb2;
+          const bool group = upper ? group2 : (same && (oneSided ? (all0 && (int)(topMax & 0xFFFFu) < gb0) : (all1 && (int)(topMax >> 16) < gb0)));
+          const int tailA = group && cmN != cmT ? (upper ? gb2 : gb0) : GD_VH;
+          const bool otherTail = !upper && !oneSided && upRange && group2 && cmN != cmT;
+          const int oTailA = otherTail ? max(ctop, gb2) : 0, oTailB = otherTail ? cupbot : 0;
+          const int4 ti = *reinterpret_cast<const int4 *>(&p.sc.texInfo[texId * 4]);
+          const int hbits = ti.w;
+          const unsigned u = (unsigned)gd_pymod_width(column, ti.x);
+          const i64 vstep = vstepBase * (1LL << (14 - hbits));
+          const i64 texMid = gd_rint((originZ - v.viewZ) * 65536.0f + sd.yoff * 65536.0f);
+          /* frac(y) = (texMid << (16-bits)) + ((vstep * (y*FU - center + FU)) >> 16); the
+           * y term is a multiple of 2^16 inside the shift, so it steps by vstep exactly. */
+          const unsigned frac0 = (unsigned)(gd_shl(texMid, 16 - hbits) + (gd_wmul(vstep, GD_FU - v.center) >> 16));
+          const unsigned step = (unsigned)vstep;
+          const unsigned texel0 = ((unsigned)texId * (unsigned)p.sc.texW + u) * (unsigned)p.sc.texH;
+          const int shift = 32 - hbits;
+#pragma unroll 1
+          for (int k = ya >> 5; k <= (yb - 1) >> 5; ++k) {
+            const unsigned have = filled[k * GD_SW];
+            unsigned m = gd_range_word(k, ya, yb) & ~gd_range_word(k, ea, eb) & ~have;
+            if (!m) continue;
+            filled[k * GD_SW] = have | m;
+            const unsigned tailM = gd_range_word(k, tailA, GD_VH) | gd_range_word(k, oTailA, oTailB);
+            const int y0 = k << 5;
+#pragma unroll 1
+            while (m) {
+              const int b0 = __ffs(m) - 1;
+              m &= m - 1;
+              const int b1 = m ? __ffs(m) - 1 : b0;
+              m &= m - 1;
+              const unsigned f0 = frac0 + (unsigned)(y0 + b0) * step, f1 = frac0 + (unsigned)(y0 + b1) * step;
+              const unsigned t0 = p.sc.texAtlasCol[texel0 + (f0 >> shift)], t1 = p.sc.texAtlasCol[texel0 + (f1 >> shift)];
+              const uint8_t p0 = gd_smem[GD_OFF_COLORMAP + ((tailM >> b0) & 1u ? cmT : cmN) + t0];
+              const uint8_t p1 = gd_smem[GD_OFF_COLORMAP + ((tailM >> b1) & 1u ? cmT : cmN) + t1];
+              frame[(unsigned)((y0 + b0) * GD_SW + x)] = p0;
+              frame[(unsigned)((y0 + b1) * GD_SW + x)] = p1;
+            }
+          }
+        }
+      }
+      /* clip updates (engine.py:12885-12913) */
+      const bool masked = sd.tex[0] >= 0;
+      if (!oneSided) {
+        const bool drawsUpper = (flags & GD_C_UPPER) && sd.tex[2] >= 0, drawsLower = (flags & GD_C_LOWER) && sd.tex[1] >= 0;
+        if (drawsUpper || (flags & GD_C_MARK_CEIL)) ceilClip = drawsUpper ? cupbot : ctop;
+        if (drawsLower || (flags & GD_C_MARK_FLOOR)) floorClip = drawsLower ? clowtop : cbot;
+        /* masked drawseg snapshot (engine.py:12914-12939) */
+        if (masked && p.sc.M > 0 && dist < *maskedDist) {
+          *maskedDist = dist;
+          *maskedInfo = ((unsigned)wall << 16) | ((unsigned)ceilClip << 8) | (unsigned)floorClip;
+        }
+      }
+      if (wantEvents) {
+        /* sprite silhouettes (engine.py:12940-12964); a crossing that draws, marks and clips nothing leaves no trace */
+        const bool bottomSil = !oneSided && ((flags & GD_C_FLOOR_ABOVE) || v.viewZ < there.x || masked);
+        const bool topSil = !oneSided && ((flags & GD_C_CEIL_BELOW) || v.viewZ > there.y || masked);
+        const int fa = max(cbot, oldCeil), cb = min(ctop, oldFloor);
+        const bool floorOn = (flags & GD_C_MARK_FLOOR) && fa < oldFloor, ceilOn = (flags & GD_C_MARK_CEIL) && oldCeil < cb;
+        const bool mid = oneSided && ctop < cbot;
+        const unsigned sil = (topSil ? (unsigned)ceilClip : 0u) | ((bottomSil ? (unsigned)floorClip : 255u) << 8);
+        const unsigned tiers = (mid ? (unsigned)ctop | ((unsigned)cbot << 8) : (upRange ? (unsigned)ctop | ((unsigned)cupbot << 8) : 0u)) |
+                               (lowRange ? ((unsigned)clowtop << 16) | ((unsigned)cbot << 24) : 0u);
+        if (mid || upRange || lowRange || sil != (255u << 8) || floorOn || ceilOn) {
+          const unsigned drawn = ((mid && masked) || (upRange && sd.tex[2] >= 0) ? 1u : 0u) | (lowRange && sd.tex[1] >= 0 ? 2u : 0u);
+          gd_put_event(events, nEvents, x, dist, wall, rc, tiers,
+                       sil | (ceilOn ? ((unsigned)oldCeil << 16) | ((unsigned)cb << 24) : 0u),
+                       (floorOn ? (unsigned)fa | ((unsigned)oldFloor << 8) : 0u) | (drawn << 16));
         }
       }
     }
-    /* clip updates (engine.py:12885-12913) */
-    bool hasUpper = it.tex[2] >= 0, hasLower = it.tex[1] >= 0;
-    bool drawsUpper = (it.viewCeil > it.otherCeil) && hasUpper;
-    bool drawsLower = (it.viewFloor < it.otherFloor) && hasLower;
-    if (it.rasterValid && !it.oneSided && (drawsUpper || it.markCeil)) c.ceilClip = drawsUpper ? it.cupbot : it.ctop;
-    if (it.rasterValid && !it.oneSided && (drawsLower || it.markFloor)) c.floorClip = drawsLower ? it.clowtop : it.cbot;
-    /* masked drawseg snapshot (engine.py:12914-12939) */
-    if (sc.M > 0 && it.rasterValid && !it.oneSided && it.tex[0] >= 0 && it.distance < sh.maskedDist[x]) {
-      sh.maskedDist[x] = it.distance;
-      sh.maskedInfo[x] = ((unsigned)wallIndex << 16) | ((unsigned)c.ceilClip << 8) | (unsigned)c.floorClip;
+    if (flags & GD_C_PORTAL) {
+      const int2 clips = gd_portal_clips<kSplit>(sc, v, sh, x, o, ceilClip | (floorClip << 8), wantEvents ? events : nullptr, nEvents);
+      ceilClip = clips.x & 255; floorClip = clips.x >> 8; nEvents = clips.y;
     }
-    /* sprite silhouettes (engine.py:12940-12964) */
-    if (it.rasterValid) {
-      bool masked = it.tex[0] >= 0;
-      bool bottomSil = !it.oneSided && ((it.viewFloor > it.otherFloor) || (v.viewZ < it.otherFloor) || masked);
-      bool topSil = !it.oneSided && ((it.viewCeil < it.otherCeil) || (v.viewZ > it.otherCeil) || masked);
-      if (bottomSil) ev.silBot = (unsigned char)c.floorClip;
-      if (topSil) ev.silTop = (unsigned char)c.ceilClip;
-      /* a crossing that draws, marks and clips nothing leaves no trace */
-      bool empty = ev.t0a == ev.t0b && ev.t1a == ev.t1b && ev.silTop == 0 && ev.silBot == 255 &&
-                   ev.ceilA == ev.ceilB && ev.floorA == ev.floorB;
-      if (!empty) {
-        if (nEvents < GD_MAX_EVENTS) events[nEvents * GD_SW + x] = ev; else overflow = true;
-        nEvents++;
-      }
-    }
-    /* clips contributed by the portal crossed behind a projected solid
-     * (engine.py:12965-13069) */
-    if (it.pskpp) {
-      int pIdx = it.psPathIndex;
-      int pSafeOther = it.psOther < 0 ? 0 : it.psOther;
-      float pOtherFloor = gd_sec_floor(sc, pSafeOther), pOtherCeil = gd_sec_ceil(sc, pSafeOther);
-      int pSide = it.psFromFront ? 0 : 1;
-      const int32_t *ptex = &sc.sideTex[(pIdx * 2 + pSide) * 3];
-      int pTop = gd_rows<kSplit>(sc, v, sh, pIdx, it.viewCeil, x), pBottom = gd_rows<kSplit>(sc, v, sh, pIdx, it.viewFloor, x);
-      int pLowerTop = gd_rows<kSplit>(sc, v, sh, pIdx, pOtherFloor, x);
-      int pUpperBottom = gd_rows<kSplit>(sc, v, sh, pIdx, pOtherCeil, x);
-      int pct = max(pTop, c.ceilClip), pcb = min(pBottom, c.floorClip);
-      int pcub = max(min(pUpperBottom, c.floorClip), pct);
-      int pclt = min(max(pLowerTop, c.ceilClip), pcb);
-      int4 ri = gd_sec_info(sc, it.renderCurrent), oi = gd_sec_info(sc, pSafeOther);
-      bool ld = ri.x != oi.x;
-      bool pDrawsUpper = (it.viewCeil > pOtherCeil) && ptex[2] >= 0;
-      bool pMarksCeil = (it.viewCeil != pOtherCeil) || ri.z != oi.z || ld;
-      if (pDrawsUpper || pMarksCeil) c.ceilClip = pDrawsUpper ? pcub : pct;
-      bool pDrawsLower = (it.viewFloor < pOtherFloor) && ptex[1] >= 0;
-      bool pMarksFloor = (it.viewFloor != pOtherFloor) || ri.y != oi.y || ld;
-      if (pDrawsLower || pMarksFloor) c.floorClip = pDrawsLower ? pclt : pcb;
-      bool pMasked = ptex[0] >= 0;
-      bool pBottomSil = (it.viewFloor > pOtherFloor) || (v.viewZ < pOtherFloor) || pMasked;
-      bool pTopSil = (it.viewCeil < pOtherCeil) || (v.viewZ > pOtherCeil) || pMasked;
-      GdEvent pe;
-      pe.dist = it.psDist; pe.wall = (short)pIdx; pe.sector = -1;
-      pe.t0a = pe.t0b = pe.t1a = pe.t1b = 0; pe.pad0 = 0; pe.pad1 = 0;
-      pe.ceilA = pe.ceilB = pe.floorA = pe.floorB = 0;
-      pe.silBot = pBottomSil ? (unsigned char)c.floorClip : 255;
-      pe.silTop = pTopSil ? (unsigned char)c.ceilClip : 0;
-      if (pBottomSil || pTopSil) {
-        if (nEvents < GD_MAX_EVENTS) events[nEvents * GD_SW + x] = pe; else overflow = true;
-        nEvents++;
-      }
-    }
-    /* traversal update (engine.py:13242-13371) */
-    float prior = c.prev;
-    float np = prior;
-    if (it.valid) {
-      if (it.nokpp) np = it.nopDist;
-      else if (it.pskpp) np = it.psDist;
-      else if (it.entersShared && (it.osd < it.distance)) np = prior;
-      else if (it.usesGeo) np = it.gpDist;
-      else np = it.distance;
-    }
-    if (it.valid && it.epb) np = prior;
-    if (it.valid && it.cppb) np = fmaxf(it.distance, c.pendPortalBridgeExit);
-    c.prev = np;
-    if (it.startsOwner) { c.pendOwnerEpX = it.selEpX; c.pendOwnerEpY = it.selEpY; }
-    c.pendOwnerBoundary = it.startsOwner || (c.pendOwnerBoundary && it.continuesOwner);
-    if (it.endpointOnly) { c.pendEpEpX = it.epEpX; c.pendEpEpY = it.epEpY; c.pendEpWall = wallIndex; }
-    c.pendEpBoundary = it.endpointOnly;
-    if (it.pendEpHasFwd) c.pendEpBridgeIndex = it.epFwdIdx;
-    c.pendEpBridgeBoundary = it.pendEpHasFwd;
-    int next;
-    if (it.nokpp) next = it.nopOther;
-    else if (it.pskpp) next = it.psOther;
-    else if (it.usesGeo) next = it.gpOther;
-    else if (it.valid && !it.oneSided && (it.geometric || it.entersOther || it.entersShared)) next = it.otherSector;
-    else if (it.endpointOnly) next = c.cur;
-    else next = -1;
-    if (it.epb) next = it.otherSector;
-    if (it.cppb) next = c.pendPortalBridgeSector;
-    if (it.epb) {
-      c.pendPortalBridgeIndex = it.ppbIdx;
-      c.pendPortalBridgeSector = it.gpOther;
-      c.pendPortalBridgeExit = it.gpDist;
-    }
-    c.pendPortalBridge = it.epb;
-    c.cur = next;
-    /* A column that has left the map repeats the same decision on the same
-     * state forever; once an iteration changes nothing and draws nothing it can
-     * stop. */
-    if (before.cur < 0 && !it.rasterValid && !it.pskpp && gd_state_equal(before, c)) settled = true;
-    if (c.cur < 0 && stopsOutside) settled = true;
+    cur = next; prev = nextPrev;
   }
   eventCount[x] = nEvents < GD_MAX_EVENTS ? nEvents : GD_MAX_EVENTS;
-  if (overflow) atomicOr(status, GD_STATUS_EVENT_OVERFLOW);
-
+  if (nEvents > GD_MAX_EVENTS) atomicOr(p.status, GD_STATUS_EVENT_OVERFLOW);
 }
 
 #endif
