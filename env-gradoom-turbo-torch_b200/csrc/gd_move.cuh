@@ -404,14 +404,11 @@ struct GdMoveParams {
 
 #define GDM_BLOCK 128      /* four lanes per block */
 
-__global__ void __launch_bounds__(GDM_BLOCK) gd_player_tics_kernel(const GdMoveParams q) {
-  const int l = (int)(((size_t)blockIdx.x * GDM_BLOCK + threadIdx.x) >> 5);
-  if (l >= q.n) return;                                        /* whole warps leave */
-  int32_t p[GD_PLAYER_WORDS];
+/* All tics of lane l by one warp; every thread ends with the new record in `p`. */
+__device__ __forceinline__ void gd_player_advance(const GdMoveParams &q, int l, uint32_t buttons, int32_t (&p)[GD_PLAYER_WORDS]) {
 #pragma unroll
   for (int k = 0; k < GD_PLAYER_WORDS; ++k) p[k] = q.players[(size_t)l * GD_PLAYER_WORDS + k];
   GdmSolids so = {q.hasActors ? &q.actors : nullptr, l};
-  const uint32_t buttons = q.buttons[l];
   for (int t = 0; t < q.tics; ++t) gdm_player_tic(&q.map, &so, p, buttons, q.episodeTimeout);
   if (GDM_T != 0) return;                                      /* every thread holds the same record */
 #pragma unroll
@@ -432,6 +429,24 @@ __global__ void __launch_bounds__(GDM_BLOCK) gd_player_tics_kernel(const GdMoveP
     o[GD_L_EPISODE_TIME] = p[GD_P_EPISODE_TIME];
     o[GD_L_FLAGS] = (o[GD_L_FLAGS] & ~1) | ((p[GD_P_FLAGS] & GD_PLAYER_DEAD) ? 1 : 0);
   }
+}
+
+__global__ void __launch_bounds__(GDM_BLOCK) gd_player_tics_kernel(const GdMoveParams q) {
+  const int l = (int)(((size_t)blockIdx.x * GDM_BLOCK + threadIdx.x) >> 5);
+  if (l >= q.n) return;                                        /* whole warps leave */
+  int32_t p[GD_PLAYER_WORDS];
+  gd_player_advance(q, l, q.buttons[l], p);
+}
+
+/* the scene's map, no actors */
+static void gd_move_params(const gd_renderer *r, GdMoveParams &q) {
+  const GdScene &sc = r->base.sc;
+  q.map.W = sc.W; q.map.S = sc.S; q.map.nStarts = r->header[GD_H_STARTS];
+  q.map.walls = sc.walls; q.map.wsec = sc.wsec; q.map.edgeOff = sc.edgeOff; q.map.edgeWalls = sc.edgeWalls;
+  q.map.fineSine = sc.fineSine; q.map.secF = sc.secF;
+  q.map.starts = (const float *)gd_section((const uint8_t *)r->blobDev, r->header, GD_S_STARTS);
+  q.hasActors = 0;
+  memset(&q.actors, 0, sizeof q.actors);
 }
 
 #undef FU
@@ -459,13 +474,9 @@ extern "C" int gd_player_tics(const gd_renderer *r, int32_t *players, const uint
   if (cudaGetDevice(&current) != cudaSuccess) return GD_ERR_CUDA;
   if (current != r->device) return GD_ERR_DEVICE;
   GdMoveParams q;
-  const GdScene &sc = r->base.sc;
-  q.map.W = sc.W; q.map.S = sc.S; q.map.nStarts = r->header[GD_H_STARTS];
-  q.map.walls = sc.walls; q.map.wsec = sc.wsec; q.map.edgeOff = sc.edgeOff; q.map.edgeWalls = sc.edgeWalls;
-  q.map.fineSine = sc.fineSine; q.map.secF = sc.secF;
-  q.map.starts = (const float *)gd_section((const uint8_t *)r->blobDev, r->header, GD_S_STARTS);
+  gd_move_params(r, q);
   q.hasActors = actors && actors->enemy_slots > 0;
-  if (q.hasActors) q.actors = *actors; else memset(&q.actors, 0, sizeof q.actors);
+  if (q.hasActors) q.actors = *actors;
   q.players = players; q.buttons = buttons; q.n = n; q.tics = tics; q.episodeTimeout = episode_timeout; q.lanes = lanes;
   const int lanesPerBlock = GDM_BLOCK / 32;
   gd_player_tics_kernel<<<(n + lanesPerBlock - 1) / lanesPerBlock, GDM_BLOCK, 0, (cudaStream_t)stream>>>(q);

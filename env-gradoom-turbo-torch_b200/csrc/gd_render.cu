@@ -525,3 +525,4 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
 #include "gd_state.cuh"
 #include "gd_state_abi.cuh"
 #include "gd_move.cuh"
+#include "gd_stepper.cuh"

@@ -427,10 +427,15 @@ class GraDoomVecEnv:
         if availability is None:
             availability = torch.ones(self.num_envs, dtype=torch.bool, device=self.device)
         signals = self._producer.signal_buffer
+        # one conversion and one copy for all names: every entry is a row of its own
+        width = len(DEVICE_SIGNAL_NAMES)
+        values = torch.empty((width, self.num_envs), dtype=torch.float64, device=self.device)
+        values.copy_(signals[:, :width].t())
+        present = availability.expand(width, -1).contiguous()
         result = {}
-        for index, name in enumerate(DEVICE_SIGNAL_NAMES):
-            result[name] = signals[:, index].to(torch.float64)
-            result[f"_{name}"] = availability.clone()
+        for name, value, mask in zip(DEVICE_SIGNAL_NAMES, values.unbind(0), present.unbind(0)):
+            result[name] = value
+            result[f"_{name}"] = mask
         return result
 
     def seed(self, seed=None):
@@ -446,7 +451,8 @@ class GraDoomVecEnv:
         else:
             mask = require_device_tensor(raw_mask, "options['reset_mask']", device=self.device,
                                          shape=(self.num_envs,), dtypes=(torch.bool,))
-        if not bool(torch.any(mask)):
+        lanes = torch.nonzero(mask).flatten().tolist()
+        if not lanes:
             raise ValueError("options['reset_mask'] must select at least one lane")
         state_indices = reset_options.pop("state_indices", None)
         if state_indices is not None:
@@ -458,7 +464,7 @@ class GraDoomVecEnv:
             raise ValueError(f"unsupported reset options: {sorted(reset_options)}")
         seed_values = _normalize_seed(seed, self.num_envs) if seed is not None else self._seed_values
         game_seeds = [0] * self.num_envs
-        for lane in torch.nonzero(mask, as_tuple=False).flatten().to("cpu").tolist():
+        for lane in lanes:
             if seed_values[lane] is not None:
                 self._reset_rngs[lane] = np.random.default_rng(seed_values[lane])
             game_seeds[lane] = int(self._reset_rngs[lane].integers(0, np.iinfo(np.uint32).max + 1, dtype=np.uint32))
@@ -473,15 +479,25 @@ class GraDoomVecEnv:
         """Validated step (host synchronising, like the reference's gym ``step``)."""
 
         self._require_open("step")
-        if not bool(torch.all(self._initialized)):
-            raise RuntimeError("all lanes must be reset before the first step")
         pending = self._producer.pending_reset
-        if bool(torch.any(pending)):
+        lanes = torch.stack((self._initialized, pending == 0)).all(dim=1)
+        try:
+            indices = require_device_tensor(actions, "actions", device=self.device, shape=(self.num_envs,),
+                                            dtypes=_ACTION_DTYPES).to(torch.int64)
+            low, high = indices.aminmax()
+            initialized, running, low, high = torch.stack((*lanes.unbind(), low, high)).tolist()
+            refusal = None
+        except (TypeError, ValueError) as error:        # the lanes' own refusals come first
+            initialized, running = lanes.tolist()
+            refusal = error
+        if not initialized:
+            raise RuntimeError("all lanes must be reset before the first step")
+        if not running:
             lanes = torch.nonzero(pending).flatten().to("cpu").tolist()
             raise RuntimeError(f"terminal lanes must be reset before step: {lanes}")
-        indices = require_device_tensor(actions, "actions", device=self.device, shape=(self.num_envs,),
-                                        dtypes=_ACTION_DTYPES).to(torch.int64)
-        if bool(torch.any((indices < 0) | (indices >= len(self.action_table)))):
+        if refusal is not None:
+            raise refusal
+        if low < 0 or high >= len(self.action_table):
             raise ValueError("actions fall outside the declared action space")
         t = self.step_device(indices)
         rewards = t.rewards if self._reward_clip is None else t.rewards.clamp(*self._reward_clip)

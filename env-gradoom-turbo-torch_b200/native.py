@@ -28,7 +28,7 @@ EXPORTS = (
     "gd_error_string", "gd_renderer_create", "gd_renderer_destroy", "gd_renderer_scratch_bytes",
     "gd_renderer_ctas", "gd_renderer_shared_bytes", "gd_renderer_shared_bytes_view", "gd_render_step", "gd_render_reset", "gd_render_frames",
     "gd_render_step_frames", "gd_render_step_host", "gd_render_step_ring", "gd_render_reset_ring", "gd_static_scratch_bytes", "gd_static_max_walls", "gd_render_step_static",
-    "gd_pack_state_scratch_bytes", "gd_pack_state", "gd_player_tics", "gd_renderer_bind_decals", "gd_probe_libm",
+    "gd_pack_state_scratch_bytes", "gd_pack_state", "gd_player_tics", "gd_stepper_step", "gd_stepper_reset", "gd_renderer_bind_decals", "gd_probe_libm",
 )
 
 _libs = {}
@@ -89,6 +89,10 @@ def load(checked: bool = False) -> ctypes.CDLL:
         lib.gd_pack_state.argtypes = [vp, vp, vp, vp, vp, sz, vp, vp]
         lib.gd_player_tics.restype = ci
         lib.gd_player_tics.argtypes = [vp, vp, vp, vp, ci, ci, ci, vp, vp, vp]
+        lib.gd_stepper_step.restype = ci
+        lib.gd_stepper_step.argtypes = [vp, vp, ci, vp, ci, ci, ci, ctypes.c_longlong, vp, vp, vp, vp]
+        lib.gd_stepper_reset.restype = ci
+        lib.gd_stepper_reset.argtypes = [vp, vp, ci, vp, vp, ctypes.c_double, vp]
         lib.gd_renderer_bind_decals.restype = ci
         lib.gd_renderer_bind_decals.argtypes = [vp, vp, ci]
         lib.gd_probe_libm.restype = ci
@@ -122,6 +126,14 @@ def probe_libm(function: int, a: torch.Tensor, b: torch.Tensor | None = None) ->
         _check(load().gd_probe_libm(int(function), a.data_ptr(), _ptr(b), out.data_ptr(), a.numel(),
                                     torch.cuda.current_stream(a.device).cuda_stream), "gd_probe_libm")
     return out
+
+
+class StepperState(ctypes.Structure):
+    """``gd_stepper_state``: the device buffers of a lane stepper."""
+
+    _fields_ = [(name, ctypes.c_void_p) for name in ("lanes", "players", "things", "signals", "pending", "floors",
+                                                     "ceilings")] \
+        + [(name, ctypes.c_int32) for name in ("max_things", "k", "cols", "rows")]
 
 
 class Renderer:
@@ -245,6 +257,24 @@ class Renderer:
                    "gd_player_tics")
         self.launches += 1
 
+    def stepper_step(self, state, n, buttons, tics, episode_timeout, tick, rewards, terminated, truncated):
+        """One step of the built-in lane stepper (``stepper.LaneStepper``; ``state``: its ``StepperState``)."""
+
+        with torch.cuda.device(self.device):
+            _check(self.lib.gd_stepper_step(self.handle, ctypes.byref(state), n, buttons.data_ptr(), buttons.shape[1],
+                                            int(tics), int(episode_timeout), tick, rewards.data_ptr(),
+                                            terminated.data_ptr(), truncated.data_ptr(), self._stream()),
+                   "gd_stepper_step")
+        self.launches += 1
+
+    def stepper_reset(self, state, n, mask, seeds, room):
+        """Seeded placement of the lanes of ``mask`` by the built-in lane stepper."""
+
+        with torch.cuda.device(self.device):
+            _check(self.lib.gd_stepper_reset(self.handle, ctypes.byref(state), n, mask.data_ptr(), seeds.data_ptr(),
+                                             float(room), self._stream()), "gd_stepper_reset")
+        self.launches += 1
+
     def step(self, lanes, things, stack, mask_hud=True):
         n = self._inputs(lanes, things)
         self._check_stack(stack, n)
@@ -291,11 +321,9 @@ class Renderer:
         self._check_stack(stack, n)
         if reset_mask.dtype not in (torch.bool, torch.uint8) or tuple(reset_mask.shape) != (n,):
             raise TypeError("reset_mask must be a bool (N,) tensor")
-        mask = reset_mask.contiguous().view(torch.uint8) if reset_mask.dtype == torch.bool else reset_mask
-        mask16 = torch.zeros(((n + 15) // 16) * 16, dtype=torch.uint8, device=self.device)
-        mask16[:n] = mask
+        mask = reset_mask.to(self.device).contiguous()
         _check(self.lib.gd_render_reset(self.handle, lanes.data_ptr(), things.data_ptr(), n, int(mask_hud),
-                                        mask16.data_ptr(), stack.data_ptr(), self.scratch.data_ptr(),
+                                        mask.data_ptr(), stack.data_ptr(), self.scratch.data_ptr(),
                                         self.scratch_bytes, self.status.data_ptr(), self._stream()),
                "gd_render_reset")
         self.launches += 1

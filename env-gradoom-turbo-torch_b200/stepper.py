@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import numpy as np
 
+from . import native
 from . import scene as gdscene
 from . import state as gdstate
 
@@ -237,6 +238,28 @@ class LaneStepper:
         fresh[:, gdstate.P_EPISODE_TIME] = lanes[:, gdstate.L_EPISODE_TIME]
         players.copy_(torch.where(mask[:, None], fresh, players))
 
+    def _native_state(self):
+        """The stepper's buffers as the library takes them; None without a renderer on their device or when a
+        buffer was replaced by one of another layout."""
+
+        renderer, n = self.renderer, self.num_envs
+        if renderer is None or renderer.device != self.lanes.device:
+            return None
+        torch, spec, sectors = self.torch, self.spec, self.floors.shape[0]
+        for t, dtype, shape in ((self.lanes, torch.int32, (n, gdstate.LANE_WORDS)),
+                                (self.players, torch.int32, (n, gdstate.PLAYER_WORDS)),
+                                (self.things, torch.int32, (n, max(self.max_things, 1), 4)),
+                                (self.signal_buffer, torch.float32, (n, self.SIGNALS)),
+                                (self.pending_reset, torch.bool, (n,)), (self.floors, torch.float32, (sectors,)),
+                                (self.ceilings, torch.float32, (sectors,))):
+            if t.dtype != dtype or t.shape != shape or t.device != renderer.device or not t.is_contiguous():
+                return None
+        if sectors < spec.cols * spec.rows:
+            return None
+        return native.StepperState(self.lanes.data_ptr(), self.players.data_ptr(), self.things.data_ptr(),
+                                   self.signal_buffer.data_ptr(), self.pending_reset.data_ptr(), self.floors.data_ptr(),
+                                   self.ceilings.data_ptr(), self.things.shape[1], self.k, spec.cols, spec.rows)
+
     # deterministic per-lane pseudo random numbers in [0, 1)
     def _uniform(self, seeds, salt):
         torch = self.torch
@@ -273,6 +296,12 @@ class LaneStepper:
 
     def reset(self, mask, seeds):
         torch = self.torch
+        state = self._native_state()
+        if state is not None and mask.dtype == torch.bool and mask.device == seeds.device == self.lanes.device \
+                and mask.shape == seeds.shape == (self.num_envs,):
+            self.renderer.stepper_reset(state, self.num_envs, mask.contiguous(), seeds.to(torch.int64).contiguous(),
+                                        self.spec.room)
+            return
         width = self.spec.cols * self.spec.room
         height = self.spec.rows * self.spec.room
         room_fixed = int(self.spec.room * FIXED_UNIT)
@@ -314,6 +343,23 @@ class LaneStepper:
             raise RuntimeError("the lane stepper moves its players with the renderer's library: "
                                "bind_renderer() first (GraDoomVecEnv does it)")
         self._tick += 1
+        state = self._native_state()
+        if state is None or buttons.dtype != torch.bool or buttons.device != lanes.device or buttons.dim() != 2 \
+                or buttons.shape[0] != self.num_envs or buttons.shape[1] == 0:
+            return self._step_tensors(buttons)
+        rewards = torch.empty(self.num_envs, dtype=torch.float32, device=self.device)
+        terminated = torch.empty(self.num_envs, dtype=torch.bool, device=self.device)
+        truncated = torch.empty_like(terminated)
+        self.renderer.stepper_step(state, self.num_envs, buttons.contiguous(), self.frame_skip, self.episode_timeout,
+                                   self._tick, rewards, terminated, truncated)
+        return rewards, terminated, truncated
+
+    def _step_tensors(self, buttons):
+        """The step as tensor operations around the kinematics kernel: buttons that are not booleans, and
+        buffers that were replaced by ones of another layout."""
+
+        torch = self.torch
+        lanes = self.lanes
         b = buttons.to(torch.int64)
         if self.button_weights is None or self.button_weights.shape[0] != b.shape[1]:
             self.button_weights = 1 << torch.arange(b.shape[1], device=self.device, dtype=torch.int64)

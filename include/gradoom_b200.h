@@ -302,6 +302,31 @@ int gd_player_tics(const gd_renderer *r, int32_t *players, const uint32_t *butto
                    int n, int tics, int episode_timeout, int32_t *lanes, int *status, void *stream);
 
 /*
+ * The built-in lane stepper (players with the reference's kinematics; seeded placement, standing things, a
+ * kill now and then and episode timeouts of its own): one launch per step and one per reset.
+ * lanes, players, things: n x 32 / n x GD_PLAYER_WORDS / n x max_things x 4 words, things may be NULL when
+ * k is 0; signals: n x 27 f32; pending: n bytes; floors, ceilings: cols * rows f32, the map's rooms row by row.
+ */
+typedef struct gd_stepper_state {
+  int32_t *lanes, *players, *things;
+  float *signals;
+  uint8_t *pending;
+  const float *floors, *ceilings;
+  int32_t max_things, k;          /* thing records and things per lane */
+  int32_t cols, rows;
+} gd_stepper_state;
+
+/* `tics` game tics, the kill, the timeout and the signals.  buttons: n x columns bytes, nonzero where
+ * button i of a lane is pressed (those past the first 32 move nothing).  Writes rewards (n f32), terminated and truncated (n bytes). */
+int gd_stepper_step(const gd_renderer *r, const gd_stepper_state *st, int n, const uint8_t *buttons, int columns, int tics,
+                    int episode_timeout, long long tick, float *rewards, uint8_t *terminated, uint8_t *truncated,
+                    void *stream);
+
+/* Places the lanes whose mask byte is set by their seeds in square rooms of `room` units. */
+int gd_stepper_reset(const gd_renderer *r, const gd_stepper_state *st, int n, const uint8_t *mask, const long long *seeds,
+                     double room, void *stream);
+
+/*
  * No counterpart in the reference.  gd_render_step for callers that may not
  * allocate device memory -- a plugin inside a host process whose GPU memory
  * pool is owned and budgeted by the embedding application, or code running
