@@ -76,6 +76,44 @@ __global__ void gd_side_setup_kernel(GdScene sc, GdSide *sides, int *fragLine) {
   sides[i] = o;
 }
 
+/* The cells of the map: one block, whose threads first agree on the area that the sectors' boxes cover, then fill a
+ * cell each.  A cell lists a sector when the box outside of which gd_point_in_sector says no, grown by a unit for
+ * rounding, reaches it; a sector whose edges are not closed may also contain points left of its box. */
+__global__ void __launch_bounds__(GD_CELLS * GD_CELLS) gd_cells_kernel(GdScene sc, GdCells *cells) {
+  __shared__ float low[2][32], high[2][32];
+  const int t = threadIdx.x;
+  float x0 = CUDART_INF_F, x1 = -CUDART_INF_F, y0 = CUDART_INF_F, y1 = -CUDART_INF_F;
+  for (int s = t; s < sc.S; s += GD_CELLS * GD_CELLS) {
+    const float4 bb = *reinterpret_cast<const float4 *>(&sc.secBBox[s * 4]);
+    x0 = fminf(x0, bb.x); x1 = fmaxf(x1, bb.y); y0 = fminf(y0, bb.z); y1 = fmaxf(y1, bb.w);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o)); x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+    y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o)); y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+  }
+  if ((t & 31) == 0) { low[0][t >> 5] = x0; high[0][t >> 5] = x1; low[1][t >> 5] = y0; high[1][t >> 5] = y1; }
+  __syncthreads();
+  for (int k = 0; k < GD_CELLS * GD_CELLS / 32; ++k) {
+    x0 = fminf(x0, low[0][k]); x1 = fmaxf(x1, high[0][k]); y0 = fminf(y0, low[1][k]); y1 = fmaxf(y1, high[1][k]);
+  }
+  /* coordinates that are not finite, or so large that a unit is lost in them: every list counts as too long */
+  const bool usable = fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(y0), fabsf(y1))) < 100000.0f;
+  const float perX = (float)GD_CELLS / fmaxf(x1 - x0, 1.0f), perY = (float)GD_CELLS / fmaxf(y1 - y0, 1.0f);
+  if (t == 0) { cells->x0 = usable ? x0 : 0.0f; cells->y0 = usable ? y0 : 0.0f; cells->perX = usable ? perX : 0.0f; cells->perY = usable ? perY : 0.0f; }
+  const int cx = t % GD_CELLS, cy = t / GD_CELLS;
+  int n = usable ? 0 : 255;
+  for (int s = 0; s < sc.S && n <= GD_CELL_SECTORS; ++s) {
+    const float4 bb = *reinterpret_cast<const float4 *>(&sc.secBBox[s * 4]);
+    const bool open = sc.secI[s * 4 + 3] == 0;
+    const int left = open ? 0 : gd_cell_axis(bb.x - 2.0f, x0, perX), right = gd_cell_axis(bb.y + 2.0f, x0, perX);
+    const int bottom = gd_cell_axis(bb.z - 1.0f, y0, perY), top = gd_cell_axis(bb.w + 1.0f, y0, perY);
+    if (cx < left || cx > right || cy < bottom || cy > top) continue;
+    if (n < GD_CELL_SECTORS) cells->cell[t][1 + n] = (unsigned short)s;
+    ++n;
+  }
+  cells->cell[t][0] = (unsigned short)(n <= GD_CELL_SECTORS ? n : 255);
+}
+
 static const void *gd_section(const uint8_t *dev, const int32_t *h, int s) { return dev + h[GD_HDR_SECTION0 + s]; }
 
 extern "C" const char *gd_error_string(int code) {
@@ -247,8 +285,10 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
   if (rc == GD_OK) {
     void *sides = nullptr, *mem = nullptr, *rows = nullptr;
     const size_t sideBytes = (size_t)sc.W * 2 * sizeof(GdSide);
-    if (cudaMalloc(&sides, sideBytes + (size_t)sc.F * 4) != cudaSuccess) rc = GD_ERR_CUDA;
+    const size_t lineBytes = gd_align16((size_t)sc.F * 4);
+    if (cudaMalloc(&sides, sideBytes + lineBytes + sizeof(GdCells)) != cudaSuccess) rc = GD_ERR_CUDA;
     r->sides = (GdSide *)sides;
+    sc.cells = (GdCells *)((uint8_t *)sides + sideBytes + lineBytes);
     r->fragLine = (int *)((uint8_t *)sides + sideBytes);
     if (rc == GD_OK && sc.F > 0) {
       if (cudaMalloc(&mem, (size_t)r->ctas * sc.F * sizeof(GdWall)) != cudaSuccess) rc = GD_ERR_CUDA;
@@ -258,6 +298,7 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
     }
     if (rc == GD_OK) {
       gd_side_setup_kernel<<<(sc.W * 2 + 127) / 128, 128>>>(sc, r->sides, r->fragLine);
+      gd_cells_kernel<<<1, GD_CELLS * GD_CELLS>>>(sc, (GdCells *)sc.cells);
       if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) rc = GD_ERR_CUDA;
     }
   }

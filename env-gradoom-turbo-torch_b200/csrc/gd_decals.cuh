@@ -45,6 +45,7 @@ __device__ __noinline__ void gd_decals(const GdScene &sc_, const GdView &v_, con
   __syncthreads();
   const float width = (float)sc.decalW;
   /* ---- project the chips in use (engine.py:13797-13883) ---- */
+#pragma unroll 1
   for (int s = tid; s < slots; s += GD_THREADS) {
     const int4 raw = *reinterpret_cast<const int4 *>(&ring[s]);
     const int serial = raw.x;
@@ -106,9 +107,11 @@ __device__ __noinline__ void gd_decals(const GdScene &sc_, const GdView &v_, con
   short *ranked = (short *)sh.hitD;                  /* GD_MAX_DECAL_SLOTS x 2 bytes */
   unsigned *spans = (unsigned *)sh.hitA;             /* GD_MAX_DECAL_SLOTS x 4 bytes: first column | end column << 16 */
   static_assert(GD_MAX_DECAL_SLOTS * 4 <= 8 * GD_SW * 4, "the chip list fits the hit cache");
+#pragma unroll 1
   for (int i = tid; i < n; i += GD_THREADS) {
     const int si = proj[i].serial, li = proj[i].slotStyle & 1023;
     int rank = 0;
+#pragma unroll 1
     for (int j = 0; j < n; ++j) {
       const int sj = proj[j].serial;
       rank += (sj < si) || (sj == si && (proj[j].slotStyle & 1023) < li);

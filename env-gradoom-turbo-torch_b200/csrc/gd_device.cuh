@@ -34,6 +34,15 @@ typedef long long i64;
 #define GD_STATUS_BAD_INDEX 8        /* checked build: a wall, texture, sprite or patch index outside its table */
 #define GD_STATUS_BAD_STATE 16       /* checked build: a lane or thing record with a value outside its range */
 
+/* A map's area in GD_CELLS x GD_CELLS cells; a cell lists, in ascending order, every sector that may contain a point
+ * of it (points outside belong to the nearest cell).  One 16-byte load fetches a cell. */
+#define GD_CELLS 32
+#define GD_CELL_SECTORS 7
+struct __align__(16) GdCells {
+  float x0, y0, perX, perY;       /* cell of a coordinate: (c - x0) * perX */
+  unsigned short cell[GD_CELLS * GD_CELLS][1 + GD_CELL_SECTORS];   /* count (255: more than the list holds), sectors */
+};
+
 struct GdScene {
   int W, S, T, texH, texW, P, sprH, sprW, Q, wpnH, wpnW, wpnTics, nStarts, B, nbDirect, wpnAvailable, hudPatches;
   const float *walls;
@@ -70,6 +79,7 @@ struct GdScene {
   /* projection fragments of the lines a node builder split: total count, CSR per line, 16.16 endpoints */
   int F;
   const int32_t *fragOff, *fragFixed;
+  const GdCells *cells;         /* the sectors that may hold a point, by where it lies (built with the renderer) */
   /* bullet-chip decals: variants (0 = none), atlas slice height / width */
   int decals, decalH, decalW;
   const int32_t *decalInfo, *wallFine;

@@ -25,6 +25,36 @@ __device__ __forceinline__ bool gd_point_in_sector(const GdScene &sc, int s, flo
   return crossings & 1;
 }
 
+/* The cell of a point; any cell will do for a point that is not a number, no sector contains it. */
+__device__ __forceinline__ int gd_cell_axis(float c, float c0, float per) { return min(max((int)((c - c0) * per), 0), GD_CELLS - 1); }
+__device__ __forceinline__ int gd_cell(const GdCells &g, float px, float py) {
+  return gd_cell_axis(py, g.y0, g.perY) * GD_CELLS + gd_cell_axis(px, g.x0, g.perX);
+}
+
+/* The lowest-numbered sector of height group g (f: floors, else ceilings) below `end` that contains the point,
+ * or -1.  A point's cell names the one to four sectors that can; testing all of a group's took most of the
+ * time of views with many such pixels (a lane of the 256-sector map: 11 million cycles at worst, now 4). */
+__device__ __noinline__ int gd_group_sector(const GdScene &sc_, int f, int g, float px, float py, int end) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  const GdCells &cells = *sc.cells;
+  uint4 list = *reinterpret_cast<const uint4 *>(cells.cell[gd_cell(cells, px, py)]);
+  const int count = (int)(list.x & 0xFFFFu);
+  const bool listed = count <= GD_CELL_SECTORS;
+  const float height = sc.groupH[f][g];
+  int k = listed ? 0 : sc.groupOff[f][g];
+  const int k1 = listed ? count : sc.groupOff[f][g + 1];
+#pragma unroll 1
+  for (; k < k1; ++k) {
+    list.x = __funnelshift_r(list.x, list.y, 16); list.y = __funnelshift_r(list.y, list.z, 16);
+    list.z = __funnelshift_r(list.z, list.w, 16); list.w >>= 16;
+    const int s = listed ? (int)(list.x & 0xFFFFu) : sc.groupSec[f][k];
+    if (s >= end) break;
+    if (listed && sc.secF[s * 2 + (f ? 0 : 1)] != height) continue;
+    if (gd_point_in_sector(sc, s, px, py)) return s;
+  }
+  return -1;
+}
+
 /* Flat-fallback resolution of a pixel (engine.py:10961-11026): true when the
  * column ray meets no sector's plane inside that sector's polygon. */
 __device__ __noinline__ bool gd_pixel_unresolved(const GdScene &sc_, const GdView &v_, int x, int y, float rc, float rs,
@@ -48,7 +78,6 @@ __device__ __noinline__ bool gd_pixel_unresolved(const GdScene &sc_, const GdVie
   }
   const int f = floorPixel ? 1 : 0;
   const float *gh = sc.groupH[f];
-  const int32_t *goff = sc.groupOff[f], *gsec = sc.groupSec[f];
 #pragma unroll 1
   for (int g = 0; g < sc.groups[f]; ++g) {
     float ph = floorPixel ? (v.viewZ - gh[g]) : (gh[g] - v.viewZ);
@@ -56,9 +85,7 @@ __device__ __noinline__ bool gd_pixel_unresolved(const GdScene &sc_, const GdVie
     float cd = perp / cc;
     if (!(ph > 0) || !isfinite(cd) || !(cd > 0)) continue;
     float px = v.x + rc * cd, py = v.y + rs * cd;
-#pragma unroll 1
-    for (int k = goff[g]; k < goff[g + 1]; ++k)
-      if (gd_point_in_sector(sc, gsec[k], px, py)) return false;
+    if (gd_group_sector(sc, f, g, px, py, 0x7fffffff) >= 0) return false;
   }
   return true;
 }
@@ -114,6 +141,7 @@ __device__ void gd_flat_bounds_setup(const GdScene &sc, const GdView &v, int *mi
   const int lane = threadIdx.x & 31;
   float phF = GD_INF, phC = GD_INF, xHi = -GD_INF, xLo = GD_INF, yHi = -GD_INF, yLo = GD_INF;
   int closed = 1;
+#pragma unroll 1
   for (int s = lane; s < sc.S; s += 32) {
     float f = v.viewZ - sc.secF[s * 2], c = sc.secF[s * 2 + 1] - v.viewZ;
     if (f > 0) phF = fminf(phF, f);
@@ -125,7 +153,7 @@ __device__ void gd_flat_bounds_setup(const GdScene &sc, const GdView &v, int *mi
     yLo = fminf(yLo, bb.z);
     closed &= sc.secI[s * 4 + 3] != 0;
   }
-#pragma unroll
+#pragma unroll 1
   for (int o = 16; o > 0; o >>= 1) {
     phF = fminf(phF, __shfl_xor_sync(0xffffffffu, phF, o));
     phC = fminf(phC, __shfl_xor_sync(0xffffffffu, phC, o));
@@ -191,7 +219,6 @@ __device__ __noinline__ GdFlatProbe gd_flat_probe(const GdScene &sc_, const GdVi
   float best = GD_INF;
   const int f = out.isFloor ? 1 : 0;
   const float *gh = sc.groupH[f];
-  const int32_t *goff = sc.groupOff[f], *gsec = sc.groupSec[f];
 #pragma unroll 1
   for (int g = 0; g < sc.groups[f]; ++g) {
     float ph = out.isFloor ? (v.viewZ - gh[g]) : (gh[g] - v.viewZ);
@@ -200,12 +227,8 @@ __device__ __noinline__ GdFlatProbe gd_flat_probe(const GdScene &sc_, const GdVi
     if (!(ph > 0) || !isfinite(cd) || !(cd > 0)) continue;
     if (cd > best) break;
     float px = v.x + r.rc * cd, py = v.y + r.rs * cd;
-#pragma unroll 1
-    for (int k = goff[g]; k < goff[g + 1]; ++k) {
-      int s = gsec[k];
-      if (cd == best && s > out.sector) break;
-      if (gd_point_in_sector(sc, s, px, py)) { best = cd; out.sector = s; break; }
-    }
+    const int s = gd_group_sector(sc, f, g, px, py, cd == best ? out.sector + 1 : 0x7fffffff);
+    if (s >= 0) { best = cd; out.sector = s; }
   }
   out.unresolved = !isfinite(best);
   return out;
@@ -236,6 +259,7 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
   if (warp == 0) gd_flat_bounds_setup(sc, v, sh.misc);
   __syncthreads();
   const GdFlatBounds b = gd_flat_bounds_load(sh.misc);
+#pragma unroll 1
   for (int i = tid; i < count; i += GD_THREADS) {
     const int px = queue[i] & 0xFFFF, py = queue[i] >> 16;
     const GdFlatRay r = gd_flat_ray(sc, v, px);
@@ -256,6 +280,7 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
     {
       const unsigned *filled = sh.masks + tid, *own = owned + tid;
       int lo = GD_VH, hi = -1;
+#pragma unroll 1
       for (int k = 0; k < 7; ++k) {
         unsigned m = gd_range_word(k, 0, GD_VH) & ~filled[k * GD_SW] & ~own[k * GD_SW];
         if (m) { lo = min(lo, (k << 5) + __ffs(m) - 1); hi = max(hi, (k << 5) + 31 - __clz(m)); }
@@ -298,6 +323,7 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
     __threadfence_block();
     __syncthreads();
   }
+#pragma unroll 1
   for (int i = tid; i < count; i += GD_THREADS) {
     if (queue[i] < 0) continue;
     const int px = queue[i] & 0xFFFF, py = queue[i] >> 16;

@@ -96,8 +96,13 @@ __device__ __noinline__ void gd_project_fixed(const GdView &v, const i64 fx[2], 
   i64 sl, sr, dl, dr;
   gd_fwall_coords(tx[a], ty[a], tx[b], ty[b], sl, sr, dl, dr);
   out.sl = sl; out.sr = sr; out.dl = dl; out.dr = dr;
-  gd_wall_visibility(tx[0], ty[0], tx[1], ty[1], out.visL[0], out.visStep[0], out.visSl[0]);
-  gd_wall_visibility(tx[1], ty[1], tx[0], ty[0], out.visL[1], out.visStep[1], out.visSl[1]);
+  i64 ax = tx[0], ay = ty[0], bx = tx[1], by = ty[1];
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    gd_wall_visibility(ax, ay, bx, by, out.visL[side], out.visStep[side], out.visSl[side]);
+    const i64 x = ax, y = ay;
+    ax = bx; ay = by; bx = x; by = y;
+  }
 }
 
 /* Project wall w of the map for this lane (engine.py:10747-10869, 11207-11302,
@@ -574,6 +579,36 @@ __device__ __forceinline__ bool gd_wall_in_frustum(const float4 wl, const GdView
   return true;
 }
 
+/* First and last column whose ray crosses a wall, as a span word, found at the projections of its ends.
+ * A ray's cross product with an endpoint is linear in the column, with a slope of its depth / 160.  With both ends
+ * at least 8 units deep and no coordinate above 16384 the rounding of the test moves a crossing's edge by less than
+ * half a column, and that of the projections below by less than a tenth: every column more than one inside the
+ * projected ends gives the same answer, and every one more than one outside is not crossed.  So the four columns
+ * around either end decide.  A wall that does not qualify gets GD_SPAN_SWEEP: all columns are tried. */
+#define GD_SPAN_SWEEP 0xFFFEFFFEu
+__device__ __forceinline__ unsigned gd_crossed_columns(const GdView &v, const GdHot &h) {
+  const float bx = h.offx + h.segx, by = h.offy + h.segy;
+  const float size = fmaxf(fmaxf(fabsf(h.offx), fabsf(h.offy)), fmaxf(fabsf(bx), fabsf(by)));
+  const float da = h.offx * v.fcos + h.offy * v.fsin, db = bx * v.fcos + by * v.fsin;
+  if (!(size <= 16384.0f && fminf(da, db) >= 8.0f)) return GD_SPAN_SWEEP;
+  const float ca = 160.0f + 160.0f * ((h.offx * v.fsin - h.offy * v.fcos) / da);
+  const float cb = 160.0f + 160.0f * ((bx * v.fsin - by * v.fcos) / db);
+  const float low = floorf(fminf(ca, cb)) - 1.0f, high = ceilf(fmaxf(ca, cb)) + 1.0f;
+  if (high < 0.0f || low > (float)(GD_SW - 1)) return 0xFFFFu;
+  const int lo = (int)fmaxf(low, 0.0f), hi = (int)fminf(high, (float)(GD_SW - 1));
+  int first = -1, last = -1;
+#pragma unroll 1
+  for (int k = 0; k < 8; ++k) {
+    const int x = min(max(k < 4 ? lo + k : hi - 7 + k, lo), hi);
+    float rx, ry;
+    gd_ray(v, x, rx, ry);
+    if (!gd_ray_geo(h, rx, ry)) continue;
+    if (first < 0) first = x;
+    last = max(last, x);
+  }
+  return ((unsigned)first & 0xFFFFu) | ((unsigned)(last + 1) << 16);
+}
+
 /* Lists the walls that a column ray may cross, and with them wall 0 and the first blocking wall, which the
  * rules fall back to; projects them; finds their ray-owned spans.  Every other wall gets the record no ray
  * meets.  The list stays in aux until the walk begins. */
@@ -588,6 +623,7 @@ __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShar
   if (threadIdx.x == 0) *listed = 0;
   __syncthreads();
   const int block0 = GD_CHECK_INDEX(sc.blocking[0], sc.W);
+#pragma unroll 1
   for (int w = threadIdx.x; w < sc.W; w += GD_THREADS) {
     const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
     if (gd_wall_in_frustum(wl, v) || w == 0 || w == block0) {
@@ -599,22 +635,24 @@ __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShar
   }
   __syncthreads();
   const int n = *listed;
+#pragma unroll 1
   for (int i = threadIdx.x; i < n; i += GD_THREADS) {
     const int w = list[i];
     gd_project_wall(sc, v, w, walls[w], gd_hot(w));
+    gd_hot(w).span = gd_crossed_columns(v, gd_hot(w));
   }
   __syncthreads();
-  float rxs[GD_SW / 32], rys[GD_SW / 32];
-#pragma unroll
-  for (int chunk = 0; chunk < GD_SW / 32; ++chunk) gd_ray(v, chunk * 32 + lane, rxs[chunk], rys[chunk]);
-  /* first and last column whose ray crosses the wall */
+#pragma unroll 1
   for (int i = warp; i < n; i += GD_WARPS) {
     const int w = list[i];
+    if (gd_hot(w).span != GD_SPAN_SWEEP) continue;
     const GdHot h = gd_hot(w);
     int first = -1, last = -1;
-#pragma unroll
+#pragma unroll 1
     for (int chunk = 0; chunk < GD_SW / 32; ++chunk) {
-      unsigned m = __ballot_sync(0xffffffffu, gd_ray_geo(h, rxs[chunk], rys[chunk]));
+      float rx, ry;
+      gd_ray(v, chunk * 32 + lane, rx, ry);
+      const unsigned m = __ballot_sync(0xffffffffu, gd_ray_geo(h, rx, ry));
       if (m) {
         if (first < 0) first = chunk * 32 + __ffs(m) - 1;
         last = chunk * 32 + 31 - __clz(m);
@@ -623,6 +661,7 @@ __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShar
     if (lane == 0) gd_hot(w).span = ((unsigned)first & 0xFFFFu) | ((unsigned)(last + 1) << 16);
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = threadIdx.x; i < n; i += GD_THREADS) {
     const int w = list[i];
     const GdWall &wv = walls[w];

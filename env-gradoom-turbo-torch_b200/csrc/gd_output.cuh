@@ -5,45 +5,67 @@
 
 /* ---- phase: 320x240 -> 84x84 area resize + grayscale ---------------------
  * Integer definition: src/gradoom/_triton_kernels.py:120-177.  The weights
- * (y_overlap*x_overlap)/48 factor exactly into (y_overlap/12)*(x_overlap/4). */
-__device__ void gd_resize(const uint8_t *frame, const unsigned long long *pal64, int srcRows, uint8_t *out) {
-  pal64 = gd_as_shared(pal64); out = gd_as_shared(out);
-  for (int o = threadIdx.x; o < GD_OBS * GD_OBS; o += GD_THREADS) {
-    int oy = o / GD_OBS, ox = o - oy * GD_OBS;
-    int ys = oy * 240, ye = ys + 240, xs = ox * 320, xe = xs + 320;
-    /* An output pixel overlaps at most 4 source rows and 5 source columns; taps
-     * past the overlap get weight zero, so the tap loops have fixed trip counts
-     * and their loads are independent. */
-    const int sy0 = ys / 84, sx0 = xs / 84;
-    if (sy0 >= srcRows) { out[o] = 0; continue; }    /* only masked status-bar rows: black */
-    unsigned wx[5];
-    int cx[5];
-#pragma unroll
-    for (int j = 0; j < 5; ++j) {
-      int sx = sx0 + j;
-      int xo = min(xe, (sx + 1) * 84) - max(xs, sx * 84);
-      wx[j] = xo > 0 ? (unsigned)xo / 4u : 0u;
-      cx[j] = min(sx, GD_SW - 1);
+ * (y_overlap*x_overlap)/48 factor exactly into (y_overlap/12)*(x_overlap/4): twenty source rows of 7 units each
+ * become seven output rows of 20 units, and a source column of 21 units goes to output columns of 80.
+ *
+ * Thread x sums its column's twenty rows into seven output rows (every pixel looks its colour up once; the weights
+ * are constants of the unrolled rows), then the threads sum four or five columns each into the 7 x 84 pixels.
+ * What bounds it is instructions: twenty lookups and 64-bit products per output pixel, as a loop over the output,
+ * took 57 of a lane's 557 thousand cycles. */
+#define GD_RESIZE_ROWS 20
+#define GD_RESIZE_OUT 7
+static_assert(GD_SCREEN_H % GD_RESIZE_ROWS == 0 && GD_RESIZE_OUT * GD_SW * 8 <= 14 * GD_SW * 4, "the sums fit the column masks");
+
+__device__ __noinline__ void gd_resize(const uint8_t *frame, int srcRows, uint8_t *out_) {
+  uint8_t *out = gd_as_shared(out_);
+  const uint2 *pal = (const uint2 *)(gd_smem + GD_OFF_PAL64);
+  uint2 *sums = (uint2 *)(gd_smem + GD_OFF_MASKS);       /* [7][320]: R | B << 16, G; the masks are done with */
+  const int x = threadIdx.x;
+  const uint8_t *column = frame + x;
+#pragma unroll 1
+  for (int y0 = 0, o0 = 0; y0 < GD_SCREEN_H; y0 += GD_RESIZE_ROWS, o0 += GD_RESIZE_OUT * GD_OBS) {
+    if (y0 >= srcRows) {                                 /* masked status-bar rows: black */
+#pragma unroll 1
+      for (int i = x; i < GD_RESIZE_OUT * GD_OBS; i += GD_THREADS) out[o0 + i] = 0;
+      continue;
     }
-    unsigned long long acc = 0;
+    unsigned index[GD_RESIZE_ROWS];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int sy = sy0 + i;
-      int yo = min(ye, (sy + 1) * 84) - max(ys, sy * 84);
-      unsigned wy = (yo > 0 && sy < srcRows) ? (unsigned)yo / 12u : 0u;
-      const uint8_t *row = frame + min(sy, srcRows - 1) * GD_SW;      /* rows beyond srcRows weigh nothing */
-      unsigned long long racc = 0;
+    for (int r = 0; r < GD_RESIZE_ROWS; ++r) index[r] = y0 + r < srcRows ? column[(y0 + r) * GD_SW] : 256u;
+    unsigned rb[GD_RESIZE_OUT], g[GD_RESIZE_OUT];
 #pragma unroll
-      for (int j = 0; j < 5; ++j) racc += (unsigned long long)wx[j] * pal64[row[cx[j]]];
-      acc += racc * wy;
+    for (int o = 0; o < GD_RESIZE_OUT; ++o) rb[o] = g[o] = 0u;
+#pragma unroll
+    for (int r = 0; r < GD_RESIZE_ROWS; ++r) {
+      const uint2 c = index[r] < 256u ? pal[index[r]] : make_uint2(0u, 0u);
+      const int o = 7 * r / 20;
+      const unsigned first = 7 * r + 7 <= 20 * (o + 1) ? 7u : 20u * (o + 1) - 7u * r;
+      rb[o] += first * c.x; g[o] += first * c.y;
+      if (first < 7u) { rb[o + 1] += (7u - first) * c.x; g[o + 1] += (7u - first) * c.y; }
     }
-    unsigned r = (unsigned)(acc & 0xFFFFF), g = (unsigned)((acc >> 20) & 0xFFFFF), b = (unsigned)((acc >> 40) & 0xFFFFF);
-    r = (r + 800) / 1600; g = (g + 800) / 1600; b = (b + 800) / 1600;
-    out[o] = (uint8_t)((r * 77 + g * 150 + b * 29 + 128) >> 8);
+    __syncthreads();                                     /* the sums of the rows before have been read */
+#pragma unroll
+    for (int o = 0; o < GD_RESIZE_OUT; ++o) sums[o * GD_SW + x] = make_uint2(rb[o], g[o]);
+    __syncthreads();
+#pragma unroll 1
+    for (int i = x; i < GD_RESIZE_OUT * GD_OBS; i += GD_THREADS) {
+      const int o = i / GD_OBS, ox = i - o * GD_OBS, c0 = 80 * ox / 21;
+      const uint2 *row = sums + o * GD_SW;
+      const unsigned w0 = 21u * (c0 + 1) - 80u * ox;
+      const unsigned weight[5] = {w0, 21u, 21u, min(38u - w0, 21u), w0 < 17u ? 17u - w0 : 0u};
+      unsigned r = 0, gg = 0, b = 0;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        const uint2 c = row[min(c0 + k, GD_SW - 1)];     /* a column past the edge weighs nothing */
+        r += weight[k] * (c.x & 0xFFFFu); b += weight[k] * (c.x >> 16); gg += weight[k] * c.y;
+      }
+      r = (r + 800) / 1600; gg = (gg + 800) / 1600; b = (b + 800) / 1600;
+      out[o0 + i] = (uint8_t)((r * 77 + gg * 150 + b * 29 + 128) >> 8);
+    }
   }
 }
 
-/* PLAYPAL of the lane in shared memory, as packed 3 x 20-bit words for the
+/* PLAYPAL of the lane in shared memory, as R | B << 16 | G << 32 for the
  * resize and as RGB24 words: the scene's palette, or its bonus / damage blends when
  * the lane's flags ask for screen flashes (engine.py:15381-15398; float32,
  * separately rounded, truncating conversion). */
@@ -70,7 +92,7 @@ __device__ void gd_lane_palette(const GdScene &sc, const GdShared &sh, int flags
     }
     ch[c] = v;
   }
-  sh.pal64[i] = (unsigned long long)ch[0] | ((unsigned long long)ch[1] << 20) | ((unsigned long long)ch[2] << 40);
+  sh.pal64[i] = (unsigned long long)(ch[0] | (ch[2] << 16)) | ((unsigned long long)ch[1] << 32);
   sh.pal32[i] = ch[0] | (ch[1] << 8) | (ch[2] << 16);
 }
 

@@ -37,7 +37,6 @@
 #include "gd_device.cuh"
 
 #define GD_THREADS 320
-#define GD_HUD_MAX_PATCHES 48
 #define GD_WARPS (GD_THREADS / 32)
 #define GD_INF CUDART_INF_F
 
@@ -116,7 +115,7 @@ struct GdActor {
  * scratch, which stays in L2: its pixels are stored once each, a warp's 32 columns of a row in one sector,
  * and the 77 KB that leaves free on chip let two lanes share an SM. */
 #define GD_OFF_COLORMAP 0                                  /* 32 x 256 */
-#define GD_OFF_PAL64 (GD_OFF_COLORMAP + 32 * 256)          /* 256: R | G<<20 | B<<40 */
+#define GD_OFF_PAL64 (GD_OFF_COLORMAP + 32 * 256)          /* 256: R | B << 16 | G << 32 */
 #define GD_OFF_PAL32 (GD_OFF_PAL64 + 256 * 8)              /* 256: r | g << 8 | b << 16, for the RGB24 output */
 #define GD_OFF_YSLOPE (GD_OFF_PAL32 + 256 * 4)             /* 208 */
 #define GD_OFF_LANE (GD_OFF_YSLOPE + GD_VIEW_H * 4)        /* 32 */
@@ -131,9 +130,9 @@ struct GdActor {
 #define GD_OFF_MASKED_INFO (GD_OFF_MASKED_DIST + 320 * 4)  /* ... its wall << 16 | ceiling clip << 8 | floor clip; 0xFFFF0000 | .. = none */
 #define GD_OFF_CAND (GD_OFF_MASKED_INFO + 320 * 4)         /* 320 x 64 bits: things that may show in the column */
 #define GD_OFF_AUX (GD_OFF_CAND + 320 * 8)                 /* 10,240 bytes for one phase at a time: listed walls, fallback queue,
-                                                              chip ranks, status-bar list, 84 x 84 result */
+                                                              chip ranks, 84 x 84 result */
 #define GD_AUX_BYTES (8 * 320 * 4)
-#define GD_OFF_AUX2 (GD_OFF_AUX + GD_AUX_BYTES)            /* 4,096: sectors of points, sprite columns, chip spans */
+#define GD_OFF_AUX2 (GD_OFF_AUX + GD_AUX_BYTES)            /* 4,096: sectors of points, status-bar list, sprite columns, chip spans */
 #define GD_OFF_HOT (GD_OFF_AUX2 + 4096)                    /* W wall records */
 static_assert(GD_OFF_HOT % 16 == 0 && GD_OFF_AUX % 16 == 0, "vector loads");
 
@@ -313,6 +312,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       gd_view_setup(sc, sh.lane, sView);
     } else if (tid >= 32) {
       const int pairs = (nThings + 1) * sc.S;
+#pragma unroll 1
       for (int i = tid - 32; i < pairs; i += GD_THREADS - 32) {
         int t = i / sc.S, s = i - t * sc.S;
         float px, py;
@@ -338,14 +338,17 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       ((unsigned *)(gd_smem + GD_OFF_YSLOPE))[tid] = (unsigned)ys;
     }
     if (kSplit)
+#pragma unroll 1
       for (int f = tid; f < sc.F; f += GD_THREADS) {
         GdWall &q = sh.frags[f];
         gd_project_fragment(sc, v, f, q);
         const unsigned sl = (unsigned)gd_clamp(q.sl, 0, GD_SW), sr = (unsigned)gd_clamp(q.sr, 0, GD_SW);
         ((unsigned *)(gd_smem + p.offFrags))[f] = q.sr > q.sl ? sl | (sr << 16) : 0u;
       }
+#pragma unroll 1
     for (int idx = GD_THREADS - 1 - tid; idx < sc.S * 2; idx += GD_THREADS)   /* the threads the things leave idle */
       gd_plane_entry_setup(sc, v, idx >> 1, (idx & 1) != 0, sh.planeTab[idx], planes[idx]);
+#pragma unroll 1
     for (int a = tid; a < nThings; a += GD_THREADS) {
       int sector = pointSector[a] == 0x7fffffff ? 0 : pointSector[a];
       gd_actor_setup(sc, v, p.things[(size_t)l * p.maxThings + a], sector, sh.actors[a]);
@@ -358,6 +361,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     /* row projections, light and column operands of the listed walls (the walk selects no other wall) and of the
      * fragments in view */
     const int fragTasks = kSplit ? sc.F * 4 : 0;
+#pragma unroll 1
     for (int idx = tid; idx < frustumListed * 4 + fragTasks; idx += GD_THREADS) {
       const bool piece = kSplit && idx >= frustumListed * 4;
       const int f = piece ? (idx - frustumListed * 4) >> 2 : 0, slot = idx & 3;
@@ -378,6 +382,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       }
       (piece ? fragRows + f * 4 : rows + w * 4)[slot] = row;
     }
+#pragma unroll 1
     for (int i = tid; i < frustumListed; i += GD_THREADS) {   /* walls outside the frustum own no column */
       const int w = frustumList[i];
       prep[w] = gd_prep_setup(sh.walls[w]);
@@ -391,6 +396,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       }
     }
     gd_mark_afterlife_columns(sc, sh);
+    if (p.flags & GD_F_DRAW_HUD) gd_hud_list(sc, sh.lane, (int4 *)sh.hitA);   /* the sectors of points have been read */
     {
       float rx, ry, wd = 0.0f;
       int bw = 0;
@@ -402,6 +408,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     }
     __syncthreads();
     gd_walk<kSplit, kChip>(p, sc, v, sh, frame, tables, events, eventCount, rowproj, sh.misc[0]);
+    if (p.flags & GD_F_DRAW_HUD) gd_hud_column(sc, (const int4 *)sh.hitA, frame + GD_VH * GD_SW);
     __syncthreads();
     /* Rows no seg ever claimed show the per-pixel flat fallback.  They are
      * queued (the hit cache is free once every column has finished its walk)
@@ -410,8 +417,10 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     bool sweepDone = false;                          /* CTA-uniform */
     for (;;) {
       const unsigned *filled = sh.masks + tid, *owned = sh.masks + 7 * GD_SW + tid;
+#pragma unroll 1
       for (int k = 0; k < 7; ++k) {
         unsigned m = gd_range_word(k, 0, GD_VH) & ~filled[k * GD_SW] & ~owned[k * GD_SW];
+#pragma unroll 1
         while (m) {
           int y = (k << 5) + __ffs(m) - 1;
           m &= m - 1;
@@ -441,9 +450,8 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     gd_weapon(sc, sh.lane, sh.frame);
     __syncthreads();
     const bool wantFull = p.indexedOut != nullptr || p.rgbOut != nullptr;
-    if (p.flags & GD_F_DRAW_HUD) {
-      gd_hud(sc, sh, sh.lane, sh.frame + GD_VH * GD_SW);
-    } else if (wantFull) {
+    if (wantFull && !(p.flags & GD_F_DRAW_HUD)) {
+#pragma unroll 1
       for (int i = tid; i < GD_HUD_H * GD_SW / 4; i += GD_THREADS) ((unsigned *)(sh.frame + GD_VH * GD_SW))[i] = 0;
       __syncthreads();
     }
@@ -467,24 +475,27 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     }
     if (p.stack || p.obsOut) {
       int srcRows = (p.flags & GD_F_MASK_HUD) ? GD_VH : GD_SCREEN_H;
-      gd_resize(sh.frame, sh.pal64, srcRows, sh.obs);
+      gd_resize(sh.frame, srcRows, sh.obs);
       __syncthreads();
       const uint4 *src = (const uint4 *)sh.obs;
       const int vecs = GD_OBS * GD_OBS / 16;  /* 441 */
       if (p.obsOut) {
         uint4 *dst = (uint4 *)(p.obsOut + (size_t)l * GD_OBS * GD_OBS);
+#pragma unroll 1
         for (int i = tid; i < vecs; i += GD_THREADS) dst[i] = src[i];
       }
       if (p.stack && (p.flags & GD_F_STACK_RING)) {
         /* mirrored ring: no old slot is read or moved */
         uint4 *s0 = (uint4 *)(p.stack + (size_t)l * 2 * GD_STACK * GD_OBS * GD_OBS);
         if (p.flags & GD_F_STACK_FILL) {
+#pragma unroll 1
           for (int i = tid; i < vecs; i += GD_THREADS) {
             uint4 val = src[i];
 #pragma unroll
             for (int k = 0; k < 2 * GD_STACK; ++k) s0[k * vecs + i] = val;
           }
         } else {
+#pragma unroll 1
           for (int i = tid; i < vecs; i += GD_THREADS) {
             uint4 val = src[i];
             s0[p.ringHead * vecs + i] = val;
@@ -494,11 +505,13 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       } else if (p.stack) {
         uint4 *s0 = (uint4 *)(p.stack + (size_t)l * GD_STACK * GD_OBS * GD_OBS);
         if (p.flags & GD_F_STACK_FILL) {
+#pragma unroll 1
           for (int i = tid; i < vecs; i += GD_THREADS) {
             uint4 val = src[i];
             s0[i] = val; s0[vecs + i] = val; s0[2 * vecs + i] = val; s0[3 * vecs + i] = val;
           }
         } else if (p.flags & GD_F_STACK_ROLL) {
+#pragma unroll 1
           for (int i = tid; i < vecs; i += GD_THREADS) {
             s0[i] = s0[vecs + i];
             s0[vecs + i] = s0[2 * vecs + i];
@@ -506,6 +519,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
             s0[3 * vecs + i] = src[i];
           }
         } else {
+#pragma unroll 1
           for (int i = tid; i < vecs; i += GD_THREADS) s0[3 * vecs + i] = src[i];
         }
       }

@@ -86,7 +86,11 @@ __device__ __noinline__ unsigned long long gd_sprite_candidates(const GdScene &s
 /* Sprites cluster in a few screen columns, so the drawing is spread by rows:
  * the columns with candidates are listed; then the warps take
  * the listed columns from a counter and draw each candidate's rows 32 at a
- * time, far to near. */
+ * time, far to near.  A column's clip events are fetched once, by all threads of the warp at once, into its
+ * share of shared memory, and what a thing's depth says about each of them (gd_behind) is decided once per thing,
+ * one event a thread, so that a row's loop over the events reads nothing from global memory. */
+#define GD_SPRITE_EVENTS (GD_MAX_EVENTS * 20)      /* bytes per warp: 16 of clip rows and 4 of wall and sector an event */
+static_assert(GD_SPRITE_EVENTS * GD_WARPS <= GD_AUX_BYTES && GD_SPRITE_EVENTS % 16 == 0, "staged events");
 __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared &sh_, const GdEvent *events,
                            const int *eventCount, int nThings) {
   const GdScene &sc = *gd_as_shared(&sc_);
@@ -102,6 +106,8 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
   if (candOf[x0]) list[atomicAdd(&counters[0], 1)] = (short)x0;
   __syncthreads();
   const int listed = counters[0];
+  uint4 *staged = (uint4 *)(gd_smem + GD_OFF_AUX + (x0 >> 5) * GD_SPRITE_EVENTS);   /* distance, tiers, silhouettes, plane marks */
+  unsigned *owners = (unsigned *)(staged + GD_MAX_EVENTS);
   for (;;) {
     int slot = 0;
     if (lane == 0) slot = atomicAdd(&counters[1], 1);
@@ -110,14 +116,23 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
     const int x = list[slot];
     unsigned long long cand = candOf[x];
     const int nEv = eventCount[x];
-    const float rayAngle = v.angle + sc.rayOffsets[x];
-    const float rayCos = cosf(rayAngle), raySin = sinf(rayAngle);
+    __syncwarp();                                      /* the column before has read its events */
+#pragma unroll 1
+    for (int e = lane; e < nEv; e += 32) {
+      const unsigned *ev = (const unsigned *)&events[e * GD_SW + x];
+      staged[e] = make_uint4(ev[0], ev[2], ev[3], ev[4]);
+      owners[e] = ev[1];
+    }
+    __syncwarp();
+    const GdFlatRay ray = gd_flat_ray(sc, v, x);
     /* far to near: repeatedly take the remaining candidate with the largest
      * (depth, index) key */
+#pragma unroll 1
     while (cand) {
       int pick = -1;
       float pd = 0.0f;
       unsigned long long m = cand;
+#pragma unroll 1
       while (m) {
         int a = __ffsll((long long)m) - 1;
         m &= m - 1;
@@ -140,6 +155,12 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
         y0 = (int)gd_clamp(ya, 0, GD_VH);
         y1 = (int)gd_clamp(yb, 0, GD_VH);
       }
+      unsigned long long behind = 0;                 /* events whose wall lies behind the thing */
+#pragma unroll 1
+      for (int e0 = 0; e0 < nEv; e0 += 32) {
+        const int wall = e0 + lane < nEv ? (int)(short)(owners[e0 + lane] & 0xFFFFu) : -1;
+        behind |= (unsigned long long)__ballot_sync(0xffffffffu, wall >= 0 && gd_behind(sc, sh.walls[wall], wall, ac)) << e0;
+      }
       __syncwarp();                                  /* the farther sprite's pixels are in place */
 #pragma unroll 1
       for (int y = y0 + lane; y < y1; y += 32) {
@@ -147,42 +168,47 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
         i64 tv = frac >> 16;
         if (tv < 0 || tv >= ac.h) continue;
         size_t si = ((size_t)ac.sprite * sc.sprH + (size_t)tv) * sc.sprW + (size_t)u;
-        uint8_t post = sc.sprPost[si];
+        const uint8_t post = sc.sprPost[si], source = sc.sprAtlas[si];
         if (post == 255) continue;
         i64 postTop = (ac.topFixed + ac.yscale * (i64)post) >> 16;
         if (y < postTop) continue;
         /* nearest clip event covering this pixel */
         float bestD = GD_INF;
-        int bestW = -1, ownerSector = -1;
+        int bestE = -1, ownerSector = -1;
         bool filled = false, ownerFloor = false;
+        const unsigned row = (unsigned)y;
 #pragma unroll 1
         for (int e = 0; e < nEv; ++e) {
-          const GdEvent ev = events[e * GD_SW + x];
-          bool inLower = y >= ev.t1a && y < ev.t1b, inUpper = y >= ev.t0a && y < ev.t0b;
-          bool drawn = inLower ? ((ev.pad0 & 2) != 0) : (inUpper ? ((ev.pad0 & 1) != 0) : false);
-          bool covers = (y < ev.silTop) || (y >= ev.silBot);
+          const uint4 q = staged[e];
+          const bool inLower = row >= ((q.y >> 16) & 255u) && row < (q.y >> 24), inUpper = row >= (q.y & 255u) && row < ((q.y >> 8) & 255u);
+          const bool drawn = inLower ? (q.w & (2u << 16)) != 0 : (inUpper && (q.w & (1u << 16)) != 0);
+          bool covers = row < (q.z & 255u) || row >= ((q.z >> 8) & 255u);
           if (drawn && !filled) { filled = true; covers = true; }
-          if (covers && ev.dist < bestD) { bestD = ev.dist; bestW = ev.wall; }
-          if (ownerSector < 0 && ev.sector >= 0) {
-            if (y >= ev.floorA && y < ev.floorB) { ownerSector = ev.sector; ownerFloor = true; }
-            else if (y >= ev.ceilA && y < ev.ceilB) ownerSector = ev.sector;
+          const float d = __uint_as_float(q.x);
+          if (covers && d < bestD) { bestD = d; bestE = e; }
+          if (ownerSector < 0) {
+            const bool onFloor = row >= (q.w & 255u) && row < ((q.w >> 8) & 255u);
+            if (onFloor || (row >= ((q.z >> 16) & 255u) && row < (q.z >> 24))) {
+              const int sector = (int)(short)(owners[e] >> 16);
+              if (sector >= 0) { ownerSector = sector; ownerFloor = onFloor; }
+            }
           }
         }
         bool visible;
-        if (bestW >= 0) {
-          visible = gd_behind(sc, sh.walls[bestW], bestW, ac);
+        if (bestE >= 0) {
+          visible = (behind >> bestE) & 1ull;
         } else {
-          float limit = GD_INF;
-          if (!filled && ownerSector >= 0 && gd_pixel_unresolved(sc, v, x, y, rayCos, raySin, ownerSector))
-            limit = gd_plane_depth(sc, v, ownerSector, ownerFloor, y);
-          visible = ac.depth < limit;
+          /* The plane's depth limits the thing only where the pixel resolves to no sector: that search (a point
+           * test of every sector, up to 3.2 million cycles for a thing that fills the view) is left for things
+           * beyond the plane. */
+          visible = ac.depth < GD_INF &&
+                    (filled || ownerSector < 0 || ac.depth < gd_plane_depth(sc, v, ownerSector, ownerFloor, y) ||
+                     !gd_pixel_unresolved(sc, v, x, y, ray.rc, ray.rs, ownerSector));
         }
         if (!visible) continue;
-        uint8_t lit = cm[sc.sprAtlas[si]];
-        uint8_t dst = sh.frame[y * GD_SW + x];
-        uint8_t out = lit;
-        if (ac.style == -2) out = sc.transLut[dst * 256 + lit];
-        else if (ac.style >= 0) out = sc.addLut[((ac.style > 1 ? 1 : ac.style) * 256 + dst) * 256 + lit];
+        uint8_t out = cm[source];
+        if (ac.style == -2) out = sc.transLut[sh.frame[y * GD_SW + x] * 256 + out];
+        else if (ac.style >= 0) out = sc.addLut[((ac.style > 1 ? 1 : ac.style) * 256 + sh.frame[y * GD_SW + x]) * 256 + out];
         sh.frame[y * GD_SW + x] = out;
       }
     }
@@ -209,6 +235,7 @@ __device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, uint8_t *frame,
   const i64 lo = -base, hi = (i64)h * GD_FU - base;
   const int y0 = (int)gd_clamp(lo <= 0 ? 0 : gd_div(lo + iscale - 1, iscale), 0, GD_VH);
   const int y1 = (int)gd_clamp(hi <= 0 ? 0 : gd_div(hi + iscale - 1, iscale), 0, GD_VH);
+#pragma unroll 1
   for (int idx = threadIdx.x; idx < (y1 - y0) * w; idx += GD_THREADS) {
     int y = y0 + idx / w, sx = idx - (y - y0) * w;
     i64 xx = screenLeft + sx;
@@ -217,7 +244,8 @@ __device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, uint8_t *frame,
     if (sy < 0 || sy >= h) continue;
     i64 cy = gd_min(sy, sc.wpnH - 1), cx = gd_min((i64)sx, (i64)sc.wpnW - 1);
     size_t si = ((size_t)id * sc.wpnH + (size_t)cy) * sc.wpnW + (size_t)cx;
-    if (sc.wpnOpaque[si]) frame[y * GD_SW + (int)xx] = sc.wpnAtlas[si];
+    const uint8_t opaque = sc.wpnOpaque[si], texel = sc.wpnAtlas[si];   /* both on their way at once */
+    if (opaque) frame[y * GD_SW + (int)xx] = texel;
   }
 }
 
@@ -248,61 +276,54 @@ __device__ void gd_weapon(const GdScene &sc_, const int32_t *lane, uint8_t *fram
 }
 
 /* ---- phase: status bar (engine.py:15158-15267) --------------------------- */
-/* The status bar is a list of up to GD_HUD_MAX_PATCHES opaque-masked blits drawn
- * in a fixed order, later ones on top.  Thread 0 lists (patch, x, y), one thread
- * per entry clips it against the canvas, and then every column thread resolves
- * its 32 pixels from the entries that cross its column, topmost first. */
+/* The status bar is a list of opaque-masked blits drawn in a fixed order, later ones on top.  Every glyph that may
+ * be drawn has its place in the list: one thread fills in one place (patch, position, clipped against the canvas),
+ * and then every column thread resolves its 32 pixels from the entries that cross its column, topmost first.
+ * What bounds it is latency (listing by one thread and dependent loads, row after row, took 15 % of a lane's time),
+ * so the list is made beside the other setup, and a warp draws its columns when its walk has ended, while others
+ * still walk. */
+#define GD_HUD_PATCHES 44      /* bar, arms panel, 3 + 3 + 1 + 3 + 1 large glyphs, face, 6 weapons, 4 x 6 small digits */
 
-struct GdHudList { int4 *entries; int *count; int patches; };
-
-__device__ __forceinline__ void gd_hud_push(const GdHudList &hl, int patch, int x, int y) {
-  int n = *hl.count;
-#ifdef GD_CHECKED
-  if (patch < 0 || patch >= hl.patches) { atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX); return; }
-#endif
-  if (n < GD_HUD_MAX_PATCHES) { hl.entries[n] = make_int4(patch, x, y, 0); *hl.count = n + 1; }
+/* Place `slot` of a number drawn right-aligned at `right` (engine.py:15180-15210); patch -1: no digit there. */
+__device__ __forceinline__ int3 gd_hud_digit(const GdScene &sc, int value, int right, int y, bool small, int slot) {
+  const int vc = value < -99 ? -99 : (value > 999 ? 999 : value);
+  const int mag = vc < 0 ? -vc : vc;
+  const int n = mag > 99 ? 3 : (mag > 9 ? 2 : 1);
+  if (slot >= n) return make_int3(-1, 0, 0);
+  const int place = n - 1 - slot;                      /* the most significant digit comes first */
+  const int digit = place == 2 ? mag / 100 : (place == 1 ? mag / 10 % 10 : mag % 10);
+  const int dw = small ? 4 : 14, patch = (small ? 28 : 2) + digit;
+  const int4 hi = *reinterpret_cast<const int4 *>(&sc.hudInfo[patch * 4]);
+  return make_int3(patch, right - (n - slot) * dw - hi.z, y - hi.w);   /* the blit subtracts the glyph offsets once more */
 }
 
-__device__ void gd_hud_number(const GdScene &sc, const GdHudList &hl, int value, int right, int y, bool small) {
-  int vc = value < -99 ? -99 : (value > 999 ? 999 : value);
-  int neg = vc < 0;
-  int mag = neg ? -vc : vc;
-  int digits[3], n = 0;
-  do { digits[n++] = mag % 10; mag /= 10; } while (mag > 0);
-  int len = n + neg;
-  int dw = small ? 4 : 14, base = small ? 28 : 2;
-  int x = right - len * dw;
-  if (neg) x += dw;
-  for (int k = n - 1; k >= 0; --k) {
-    int patch = base + digits[k];
-    const int4 hi = *reinterpret_cast<const int4 *>(&sc.hudInfo[patch * 4]);
-    gd_hud_push(hl, patch, x - hi.z, y - hi.w);   /* the blit subtracts the glyph offsets once more */
-    x += dw;
-  }
-}
-
-__device__ __noinline__ void gd_hud(const GdScene &sc_, const GdShared &sh_, const int32_t *lane, uint8_t *canvas) {
+/* Threads 0 .. GD_HUD_PATCHES - 1: entries (tx | ty << 16, cw | ch << 16, sx | sy << 16, patch); cw = 0 when
+ * nothing is left. */
+__device__ __noinline__ void gd_hud_list(const GdScene &sc_, const int32_t *lane, int4 *entries) {
   const GdScene &sc = *gd_as_shared(&sc_);
-  const GdShared &sh = *gd_as_shared(&sh_);
-  GdHudList hl;
-  hl.entries = (int4 *)sh.obs;                       /* free until the resize */
-  hl.count = (int *)(sh.obs + GD_HUD_MAX_PATCHES * sizeof(int4));
-  hl.patches = sc.hudPatches;
-  if (threadIdx.x == 0) {
-    *hl.count = 0;
-    gd_hud_push(hl, 0, 0, 0);
-    gd_hud_push(hl, 1, 104, 0);
-    int weapon = lane[GD_L_WEAPON];
-    int ammoSlot = weapon < 2 ? -1 : (int)((0x54122100u >> (4 * (weapon > 7 ? 7 : weapon))) & 0xF);   /* -,-,1,2,2,1,4,5 */
-    int ammo = ammoSlot < 0 ? 0 : (int)__int_as_float(lane[GD_L_READY_AMMO]);
-    float hf = __int_as_float(lane[GD_L_HEALTH]), af = __int_as_float(lane[GD_L_ARMOR]);
-    int health = (int)(hf < 0 ? 0.0f : (hf > 999 ? 999.0f : hf));
-    int armor = (int)(af < 0 ? 0.0f : (af > 999 ? 999.0f : af));
-    gd_hud_number(sc, hl, ammo, 44, 3, false);
-    gd_hud_number(sc, hl, health, 90, 3, false);
-    gd_hud_push(hl, 12, 90, 3);
-    gd_hud_number(sc, hl, armor, 221, 3, false);
-    gd_hud_push(hl, 12, 221, 3);
+  const int t = threadIdx.x;
+  if (t >= GD_HUD_PATCHES) return;
+  const float hf = __int_as_float(lane[GD_L_HEALTH]), af = __int_as_float(lane[GD_L_ARMOR]);
+  const int health = (int)(hf < 0 ? 0.0f : (hf > 999 ? 999.0f : hf));
+  const int armor = (int)(af < 0 ? 0.0f : (af > 999 ? 999.0f : af));
+  int3 e = make_int3(-1, 0, 0);                        /* patch, x, y */
+  int number = 0, right = -1, top = 3, slot = t - 2;   /* right < 0: not a digit */
+  if (t < 2) {
+    e = make_int3(t, t ? 104 : 0, 0);
+  } else if (t < 5) {
+    const int weapon = lane[GD_L_WEAPON];
+    const int ammoSlot = weapon < 2 ? -1 : (int)((0x54122100u >> (4 * (weapon > 7 ? 7 : weapon))) & 0xF);   /* -,-,1,2,2,1,4,5 */
+    number = ammoSlot < 0 ? 0 : (int)__int_as_float(lane[GD_L_READY_AMMO]);
+    right = 44;
+  } else if (t < 8) {
+    number = health; right = 90; slot = t - 5;
+  } else if (t == 8) {
+    e = make_int3(12, 90, 3);
+  } else if (t < 12) {
+    number = armor; right = 221; slot = t - 9;
+  } else if (t == 12) {
+    e = make_int3(12, 221, 3);
+  } else if (t == 13) {
     int pain = (100 - health) >= 0 ? (100 - health) / 20 : -((health - 100 + 19) / 20);
     pain = pain < 0 ? 0 : (pain > 4 ? 4 : pain);
     int face = 13 + pain * 3 + lane[GD_L_FACE_INDEX];
@@ -316,57 +337,63 @@ __device__ __noinline__ void gd_hud(const GdScene &sc_, const GdShared &sh_, con
       }
     } else if (lane[GD_L_ATTACK_HELD] >= 70) face = 49 + pain;
     if (health <= 0) face = 69;
-    gd_hud_push(hl, face < 0 ? 0 : (face > 69 ? 69 : face), 143, 0);
-    for (int wi = 0; wi < 6; ++wi) {
-      bool owned = wi < 5 && ((lane[GD_L_WEAPONS_OWNED] >> (wi + 1)) & 1);
-      gd_hud_push(hl, owned ? 28 + wi + 2 : 38 + wi, 111 + 12 * (wi % 3), wi < 3 ? 4 : 14);
-    }
-    for (int row = 0; row < 4; ++row) {
-      int y = 5 + row * 6;
-      gd_hud_number(sc, hl, (int)__int_as_float(lane[GD_L_AMMO0 + row]), 288, y, true);
-      gd_hud_number(sc, hl, row == 0 ? 200 : (row == 3 ? 300 : 50), 314, y, true);   /* ammo maxima */
-    }
+    e = make_int3(face < 0 ? 0 : (face > 69 ? 69 : face), 143, 0);
+  } else if (t < 20) {
+    const int wi = t - 14;
+    const bool owned = wi < 5 && ((lane[GD_L_WEAPONS_OWNED] >> (wi + 1)) & 1);
+    e = make_int3(owned ? 28 + wi + 2 : 38 + wi, 111 + 12 * (wi % 3), wi < 3 ? 4 : 14);
+  } else {
+    const int row = (t - 20) / 6;
+    slot = (t - 20) % 6;
+    top = 5 + row * 6;
+    if (slot < 3) { number = (int)__int_as_float(lane[GD_L_AMMO0 + row]); right = 288; }
+    else { number = row == 0 ? 200 : (row == 3 ? 300 : 50); right = 314; slot -= 3; }   /* ammo maxima */
   }
-  __syncthreads();
-  const int n = *hl.count;
-  if (threadIdx.x < n) {
-    /* clip against the canvas: (tx | ty << 16, cw | ch << 16, sx | sy << 16, patch); cw = 0 when nothing is left */
-    int4 e = hl.entries[threadIdx.x];
-    const int patch = e.x;
-    const int4 hi = *reinterpret_cast<const int4 *>(&sc.hudInfo[patch * 4]);
-    int x = e.y - hi.z, y = e.z - hi.w;
-    int w = hi.x, h = hi.y;
-    int sx = x < 0 ? -x : 0, sy = y < 0 ? -y : 0;
-    int tx = x > 0 ? x : 0, ty = y > 0 ? y : 0;
-    int cw = min(w - sx, GD_SW - tx), ch = min(h - sy, GD_HUD_H - ty);
-    if (w <= 0 || h <= 0 || cw <= 0 || ch <= 0) { cw = 0; ch = 0; }
-    hl.entries[threadIdx.x] = make_int4(tx | (ty << 16), cw | (ch << 16), sx | (sy << 16), patch);
+  if (right >= 0) e = gd_hud_digit(sc, number, right, top, t >= 20, slot);
+#ifdef GD_CHECKED
+  if (e.x >= sc.hudPatches) { atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX); e.x = -1; }
+#endif
+  int tx = 0, ty = 0, cw = 0, ch = 0, sx = 0, sy = 0;
+  if (e.x >= 0) {
+    const int4 hi = *reinterpret_cast<const int4 *>(&sc.hudInfo[e.x * 4]);
+    const int x = e.y - hi.z, y = e.z - hi.w;
+    sx = x < 0 ? -x : 0; sy = y < 0 ? -y : 0;
+    tx = x > 0 ? x : 0; ty = y > 0 ? y : 0;
+    cw = min(hi.x - sx, GD_SW - tx); ch = min(hi.y - sy, GD_HUD_H - ty);
+    if (hi.x <= 0 || hi.y <= 0 || cw <= 0 || ch <= 0) { cw = 0; ch = 0; }
   }
-  __syncthreads();
-  {
-    const int x = threadIdx.x;
-    unsigned long long mine = 0;                       /* entries that cross this column */
-    for (int k = 0; k < n; ++k) {
-      int4 e = hl.entries[k];
-      int tx = e.x & 0xFFFF, cw = e.y & 0xFFFF;
-      if (x >= tx && x < tx + cw) mine |= 1ull << k;
-    }
-    for (int y = 0; y < GD_HUD_H; ++y) {
-      uint8_t value = 0;
-      unsigned long long m = mine;
-      while (m) {
-        int k = 63 - __clzll((long long)m);            /* topmost remaining entry */
-        m &= ~(1ull << k);
-        int4 e = hl.entries[k];
-        int tx = e.x & 0xFFFF, ty = e.x >> 16, ch = e.y >> 16, sx = e.z & 0xFFFF, sy = e.z >> 16;
-        if (y < ty || y >= ty + ch) continue;
-        size_t si = ((size_t)e.w * GD_HUD_H + (size_t)(sy + y - ty)) * GD_SW + (size_t)(sx + x - tx);
-        if (sc.hudOpaque[si]) { value = sc.hudAtlas[si]; break; }
-      }
-      canvas[y * GD_SW + x] = value;
-    }
+  entries[t] = make_int4(tx | (ty << 16), cw | (ch << 16), sx | (sy << 16), e.x < 0 ? 0 : e.x);
+}
+
+/* Column threadIdx.x of the status bar; the list is complete. */
+__device__ __noinline__ void gd_hud_column(const GdScene &sc_, const int4 *entries_, uint8_t *canvas) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  const int4 *entries = gd_as_shared(entries_);
+  const int x = threadIdx.x;
+  unsigned long long mine = 0;                         /* entries that cross this column */
+#pragma unroll 1
+  for (int k = 0; k < GD_HUD_PATCHES; ++k) {
+    const int4 e = entries[k];
+    const int tx = e.x & 0xFFFF;
+    if (x >= tx && x < tx + (e.y & 0xFFFF)) mine |= 1ull << k;
   }
-  __syncthreads();
+#pragma unroll 1
+  for (int y = 0; y < GD_HUD_H; ++y) {
+    uint8_t value = 0;
+    unsigned long long m = mine;
+#pragma unroll 1
+    while (m) {
+      const int k = 63 - __clzll((long long)m);        /* topmost remaining entry */
+      m &= ~(1ull << k);
+      const int4 e = entries[k];
+      const int ty = e.x >> 16;
+      if (y < ty || y >= ty + (e.y >> 16)) continue;
+      const int si = (e.w * GD_HUD_H + (e.z >> 16) + y - ty) * GD_SW + (e.z & 0xFFFF) + x - (e.x & 0xFFFF);
+      const uint8_t opaque = sc.hudOpaque[si], texel = sc.hudAtlas[si];   /* both on their way at once */
+      if (opaque) { value = texel; break; }
+    }
+    canvas[y * GD_SW + x] = value;
+  }
 }
 
 #endif

@@ -715,9 +715,10 @@ __device__ __noinline__ void gd_masked_pass(const GdScene &sc_, const GdView &v_
 /* A column that has left the map (current sector -1) still takes part in the reference's
  * vectorised iterations: its decision is made against sector 0 with wall 0 selected at an
  * infinite distance (engine.py:11561-11588 clamp the sector index).  That decision can only
- * become a valid crossing through a projected left-edge owner: a wall of sector 0, or a
- * neighbour of wall 0 at one of its endpoints, whose ray-owned span starts at this very
- * column (engine.py:11589-11730, 11905-11990, 12005-12072), or through the rules that need
+ * become a valid crossing through a projected left-edge owner: a one-sided wall of sector 0
+ * that shares an endpoint with wall 0 (engine.py:11905-11930), or a neighbour of wall 0 at one
+ * of its endpoints (11589-11730), whose ray-owned span starts at this very column, or
+ * through the rules that need
  * wall 0's projected span to end at this column (engine.py:11930-11962, 12073-12164).  Every
  * other column draws nothing, records nothing and changes nothing the frame depends on once
  * it is outside, so its walk can stop there.  This marks the columns that may have to go on; all these rules
@@ -727,6 +728,7 @@ __device__ void gd_mark_afterlife_columns(const GdScene &sc, const GdShared &sh)
   const int n0 = sc.secOff[1] - sc.secOff[0];
   const int nb0 = sc.nbDirect ? 0 : sc.nbOff[0], nb1 = sc.nbDirect ? 2 : sc.nbOff[1];
   const int total = n0 + (nb1 - nb0) + 1;
+#pragma unroll 1
   for (int i = threadIdx.x; i < total; i += GD_THREADS) {
     int xl;
     if (i == total - 1) {
@@ -737,6 +739,7 @@ __device__ void gd_mark_afterlife_columns(const GdScene &sc, const GdShared &sh)
                      : (sc.nbDirect ? sc.nbDirectTab[i - n0] : sc.nbIdx[nb0 + (i - n0)]);
       if (w < 0) continue;                            /* no neighbour at that endpoint */
       w = GD_CHECK_INDEX(w, sc.W);
+      if (i < n0 && (!(gd_hot(w).bits & GD_HOT_ONESIDED) || !gd_shares_endpoint(sc, w, 0))) continue;
       xl = (int)(short)(gd_hot(w).span & 0xFFFFu);
     }
     if (xl >= 0 && xl < GD_SW) atomicOr(&busy[xl >> 5], 1u << (xl & 31));
@@ -902,9 +905,14 @@ __device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, co
         else if (pendEnd) slow = true;
         else if (kind == 2u) slow = !gd_quiet_crossing(sc, secWalls, secOff[cur], k1, wall, x, rx, ry, spanStarts);
         else if (kind == 1u) slow = !(gd_hot(wall).bits & GD_HOT_ONESIDED);     /* a one-sided end of the column either way */
-        else slow = spanStarts;
+        else slow = !stopsOutside;
         if (!slow && kind == 0u) {
-          /* no wall is left and no span starts here: no rule finds another one, the column leaves the map */
+          /* no wall of the sector is left and nothing is pending: the rules start from wall 0 at an infinite distance
+           * like those of a column outside the map, and of the sector's walls none can take over, because a
+           * projected one would have been found.  What can is a neighbour of wall 0 whose span starts here
+           * (engine.py:11650-11730), which gd_mark_afterlife_columns marks; every other column leaves the map.
+           * (Any span's start used to send the column to gd_slow_step: 5.7 of 9 such steps per lane of the
+           * 64-sector map, each a warp's wait of 28 thousand cycles.) */
           wall = -1 - x;
         } else
         if (!slow) {
