@@ -99,6 +99,10 @@ __global__ void __launch_bounds__(GD_CELLS * GD_CELLS) gd_cells_kernel(GdScene s
   /* coordinates that are not finite, or so large that a unit is lost in them: every list counts as too long */
   const bool usable = fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(y0), fabsf(y1))) < 100000.0f;
   const float perX = (float)GD_CELLS / fmaxf(x1 - x0, 1.0f), perY = (float)GD_CELLS / fmaxf(y1 - y0, 1.0f);
+  bool closed = true;
+  for (int s = t; s < sc.S; s += GD_CELLS * GD_CELLS) closed = closed && sc.secI[s * 4 + 3] != 0;
+  closed = __syncthreads_and(closed);
+  if (t == 0) { cells->xLo = closed ? x0 - 1.0f : -CUDART_INF_F; cells->xHi = x1 + 1.0f; cells->yLo = y0; cells->yHi = y1; }
   if (t == 0) { cells->x0 = usable ? x0 : 0.0f; cells->y0 = usable ? y0 : 0.0f; cells->perX = usable ? perX : 0.0f; cells->perY = usable ? perY : 0.0f; }
   const int cx = t % GD_CELLS, cy = t / GD_CELLS;
   int n = usable ? 0 : 255;

@@ -40,6 +40,7 @@ typedef long long i64;
 #define GD_CELL_SECTORS 7
 struct __align__(16) GdCells {
   float x0, y0, perX, perY;       /* cell of a coordinate: (c - x0) * perX */
+  float xLo, xHi, yLo, yHi;       /* no sector contains a point with x > xHi, y >= yHi, y < yLo or (all closed) x < xLo */
   unsigned short cell[GD_CELLS * GD_CELLS][1 + GD_CELL_SECTORS];   /* count (255: more than the list holds), sectors */
 };
 

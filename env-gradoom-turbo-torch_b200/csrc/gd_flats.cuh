@@ -31,6 +31,12 @@ __device__ __forceinline__ int gd_cell(const GdCells &g, float px, float py) {
   return gd_cell_axis(py, g.y0, g.perY) * GD_CELLS + gd_cell_axis(px, g.x0, g.perX);
 }
 
+/* Along a ray (rc, rs) the points only move on: once one is past every sector in the ray's direction (the roundings
+ * are monotone, so is the distance from group to group), no later one lies in a sector. */
+__device__ __forceinline__ bool gd_past_map(const GdCells &g, float px, float py, float rc, float rs) {
+  return (rc > 0 && px > g.xHi) || (rc < 0 && px < g.xLo) || (rs > 0 && py >= g.yHi) || (rs < 0 && py < g.yLo);
+}
+
 /* The lowest-numbered sector of height group g (f: floors, else ceilings) below `end` that contains the point,
  * or -1.  A point's cell names the one to four sectors that can; testing all of a group's took most of the
  * time of views with many such pixels (a lane of the 256-sector map: 11 million cycles at worst, now 4). */
@@ -85,6 +91,7 @@ __device__ __noinline__ bool gd_pixel_unresolved(const GdScene &sc_, const GdVie
     float cd = perp / cc;
     if (!(ph > 0) || !isfinite(cd) || !(cd > 0)) continue;
     float px = v.x + rc * cd, py = v.y + rs * cd;
+    if (gd_past_map(*sc.cells, px, py, rc, rs)) break;
     if (gd_group_sector(sc, f, g, px, py, 0x7fffffff) >= 0) return false;
   }
   return true;
@@ -227,6 +234,7 @@ __device__ __noinline__ GdFlatProbe gd_flat_probe(const GdScene &sc_, const GdVi
     if (!(ph > 0) || !isfinite(cd) || !(cd > 0)) continue;
     if (cd > best) break;
     float px = v.x + r.rc * cd, py = v.y + r.rs * cd;
+    if (gd_past_map(*sc.cells, px, py, r.rc, r.rs)) break;
     const int s = gd_group_sector(sc, f, g, px, py, cd == best ? out.sector + 1 : 0x7fffffff);
     if (s >= 0) { best = cd; out.sector = s; }
   }
