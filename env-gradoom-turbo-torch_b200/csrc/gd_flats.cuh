@@ -61,12 +61,26 @@ __device__ __noinline__ int gd_group_sector(const GdScene &sc_, int f, int g, fl
   return -1;
 }
 
+/* Lowest-numbered sector that contains a point (engine.py:9598-9617), 0x7fffffff for none; by a whole warp. */
+__device__ __forceinline__ int gd_sector_of_point(const GdScene &sc, float px, float py) {
+  const unsigned short *cell = sc.cells->cell[gd_cell(*sc.cells, px, py)];
+  const bool listed = cell[0] <= GD_CELL_SECTORS;
+  const int count = listed ? cell[0] : sc.S;
+  unsigned found = 0x7fffffff;
+#pragma unroll 1
+  for (int k = threadIdx.x & 31; k < count; k += 32) {
+    const int s = listed ? cell[1 + k] : k;
+    if (gd_point_in_sector(sc, s, px, py)) { found = (unsigned)s; break; }
+  }
+  return (int)__reduce_min_sync(0xffffffffu, found);
+}
+
 /* Flat-fallback resolution of a pixel (engine.py:10961-11026): true when the
  * column ray meets no sector's plane inside that sector's polygon. */
-__device__ __noinline__ bool gd_pixel_unresolved(const GdScene &sc_, const GdView &v_, int x, int y, float rc, float rs,
-                                                 int hint) {
+__device__ __noinline__ bool gd_pixel_unresolved(const GdScene &sc_, const GdView &v_, int x, int y, int hint) {
   const GdScene &sc = *gd_as_shared(&sc_);
   const GdView &v = *gd_as_shared(&v_);
+  const float rayAngle = v.angle + sc.rayOffsets[x], rc = cosf(rayAngle), rs = sinf(rayAngle);
   i64 ti = gd_clamp((GD_ANG90 - v.pitchBam) >> 19, 0, 4095);
   i64 offFixed = ((i64)sc.fineTan[ti] * 12582912LL) >> 16;
   float center = 103.5f + (float)offFixed / 65536.0f;
@@ -97,12 +111,13 @@ __device__ __noinline__ bool gd_pixel_unresolved(const GdScene &sc_, const GdVie
   return true;
 }
 
-__device__ float gd_plane_depth(const GdScene &sc_, const GdView &v_, int sector, bool isFloor, int y) {
-  const GdScene &sc = *gd_as_shared(&sc_);
-  const GdView &v = *gd_as_shared(&v_);
+/* Row of the horizon, for gd_plane_depth. */
+__device__ __forceinline__ float gd_flat_center(const GdScene &sc, const GdView &v) {
   i64 ti = gd_clamp((GD_ANG90 - v.pitchBam) >> 19, 0, 4095);
   i64 offFixed = ((i64)sc.fineTan[ti] * 12582912LL) >> 16;
-  float flatCenter = (103.0f + (float)offFixed / 65536.0f) + 0.5f;
+  return (103.0f + (float)offFixed / 65536.0f) + 0.5f;
+}
+__device__ __forceinline__ float gd_plane_depth(const GdScene &sc, const GdView &v, float flatCenter, int sector, bool isFloor, int y) {
   float ph = isFloor ? (v.viewZ - gd_sec_floor(sc, sector)) : (gd_sec_ceil(sc, sector) - v.viewZ);
   float den = fmaxf(fabsf((float)y - flatCenter), 0.5f);
   return ph * 192.0f / den;

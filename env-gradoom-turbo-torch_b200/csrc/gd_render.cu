@@ -271,10 +271,9 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     if (tid < GD_OWNER_WORDS) sh.ownerMask[tid] = 0;
     if (tid == 0) sh.misc[1] = 0;
     /* sector of every thing and of the player (slot 64): lowest index that
-     * contains the point (engine.py:9598-9617), found by all threads together
+     * contains the point (engine.py:9598-9617), found by warps 1 to 9
      * while thread 0 sets up the view */
     int *pointSector = (int *)sh.hitA;
-    if (tid <= 64) pointSector[tid] = 0x7fffffff;
     __syncthreads();
     {
       const int laneFlags = sh.lane[GD_L_FLAGS];
@@ -311,19 +310,16 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     if (tid == 0) {
       gd_view_setup(sc, sh.lane, sView);
     } else if (tid >= 32) {
-      const int pairs = (nThings + 1) * sc.S;
+      /* one warp a point: its cell of the map names the sectors to test */
 #pragma unroll 1
-      for (int i = tid - 32; i < pairs; i += GD_THREADS - 32) {
-        int t = i / sc.S, s = i - t * sc.S;
-        float px, py;
+      for (int t = (tid >> 5) - 1; t <= nThings; t += GD_WARPS - 1) {
+        float px = __int_as_float(sh.lane[GD_L_X]), py = __int_as_float(sh.lane[GD_L_Y]);
         if (t < nThings) {
           const gd_thing &th = p.things[(size_t)l * p.maxThings + t];
           px = th.x; py = th.y;
-        } else {
-          px = __int_as_float(sh.lane[GD_L_X]); py = __int_as_float(sh.lane[GD_L_Y]);
-          t = 64;
         }
-        if (gd_point_in_sector(sc, s, px, py)) atomicMin(&pointSector[t], s);
+        const int s = gd_sector_of_point(sc, px, py);
+        if ((tid & 31) == 0) pointSector[t < nThings ? t : 64] = s;
       }
     }
     __syncthreads();

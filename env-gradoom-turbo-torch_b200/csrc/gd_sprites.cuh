@@ -106,6 +106,7 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
   if (candOf[x0]) list[atomicAdd(&counters[0], 1)] = (short)x0;
   __syncthreads();
   const int listed = counters[0];
+  const float flatCenter = gd_flat_center(sc, v);
   uint4 *staged = (uint4 *)(gd_smem + GD_OFF_AUX + (x0 >> 5) * GD_SPRITE_EVENTS);   /* distance, tiers, silhouettes, plane marks */
   unsigned *owners = (unsigned *)(staged + GD_MAX_EVENTS);
   for (;;) {
@@ -124,7 +125,6 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
       owners[e] = ev[1];
     }
     __syncwarp();
-    const GdFlatRay ray = gd_flat_ray(sc, v, x);
     /* far to near: repeatedly take the remaining candidate with the largest
      * (depth, index) key */
 #pragma unroll 1
@@ -202,8 +202,8 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
            * test of every sector, up to 3.2 million cycles for a thing that fills the view) is left for things
            * beyond the plane. */
           visible = ac.depth < GD_INF &&
-                    (filled || ownerSector < 0 || ac.depth < gd_plane_depth(sc, v, ownerSector, ownerFloor, y) ||
-                     !gd_pixel_unresolved(sc, v, x, y, ray.rc, ray.rs, ownerSector));
+                    (filled || ownerSector < 0 || ac.depth < gd_plane_depth(sc, v, flatCenter, ownerSector, ownerFloor, y) ||
+                     !gd_pixel_unresolved(sc, v, x, y, ownerSector));
         }
         if (!visible) continue;
         uint8_t out = cm[source];

@@ -639,6 +639,10 @@ __device__ __noinline__ void gd_masked_pass(const GdScene &sc_, const GdView &v_
 #pragma unroll 1
   for (int i = 0; i < sc.M; ++i) {
     const int k = GD_CHECK_INDEX(sc.maskedWalls[i], sc.W);
+#ifndef GD_CHECKED
+    const unsigned span = gd_hot(k).span;              /* the wall has to own the column */
+    if (x < (int)(short)(span & 0xFFFFu) || x >= (int)(span >> 16)) continue;
+#endif
     const int sd = (gd_hot(k).bits & GD_HOT_FRONT) ? 0 : 1;
     const int t = sc.sideTex[(k * 2 + sd) * 3];
     if (t < 0) continue;
