@@ -371,10 +371,11 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       if (sector >= 0) {
         GdRowProj unused;
         gd_rowproj_setup(v, q, sc.secF[sector * 2 + (slot & 1)], piece ? unused : rowproj[w * 4 + slot], row);
-        /* the light of the side, modulo 2^32 as well: exact while the owned columns' values fit */
+        /* the light of the side, modulo 2^32 as well: exact while the owned columns' values fit.  Nothing below
+         * -2^30 is left to this form either: gd_shade takes the light from a base below 2^30 in 32 bits */
         const i64 step = q.visStep[sd], origin = q.visL[sd] - gd_wmul(q.visSl[sd], step);
         const i64 l0 = origin + gd_wmul(gd_max(q.sl, 0), step), l1 = origin + gd_wmul(gd_min(q.sr, GD_SW) - 1, step);
-        if (l0 != (i64)(int)l0 || l1 != (i64)(int)l1) row.lim |= GD_ROW_LIGHT_WIDE;
+        if (gd_min(l0, l1) < -(1LL << 30) || gd_max(l0, l1) >= (1LL << 31)) row.lim |= GD_ROW_LIGHT_WIDE;
         row.vis = (int)((slot & 1) ? step : origin);
       }
       (piece ? fragRows + f * 4 : rows + w * 4)[slot] = row;

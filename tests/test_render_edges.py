@@ -68,6 +68,19 @@ def test_views_from_outside_rooms_and_close_to_walls(pkg, oracle, rows, cols, ro
     _equal(oracle, sc, lanes, things, k)
 
 
+def test_wall_light_below_the_range_of_the_shade(pkg, oracle, scenes):
+    """A viewer outside every room sees a wall of another sector from its far side: the light of the first column is
+    -2 147 316 498, which the shade's base less it does not fit 32 bits.  The column is the darkest, not the brightest."""
+
+    sc, _ = scenes("c2")
+    lanes, things = stepper.random_lanes(sc, 3, 0, seed=3)
+    _place(lanes, slice(0, 3), [302.71452, 302.71452, 303.0], [-24.25008, -24.2, -24.25008])
+    lanes[:, gdstate.L_ANGLE_BAM] = 770460205
+    lanes.view(np.float32)[:, gdstate.L_ANGLE] = np.float32(770460205) * np.float32(gdstate.BAM_TO_RADIANS)
+    lanes.view(np.float32)[:, gdstate.L_VIEW_Z] = 150.0
+    _equal(oracle, sc, lanes, things, 0)
+
+
 def test_status_bar_numbers(pkg, oracle, scenes):
     """One, two and three digits, the sign that is not drawn, and values past the bar's range."""
 
