@@ -239,12 +239,16 @@ class LaneStepper:
         players.copy_(torch.where(mask[:, None], fresh, players))
 
     def _native_state(self):
-        """The stepper's buffers as the library takes them; None without a renderer on their device or when a
-        buffer was replaced by one of another layout."""
+        """The stepper's buffers as the library takes them; None without a renderer on their device, when a buffer
+        was replaced by one of another layout, or when one of the rules that the library's kernels restate was
+        overridden by a subclass or on the object."""
 
         renderer, n = self.renderer, self.num_envs
         if renderer is None or renderer.device != self.lanes.device:
             return None
+        for rule in ("_uniform", "_refresh_pose", "_players_from_lanes"):
+            if getattr(getattr(self, rule), "__func__", None) is not getattr(LaneStepper, rule):
+                return None
         torch, spec, sectors = self.torch, self.spec, self.floors.shape[0]
         for t, dtype, shape in ((self.lanes, torch.int32, (n, gdstate.LANE_WORDS)),
                                 (self.players, torch.int32, (n, gdstate.PLAYER_WORDS)),
@@ -355,8 +359,8 @@ class LaneStepper:
         return rewards, terminated, truncated
 
     def _step_tensors(self, buttons):
-        """The step as tensor operations around the kinematics kernel: buttons that are not booleans, and
-        buffers that were replaced by ones of another layout."""
+        """The step as tensor operations around the kinematics kernel: buttons that are not booleans, buffers that
+        were replaced by ones of another layout, and steppers with rules of their own."""
 
         torch = self.torch
         lanes = self.lanes

@@ -306,3 +306,32 @@ def test_wall_fine_angles_of_axis_aligned_and_diagonal_lines(pkg):
     fine = gdscene.wall_fine_angles(walls)
     assert fine[:, 0].tolist() == [0, 2048, 4096, 6144, 1024, 5120, 7168]
     assert fine[:, 1].tolist() == [4096, 6144, 0, 2048, 5120, 1024, 3072]
+
+
+@pytest.mark.parametrize("rule", [None, "_uniform", "_refresh_pose", "_players_from_lanes"])
+@pytest.mark.parametrize("where", ["class", "object"])
+def test_lane_stepper_rules_that_were_overridden_are_used(rule, where, pkg, scenes):
+    """The library's stepper kernels restate the stepper's own rules, so they serve no stepper that has others."""
+
+    from gradoom_b200 import stepper
+
+    sc, _ = scenes("c1")
+    fused, used = [], []
+    renderer = types.SimpleNamespace(device=torch.device("cpu"), player_tics=lambda *a, **k: None,
+                                     stepper_step=lambda *a: fused.append("step"),
+                                     stepper_reset=lambda *a: fused.append("reset"))
+
+    def other(self, *args):
+        used.append(rule)
+        return getattr(stepper.LaneStepper, rule)(self, *args)
+
+    members = {rule: other} if rule and where == "class" else {}
+    s = type("Stepper", (stepper.LaneStepper,), members)(sc, 5, device="cpu", k_things=2)
+    if rule and where == "object":
+        setattr(s, rule, types.MethodType(other, s))
+    s.bind_renderer(renderer)
+    used.clear()
+    s.reset(torch.ones(5, dtype=torch.bool), torch.arange(5))
+    s.step(torch.ones((5, 3), dtype=torch.bool))
+    assert fused == ([] if rule else ["reset", "step"])
+    assert bool(used) == bool(rule)
