@@ -10,6 +10,10 @@
 #include <string.h>
 
 #define GD_HOST_CHUNKS 4
+/* limits of the scratch array built into the library (gd_render_step_static) */
+#define GD_STATIC_MAX_CTAS 32
+#define GD_STATIC_MAX_WALLS 256
+static bool gd_fits_static(const GdScene &sc) { return sc.W <= GD_STATIC_MAX_WALLS && sc.S <= GD_STATIC_MAX_WALLS; }
 
 struct gd_renderer {
   int32_t header[GD_HDR_WORDS];
@@ -31,8 +35,8 @@ struct gd_renderer {
   size_t decalScratchBytes;
   GdSide *sides;             /* 2 W crossing records, the line of every fragment */
   int *fragLine;
-  GdWall *fragScratch;       /* ctas x F records, allocated with the renderer when the scene has split lines */
-  GdRow *fragRows;
+  size_t fragBytes;          /* a CTA's records of split lines: behind its scratch; F is not bounded, so */
+  uint8_t *staticFrags;      /* those of the built-in array's CTAs are allocated with the renderer */
 };
 
 /* Crossing records of the scene, once per renderer.  Texture indices are passed on as they are (the checked build
@@ -205,7 +209,7 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
   r->copyStream = nullptr;
   r->copiesDone = nullptr;
   r->decalScratch = nullptr;
-  r->fragScratch = nullptr; r->fragRows = nullptr; r->sides = nullptr; r->fragLine = nullptr;
+  r->staticFrags = nullptr; r->fragBytes = 0; r->sides = nullptr; r->fragLine = nullptr;
   for (int c = 0; c < GD_HOST_CHUNKS; ++c) r->chunkDone[c] = nullptr;
   memcpy(r->header, h, sizeof r->header);
   r->device = device;
@@ -287,18 +291,17 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
       r->ctas = sms * perSm;  /* one persistent CTA per resident slot */
   }
   if (rc == GD_OK) {
-    void *sides = nullptr, *mem = nullptr, *rows = nullptr;
+    void *sides = nullptr, *mem = nullptr;
     const size_t sideBytes = (size_t)sc.W * 2 * sizeof(GdSide);
     const size_t lineBytes = gd_align16((size_t)sc.F * 4);
     if (cudaMalloc(&sides, sideBytes + lineBytes + sizeof(GdCells)) != cudaSuccess) rc = GD_ERR_CUDA;
     r->sides = (GdSide *)sides;
     sc.cells = (GdCells *)((uint8_t *)sides + sideBytes + lineBytes);
     r->fragLine = (int *)((uint8_t *)sides + sideBytes);
-    if (rc == GD_OK && sc.F > 0) {
-      if (cudaMalloc(&mem, (size_t)r->ctas * sc.F * sizeof(GdWall)) != cudaSuccess) rc = GD_ERR_CUDA;
-      r->fragScratch = (GdWall *)mem;
-      if (!r->chip && cudaMalloc(&rows, (size_t)r->ctas * sc.F * 4 * sizeof(GdRow)) != cudaSuccess) rc = GD_ERR_CUDA;
-      r->fragRows = (GdRow *)rows;
+    if (sc.F > 0) r->fragBytes = gd_frag_bytes(sc.F, r->chip);
+    if (rc == GD_OK && sc.F > 0 && gd_fits_static(sc)) {
+      if (cudaMalloc(&mem, GD_STATIC_MAX_CTAS * r->fragBytes) != cudaSuccess) rc = GD_ERR_CUDA;
+      r->staticFrags = (uint8_t *)mem;
     }
     if (rc == GD_OK) {
       gd_side_setup_kernel<<<(sc.W * 2 + 127) / 128, 128>>>(sc, r->sides, r->fragLine);
@@ -307,9 +310,9 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
     }
   }
   r->base.maxThings = max_things;
-  r->base.sides = r->sides; r->base.fragLine = r->fragLine; r->base.fragScratch = r->fragScratch; r->base.fragRows = r->fragRows;
+  r->base.sides = r->sides; r->base.fragLine = r->fragLine;
   r->base.secWallsN = secWallsN;
-  r->base.perCta = gd_scratch_per_cta(sc.W, sc.S);
+  r->base.perCta = r->base.fragStride = gd_scratch_per_cta(sc.W, sc.S) + r->fragBytes;
   r->base.queueOffset = (size_t)r->ctas * r->base.perCta;
   r->copyStream = nullptr;
   r->copiesDone = nullptr;
@@ -336,8 +339,7 @@ extern "C" void gd_renderer_destroy(gd_renderer *r) {
   if (r->copiesDone) cudaEventDestroy(r->copiesDone);
   if (r->copyStream) cudaStreamDestroy(r->copyStream);
   if (r->decalScratch) cudaFree(r->decalScratch);
-  if (r->fragScratch) cudaFree(r->fragScratch);
-  if (r->fragRows) cudaFree(r->fragRows);
+  if (r->staticFrags) cudaFree(r->staticFrags);
   if (r->sides) cudaFree(r->sides);
   if (switched) cudaSetDevice(prev);
   delete r;
@@ -391,6 +393,7 @@ static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing 
   p.lanes = lanes; p.things = things; p.n = n; p.flags = flags;
   p.stack = stack; p.ringHead = ring_head; p.resetMask = reset_mask; p.obsOut = obs_out; p.indexedOut = indexed_out; p.rgbOut = rgb_out;
   p.scratch = (uint8_t *)scratch; p.status = status;
+  p.frags = p.scratch + gd_scratch_per_cta(r->base.sc.W, r->base.sc.S);
   p.decals = r->decals; p.decalSlots = r->decalSlots; p.decalScratch = r->decalScratch;
   int grid = n < r->ctas ? n : r->ctas;
   gd_kernel_for(r)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
@@ -543,8 +546,6 @@ extern "C" int gd_render_step_host(const gd_renderer *r, const int32_t *lanes_ho
  * library image.  Every GPU that loads the library holds GD_STATIC_SCRATCH_BYTES
  * of it until the process exits.
  */
-#define GD_STATIC_MAX_CTAS 32
-#define GD_STATIC_MAX_WALLS 256
 /* a scene of W walls has fewer than W sectors (three walls bound a sector, a wall bounds two) */
 #define GD_STATIC_PER_CTA ((GD_SCRATCH_FIXED + GD_STATIC_MAX_WALLS * (2 * GD_PLANE_ENTRY_BYTES + 2 * GD_PLANE_BYTES + \
                             sizeof(GdWall) + 4 * sizeof(GdRowProj) + 4 * sizeof(GdRow) + 16) + 127) & ~(size_t)63)
@@ -565,7 +566,7 @@ extern "C" int gd_render_step_static(const gd_renderer *r, const int32_t *lanes,
   if (!r || !lanes || !stack || !status) return GD_ERR_NULL;
   if (r->maxThings > 0 && !things) return GD_ERR_NULL;
   if (n < 0) return GD_ERR_SIZE;
-  if (r->base.sc.W > GD_STATIC_MAX_WALLS || r->base.sc.S > GD_STATIC_MAX_WALLS) return GD_ERR_STATIC_LIMIT;
+  if (!gd_fits_static(r->base.sc)) return GD_ERR_STATIC_LIMIT;
   if (r->device < 0 || r->device >= GD_STATIC_MAX_DEVICES) return GD_ERR_STATIC_LIMIT;
   if (n == 0) return GD_OK;
   uintptr_t align = (uintptr_t)lanes | (uintptr_t)things | (uintptr_t)stack;
@@ -590,6 +591,8 @@ extern "C" int gd_render_step_static(const gd_renderer *r, const int32_t *lanes,
   p.flags = GD_F_STACK_ROLL | (mask_hud ? GD_F_MASK_HUD : GD_F_DRAW_HUD);
   p.stack = stack; p.ringHead = 0; p.resetMask = nullptr; p.obsOut = nullptr; p.indexedOut = nullptr; p.rgbOut = nullptr;
   p.scratch = scratch; p.status = status;
+  p.perCta = gd_scratch_per_cta(r->base.sc.W, r->base.sc.S);
+  p.frags = r->staticFrags; p.fragStride = r->fragBytes;
   /* lane queue: the last 16 bytes of the array; zero when the library is
    * loaded and left at zero by every launch */
   p.queueOffset = (size_t)GD_STATIC_MAX_CTAS * GD_STATIC_PER_CTA;

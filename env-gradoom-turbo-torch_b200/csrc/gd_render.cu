@@ -75,8 +75,10 @@ struct GdParams {
   const gd_decal *decals;    /* n x decalSlots rings of bullet chips, or null */
   int decalSlots;
   uint8_t *decalScratch;     /* ctas x gd_decal_scratch_per_cta(decalSlots) */
-  GdWall *fragScratch;       /* ctas x F fragment records, when the scene has split lines */
-  GdRow *fragRows;           /* ctas x F x 4 row projections of the fragments, when they are not on chip */
+  /* scenes with split lines: a CTA's F fragment records, then their F x 4 row projections when those are not on
+   * chip; in the launch's own scratch like all that a CTA writes, so that launches of one renderer may overlap */
+  uint8_t *frags;
+  size_t fragStride;         /* from CTA to CTA */
 };
 
 #define GD_SCRATCH_EVENTS_BYTES (GD_MAX_EVENTS * GD_SW * (int)sizeof(GdEvent))
@@ -99,6 +101,8 @@ __host__ __device__ inline size_t gd_table_bytes(int W, int S) {
   return (size_t)W * 4 * sizeof(GdRow) + (size_t)W * 16 + (size_t)S * 2 * GD_PLANE_BYTES;
 }
 __host__ __device__ inline size_t gd_scratch_per_cta(int W, int S) { return gd_scratch_tables(W, S) + gd_table_bytes(W, S); }
+__host__ __device__ inline size_t gd_frag_wall_bytes(int F) { return gd_align16((size_t)F * sizeof(GdWall)); }
+inline size_t gd_frag_bytes(int F, bool chip) { return gd_frag_wall_bytes(F) + (chip ? 0 : (size_t)F * 4 * sizeof(GdRow)); }
 
 struct GdActor {
   float x, y, depth;
@@ -198,8 +202,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     sh.lane = (int32_t *)(gd_smem + GD_OFF_LANE);
     sh.ownerMask = (unsigned *)(gd_smem + GD_OFF_OWNER);
     sh.walls = (GdWall *)(myScratch + gd_scratch_walls(sc.W, sc.S));
-    sh.frags = p.fragScratch ? p.fragScratch + (size_t)blockIdx.x * sc.F : nullptr;
-    if (!sh.frags) sc.F = 0;
+    sh.frags = (GdWall *)(p.frags + blockIdx.x * p.fragStride);
     sh.anchors = (unsigned *)(myScratch + GD_SCRATCH_ANCHORS);
     sh.actors = (GdActor *)(gd_smem + p.offActors);
     sh.pal64 = (unsigned long long *)(gd_smem + GD_OFF_PAL64);
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
   unsigned short *vsec = (unsigned short *)(myScratch + GD_SCRATCH_VSEC);
   GdRowProj *rowproj = (GdRowProj *)(myScratch + gd_scratch_rowproj(sc.W, sc.S));
   GdRow *rows = (GdRow *)(kChip ? gd_smem + p.offRows : tables + p.offRows);
-  GdRow *fragRows = kChip ? rows + sc.W * 4 : p.fragRows + (size_t)blockIdx.x * sc.F * 4;
+  GdRow *fragRows = kChip ? rows + sc.W * 4 : (GdRow *)(p.frags + blockIdx.x * p.fragStride + gd_frag_wall_bytes(sc.F));
   float4 *prep = (float4 *)(kChip ? gd_smem + p.offPrep : tables + p.offPrep);
   GdPlane *planes = (GdPlane *)(kChip ? gd_smem + p.offPlanes : tables + p.offPlanes);
 

@@ -89,7 +89,9 @@ int gd_renderer_bind_decals(gd_renderer *r, const void *decals, int slots);
 /* Scratch the caller must provide to every render call: clip events of the
  * lanes being drawn plus, in its last 16 bytes, the kernel's lane queue.  Zero
  * the buffer once after allocating it; every launch leaves the queue at zero.
- * Launches that share a scratch buffer must not overlap on the device. */
+ * Launches that share a scratch buffer must not overlap on the device; launches
+ * of one renderer with a scratch buffer each may, unless decals are bound (their
+ * projections are the renderer's own scratch). */
 size_t gd_renderer_scratch_bytes(const gd_renderer *r);
 /* Launch shape, for reports: persistent CTAs and dynamic shared memory per CTA. */
 int gd_renderer_ctas(const gd_renderer *r);
