@@ -33,94 +33,21 @@ struct gd_renderer {
   int decalSlots;
   uint8_t *decalScratch;
   size_t decalScratchBytes;
-  GdSide *sides;             /* 2 W crossing records, the line of every fragment */
-  int *fragLine;
   size_t fragBytes;          /* a CTA's records of split lines: behind its scratch; F is not bounded, so */
   uint8_t *staticFrags;      /* those of the built-in array's CTAs are allocated with the renderer */
+  size_t sidesOffset;        /* crossing records of maps whose tables are not on chip: behind the CTAs' scratch */
 };
 
-/* Crossing records of the scene, once per renderer.  Texture indices are passed on as they are (the checked build
- * tests them where they are drawn); sectors out of range count as absent. */
-__global__ void gd_side_setup_kernel(GdScene sc, GdSide *sides, int *fragLine) {
+/* The crossing records of a map that reads them from scratch, before every draw of it (the others build theirs on
+ * chip): a few microseconds beside draws of milliseconds, and the renderer keeps nothing of the blob's. */
+__global__ void gd_side_setup_kernel(const __grid_constant__ GdScene sc, GdSide *sides) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= sc.W * 2) return;
-  const int w = i >> 1, side = i & 1;
-  if (side == 0 && sc.F > 0)
-    for (int f = sc.fragOff[w]; f < sc.fragOff[w + 1] && f < sc.F; ++f)
-      if (f >= 0) fragLine[f] = w;
-  int here = sc.wsec[i], there = sc.wsec[i ^ 1];
-  if (here < 0 || here >= sc.S) here = 0;
-  if (there < -1 || there >= sc.S) there = -1;
-  const bool oneSided = there < 0;
-  const int other = oneSided ? 0 : there;
-  const float vf = sc.secF[here * 2], vc = sc.secF[here * 2 + 1], of = sc.secF[other * 2], oc = sc.secF[other * 2 + 1];
-  const int4 ri = *reinterpret_cast<const int4 *>(&sc.secI[here * 4]), oi = *reinterpret_cast<const int4 *>(&sc.secI[other * 4]);
-  const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
-  const bool horizontal = fabsf(wl.w - wl.y) < 1e-6f, vertical = fabsf(wl.z - wl.x) < 1e-6f;
-  GdSide o;
-  for (int k = 0; k < 3; ++k) o.tex[k] = sc.sideTex[i * 3 + k];
-  o.contrast = vertical ? 16 : (horizontal ? -16 : 0);
-  o.tox = gd_rint(sc.sideOff[i * 2] * 65536.0f);
-  o.yoff = sc.sideOff[i * 2 + 1];
-  o.repeat = gd_rint(sc.wlen[w] * 65536.0f);
-  o.pad = 0;
-  unsigned f = GD_C_RASTER | GD_C_VALID;
-  const bool lightDiff = ri.x != oi.x;
-  if (oneSided || vc != oc || ri.z != oi.z || lightDiff) f |= GD_C_MARK_CEIL;
-  if (oneSided || vf != of || ri.y != oi.y || lightDiff) f |= GD_C_MARK_FLOOR;
-  if (oneSided) {
-    f |= GD_C_ONE_SIDED | (o.tex[0] >= 0 ? GD_C_TIER0 : 0u);
-  } else {
-    if (vf < of) f |= GD_C_LOWER | (o.tex[1] >= 0 ? GD_C_TIER1 : 0u);
-    if (vc > oc) f |= GD_C_UPPER | (o.tex[2] >= 0 ? GD_C_TIER2 : 0u);
-    if (vf > of) f |= GD_C_FLOOR_ABOVE;
-    if (vc < oc) f |= GD_C_CEIL_BELOW;
-  }
-  o.flags = f;
-  sides[i] = o;
+  if (i < sc.W * 2) gd_side_setup(sc, i, sides[i]);
 }
 
-/* The cells of the map: one block, whose threads first agree on the area that the sectors' boxes cover, then fill a
- * cell each.  A cell lists a sector when the box outside of which gd_point_in_sector says no, grown by a unit for
- * rounding, reaches it; a sector whose edges are not closed may also contain points left of its box. */
-__global__ void __launch_bounds__(GD_CELLS * GD_CELLS) gd_cells_kernel(GdScene sc, GdCells *cells) {
-  __shared__ float low[2][32], high[2][32];
-  const int t = threadIdx.x;
-  float x0 = CUDART_INF_F, x1 = -CUDART_INF_F, y0 = CUDART_INF_F, y1 = -CUDART_INF_F;
-  for (int s = t; s < sc.S; s += GD_CELLS * GD_CELLS) {
-    const float4 bb = *reinterpret_cast<const float4 *>(&sc.secBBox[s * 4]);
-    x0 = fminf(x0, bb.x); x1 = fmaxf(x1, bb.y); y0 = fminf(y0, bb.z); y1 = fmaxf(y1, bb.w);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o)); x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-    y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o)); y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-  }
-  if ((t & 31) == 0) { low[0][t >> 5] = x0; high[0][t >> 5] = x1; low[1][t >> 5] = y0; high[1][t >> 5] = y1; }
-  __syncthreads();
-  for (int k = 0; k < GD_CELLS * GD_CELLS / 32; ++k) {
-    x0 = fminf(x0, low[0][k]); x1 = fmaxf(x1, high[0][k]); y0 = fminf(y0, low[1][k]); y1 = fmaxf(y1, high[1][k]);
-  }
-  /* coordinates that are not finite, or so large that a unit is lost in them: every list counts as too long */
-  const bool usable = fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(y0), fabsf(y1))) < 100000.0f;
-  const float perX = (float)GD_CELLS / fmaxf(x1 - x0, 1.0f), perY = (float)GD_CELLS / fmaxf(y1 - y0, 1.0f);
-  bool closed = true;
-  for (int s = t; s < sc.S; s += GD_CELLS * GD_CELLS) closed = closed && sc.secI[s * 4 + 3] != 0;
-  closed = __syncthreads_and(closed);
-  if (t == 0) { cells->xLo = closed ? x0 - 1.0f : -CUDART_INF_F; cells->xHi = x1 + 1.0f; cells->yLo = y0; cells->yHi = y1; }
-  if (t == 0) { cells->x0 = usable ? x0 : 0.0f; cells->y0 = usable ? y0 : 0.0f; cells->perX = usable ? perX : 0.0f; cells->perY = usable ? perY : 0.0f; }
-  const int cx = t % GD_CELLS, cy = t / GD_CELLS;
-  int n = usable ? 0 : 255;
-  for (int s = 0; s < sc.S && n <= GD_CELL_SECTORS; ++s) {
-    const float4 bb = *reinterpret_cast<const float4 *>(&sc.secBBox[s * 4]);
-    const bool open = sc.secI[s * 4 + 3] == 0;
-    const int left = open ? 0 : gd_cell_axis(bb.x - 2.0f, x0, perX), right = gd_cell_axis(bb.y + 2.0f, x0, perX);
-    const int bottom = gd_cell_axis(bb.z - 1.0f, y0, perY), top = gd_cell_axis(bb.w + 1.0f, y0, perY);
-    if (cx < left || cx > right || cy < bottom || cy > top) continue;
-    if (n < GD_CELL_SECTORS) cells->cell[t][1 + n] = (unsigned short)s;
-    ++n;
-  }
-  cells->cell[t][0] = (unsigned short)(n <= GD_CELL_SECTORS ? n : 255);
-}
+/* for blobs without GD_S_CELLS: every list is too long, no point lies past the map */
+#define GD_FLOAT_INF __builtin_huge_valf()
+static __device__ const GdCells gd_no_cells = {0.0f, 0.0f, 0.0f, 0.0f, -GD_FLOAT_INF, GD_FLOAT_INF, -GD_FLOAT_INF, GD_FLOAT_INF, {{255}}};
 
 static const void *gd_section(const uint8_t *dev, const int32_t *h, int s) { return dev + h[GD_HDR_SECTION0 + s]; }
 
@@ -209,7 +136,7 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
   r->copyStream = nullptr;
   r->copiesDone = nullptr;
   r->decalScratch = nullptr;
-  r->staticFrags = nullptr; r->fragBytes = 0; r->sides = nullptr; r->fragLine = nullptr;
+  r->staticFrags = nullptr; r->fragBytes = 0;
   for (int c = 0; c < GD_HOST_CHUNKS; ++c) r->chunkDone[c] = nullptr;
   memcpy(r->header, h, sizeof r->header);
   r->device = device;
@@ -260,6 +187,7 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
   sc.decalAtlas = SECP(uint8_t, GD_S_DECAL_ATLAS); sc.decalOpacity = SECP(uint8_t, GD_S_DECAL_OPACITY);
   sc.decalBlack = SECP(uint8_t, GD_S_DECAL_BLACK);
   sc.F = h[GD_H_FRAGMENTS]; sc.fragOff = SECP(int32_t, GD_S_FRAG_OFF); sc.fragFixed = SECP(int32_t, GD_S_FRAG_FIXED);
+  sc.cells = SECP(GdCells, GD_S_CELLS);
   r->decals = nullptr; r->decalSlots = 0; r->decalScratch = nullptr; r->decalScratchBytes = 0;
 #undef SECP
   const int secWallsN = h[GD_H_SEC_WALLS_N];
@@ -290,30 +218,22 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
     else
       r->ctas = sms * perSm;  /* one persistent CTA per resident slot */
   }
-  if (rc == GD_OK) {
-    void *sides = nullptr, *mem = nullptr;
-    const size_t sideBytes = (size_t)sc.W * 2 * sizeof(GdSide);
-    const size_t lineBytes = gd_align16((size_t)sc.F * 4);
-    if (cudaMalloc(&sides, sideBytes + lineBytes + sizeof(GdCells)) != cudaSuccess) rc = GD_ERR_CUDA;
-    r->sides = (GdSide *)sides;
-    sc.cells = (GdCells *)((uint8_t *)sides + sideBytes + lineBytes);
-    r->fragLine = (int *)((uint8_t *)sides + sideBytes);
-    if (sc.F > 0) r->fragBytes = gd_frag_bytes(sc.F, r->chip);
-    if (rc == GD_OK && sc.F > 0 && gd_fits_static(sc)) {
-      if (cudaMalloc(&mem, GD_STATIC_MAX_CTAS * r->fragBytes) != cudaSuccess) rc = GD_ERR_CUDA;
-      r->staticFrags = (uint8_t *)mem;
-    }
-    if (rc == GD_OK) {
-      gd_side_setup_kernel<<<(sc.W * 2 + 127) / 128, 128>>>(sc, r->sides, r->fragLine);
-      gd_cells_kernel<<<1, GD_CELLS * GD_CELLS>>>(sc, (GdCells *)sc.cells);
-      if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) rc = GD_ERR_CUDA;
-    }
+  if (sc.F > 0) r->fragBytes = gd_frag_bytes(sc.F, r->chip);
+  if (rc == GD_OK && sc.F > 0 && gd_fits_static(sc)) {
+    void *mem = nullptr;
+    if (cudaMalloc(&mem, GD_STATIC_MAX_CTAS * r->fragBytes) != cudaSuccess) rc = GD_ERR_CUDA;
+    r->staticFrags = (uint8_t *)mem;
+  }
+  if (rc == GD_OK && h[GD_HDR_SECTION0 + GD_S_CELLS] == 0) {
+    void *address = nullptr;
+    if (cudaGetSymbolAddress(&address, gd_no_cells) != cudaSuccess) rc = GD_ERR_CUDA;
+    sc.cells = (const GdCells *)address;
   }
   r->base.maxThings = max_things;
-  r->base.sides = r->sides; r->base.fragLine = r->fragLine;
   r->base.secWallsN = secWallsN;
   r->base.perCta = r->base.fragStride = gd_scratch_per_cta(sc.W, sc.S) + r->fragBytes;
-  r->base.queueOffset = (size_t)r->ctas * r->base.perCta;
+  r->sidesOffset = (size_t)r->ctas * r->base.perCta;
+  r->base.queueOffset = r->sidesOffset + (r->chip ? 0 : (size_t)sc.W * 2 * sizeof(GdSide));
   r->copyStream = nullptr;
   r->copiesDone = nullptr;
   for (int c = 0; c < GD_HOST_CHUNKS; ++c) r->chunkDone[c] = nullptr;
@@ -340,7 +260,6 @@ extern "C" void gd_renderer_destroy(gd_renderer *r) {
   if (r->copyStream) cudaStreamDestroy(r->copyStream);
   if (r->decalScratch) cudaFree(r->decalScratch);
   if (r->staticFrags) cudaFree(r->staticFrags);
-  if (r->sides) cudaFree(r->sides);
   if (switched) cudaSetDevice(prev);
   delete r;
 }
@@ -367,12 +286,18 @@ extern "C" int gd_renderer_bind_decals(gd_renderer *r, const void *decals, int s
 }
 
 extern "C" size_t gd_renderer_scratch_bytes(const gd_renderer *r) {
-  return r ? (size_t)r->ctas * r->base.perCta + 16 : 0;
+  return r ? r->base.queueOffset + 16 : 0;
 }
 
 extern "C" int gd_renderer_ctas(const gd_renderer *r) { return r ? r->ctas : 0; }
 extern "C" size_t gd_renderer_shared_bytes(const gd_renderer *r) { return r ? r->smemBytes : 0; }
 extern "C" size_t gd_renderer_shared_bytes_view(const gd_renderer *r) { return r ? r->smemBytes : 0; }
+
+static int gd_draw(const gd_renderer *r, const GdParams &p, int grid, void *stream) {
+  if (!r->chip) gd_side_setup_kernel<<<(p.sc.W * 2 + 127) / 128, 128, 0, (cudaStream_t)stream>>>(p.sc, p.sides);
+  gd_kernel_for(r)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
+  return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
+}
 
 static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing *things, int n, int flags,
                      uint8_t *stack, const uint8_t *reset_mask, uint8_t *obs_out, uint8_t *indexed_out,
@@ -393,11 +318,10 @@ static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing 
   p.lanes = lanes; p.things = things; p.n = n; p.flags = flags;
   p.stack = stack; p.ringHead = ring_head; p.resetMask = reset_mask; p.obsOut = obs_out; p.indexedOut = indexed_out; p.rgbOut = rgb_out;
   p.scratch = (uint8_t *)scratch; p.status = status;
+  p.sides = (GdSide *)(p.scratch + r->sidesOffset);
   p.frags = p.scratch + gd_scratch_per_cta(r->base.sc.W, r->base.sc.S);
   p.decals = r->decals; p.decalSlots = r->decalSlots; p.decalScratch = r->decalScratch;
-  int grid = n < r->ctas ? n : r->ctas;
-  gd_kernel_for(r)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
+  return gd_draw(r, p, n < r->ctas ? n : r->ctas, stream);
 }
 
 extern "C" int gd_render_step(const gd_renderer *r, const int32_t *lanes, const void *things, int n, int mask_hud,
@@ -549,7 +473,9 @@ extern "C" int gd_render_step_host(const gd_renderer *r, const int32_t *lanes_ho
 /* a scene of W walls has fewer than W sectors (three walls bound a sector, a wall bounds two) */
 #define GD_STATIC_PER_CTA ((GD_SCRATCH_FIXED + GD_STATIC_MAX_WALLS * (2 * GD_PLANE_ENTRY_BYTES + 2 * GD_PLANE_BYTES + \
                             sizeof(GdWall) + 4 * sizeof(GdRowProj) + 4 * sizeof(GdRow) + 16) + 127) & ~(size_t)63)
-#define GD_STATIC_SCRATCH_BYTES (GD_STATIC_MAX_CTAS * GD_STATIC_PER_CTA + 16)
+#define GD_STATIC_SIDES (GD_STATIC_MAX_CTAS * GD_STATIC_PER_CTA)
+#define GD_STATIC_QUEUE (GD_STATIC_SIDES + GD_STATIC_MAX_WALLS * 2 * sizeof(GdSide))
+#define GD_STATIC_SCRATCH_BYTES (GD_STATIC_QUEUE + 16)
 #define GD_STATIC_MAX_DEVICES 64
 
 static __device__ __align__(256) unsigned char gd_static_scratch[GD_STATIC_SCRATCH_BYTES];
@@ -595,12 +521,12 @@ extern "C" int gd_render_step_static(const gd_renderer *r, const int32_t *lanes,
   p.frags = r->staticFrags; p.fragStride = r->fragBytes;
   /* lane queue: the last 16 bytes of the array; zero when the library is
    * loaded and left at zero by every launch */
-  p.queueOffset = (size_t)GD_STATIC_MAX_CTAS * GD_STATIC_PER_CTA;
+  p.queueOffset = GD_STATIC_QUEUE;
+  p.sides = (GdSide *)(scratch + GD_STATIC_SIDES);
   p.decals = r->decals; p.decalSlots = r->decalSlots; p.decalScratch = r->decalScratch;
   int grid = n < r->ctas ? n : r->ctas;
   if (grid > GD_STATIC_MAX_CTAS) grid = GD_STATIC_MAX_CTAS;
-  gd_kernel_for(r)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
+  return gd_draw(r, p, grid, stream);
 }
 
 /* ---- diagnostic: the device's float32 libm on caller-given arguments -------------------- */

@@ -80,7 +80,7 @@ struct GdScene {
   /* projection fragments of the lines a node builder split: total count, CSR per line, 16.16 endpoints */
   int F;
   const int32_t *fragOff, *fragFixed;
-  const GdCells *cells;         /* the sectors that may hold a point, by where it lies (built with the renderer) */
+  const GdCells *cells;         /* the sectors that may hold a point, by where it lies */
   /* bullet-chip decals: variants (0 = none), atlas slice height / width */
   int decals, decalH, decalW;
   const int32_t *decalInfo, *wallFine;
@@ -221,8 +221,8 @@ struct __align__(16) GdHot {
 #define GD_HOT_BRIDGE1 (1u << 25)
 #define GD_HOT_STATIC (GD_HOT_SPLIT | GD_HOT_NEIGHBOUR | GD_HOT_BRIDGE0 | GD_HOT_BRIDGE1)
 
-/* Everything of a crossing that depends on the wall and the side it is seen from alone; built once per
- * scene.  The flags assume that the sectors of the crossing are the wall's own two. */
+/* Everything of a crossing that depends on the wall and the side it is seen from alone; built by every
+ * launch.  The flags assume that the sectors of the crossing are the wall's own two. */
 struct __align__(16) GdSide {
   int tex[3];                     /* middle, lower, upper texture, -1: none */
   int contrast;                   /* fake contrast: +16 vertical, -16 horizontal */

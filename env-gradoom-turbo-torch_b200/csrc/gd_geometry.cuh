@@ -105,6 +105,43 @@ __device__ __noinline__ void gd_project_fixed(const GdView &v, const i64 fx[2], 
   }
 }
 
+/* Crossing record of side i & 1 of wall i >> 1.  Texture indices are passed on as they are (the checked build tests
+ * them where they are drawn); sectors out of range count as absent.  Inline: as a function of its own it moves the
+ * walk's functions to addresses that cost 4096 lanes of the 64-sector map 3.46 instead of 3.40 ms. */
+__device__ __forceinline__ void gd_side_setup(const GdScene &sc, int i, GdSide &out) {
+  const int w = i >> 1;
+  int here = sc.wsec[i], there = sc.wsec[i ^ 1];
+  if (here < 0 || here >= sc.S) here = 0;
+  if (there < -1 || there >= sc.S) there = -1;
+  const bool oneSided = there < 0;
+  const int other = oneSided ? 0 : there;
+  const float vf = sc.secF[here * 2], vc = sc.secF[here * 2 + 1], of = sc.secF[other * 2], oc = sc.secF[other * 2 + 1];
+  const int4 ri = *reinterpret_cast<const int4 *>(&sc.secI[here * 4]), oi = *reinterpret_cast<const int4 *>(&sc.secI[other * 4]);
+  const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
+  const bool horizontal = fabsf(wl.w - wl.y) < 1e-6f, vertical = fabsf(wl.z - wl.x) < 1e-6f;
+  GdSide o;
+  for (int k = 0; k < 3; ++k) o.tex[k] = sc.sideTex[i * 3 + k];
+  o.contrast = vertical ? 16 : (horizontal ? -16 : 0);
+  o.tox = gd_rint(sc.sideOff[i * 2] * 65536.0f);
+  o.yoff = sc.sideOff[i * 2 + 1];
+  o.repeat = gd_rint(sc.wlen[w] * 65536.0f);
+  o.pad = 0;
+  unsigned f = GD_C_RASTER | GD_C_VALID;
+  const bool lightDiff = ri.x != oi.x;
+  if (oneSided || vc != oc || ri.z != oi.z || lightDiff) f |= GD_C_MARK_CEIL;
+  if (oneSided || vf != of || ri.y != oi.y || lightDiff) f |= GD_C_MARK_FLOOR;
+  if (oneSided) {
+    f |= GD_C_ONE_SIDED | (o.tex[0] >= 0 ? GD_C_TIER0 : 0u);
+  } else {
+    if (vf < of) f |= GD_C_LOWER | (o.tex[1] >= 0 ? GD_C_TIER1 : 0u);
+    if (vc > oc) f |= GD_C_UPPER | (o.tex[2] >= 0 ? GD_C_TIER2 : 0u);
+    if (vf > of) f |= GD_C_FLOOR_ABOVE;
+    if (vc < oc) f |= GD_C_CEIL_BELOW;
+  }
+  o.flags = f;
+  out = o;
+}
+
 /* Project wall w of the map for this lane (engine.py:10747-10869, 11207-11302,
  * 11359-11427), and the lane-dependent operands of its column-ray test.  The
  * ray-owned span is completed by gd_wall_spans below. */

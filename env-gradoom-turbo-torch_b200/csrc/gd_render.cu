@@ -64,8 +64,7 @@ struct GdParams {
   uint8_t *rgbOut;           /* n x 240 x 320 x 3, optional */
   uint8_t *scratch;          /* ctas x gd_scratch_per_cta(W), then the lane queue (2 words, zero between launches) */
   size_t queueOffset, perCta;
-  const GdSide *sides;       /* 2 W crossing records (built with the renderer) */
-  const int *fragLine;       /* F: the line of each projection fragment */
+  GdSide *sides;             /* 2 W crossing records of maps whose tables are not on chip, in the launch's scratch */
   /* byte offsets in shared memory; those of the last four are offsets into the CTA's scratch tables when
    * they do not fit on chip (kChip false) */
   int offSectors, offSecOff, offSecWalls, offVtx, offFrags, offActors;
@@ -75,8 +74,8 @@ struct GdParams {
   const gd_decal *decals;    /* n x decalSlots rings of bullet chips, or null */
   int decalSlots;
   uint8_t *decalScratch;     /* ctas x gd_decal_scratch_per_cta(decalSlots) */
-  /* scenes with split lines: a CTA's F fragment records, then their F x 4 row projections when those are not on
-   * chip; in the launch's own scratch like all that a CTA writes, so that launches of one renderer may overlap */
+  /* scenes with split lines: a CTA's F fragment records, the line of each, then their F x 4 row projections when
+   * those are not on chip; in the launch's own scratch like all that a CTA writes, so that launches of one renderer may overlap */
   uint8_t *frags;
   size_t fragStride;         /* from CTA to CTA */
 };
@@ -102,7 +101,8 @@ __host__ __device__ inline size_t gd_table_bytes(int W, int S) {
 }
 __host__ __device__ inline size_t gd_scratch_per_cta(int W, int S) { return gd_scratch_tables(W, S) + gd_table_bytes(W, S); }
 __host__ __device__ inline size_t gd_frag_wall_bytes(int F) { return gd_align16((size_t)F * sizeof(GdWall)); }
-inline size_t gd_frag_bytes(int F, bool chip) { return gd_frag_wall_bytes(F) + (chip ? 0 : (size_t)F * 4 * sizeof(GdRow)); }
+__host__ __device__ inline size_t gd_frag_rows(int F) { return gd_frag_wall_bytes(F) + gd_align16((size_t)F * 4); }
+inline size_t gd_frag_bytes(int F, bool chip) { return gd_frag_rows(F) + (chip ? 0 : (size_t)F * 4 * sizeof(GdRow)); }
 
 struct GdActor {
   float x, y, depth;
@@ -244,15 +244,20 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
   for (int i = tid; i < p.secWallsN; i += GD_THREADS)
     ((unsigned short *)(gd_smem + p.offSecWalls))[i] = (unsigned short)GD_CHECK_INDEX(sc.secWalls[i], sc.W);
   if (kChip)
-    for (int i = tid; i < sc.W * 2 * (int)(sizeof(GdSide) / 16); i += GD_THREADS)
-      ((uint4 *)(gd_smem + p.offSides))[i] = ((const uint4 *)p.sides)[i];
+#pragma unroll 1
+    for (int i = tid; i < sc.W * 2; i += GD_THREADS) gd_side_setup(sc, i, ((GdSide *)(gd_smem + p.offSides))[i]);
+  int *fragLine = (int *)(p.frags + blockIdx.x * p.fragStride + gd_frag_wall_bytes(sc.F));
+  if (kSplit)
+#pragma unroll 1
+    for (int w = tid; w < sc.W; w += GD_THREADS)
+      for (int f = max(sc.fragOff[w], 0); f < min(sc.fragOff[w + 1], sc.F); ++f) fragLine[f] = w;
   bool paletteBlended = false;    /* CTA-uniform: the shared palette holds a lane's screen-flash blend */
   GdEvent *events = (GdEvent *)myScratch;
   int *eventCount = (int *)(myScratch + GD_SCRATCH_EVENTS_BYTES);
   unsigned short *vsec = (unsigned short *)(myScratch + GD_SCRATCH_VSEC);
   GdRowProj *rowproj = (GdRowProj *)(myScratch + gd_scratch_rowproj(sc.W, sc.S));
   GdRow *rows = (GdRow *)(kChip ? gd_smem + p.offRows : tables + p.offRows);
-  GdRow *fragRows = kChip ? rows + sc.W * 4 : (GdRow *)(p.frags + blockIdx.x * p.fragStride + gd_frag_wall_bytes(sc.F));
+  GdRow *fragRows = kChip ? rows + sc.W * 4 : (GdRow *)(p.frags + blockIdx.x * p.fragStride + gd_frag_rows(sc.F));
   float4 *prep = (float4 *)(kChip ? gd_smem + p.offPrep : tables + p.offPrep);
   GdPlane *planes = (GdPlane *)(kChip ? gd_smem + p.offPlanes : tables + p.offPlanes);
 
@@ -366,7 +371,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       const bool piece = kSplit && idx >= frustumListed * 4;
       const int f = piece ? (idx - frustumListed * 4) >> 2 : 0, slot = idx & 3;
       if (piece && ((const unsigned *)(gd_smem + p.offFrags))[f] == 0u) continue;
-      const int w = piece ? p.fragLine[f] : frustumList[idx >> 2];
+      const int w = piece ? fragLine[f] : frustumList[idx >> 2];
       const GdWall &q = piece ? sh.frags[f] : sh.walls[w];
       const int sector = gd_wsec(sc, w * 2 + (slot >> 1)), sd = slot >> 1;
       GdRow row;

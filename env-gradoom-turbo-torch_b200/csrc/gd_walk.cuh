@@ -838,7 +838,7 @@ __device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, co
   float rx, ry;
   gd_ray(v, x, rx, ry);
   const GdRow *rows = (const GdRow *)(kChip ? gd_smem + p.offRows : tables + p.offRows);
-  const GdRow *fragRows = kChip ? rows + p.sc.W * 4 : (const GdRow *)(p.frags + blockIdx.x * p.fragStride + gd_frag_wall_bytes(p.sc.F));
+  const GdRow *fragRows = kChip ? rows + p.sc.W * 4 : (const GdRow *)(p.frags + blockIdx.x * p.fragStride + gd_frag_rows(p.sc.F));
   const float4 *prep = (const float4 *)(kChip ? gd_smem + p.offPrep : tables + p.offPrep);
   const GdPlane *planes = (const GdPlane *)(kChip ? gd_smem + p.offPlanes : tables + p.offPlanes);
   const GdSide *sides = kChip ? (const GdSide *)(gd_smem + p.offSides) : p.sides;

@@ -630,7 +630,7 @@ _SECTIONS = (
     "HUD_OPAQUE FINESINE FINETAN STARTS RAY_OFFSETS RAY_COSCORR TEX_ATLAS_COL SECTOR_BBOX "
     "MASKED_WALLS DAMAGE_ALPHA FLOOR_GROUP_H FLOOR_GROUP_OFF FLOOR_GROUP_SEC CEIL_GROUP_H CEIL_GROUP_OFF "
     "CEIL_GROUP_SEC ITEM_POS ITEM_INFO ITEM_ANIM DECAL_INFO DECAL_ATLAS DECAL_OPACITY DECAL_BLACK WALL_FINE "
-    "FRAG_OFF FRAG_FIXED"
+    "FRAG_OFF FRAG_FIXED CELLS"
 ).split()
 SEC = {name: i for i, name in enumerate(_SECTIONS)}
 
@@ -723,6 +723,38 @@ def ray_tables():
     columns = torch.arange(320, dtype=torch.float32) - 320 / 2.0
     offsets = -torch.atan(columns / (320 / 2.0))
     return offsets.numpy().copy(), torch.cos(offsets).numpy().copy()
+
+
+def sector_cells(bbox: np.ndarray, closed: np.ndarray) -> np.ndarray:
+    """The ``CELLS`` section: the map's area in 32 x 32 cells, each with the sectors that may contain a point of it
+    (points outside belong to the nearest cell).  ``bbox (S,4) float32``: xmin xmax ymin ymax of the sectors' edges;
+    ``closed (S,)``: the edges form closed loops.  A sector is listed where its box reaches, grown by more than the
+    crossing test's rounding; one that is not closed may also contain points left of its box.  The cell of a
+    coordinate is taken in float32, in the order of operations that the kernel uses."""
+
+    grid, most = 32, 7
+    limits = np.zeros(8, dtype=np.float32)
+    x0, x1, y0, y1 = bbox[:, 0].min(), bbox[:, 1].max(), bbox[:, 2].min(), bbox[:, 3].max()
+    per_x, per_y = (np.float32(grid) / np.maximum(high - low, np.float32(1.0)) for low, high in ((x0, x1), (y0, y1)))
+    limits[4:] = x0 - 1.0 if closed.all() else -np.inf, x1 + 1.0, y0, y1
+    lists = np.zeros((grid, grid, 1 + most), dtype=np.uint16)
+    counts = np.zeros((grid, grid), dtype=np.int64)
+    # coordinates so large that a unit is lost in them, or not numbers: every list counts as too long
+    if np.abs([x0, x1, y0, y1]).max() < 100000.0:
+        limits[:4] = x0, y0, per_x, per_y
+        grown = bbox + np.asarray([-2.0, 2.0, -1.0, 1.0], dtype=np.float32)
+        origin, per = np.asarray([x0, x0, y0, y0]), np.asarray([per_x, per_x, per_y, per_y])
+        reach = np.clip(((grown - origin) * per).astype(np.int64), 0, grid - 1)
+        reach[~closed, 0] = 0
+        for s, (left, right, bottom, top) in enumerate(reach):
+            block = counts[bottom:top + 1, left:right + 1]
+            rows, cols = np.nonzero(block < most)
+            lists[bottom + rows, left + cols, 1 + block[rows, cols]] = s
+            block += 1
+    else:
+        counts[:] = 255
+    lists[..., 0] = np.where(counts <= most, counts, 255)
+    return np.concatenate((limits.view(np.uint8), lists.reshape(-1).view(np.uint8)))
 
 
 def pack_scene(scene: Scene, ray_table_override=None) -> np.ndarray:
@@ -999,6 +1031,7 @@ def pack_scene(scene: Scene, ray_table_override=None) -> np.ndarray:
         "DECAL_INFO": decal_info, "DECAL_ATLAS": decal_atlas, "DECAL_OPACITY": decal_opacity,
         "DECAL_BLACK": decal_black, "WALL_FINE": wall_fine_angles(walls),
         "FRAG_OFF": frag_off, "FRAG_FIXED": frag_fixed,
+        "CELLS": sector_cells(bbox, sector_i[:, 3] != 0),
     }
     assert set(sections) == set(SEC), set(SEC) ^ set(sections)
 

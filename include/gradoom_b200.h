@@ -6,8 +6,10 @@
  * bar) and reduces it to the 84x84 grayscale policy observation, writing it
  * into the four-frame stack.  Every pointer below is a plain device or host
  * pointer; no framework types cross this boundary.  The caller owns all
- * memory: the library never allocates device memory and never blocks on the
- * host.  All device buffers must be 16-byte aligned.
+ * memory: the calls that draw, pack and step never allocate device memory and
+ * never block on the host (what a renderer itself may allocate is said at
+ * gd_renderer_create and gd_renderer_bind_decals).  All device buffers must be
+ * 16-byte aligned.
  *
  * Input formats (scene blob, lane records, thing records):
  * gradoom_b200_layout.h.
@@ -64,6 +66,11 @@ const char *gd_error_string(int code);
  * `blob_header_host` points at (at least) the first GD_HDR_WORDS*4 bytes of
  * the same blob in host memory.  `max_things` (<= 64) is the per-lane stride
  * of the thing array passed to the render calls.
+ * Of the device blob only the address is taken: nothing is launched, and its
+ * bytes have to be there when a call first draws from it.  A scene with split
+ * lines (GD_H_FRAGMENTS > 0) that gd_render_step_static can draw gets a block for
+ * that call's 32 CTAs, 172 bytes a fragment each at most; no other scene makes
+ * the creation allocate device memory.
  */
 int gd_renderer_create(const void *blob_header_host, const void *blob_dev, size_t blob_bytes, int device,
                        int max_things, gd_renderer **out);

@@ -150,6 +150,11 @@ enum gd_section {
   GD_S_FRAG_OFF,        /* W+1 i32 CSR into GD_S_FRAG_FIXED; a line that was not split has an empty range */
   GD_S_FRAG_FIXED,      /* fragments x 4 i32: x1 y1 x2 y2 in 16.16, the pieces of a split line in the node
                            builder's order (src/gradoom/scenario.py:420-455, engine.py:745-767) */
+  GD_S_CELLS,           /* the map's area in 32 x 32 cells with the sectors that may contain a point of each, for the
+                           point searches: 8 f32 (x0, y0, cells per unit in x and y; no sector contains a point with
+                           x < xlo, x > xhi, y < ylo or y >= yhi: xlo xhi ylo yhi), then 1024 x 8 u16, row by row:
+                           count (255: more than seven) and up to seven sectors, ascending.  Offset 0: not in the blob,
+                           every sector is tested */
   GD_S_COUNT
 };
 
