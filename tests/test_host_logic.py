@@ -339,7 +339,7 @@ def test_lane_stepper_rules_that_were_overridden_are_used(rule, where, pkg, scen
 
 
 @pytest.mark.parametrize("rows,cols,room,diagonals,opened", [
-    (1, 1, 512.0, False, 0), (2, 200, 96.0, False, 0), (16, 16, 128.0, True, 0), (5, 3, 96.0, True, 4)])
+    (1, 1, 512.0, False, 0), (2, 240, 96.0, False, 0), (16, 16, 128.0, True, 0), (5, 3, 96.0, True, 4)])
 def test_cells_list_every_sector_that_contains_a_point(rows, cols, room, diagonals, opened, pkg):
     from gradoom_b200 import scene as gdscene
 
@@ -354,7 +354,7 @@ def test_cells_list_every_sector_that_contains_a_point(rows, cols, room, diagona
     at = int(blob[:gdscene.GD_HDR_WORDS * 4].view(np.int32)[gdscene.GD_HDR_SECTION0 + gdscene.SEC["CELLS"]])
     x0, y0, per_x, per_y, x_low, x_high, y_low, y_high = blob[at:at + 32].view(np.float32)
     lists = blob[at + 32:at + 32 + 1024 * 16].view(np.uint16).reshape(32, 32, 8)
-    wide, high, n = cols * room, rows * room, 800
+    wide, high, n = cols * room, rows * room, 300
     x = np.concatenate((rng.uniform(-200, wide + 200, n), rng.integers(0, cols + 1, n) * room, rng.uniform(-200, wide + 200, n)))
     y = np.concatenate((rng.uniform(-200, high + 200, n), rng.uniform(-9, high + 9, n), rng.integers(0, rows + 1, n) * room))
     x, y = x.astype(np.float32), y.astype(np.float32)
@@ -366,7 +366,7 @@ def test_cells_list_every_sector_that_contains_a_point(rows, cols, room, diagona
     count = cell[:, 0]
     listed = ((cell[:, 1:] == sector[:, None]) & (np.arange(7) < count[:, None])).any(axis=1)
     assert (listed | (count == 255) | (sector < 0)).all()
-    assert (sector >= 0).sum() > n and ((count <= 7) & (sector >= 0)).any() == (cols != 200)
+    assert (sector >= 0).sum() > n and ((count <= 7) & (sector >= 0)).any() == (cols != 240)
     beyond = (x > x_high) | (x < x_low) | (y >= y_high) | (y < y_low)
     assert beyond.any() and (sector[beyond] < 0).all()
     assert np.isneginf(x_low) == bool(opened)
