@@ -103,10 +103,10 @@ __device__ __noinline__ void gd_decals(const GdScene &sc_, const GdView &v_, con
   const int n = *count;
   if (n == 0) return;                                /* block-uniform */
   /* ---- oldest first (engine.py:13763-13775); the ranked list and every chip's column span go to
-   * shared memory (the hit cache is idle here), so a column rejects the chips beside it cheaply ---- */
+   * shared memory (both aux areas are idle here), so a column rejects the chips beside it cheaply ---- */
   short *ranked = (short *)sh.hitD;                  /* GD_MAX_DECAL_SLOTS x 2 bytes */
   unsigned *spans = (unsigned *)sh.hitA;             /* GD_MAX_DECAL_SLOTS x 4 bytes: first column | end column << 16 */
-  static_assert(GD_MAX_DECAL_SLOTS * 4 <= 8 * GD_SW * 4, "the chip list fits the hit cache");
+  static_assert(GD_MAX_DECAL_SLOTS * 2 <= GD_AUX_BYTES && GD_MAX_DECAL_SLOTS * 4 <= GD_AUX2_BYTES, "the chip list and its spans");
 #pragma unroll 1
   for (int i = tid; i < n; i += GD_THREADS) {
     const int si = proj[i].serial, li = proj[i].slotStyle & 1023;
@@ -209,7 +209,7 @@ __device__ __noinline__ void gd_decals(const GdScene &sc_, const GdView &v_, con
       *px = sc.decalBlack[min((int)opacityRow[src], 64) * 256 + *px];   /* the table has 65 rows */
     }
   }
-  __syncthreads();                                   /* the chip list leaves the hit cache to the sprite pass */
+  __syncthreads();                                   /* the chip list leaves the aux areas to the sprite pass */
 }
 
 #endif

@@ -138,8 +138,11 @@ struct GdActor {
                                                               chip ranks, 84 x 84 result */
 #define GD_AUX_BYTES (8 * 320 * 4)
 #define GD_OFF_AUX2 (GD_OFF_AUX + GD_AUX_BYTES)            /* 4,096: sectors of points, status-bar list, sprite columns, chip spans */
-#define GD_OFF_HOT (GD_OFF_AUX2 + 4096)                    /* W wall records */
-static_assert(GD_OFF_HOT % 16 == 0 && GD_OFF_AUX % 16 == 0, "vector loads");
+#define GD_AUX2_BYTES 4096
+#define GD_OFF_HOT (GD_OFF_AUX2 + GD_AUX2_BYTES)           /* W wall records */
+static_assert(GD_OFF_HOT % 16 == 0 && GD_OFF_AUX % 16 == 0 && GD_OFF_AUX2 % 16 == 0, "vector loads");
+static_assert(GD_OBS * GD_OBS <= GD_AUX_BYTES && 65 * 4 <= GD_AUX2_BYTES && GD_SW * 2 <= GD_AUX2_BYTES,
+              "the result; the sectors of 64 things and the player, the sprite columns");
 
 struct GdPlaneEntry;
 
@@ -417,7 +420,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     if (p.flags & GD_F_DRAW_HUD) gd_hud_column(sc, (const int4 *)sh.hitA, frame + GD_VH * GD_SW);
     __syncthreads();
     /* Rows no seg ever claimed show the per-pixel flat fallback.  They are
-     * queued (the hit cache is free once every column has finished its walk)
+     * queued (the first aux area is free once every column has finished its walk)
      * and resolved; a frame with more such pixels than the queue holds takes
      * several rounds, each pass marking what it drew as owned. */
     bool sweepDone = false;                          /* CTA-uniform */

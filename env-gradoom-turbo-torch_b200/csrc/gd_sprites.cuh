@@ -283,6 +283,7 @@ __device__ void gd_weapon(const GdScene &sc_, const int32_t *lane, uint8_t *fram
  * so the list is made beside the other setup, and a warp draws its columns when its walk has ended, while others
  * still walk. */
 #define GD_HUD_PATCHES 44      /* bar, arms panel, 3 + 3 + 1 + 3 + 1 large glyphs, face, 6 weapons, 4 x 6 small digits */
+static_assert(GD_HUD_PATCHES * 16 <= GD_AUX2_BYTES, "the status-bar list");
 
 /* Place `slot` of a number drawn right-aligned at `right` (engine.py:15180-15210); patch -1: no digit there. */
 __device__ __forceinline__ int3 gd_hud_digit(const GdScene &sc, int value, int right, int y, bool small, int slot) {

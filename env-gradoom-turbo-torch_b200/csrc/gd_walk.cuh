@@ -715,6 +715,7 @@ __device__ __noinline__ void gd_masked_pass(const GdScene &sc_, const GdView &v_
 }
 
 #define GD_FALLBACK_MAX (8 * GD_SW)
+static_assert(GD_FALLBACK_MAX * 4 <= GD_AUX_BYTES, "the fallback queue");
 
 /* A column that has left the map (current sector -1) still takes part in the reference's
  * vectorised iterations: its decision is made against sector 0 with wall 0 selected at an
