@@ -122,28 +122,13 @@ __device__ __forceinline__ int gd_wsec(const GdScene &sc, int i) {
 /* The CTA's dynamic shared memory. */
 extern __shared__ __align__(16) uint8_t gd_smem[];
 
-/* Shared-memory accesses of the pixel loops by 32-bit shared-space address: the pointers of the shared-memory
- * map are generic (they are read from a structure), so the compiler would otherwise carry 64-bit addresses
- * and issue generic loads and stores.  The loads are for tables nothing writes while a lane is drawn. */
 __device__ __forceinline__ unsigned gd_shared_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-/* The same pointer, re-derived from the shared array itself: the compiler then knows its address space and
- * addresses everything reached through it with 32 bits and shared-space instructions. */
+/* The same pointer, re-derived from the shared array itself.  The pointers of the shared-memory map are generic (they
+ * are read from a structure); this way the compiler knows their address space and addresses everything reached through
+ * them with 32 bits and shared-space instructions. */
 template <class T>
 __device__ __forceinline__ T *gd_as_shared(T *p) {
   return (T *)(gd_smem + (int)(gd_shared_addr(p) - gd_shared_addr(gd_smem)));   /* static shared variables lie below */
-}
-__device__ __forceinline__ unsigned gd_lds8(unsigned addr) {
-  unsigned v;
-  asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ unsigned gd_lds32(unsigned addr) {
-  unsigned v;
-  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void gd_sts8(unsigned addr, unsigned v) {
-  asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ i64 gd_min(i64 a, i64 b) { return a < b ? a : b; }
 __device__ __forceinline__ i64 gd_max(i64 a, i64 b) { return a > b ? a : b; }
@@ -198,7 +183,6 @@ struct __align__(8) GdWall {
   i64 sl, sr;                         /* projected half-open span (unbounded when rejected) */
   i64 dl, dr;                         /* clipped endpoint depths, 20.12 */
   int tx[2], ty[2];                   /* view coordinates in stored endpoint order */
-  unsigned char frontF, oneSided;
 };
 
 /* What the column walk reads of a wall of the lane being drawn, kept in shared memory: the ray test's
@@ -246,7 +230,6 @@ struct __align__(16) GdSide {
 #define GD_C_FLOOR_ABOVE 512u     /* view floor above the other sector's */
 #define GD_C_CEIL_BELOW 1024u     /* view ceiling below the other sector's */
 #define GD_C_PORTAL 2048u         /* a portal behind a projected solid contributes its clips */
-#define GD_C_VALID 4096u
 
 /* One clip event of a column: what a drawn seg contributes to sprite clipping
  * and to visplane ownership. Rows are 0..208 and fit a byte. */

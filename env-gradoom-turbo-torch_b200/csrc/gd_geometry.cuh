@@ -126,7 +126,7 @@ __device__ __forceinline__ void gd_side_setup(const GdScene &sc, int i, GdSide &
   o.yoff = sc.sideOff[i * 2 + 1];
   o.repeat = gd_rint(sc.wlen[w] * 65536.0f);
   o.pad = 0;
-  unsigned f = GD_C_RASTER | GD_C_VALID;
+  unsigned f = GD_C_RASTER;
   const bool lightDiff = ri.x != oi.x;
   if (oneSided || vc != oc || ri.z != oi.z || lightDiff) f |= GD_C_MARK_CEIL;
   if (oneSided || vf != of || ri.y != oi.y || lightDiff) f |= GD_C_MARK_FLOOR;
@@ -154,7 +154,6 @@ __device__ __forceinline__ void gd_project_wall(const GdScene &sc, const GdView 
   const float segx = wl.z - wl.x, segy = wl.w - wl.y;
   const float vfsx = v.x - wl.x, vfsy = v.y - wl.y;
   const bool front = (segx * vfsy - segy * vfsx) < 0;
-  out.oneSided = oneSided; out.frontF = front;
   hot.segx = segx; hot.segy = segy;
   hot.offx = wl.x - v.x; hot.offy = wl.y - v.y;
   hot.dn = hot.offx * segy - hot.offy * segx;
@@ -168,7 +167,6 @@ __device__ __forceinline__ void gd_project_fragment(const GdScene &sc, const GdV
   const int4 q = *reinterpret_cast<const int4 *>(&sc.fragFixed[f * 4]);
   const i64 fx[2] = {q.x, q.z}, fy[2] = {q.y, q.w};
   gd_project_fixed(v, fx, fy, out);
-  out.oneSided = 0; out.frontF = 0;
 }
 
 /* Does the column ray (rx, ry) cross the wall (engine.py:11317-11331)?  The

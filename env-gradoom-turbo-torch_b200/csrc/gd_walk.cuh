@@ -495,7 +495,7 @@ __device__ __noinline__ void gd_slow_step(const GdScene &sc_, const GdView &v_, 
   o.tops = (unsigned)it.ctop | ((unsigned)it.clowtop << 16);
   o.bots = (unsigned)(255 - it.cbot) | ((unsigned)(255 - it.cupbot) << 16);
   o.vis = gd_vis_clamp(it.vis);
-  o.flags = (it.rasterValid ? GD_C_RASTER : 0u) | (it.valid ? GD_C_VALID : 0u) | (it.oneSided ? GD_C_ONE_SIDED : 0u) |
+  o.flags = (it.rasterValid ? GD_C_RASTER : 0u) | (it.oneSided ? GD_C_ONE_SIDED : 0u) |
             (it.markCeil ? GD_C_MARK_CEIL : 0u) | (it.markFloor ? GD_C_MARK_FLOOR : 0u) |
             (it.viewFloor < it.otherFloor ? GD_C_LOWER : 0u) | (it.viewCeil > it.otherCeil ? GD_C_UPPER : 0u) |
             (it.tier[0] ? GD_C_TIER0 : 0u) | (it.tier[1] ? GD_C_TIER1 : 0u) | (it.tier[2] ? GD_C_TIER2 : 0u) |

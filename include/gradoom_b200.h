@@ -46,7 +46,8 @@ enum gd_error {
 };
 
 /* device status bits */
-#define GD_STATUS_EVENT_OVERFLOW 1
+#define GD_STATUS_EVENT_OVERFLOW 1   /* a column that a thing or a chip may cover made more than 48 clip events; those of
+                                        the other columns are neither kept nor counted */
 #define GD_STATUS_THINGS_OVERFLOW 2
 /* set only by the checked build of the library (libgradoom_b200_checked.so, compiled with
  * -DGD_CHECKED), which range-tests every index taken from the blob and the records, skips the
@@ -69,7 +70,7 @@ const char *gd_error_string(int code);
  * Of the device blob only the address is taken: nothing is launched, and its
  * bytes have to be there when a call first draws from it.  A scene with split
  * lines (GD_H_FRAGMENTS > 0) that gd_render_step_static can draw gets a block for
- * that call's 32 CTAs, 172 bytes a fragment each at most; no other scene makes
+ * that call's 32 CTAs, 164 bytes a fragment each at most; no other scene makes
  * the creation allocate device memory.
  */
 int gd_renderer_create(const void *blob_header_host, const void *blob_dev, size_t blob_bytes, int device,
@@ -93,8 +94,10 @@ void gd_renderer_destroy(gd_renderer *r);
  */
 int gd_renderer_bind_decals(gd_renderer *r, const void *decals, int slots);
 
-/* Scratch the caller must provide to every render call: clip events of the
- * lanes being drawn plus, in its last 16 bytes, the kernel's lane queue.  Zero
+/* Scratch the caller must provide to every render call: for each of the persistent
+ * CTAs (two per SM) the frame, clip events and wall records of the lane being drawn,
+ * and in its last 16 bytes the kernel's lane queue.  0.55 MB a CTA for a 40-wall map,
+ * 0.6 MB for 144 walls, 0.9 MB for 800, whatever the number of lanes.  Zero
  * the buffer once after allocating it; every launch leaves the queue at zero.
  * Launches that share a scratch buffer must not overlap on the device; launches
  * of one renderer with a scratch buffer each may, unless decals are bound (their
@@ -103,9 +106,7 @@ size_t gd_renderer_scratch_bytes(const gd_renderer *r);
 /* Launch shape, for reports: persistent CTAs and dynamic shared memory per CTA. */
 int gd_renderer_ctas(const gd_renderer *r);
 size_t gd_renderer_shared_bytes(const gd_renderer *r);
-/* The same for calls that neither draw the status bar nor return a full frame (gd_render_step and
- * gd_render_reset with mask_hud, and their ring / host variants): the frame's 32 status-bar rows stay
- * off chip and their 10 KB hold more of the scene's tables (or leave the SM a larger L1). */
+/* The same number, for callers that ask for the calls without a full frame: all calls launch alike. */
 size_t gd_renderer_shared_bytes_view(const gd_renderer *r);
 
 /*
@@ -341,7 +342,7 @@ int gd_stepper_reset(const gd_renderer *r, const gd_stepper_state *st, int n, co
  * pool is owned and budgeted by the embedding application, or code running
  * after the framework's allocator has been frozen -- and therefore cannot
  * provide the scratch buffer.  The scratch lives in a fixed array inside the
- * library (gd_static_scratch_bytes(), about 16 MB, held by every GPU that loads
+ * library (gd_static_scratch_bytes(), about 22 MB, held by every GPU that loads
  * the library until the process exits); the call allocates and frees nothing.
  * Limits: scenes of at most gd_static_max_walls() walls (more: GD_ERR_STATIC_LIMIT)
  * and at most 32 concurrently drawing CTAs, so it is slower than gd_render_step
