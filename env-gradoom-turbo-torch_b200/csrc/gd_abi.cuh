@@ -466,7 +466,7 @@ extern "C" int gd_render_step_host(const gd_renderer *r, const int32_t *lanes_ho
  * process whose memory pool is owned and fully budgeted by its embedder, or
  * code that runs after the framework's allocator has been frozen.  Such a
  * caller cannot obtain the scratch buffer the other entry points ask for, so
- * this variant keeps the clip-event scratch in a fixed array inside the
+ * this variant keeps the CTAs' scratch in a fixed array inside the
  * library image.  Every GPU that loads the library holds GD_STATIC_SCRATCH_BYTES
  * of it until the process exits.
  */

@@ -62,7 +62,7 @@ struct GdParams {
   uint8_t *obsOut;           /* n x 84 x 84, optional */
   uint8_t *indexedOut;       /* n x 240 x 320, optional */
   uint8_t *rgbOut;           /* n x 240 x 320 x 3, optional */
-  uint8_t *scratch;          /* ctas x gd_scratch_per_cta(W), then the lane queue (2 words, zero between launches) */
+  uint8_t *scratch;          /* ctas x perCta, the crossing records below, the lane queue (2 words, zero between launches) */
   size_t queueOffset, perCta;
   GdSide *sides;             /* 2 W crossing records of maps whose tables are not on chip, in the launch's scratch */
   /* byte offsets in shared memory; those of the last four are offsets into the CTA's scratch tables when

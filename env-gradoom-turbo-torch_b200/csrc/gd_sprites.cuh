@@ -198,9 +198,9 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
         if (bestE >= 0) {
           visible = (behind >> bestE) & 1ull;
         } else {
-          /* The plane's depth limits the thing only where the pixel resolves to no sector: that search (a point
-           * test of every sector, up to 3.2 million cycles for a thing that fills the view) is left for things
-           * beyond the plane. */
+          /* The plane's depth limits the thing only where the pixel resolves to no sector: that search, plane by
+           * plane along the ray, is left for things beyond the plane (made for every pixel, and with a test of every
+           * sector, it took up to 3.2 million cycles for a thing that fills the view). */
           visible = ac.depth < GD_INF &&
                     (filled || ownerSector < 0 || ac.depth < gd_plane_depth(sc, v, flatCenter, ownerSector, ownerFloor, y) ||
                      !gd_pixel_unresolved(sc, v, x, y, ownerSector));

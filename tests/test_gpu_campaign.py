@@ -4,8 +4,8 @@ chips, thing count and the status bar all vary; the players walk with the kinema
 before the comparison, so some stand in doorways.  Every indexed frame and observation must be equal.  With
 GD_CAMPAIGN_LOG set, one line per specification is appended to that file; GD_CAMPAIGN_SPECS and
 GD_CAMPAIGN_FIRST widen or move the range of specification numbers (default: the first 24);
-GD_CAMPAIGN_MAX_GRID raises the largest grid side (default 8; 16 reaches 800-wall maps, which keep fewer
-tables in shared memory)."""
+GD_CAMPAIGN_MAX_GRID raises the largest grid side (default 8; 16 reaches 800-wall maps, which read the walk's
+tables from scratch)."""
 
 import dataclasses
 import json
