@@ -53,7 +53,7 @@ __device__ __noinline__ int gd_group_sector(const GdScene &sc_, int f, int g, fl
   for (; k < k1; ++k) {
     list.x = __funnelshift_r(list.x, list.y, 16); list.y = __funnelshift_r(list.y, list.z, 16);
     list.z = __funnelshift_r(list.z, list.w, 16); list.w >>= 16;
-    const int s = listed ? (int)(list.x & 0xFFFFu) : sc.groupSec[f][k];
+    const int s = GD_CHECK_SECTOR(listed ? (int)(list.x & 0xFFFFu) : sc.groupSec[f][k], sc.S);
     if (s >= end) break;
     if (listed && sc.secF[s * 2 + (f ? 0 : 1)] != height) continue;
     if (gd_point_in_sector(sc, s, px, py)) return s;
@@ -69,7 +69,7 @@ __device__ __forceinline__ int gd_sector_of_point(const GdScene &sc, float px, f
   unsigned found = 0x7fffffff;
 #pragma unroll 1
   for (int k = threadIdx.x & 31; k < count; k += 32) {
-    const int s = listed ? cell[1 + k] : k;
+    const int s = GD_CHECK_SECTOR(listed ? cell[1 + k] : k, sc.S);
     if (gd_point_in_sector(sc, s, px, py)) { found = (unsigned)s; break; }
   }
   return (int)__reduce_min_sync(0xffffffffu, found);

@@ -99,8 +99,8 @@ def _patched(pkg, blob, section, indices, value):
 
 
 def test_corrupted_blobs_are_reported_not_followed(pkg, scenes):
-    """A side texture past the atlas and a wall whose back sector lies beyond the scene: the
-    draw completes, the bit is set, the texture / the sector is treated as absent."""
+    """A side texture past the atlas, a wall whose back sector lies beyond the scene and cells that list such
+    sectors: the draw completes, the bit is set, the texture / the sector is treated as absent."""
 
     from gradoom_b200 import native, stepper
 
@@ -114,7 +114,9 @@ def test_corrupted_blobs_are_reported_not_followed(pkg, scenes):
     for section, indices, value, bit in (
             ("SIDE_TEX", lower, textures + 3, native.STATUS_BAD_INDEX),
             ("SIDE_TEX", upper, textures + 40, native.STATUS_BAD_INDEX),
-            ("WALL_SECTORS", back, sc.num_sectors + 5, native.STATUS_BAD_SECTOR)):
+            ("WALL_SECTORS", back, sc.num_sectors + 5, native.STATUS_BAD_SECTOR),
+            # every cell of the map lists one sector, which does not exist
+            ("CELLS", range(8, 8 + 1024 * 4, 4), 1 | ((sc.num_sectors + 5) << 16), native.STATUS_BAD_SECTOR)):
         r = _checked(_patched(pkg, blob, section, indices, value), 4)
         bits = 0
         for seed in range(6):                       # several poses, so that some lane looks at the wall
