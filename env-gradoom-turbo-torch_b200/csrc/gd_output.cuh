@@ -11,9 +11,11 @@
  * Thread x sums its column's twenty rows into seven output rows (every pixel looks its colour up once; the weights
  * are constants of the unrolled rows), then the threads sum four or five columns each into the 7 x 84 pixels.
  * What bounds it is instructions: twenty lookups and 64-bit products per output pixel, as a loop over the output,
- * took 57 of a lane's 557 thousand cycles. */
+ * took 57 of a lane's 557 thousand cycles; column sums first, 44 of 426; with the weights of a thread's pixel column found
+ * once, a black palette entry in place of tests, and the next rows' loads ahead of the barriers, 33. */
 #define GD_RESIZE_ROWS 20
 #define GD_RESIZE_OUT 7
+#define GD_RESIZE_GROUPS (GD_THREADS / GD_OBS)           /* rows of pixels that the threads sum at once */
 static_assert(GD_SCREEN_H % GD_RESIZE_ROWS == 0 && GD_RESIZE_OUT * GD_SW * 8 <= 14 * GD_SW * 4, "the sums fit the column masks");
 
 __device__ __noinline__ void gd_resize(const uint8_t *frame, int srcRows, uint8_t *out_) {
@@ -22,6 +24,13 @@ __device__ __noinline__ void gd_resize(const uint8_t *frame, int srcRows, uint8_
   uint2 *sums = (uint2 *)(gd_smem + GD_OFF_MASKS);       /* [7][320]: R | B << 16, G; the masks are done with */
   const int x = threadIdx.x;
   const uint8_t *column = frame + x;
+  /* the pixel column that a thread sums, in every third row: its four or five columns and their weights */
+  const int group = x / GD_OBS < GD_RESIZE_GROUPS ? x / GD_OBS : GD_RESIZE_OUT, ox = x % GD_OBS, c0 = 80 * ox / 21;
+  const unsigned w0 = 21u * (c0 + 1) - 80u * ox, w3 = min(38u - w0, 21u), w4 = w0 < 17u ? 17u - w0 : 0u;
+  const int last = w4 ? 4 : 3;                           /* a fifth column may lie past the edge */
+  unsigned index[GD_RESIZE_ROWS];                        /* the twenty rows' pixels; the next ones travel while these are summed */
+#pragma unroll
+  for (int r = 0; r < GD_RESIZE_ROWS; ++r) index[r] = column[r * GD_SW];
 #pragma unroll 1
   for (int y0 = 0, o0 = 0; y0 < GD_SCREEN_H; y0 += GD_RESIZE_ROWS, o0 += GD_RESIZE_OUT * GD_OBS) {
     if (y0 >= srcRows) {                                 /* masked status-bar rows: black */
@@ -29,38 +38,36 @@ __device__ __noinline__ void gd_resize(const uint8_t *frame, int srcRows, uint8_
       for (int i = x; i < GD_RESIZE_OUT * GD_OBS; i += GD_THREADS) out[o0 + i] = 0;
       continue;
     }
-    unsigned index[GD_RESIZE_ROWS];
-#pragma unroll
-    for (int r = 0; r < GD_RESIZE_ROWS; ++r) index[r] = y0 + r < srcRows ? column[(y0 + r) * GD_SW] : 256u;
     unsigned rb[GD_RESIZE_OUT], g[GD_RESIZE_OUT];
 #pragma unroll
     for (int o = 0; o < GD_RESIZE_OUT; ++o) rb[o] = g[o] = 0u;
 #pragma unroll
     for (int r = 0; r < GD_RESIZE_ROWS; ++r) {
-      const uint2 c = index[r] < 256u ? pal[index[r]] : make_uint2(0u, 0u);
+      const uint2 c = pal[index[r]];
       const int o = 7 * r / 20;
       const unsigned first = 7 * r + 7 <= 20 * (o + 1) ? 7u : 20u * (o + 1) - 7u * r;
       rb[o] += first * c.x; g[o] += first * c.y;
       if (first < 7u) { rb[o + 1] += (7u - first) * c.x; g[o + 1] += (7u - first) * c.y; }
+    }
+    {
+      const int next = y0 + GD_RESIZE_ROWS;
+#pragma unroll
+      for (int r = 0; r < GD_RESIZE_ROWS; ++r) index[r] = next + r < srcRows ? column[(next + r) * GD_SW] : 256u;
     }
     __syncthreads();                                     /* the sums of the rows before have been read */
 #pragma unroll
     for (int o = 0; o < GD_RESIZE_OUT; ++o) sums[o * GD_SW + x] = make_uint2(rb[o], g[o]);
     __syncthreads();
 #pragma unroll 1
-    for (int i = x; i < GD_RESIZE_OUT * GD_OBS; i += GD_THREADS) {
-      const int o = i / GD_OBS, ox = i - o * GD_OBS, c0 = 80 * ox / 21;
-      const uint2 *row = sums + o * GD_SW;
-      const unsigned w0 = 21u * (c0 + 1) - 80u * ox;
-      const unsigned weight[5] = {w0, 21u, 21u, min(38u - w0, 21u), w0 < 17u ? 17u - w0 : 0u};
-      unsigned r = 0, gg = 0, b = 0;
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        const uint2 c = row[min(c0 + k, GD_SW - 1)];     /* a column past the edge weighs nothing */
-        r += weight[k] * (c.x & 0xFFFFu); b += weight[k] * (c.x >> 16); gg += weight[k] * c.y;
-      }
+    for (int o = group; o < GD_RESIZE_OUT; o += GD_RESIZE_GROUPS) {
+      const uint2 *row = sums + o * GD_SW + c0;
+      const uint2 c[5] = {row[0], row[1], row[2], row[3], row[last]};
+      unsigned r = w0 * (c[0].x & 0xFFFFu), b = w0 * (c[0].x >> 16), gg = w0 * c[0].y;
+      r += 21u * ((c[1].x & 0xFFFFu) + (c[2].x & 0xFFFFu)); b += 21u * ((c[1].x >> 16) + (c[2].x >> 16)); gg += 21u * (c[1].y + c[2].y);
+      r += w3 * (c[3].x & 0xFFFFu); b += w3 * (c[3].x >> 16); gg += w3 * c[3].y;
+      r += w4 * (c[4].x & 0xFFFFu); b += w4 * (c[4].x >> 16); gg += w4 * c[4].y;
       r = (r + 800) / 1600; gg = (gg + 800) / 1600; b = (b + 800) / 1600;
-      out[o0 + i] = (uint8_t)((r * 77 + gg * 150 + b * 29 + 128) >> 8);
+      out[o0 + o * GD_OBS + ox] = (uint8_t)((r * 77 + gg * 150 + b * 29 + 128) >> 8);
     }
   }
 }
@@ -71,7 +78,10 @@ __device__ __noinline__ void gd_resize(const uint8_t *frame, int srcRows, uint8_
  * separately rounded, truncating conversion). */
 __device__ void gd_lane_palette(const GdScene &sc, const GdShared &sh, int flags) {
   const int i = threadIdx.x;
-  if (i >= 256) return;
+  if (i >= 256) {
+    if (i == 256) sh.pal64[i] = 0;
+    return;
+  }
   float bonus = 0.0f, flash = 0.0f;
   const bool blend = (flags & 4) != 0;
   if (blend) {

@@ -122,8 +122,8 @@ struct GdActor {
  * scratch, mostly in L2: its pixels are stored once each, a warp's 32 columns of a row in one sector,
  * and the 77 KB that leaves free on chip let two lanes share an SM. */
 #define GD_OFF_COLORMAP 0                                  /* 32 x 256 */
-#define GD_OFF_PAL64 (GD_OFF_COLORMAP + 32 * 256)          /* 256: R | B << 16 | G << 32 */
-#define GD_OFF_PAL32 (GD_OFF_PAL64 + 256 * 8)              /* 256: r | g << 8 | b << 16, for the RGB24 output */
+#define GD_OFF_PAL64 (GD_OFF_COLORMAP + 32 * 256)          /* 256: R | B << 16 | G << 32; then a zero: black rows */
+#define GD_OFF_PAL32 (GD_OFF_PAL64 + 258 * 8)              /* 256: r | g << 8 | b << 16, for the RGB24 output */
 #define GD_OFF_YSLOPE (GD_OFF_PAL32 + 256 * 4)             /* 208 */
 #define GD_OFF_LANE (GD_OFF_YSLOPE + GD_VIEW_H * 4)        /* 32 */
 #define GD_OFF_OWNER (GD_OFF_LANE + GD_LANE_WORDS * 4)     /* 10 words of column bits: boundary_has_projected_owner; words 16..25: the
