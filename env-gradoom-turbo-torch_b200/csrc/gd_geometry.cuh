@@ -747,8 +747,9 @@ __device__ void gd_blocking_raycast(const GdScene &sc_, const short *list, int l
 #pragma unroll 1
   for (int i = 0; i < listed; ++i) {
     const int w = list[i];
+    if (!(gd_hot(w).bits & GD_HOT_ONESIDED)) continue;
     const GdHot h = gd_hot(w);
-    if (!(h.bits & GD_HOT_ONESIDED) || !gd_ray_geo(h, rx, ry)) continue;
+    if (!gd_ray_geo(h, rx, ry)) continue;
     const float d = h.dn / (rx * h.segy - ry * h.segx);
     if (d < best || (d == best && w < bestWall && isfinite(d))) { best = d; bestWall = w; }
   }

@@ -408,15 +408,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     }
     gd_mark_afterlife_columns(sc, sh);
     if (p.flags & GD_F_DRAW_HUD) gd_hud_list(sc, sh.lane, (int4 *)sh.hitA);   /* the sectors of points have been read */
-    {
-      float rx, ry, wd = 0.0f;
-      int bw = 0;
-      if (nThings > 0) {
-        gd_ray(v, tid, rx, ry);
-        gd_blocking_raycast(sc, frustumList, frustumListed, rx, ry, wd, bw);
-      }
-      ((unsigned long long *)(gd_smem + GD_OFF_CAND))[tid] = gd_sprite_candidates(sc, sh, nThings, wd, bw);
-    }
+    ((unsigned long long *)(gd_smem + GD_OFF_CAND))[tid] = gd_sprite_candidates(sc, v, sh, nThings, frustumList, frustumListed);
     __syncthreads();
     gd_walk<kSplit, kChip>(p, sc, v, sh, frame, tables, events, eventCount, rowproj, sh.misc[0]);
     if (p.flags & GD_F_DRAW_HUD) gd_hud_column(sc, (const int4 *)sh.hitA, frame + GD_VH * GD_SW);
