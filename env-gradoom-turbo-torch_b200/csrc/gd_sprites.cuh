@@ -237,6 +237,7 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
 }
 
 /* ---- phase: weapon (engine.py:14994-15121) ------------------------------ */
+#define GD_WEAPON_ROWS 4
 __device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, uint8_t *frame, int id, i64 hoff, i64 voff) {
   const GdScene &sc = *gd_as_shared(&sc_);
 #ifdef GD_CHECKED
@@ -255,17 +256,31 @@ __device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, uint8_t *frame,
   const i64 lo = -base, hi = (i64)h * GD_FU - base;
   const int y0 = (int)gd_clamp(lo <= 0 ? 0 : gd_div(lo + iscale - 1, iscale), 0, GD_VH);
   const int y1 = (int)gd_clamp(hi <= 0 ? 0 : gd_div(hi + iscale - 1, iscale), 0, GD_VH);
+  /* a warp takes a row of 32 pixels, GD_WEAPON_ROWS such rows at once: what bounds it is the latency of the texels
+   * (a pixel at a time, with a division for each, 13 of a lane's 426 thousand cycles; now 11, and of a lane alone 17 and 10) */
+  const uint8_t *opaques = sc.wpnOpaque + (size_t)id * sc.wpnH * sc.wpnW, *texels = sc.wpnAtlas + (size_t)id * sc.wpnH * sc.wpnW;
 #pragma unroll 1
-  for (int idx = threadIdx.x; idx < (y1 - y0) * w; idx += GD_THREADS) {
-    int y = y0 + idx / w, sx = idx - (y - y0) * w;
-    i64 xx = screenLeft + sx;
+  for (int sx = threadIdx.x & 31; sx < w; sx += 32) {
+    const i64 xx = screenLeft + sx;
     if (xx < 0 || xx >= GD_SW) continue;
-    i64 sy = (base + (i64)y * iscale) >> 16;
-    if (sy < 0 || sy >= h) continue;
-    i64 cy = gd_min(sy, sc.wpnH - 1), cx = gd_min((i64)sx, (i64)sc.wpnW - 1);
-    size_t si = ((size_t)id * sc.wpnH + (size_t)cy) * sc.wpnW + (size_t)cx;
-    const uint8_t opaque = sc.wpnOpaque[si], texel = sc.wpnAtlas[si];   /* both on their way at once */
-    if (opaque) frame[y * GD_SW + (int)xx] = texel;
+    const int cx = min(sx, sc.wpnW - 1);
+#pragma unroll 1
+    for (int y = y0 + (threadIdx.x >> 5); y < y1; y += GD_WARPS * GD_WEAPON_ROWS) {
+      uint8_t opaque[GD_WEAPON_ROWS], texel[GD_WEAPON_ROWS];
+#pragma unroll
+      for (int r = 0; r < GD_WEAPON_ROWS; ++r) {
+        const int row = y + r * GD_WARPS;
+        const i64 sy = (base + (i64)row * iscale) >> 16;
+        opaque[r] = texel[r] = 0;
+        if (row < y1 && sy >= 0 && sy < h) {
+          const int si = (int)gd_min(sy, sc.wpnH - 1) * sc.wpnW + cx;
+          opaque[r] = opaques[si]; texel[r] = texels[si];
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < GD_WEAPON_ROWS; ++r)
+        if (opaque[r]) frame[(y + r * GD_WARPS) * GD_SW + (int)xx] = texel[r];
+    }
   }
 }
 
