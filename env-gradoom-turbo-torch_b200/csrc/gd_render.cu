@@ -464,16 +464,26 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       for (int i = tid; i < GD_SCREEN_H * GD_SW / 16; i += GD_THREADS) dst[i] = src[i];
     }
     if (p.rgbOut) {
-      /* four pixels (one word of indices) become three words of RGB24 */
-      unsigned *dst = (unsigned *)(p.rgbOut + (size_t)l * GD_SCREEN_H * GD_SW * 3);
-      const unsigned *src = (const unsigned *)sh.frame;
-      for (int q = tid; q < GD_SCREEN_H * GD_SW / 4; q += GD_THREADS) {
-        const unsigned idx = src[q];
-        const unsigned p0 = sh.pal32[idx & 0xFF], p1 = sh.pal32[(idx >> 8) & 0xFF];
-        const unsigned p2 = sh.pal32[(idx >> 16) & 0xFF], p3 = sh.pal32[idx >> 24];
-        dst[q * 3 + 0] = p0 | (p1 << 24);
-        dst[q * 3 + 1] = (p1 >> 8) | (p2 << 16);
-        dst[q * 3 + 2] = (p2 >> 16) | (p3 << 8);
+      /* sixteen pixels (one 16-byte load) become three 16-byte stores (a word at a time: 43 of a lane's 442 thousand
+       * cycles, now 19; 1024 lanes with RGB24 1396 and 1362 us) */
+      uint4 *dst = (uint4 *)(p.rgbOut + (size_t)l * GD_SCREEN_H * GD_SW * 3);
+      const uint4 *src = (const uint4 *)sh.frame;
+      const unsigned *pal32 = (const unsigned *)(gd_smem + GD_OFF_PAL32);
+#pragma unroll 1
+      for (int q = tid; q < GD_SCREEN_H * GD_SW / 16; q += GD_THREADS) {
+        const uint4 four = src[q];
+        const unsigned idx[4] = {four.x, four.y, four.z, four.w};
+        unsigned out[12];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned p0 = pal32[idx[k] & 0xFF], p1 = pal32[(idx[k] >> 8) & 0xFF];
+          const unsigned p2 = pal32[(idx[k] >> 16) & 0xFF], p3 = pal32[idx[k] >> 24];
+          out[k * 3] = p0 | (p1 << 24);
+          out[k * 3 + 1] = (p1 >> 8) | (p2 << 16);
+          out[k * 3 + 2] = (p2 >> 16) | (p3 << 8);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) dst[q * 3 + k] = make_uint4(out[k * 4], out[k * 4 + 1], out[k * 4 + 2], out[k * 4 + 3]);
       }
     }
     if (p.stack || p.obsOut) {
