@@ -277,7 +277,7 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
   const int count = min(sh.misc[1], GD_FALLBACK_MAX);
   int *queue = (int *)sh.hitD;
   unsigned *anchors = sh.anchors;                    /* [row][GD_WARPS] column bits */
-  unsigned *owned = sh.masks + 7 * GD_SW;            /* drawn pixels are marked owned */
+  unsigned *owned = sh.masks;                        /* drawn pixels are marked as claimed */
   if (tid == 0) { sh.misc[2] = GD_VH; sh.misc[3] = -1; sh.misc[11] = 0; }
   if (warp == 0) gd_flat_bounds_setup(sc, v, sh.misc);
   __syncthreads();
@@ -301,11 +301,11 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
   if (sh.misc[11] == 0) return;                       /* block-uniform: nothing unresolved */
   if (!sweepDone) {
     {
-      const unsigned *filled = sh.masks + tid, *own = owned + tid;
+      const unsigned *own = owned + tid;
       int lo = GD_VH, hi = -1;
 #pragma unroll 1
       for (int k = 0; k < 7; ++k) {
-        unsigned m = gd_range_word(k, 0, GD_VH) & ~filled[k * GD_SW] & ~own[k * GD_SW];
+        unsigned m = gd_range_word(k, 0, GD_VH) & ~own[k * GD_SW];
         if (m) { lo = min(lo, (k << 5) + __ffs(m) - 1); hi = max(hi, (k << 5) + 31 - __clz(m)); }
       }
       if (hi >= 0) { atomicMin(&sh.misc[2], lo); atomicMax(&sh.misc[3], hi); }

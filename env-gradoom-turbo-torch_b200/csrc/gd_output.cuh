@@ -16,12 +16,12 @@
 #define GD_RESIZE_ROWS 20
 #define GD_RESIZE_OUT 7
 #define GD_RESIZE_GROUPS (GD_THREADS / GD_OBS)           /* rows of pixels that the threads sum at once */
-static_assert(GD_SCREEN_H % GD_RESIZE_ROWS == 0 && GD_RESIZE_OUT * GD_SW * 8 <= 14 * GD_SW * 4, "the sums fit the column masks");
+static_assert(GD_SCREEN_H % GD_RESIZE_ROWS == 0 && GD_OFF_MASKS + GD_RESIZE_OUT * GD_SW * 8 <= GD_OFF_RESULT, "the sums lie before the result");
 
 __device__ __noinline__ void gd_resize(const uint8_t *frame, int srcRows, uint8_t *out_) {
   uint8_t *out = gd_as_shared(out_);
   const uint2 *pal = (const uint2 *)(gd_smem + GD_OFF_PAL64);
-  uint2 *sums = (uint2 *)(gd_smem + GD_OFF_MASKS);       /* [7][320]: R | B << 16, G; the masks are done with */
+  uint2 *sums = (uint2 *)(gd_smem + GD_OFF_MASKS);       /* [7][320]: R | B << 16, G */
   const int x = threadIdx.x;
   const uint8_t *column = frame + x;
   /* the pixel column that a thread sums, in every third row: its four or five columns and their weights */

@@ -132,19 +132,22 @@ struct GdActor {
 #define GD_OWNER_WORDS 48
 #define GD_OFF_MISC (GD_OFF_OWNER + GD_OWNER_WORDS * 4)                   /* 16 ints: start sector, fallback queue length, its unresolved
                                                               rows' range, GdFlatBounds */
-#define GD_OFF_MASKS (GD_OFF_MISC + 64)                    /* 14 x 320: per-column filled / plane-owned row bitmasks */
-#define GD_OFF_MASKED_DIST (GD_OFF_MASKS + 14 * 320 * 4)   /* 320: nearest masked drawseg of the column ... */
+#define GD_OFF_MASKS (GD_OFF_MISC + 64)                    /* 7 x 320: per-column row bitmasks */
+#define GD_OFF_MASKED_DIST (GD_OFF_MASKS + 7 * 320 * 4)   /* 320: nearest masked drawseg of the column ... */
 #define GD_OFF_MASKED_INFO (GD_OFF_MASKED_DIST + 320 * 4)  /* ... its wall << 16 | ceiling clip << 8 | floor clip; 0xFFFF0000 | .. = none */
 #define GD_OFF_CAND (GD_OFF_MASKED_INFO + 320 * 4)         /* 320 x 64 bits: things that may show in the column */
 #define GD_OFF_AUX (GD_OFF_CAND + 320 * 8)                 /* 10,240 bytes for one phase at a time: listed walls, fallback queue,
-                                                              chip ranks, 84 x 84 result */
+                                                              chip ranks, sprite columns' events */
 #define GD_AUX_BYTES (8 * 320 * 4)
 #define GD_OFF_AUX2 (GD_OFF_AUX + GD_AUX_BYTES)            /* 4,096: sectors of points, status-bar list, sprite columns, chip spans */
 #define GD_AUX2_BYTES 4096
 #define GD_OFF_HOT (GD_OFF_AUX2 + GD_AUX2_BYTES)           /* W wall records */
+/* the resize, when all before it is done: its sums from the masks on, the result behind them */
+#define GD_OFF_RESULT ((GD_OFF_MASKS + 7 * GD_SW * 8 + 15) / 16 * 16)
+static_assert(GD_OFF_RESULT + GD_OBS * GD_OBS <= GD_OFF_HOT, "the sums and the result");
 static_assert(GD_OFF_HOT % 16 == 0 && GD_OFF_AUX % 16 == 0 && GD_OFF_AUX2 % 16 == 0, "vector loads");
-static_assert(GD_OBS * GD_OBS <= GD_AUX_BYTES && 65 * 4 <= GD_AUX2_BYTES && GD_SW * 2 <= GD_AUX2_BYTES,
-              "the result; the sectors of 64 things and the player, the sprite columns");
+static_assert(65 * 4 <= GD_AUX2_BYTES && GD_SW * 2 <= GD_AUX2_BYTES,
+              "the sectors of 64 things and the player, the sprite columns");
 
 struct GdPlaneEntry;
 
@@ -157,9 +160,10 @@ struct GdShared {
   GdWall *walls;        /* scratch: W, the listed ones filled */
   GdWall *frags;        /* scratch: F projection fragments of split lines (only their spans, depths and light) */
   unsigned *anchors;    /* scratch: flat fallback */
+  unsigned *planeRows;  /* scratch: 7 x 320, rows of the planes of loose columns; where the fallback's sector table will be */
   GdActor *actors;      /* maxThings */
   unsigned long long *pal64;
-  uint8_t *obs;         /* 84 x 84; aux */
+  uint8_t *obs;         /* 84 x 84 */
   int *misc;
   unsigned *masks;
   unsigned *pal32;
@@ -209,9 +213,10 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     sh.walls = (GdWall *)(myScratch + gd_scratch_walls(sc.W, sc.S));
     sh.frags = (GdWall *)(p.frags + blockIdx.x * p.fragStride);
     sh.anchors = (unsigned *)(myScratch + GD_SCRATCH_ANCHORS);
+    sh.planeRows = (unsigned *)(myScratch + GD_SCRATCH_VSEC);
     sh.actors = (GdActor *)(gd_smem + p.offActors);
     sh.pal64 = (unsigned long long *)(gd_smem + GD_OFF_PAL64);
-    sh.obs = gd_smem + GD_OFF_AUX;
+    sh.obs = gd_smem + GD_OFF_RESULT;
     sh.misc = (int *)(gd_smem + GD_OFF_MISC);
     sh.masks = (unsigned *)(gd_smem + GD_OFF_MASKS);
     sh.pal32 = (unsigned *)(gd_smem + GD_OFF_PAL32);
@@ -410,7 +415,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     if (p.flags & GD_F_DRAW_HUD) gd_hud_list(sc, sh.lane, (int4 *)sh.hitA);   /* the sectors of points have been read */
     ((unsigned long long *)(gd_smem + GD_OFF_CAND))[tid] = gd_sprite_candidates(sc, v, sh, nThings, frustumList, frustumListed);
     __syncthreads();
-    gd_walk<kSplit, kChip>(p, sc, v, sh, frame, tables, events, eventCount, rowproj, sh.misc[0]);
+    const bool open = gd_walk<kSplit, kChip>(p, sc, v, sh, frame, tables, events, eventCount, rowproj, sh.misc[0]);
     if (p.flags & GD_F_DRAW_HUD) gd_hud_column(sc, (const int4 *)sh.hitA, frame + GD_VH * GD_SW);
     __syncthreads();
     /* Rows no seg ever claimed show the per-pixel flat fallback.  They are
@@ -419,10 +424,10 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
      * several rounds, each pass marking what it drew as owned. */
     bool sweepDone = false;                          /* CTA-uniform */
     for (;;) {
-      const unsigned *filled = sh.masks + tid, *owned = sh.masks + 7 * GD_SW + tid;
+      const unsigned *claimed = sh.masks + tid;
 #pragma unroll 1
-      for (int k = 0; k < 7; ++k) {
-        unsigned m = gd_range_word(k, 0, GD_VH) & ~filled[k * GD_SW] & ~owned[k * GD_SW];
+      for (int k = 0; k < 7 && open; ++k) {
+        unsigned m = gd_range_word(k, 0, GD_VH) & ~claimed[k * GD_SW];
 #pragma unroll 1
         while (m) {
           int y = (k << 5) + __ffs(m) - 1;
@@ -434,6 +439,9 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       __syncthreads();
       const int queued = sh.misc[1];
       if (queued == 0) break;                        /* block-uniform */
+      if (!open)
+#pragma unroll 1
+        for (int k = 0; k < 7; ++k) sh.masks[k * GD_SW + tid] = 0xffffffffu;
       gd_fallback_pass(sc, v, sh, sh.misc[0], vsec, sweepDone);
       if (queued <= GD_FALLBACK_MAX) break;
       if (tid == 0) sh.misc[1] = 0;

@@ -594,24 +594,96 @@ __device__ __noinline__ int2 gd_portal_clips(const GdScene &sc_, const GdView &v
   return make_int2(ceilClip | (floorClip << 8), nEvents);
 }
 
-/* Rows [ya,yb) of column x that no plane owns yet become the span's; those no wall tier filled are drawn.
- * This is the form for spans whose operands need 64 bits. */
-__device__ __noinline__ void gd_plane_rows_wide(const GdScene &sc_, const GdView &v_, const GdShared &sh_, int x, int ya, int yb,
-                                                int sector, bool isFloor) {
+/* ---- what a column's crossings claim (engine.py:10879-10954, 12637-12884) ---------------------------------- */
+/* Crossings narrow a window of open rows from above and below, and nearly every plane or tier continues the rows claimed
+ * so far: [0, top) and [bottom, GD_VH).  Such a claim can meet no other, and its rows are drawn as one run.  (Looking
+ * every claim up in masks of 32 rows, a bit at a time, took 30 of 322 million warp instructions of 1024 lanes; a step of 4096
+ * lanes took 3282 us, now 3104.)  A claim that
+ * does not continue them (a crossing behind a projected solid, tiers that overlap) makes the column loose for good: its rows
+ * are told apart by masks, tiers before planes and then the first claim, as the reference has it.
+ * Until then the column's mask holds the bounds of its tiers, a bit where a row differs from the one before; then it
+ * holds the rows of its tiers, and one in scratch those of its planes (on chip for every column it took 9 KB of what is L1
+ * now). */
+__device__ __forceinline__ bool gd_claim_fits(int top, int bottom, int ya, int yb, bool above) {
+  return above ? ya == top && yb <= bottom : yb == bottom && ya >= top;       /* top and bottom are -1 in a loose column */
+}
+__device__ __forceinline__ void gd_note_tier(unsigned *filled, int ya, int yb) {
+  filled[(ya >> 5) * GD_SW] ^= 1u << (ya & 31);
+  filled[(yb >> 5) * GD_SW] ^= 1u << (yb & 31);
+}
+static_assert(GD_VH >> 5 < 7, "the bit past the last row");
+
+struct GdTierRun { unsigned texel, frac, step; int shift; };
+
+/* A claim of a loose column, or the one that makes it loose (`bounds`: top | bottom << 8, else -1).  plane: its place in the
+ * span table, or -1 for a tier; rows: ya | yb << 8 | excluded rows << 16, << 24; tails: rows from the first byte
+ * on, and between the other two, have the second shade. */
+__device__ __noinline__ void gd_loose_claim(const GdScene &sc_, const GdView &v_, const GdShared &sh_, int x, int bounds, int plane,
+                                            GdTierRun t, unsigned rows, unsigned tails, unsigned shades) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  const GdView &v = *gd_as_shared(&v_);
+  const GdShared &sh = *gd_as_shared(&sh_);
+  unsigned *filled = (unsigned *)(gd_smem + GD_OFF_MASKS) + x, *owned = sh.planeRows + x;
+  if (bounds >= 0) {
+    unsigned carry = 0u;
+#pragma unroll 1
+    for (int k = 0; k < 7; ++k) {
+      unsigned m = filled[k * GD_SW];
+      m ^= m << 1; m ^= m << 2; m ^= m << 4; m ^= m << 8; m ^= m << 16;
+      m ^= carry;
+      carry = m >> 31 ? ~0u : 0u;
+      filled[k * GD_SW] = m;
+      owned[k * GD_SW] = gd_range_word(k, 0, bounds & 255) | gd_range_word(k, bounds >> 8, GD_VH);
+    }
+  }
+  GdPlaneSpan p;
+  if (plane >= 0) gd_plane_setup(sc, sh.planeTab, plane >> 1, (plane & 1) != 0, x, p);
+#pragma unroll 1
+  for (int k = 0; k < 7; ++k) {
+    unsigned m = gd_range_word(k, rows & 255u, (rows >> 8) & 255u) & ~gd_range_word(k, (rows >> 16) & 255u, rows >> 24);
+    if (plane >= 0) {
+      m &= ~owned[k * GD_SW];
+      owned[k * GD_SW] |= m;
+      m &= ~filled[k * GD_SW];
+    } else {
+      m &= ~filled[k * GD_SW];
+      filled[k * GD_SW] |= m;
+    }
+    const unsigned tail = gd_range_word(k, tails & 255u, GD_VH) | gd_range_word(k, (tails >> 8) & 255u, (tails >> 16) & 255u);
+#pragma unroll 1
+    while (m) {
+      const int b = __ffs(m) - 1, y = (k << 5) + b;
+      m &= m - 1;
+      unsigned pixel;
+      if (plane >= 0) {
+        pixel = gd_plane_pixel(sc, p, v.center, y);
+      } else {
+        const unsigned shade = (tail >> b) & 1u ? shades >> 8 : shades & 255u;
+        pixel = gd_smem[GD_OFF_COLORMAP + shade * 256u + sc.texAtlasCol[t.texel + ((t.frac + (unsigned)y * t.step) >> t.shift)]];
+      }
+      sh.frame[y * GD_SW + x] = (uint8_t)pixel;
+    }
+  }
+}
+
+/* Rows [ya, yb) of column x for a plane whose operands need 64 bits. */
+__device__ __noinline__ void gd_plane_rows_wide(const GdScene &sc_, const GdView &v_, const GdShared &sh_, int x, int ya, int yb, int plane) {
   const GdScene &sc = *gd_as_shared(&sc_);
   const GdView &v = *gd_as_shared(&v_);
   const GdShared &sh = *gd_as_shared(&sh_);
   GdPlaneSpan p;
-  gd_plane_setup(sc, sh.planeTab, sector, isFloor, x, p);
-  unsigned *filled = (unsigned *)(gd_smem + GD_OFF_MASKS) + x, *owned = filled + 7 * GD_SW;
+  gd_plane_setup(sc, sh.planeTab, plane >> 1, (plane & 1) != 0, x, p);
 #pragma unroll 1
-  for (int y = ya; y < yb; ++y) {
-    const unsigned bit = 1u << (y & 31);
-    const int k = (y >> 5) * GD_SW;
-    if (owned[k] & bit) continue;
-    owned[k] |= bit;
-    if (!(filled[k] & bit)) sh.frame[y * GD_SW + x] = (uint8_t)gd_plane_pixel(sc, p, v.center, y);
-  }
+  for (int y = ya; y < yb; ++y) sh.frame[y * GD_SW + x] = (uint8_t)gd_plane_pixel(sc, p, v.center, y);
+}
+
+/* The mask that the fallback reads: a bit for every claimed row. */
+__device__ __noinline__ void gd_claimed_rows(const GdShared &sh_, int x, int top, int bottom) {
+  const GdShared &sh = *gd_as_shared(&sh_);
+  unsigned *claimed = (unsigned *)(gd_smem + GD_OFF_MASKS) + x;
+#pragma unroll 1
+  for (int k = 0; k < 7; ++k)
+    claimed[k * GD_SW] = top < 0 ? claimed[k * GD_SW] | sh.planeRows[k * GD_SW + x] : gd_range_word(k, 0, top) | gd_range_word(k, bottom, GD_VH);
 }
 
 /* ---- two-sided middle textures (engine.py:13424-13745) -----------------------
@@ -752,7 +824,8 @@ __device__ void gd_mark_afterlife_columns(const GdScene &sc, const GdShared &sh)
 }
 
 /* ---- phase: per-column portal walk (engine.py:11561-13371) -------------- */
-/* Thread x walks column x front to back.  Nearly every crossing is plain: nothing is carried over from the one
+/* Thread x walks column x front to back; true: the column's mask tells which of its rows are claimed, else all
+ * are.  Nearly every crossing is plain: nothing is carried over from the one
  * before, and the nearest wall of the current sector is both crossed by the column's ray and owned by its
  * projected span.  None of the ownership rules can then change the outcome: the owner rules ask for a selected
  * wall that is not projected here (engine.py:11589-11730, 11905-12164), the endpoint rules for one that is not
@@ -831,7 +904,7 @@ __device__ __noinline__ uint3 gd_rows_outside(const GdView &v_, const GdWall &wv
 }
 
 template <bool kSplit, bool kChip>
-__device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, const GdView &v, const GdShared &sh, uint8_t *frame,
+__device__ __forceinline__ bool gd_walk(const GdParams &p, const GdScene &sc, const GdView &v, const GdShared &sh, uint8_t *frame,
                                         uint8_t *tables, GdEvent *events, int *eventCount, const GdRowProj *rowproj, int startSector) {
   const int x = threadIdx.x;
   const int quadBase = x & 28;
@@ -846,9 +919,10 @@ __device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, co
   const float4 *sectors = (const float4 *)(gd_smem + p.offSectors);
   const unsigned short *secOff = (const unsigned short *)(gd_smem + p.offSecOff), *secWalls = (const unsigned short *)(gd_smem + p.offSecWalls);
   const unsigned *yslope = (const unsigned *)(gd_smem + GD_OFF_YSLOPE);
-  unsigned *filled = (unsigned *)(gd_smem + GD_OFF_MASKS) + x, *owned = filled + 7 * GD_SW;
+  unsigned *filled = (unsigned *)(gd_smem + GD_OFF_MASKS) + x;
 #pragma unroll
-  for (int k = 0; k < 14; ++k) filled[k * GD_SW] = 0;
+  for (int k = 0; k < 7; ++k) filled[k * GD_SW] = 0;
+  int top = 0, bottom = GD_VH;      /* the rows not in between are claimed; -1: the masks tell */
   float *maskedDist = (float *)(gd_smem + GD_OFF_MASKED_DIST) + x;
   unsigned *maskedInfo = (unsigned *)(gd_smem + GD_OFF_MASKED_INFO) + x;
   if (p.sc.M > 0) { *maskedDist = GD_INF; *maskedInfo = 0xFFFF0000u | GD_VH; }
@@ -1015,17 +1089,20 @@ __device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, co
         const bool isFloor = q == 0;
         const int ya = isFloor ? max(cbot, ceilClip) : ceilClip, yb = isFloor ? floorClip : min(ctop, floorClip);
         if (!(flags & (isFloor ? GD_C_MARK_FLOOR : GD_C_MARK_CEIL)) || ya >= yb) continue;
-        const int k1 = (yb - 1) >> 5;
-        unsigned any = 0;
-#pragma unroll 1
-        for (int k = ya >> 5; k <= k1; ++k) any |= gd_range_word(k, ya, yb) & ~owned[k * GD_SW];
-        if (!any) continue;
-        const int4 *e = reinterpret_cast<const int4 *>(&planes[rc * 2 + (isFloor ? 1 : 0)]);
+        const int plane = rc * 2 + (isFloor ? 1 : 0);
+        if (!gd_claim_fits(top, bottom, ya, yb, !isFloor)) {
+          gd_loose_claim(sc, v, sh, x, top < 0 ? -1 : top | (bottom << 8), plane, GdTierRun{0u, 0u, 0u, 0},
+                         (unsigned)ya | ((unsigned)yb << 8), 255u, 0u);
+          top = bottom = -1;
+          continue;
+        }
+        if (isFloor) bottom = ya; else top = yb;
+        const int4 *e = reinterpret_cast<const int4 *>(&planes[plane]);
         const int4 e0 = e[0];
         /* rows lie farther from the viewer towards the horizon: the row that bounds the span's distance */
         const unsigned far = ya > centerRow ? yslope[ya] : (yb <= centerRow ? yslope[yb - 1] : 0xffffffffu);
         if (!((unsigned)e0.w & GD_PLANE_NARROW) || ((unsigned long long)(unsigned)e0.x * far) >> 47) {
-          gd_plane_rows_wide(sc, v, sh, x, ya, yb, rc, isFloor);
+          gd_plane_rows_wide(sc, v, sh, x, ya, yb, plane);
           continue;
         }
         const int4 e1 = e[1], e2 = e[2];
@@ -1035,26 +1112,14 @@ __device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, co
         s.basex = e1.x + (x - 159) * e1.y; s.basey = e1.z + (x - 159) * e1.w;
         s.pviewx = (unsigned)e2.x; s.pviewy = (unsigned)e2.y; s.tex = (unsigned)e2.z;
         const int center = (int)v.center;
+        /* two rows per trip; an odd last row is simply drawn twice */
 #pragma unroll 1
-        for (int k = ya >> 5; k <= k1; ++k) {
-          const unsigned have = owned[k * GD_SW];
-          const unsigned fresh = gd_range_word(k, ya, yb) & ~have;
-          if (!fresh) continue;
-          owned[k * GD_SW] = have | fresh;
-          unsigned m = fresh & ~filled[k * GD_SW];
-          const int y0 = k << 5;
-          /* two rows per trip; an odd last row is simply drawn twice */
-#pragma unroll 1
-          while (m) {
-            const int b0 = __ffs(m) - 1;
-            m &= m - 1;
-            const int b1 = m ? __ffs(m) - 1 : b0;
-            m &= m - 1;
-            const unsigned p0 = gd_plane_pixel_narrow(s, p.sc.texAtlas, p.sc.texW, center, y0 + b0);
-            const unsigned p1 = gd_plane_pixel_narrow(s, p.sc.texAtlas, p.sc.texW, center, y0 + b1);
-            frame[(unsigned)((y0 + b0) * GD_SW + x)] = (uint8_t)p0;
-            frame[(unsigned)((y0 + b1) * GD_SW + x)] = (uint8_t)p1;
-          }
+        for (int y = ya; y < yb; y += 2) {
+          const int y1 = min(y + 1, yb - 1);
+          const unsigned p0 = gd_plane_pixel_narrow(s, p.sc.texAtlas, p.sc.texW, center, y);
+          const unsigned p1 = gd_plane_pixel_narrow(s, p.sc.texAtlas, p.sc.texW, center, y1);
+          frame[(unsigned)(y * GD_SW + x)] = (uint8_t)p0;
+          frame[(unsigned)(y1 * GD_SW + x)] = (uint8_t)p1;
         }
       }
       /* wall tiers: middle or lower first, then upper; the lower one has priority where they overlap
@@ -1071,25 +1136,27 @@ __device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, co
         if (hoff >= repeat) hoff = repeat - 1;
         const i64 column = (hoff + sd.tox) >> 16;
         const int base = gd_shade_base(__float_as_int(here.z) + v.flashLight * 16 + sd.contrast);
-        const unsigned cmN = (unsigned)gd_shade(base, vis) * 256u, cmT = (unsigned)gd_shade(base, firstVis) * 256u;
+        const unsigned shadeN = (unsigned)gd_shade(base, vis), shadeT = (unsigned)gd_shade(base, firstVis);
 #pragma unroll 1
         for (int q = 0; q < 2; ++q) {
           const bool upper = q == 1;
           if (!(flags & (upper ? GD_C_TIER2 : (oneSided ? GD_C_TIER0 : GD_C_TIER1)))) continue;
           const int texId = sd.tex[upper ? 2 : (oneSided ? 0 : 1)];
 #ifdef GD_CHECKED
-          if (texId >= sc.T) { atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX); continue; }   /* the tier stays undrawn */
+          if (texId >= sc.T) {                         /* the tier stays undrawn, and its rows are nobody's */
+            atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX);
+            gd_loose_claim(sc, v, sh, x, top < 0 ? -1 : top | (bottom << 8), -1, GdTierRun{0u, 0u, 0u, 0}, 0u, 255u, 0u);
+            top = bottom = -1;
+            continue;
+          }
 #endif
           const int ya = upper || oneSided ? ctop : clowtop, yb = upper ? cupbot : cbot;
           const float originZ = upper ? there.y : (oneSided ? here.y : there.x);
-          const int ea = upper && lowRange ? clowtop : 0, eb = upper && lowRange ? cbot : 0;
           /* rows lit with the group's first-column light: below the group's highest bottom */
           const int gb0 = 255 - (int)(botMax & 0xFFFFu), gb2 = 255 - (int)(botMax >> 16);
           const bool group2 = same && all2 && (int)(topMax & 0xFFFFu) < gb2;
           const bool group = upper ? group2 : (same && (oneSided ? (all0 && (int)(topMax & 0xFFFFu) < gb0) : (all1 && (int)(topMax >> 16) < gb0)));
-          const int tailA = group && cmN != cmT ? (upper ? gb2 : gb0) : GD_VH;
-          const bool otherTail = !upper && !oneSided && upRange && group2 && cmN != cmT;
-          const int oTailA = otherTail ? max(ctop, gb2) : 0, oTailB = otherTail ? cupbot : 0;
+          const int tailA = group && shadeN != shadeT ? (upper ? gb2 : gb0) : GD_VH;
           const int4 ti = *reinterpret_cast<const int4 *>(&p.sc.texInfo[texId * 4]);
           const int hbits = ti.w;
           const unsigned u = (unsigned)gd_pymod_width(column, ti.x);
@@ -1097,31 +1164,32 @@ __device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, co
           const i64 texMid = gd_rint((originZ - v.viewZ) * 65536.0f + sd.yoff * 65536.0f);
           /* frac(y) = (texMid << (16-bits)) + ((vstep * (y*FU - center + FU)) >> 16); the
            * y term is a multiple of 2^16 inside the shift, so it steps by vstep exactly. */
-          const unsigned frac0 = (unsigned)(gd_shl(texMid, 16 - hbits) + (gd_wmul(vstep, GD_FU - v.center) >> 16));
-          const unsigned step = (unsigned)vstep;
-          const unsigned texel0 = ((unsigned)texId * (unsigned)p.sc.texW + u) * (unsigned)p.sc.texH;
-          const int shift = 32 - hbits;
+          GdTierRun t;
+          t.frac = (unsigned)(gd_shl(texMid, 16 - hbits) + (gd_wmul(vstep, GD_FU - v.center) >> 16));
+          t.step = (unsigned)vstep;
+          t.texel = ((unsigned)texId * (unsigned)p.sc.texW + u) * (unsigned)p.sc.texH;
+          t.shift = 32 - hbits;
+          if (!gd_claim_fits(top, bottom, ya, yb, upper || oneSided)) {
+            const bool otherTail = !upper && !oneSided && upRange && group2 && shadeN != shadeT;
+            const unsigned oTailA = otherTail ? (unsigned)max(ctop, gb2) : 0u, oTailB = otherTail ? (unsigned)cupbot : 0u;
+            gd_loose_claim(sc, v, sh, x, top < 0 ? -1 : top | (bottom << 8), -1, t,
+                           (unsigned)ya | ((unsigned)yb << 8) | (upper && lowRange ? ((unsigned)clowtop << 16) | ((unsigned)cbot << 24) : 0u),
+                           (unsigned)tailA | (oTailA << 8) | (oTailB << 16), shadeN | (shadeT << 8));
+            top = bottom = -1;
+            continue;
+          }
+          if (upper || oneSided) top = yb; else bottom = ya;
+          gd_note_tier(filled, ya, yb);
+          const unsigned cmN = shadeN * 256u, cmT = shadeT * 256u;
+          unsigned f = t.frac + (unsigned)ya * t.step;
 #pragma unroll 1
-          for (int k = ya >> 5; k <= (yb - 1) >> 5; ++k) {
-            const unsigned have = filled[k * GD_SW];
-            unsigned m = gd_range_word(k, ya, yb) & ~gd_range_word(k, ea, eb) & ~have;
-            if (!m) continue;
-            filled[k * GD_SW] = have | m;
-            const unsigned tailM = gd_range_word(k, tailA, GD_VH) | gd_range_word(k, oTailA, oTailB);
-            const int y0 = k << 5;
-#pragma unroll 1
-            while (m) {
-              const int b0 = __ffs(m) - 1;
-              m &= m - 1;
-              const int b1 = m ? __ffs(m) - 1 : b0;
-              m &= m - 1;
-              const unsigned f0 = frac0 + (unsigned)(y0 + b0) * step, f1 = frac0 + (unsigned)(y0 + b1) * step;
-              const unsigned t0 = p.sc.texAtlasCol[texel0 + (f0 >> shift)], t1 = p.sc.texAtlasCol[texel0 + (f1 >> shift)];
-              const uint8_t p0 = gd_smem[GD_OFF_COLORMAP + ((tailM >> b0) & 1u ? cmT : cmN) + t0];
-              const uint8_t p1 = gd_smem[GD_OFF_COLORMAP + ((tailM >> b1) & 1u ? cmT : cmN) + t1];
-              frame[(unsigned)((y0 + b0) * GD_SW + x)] = p0;
-              frame[(unsigned)((y0 + b1) * GD_SW + x)] = p1;
-            }
+          for (int y = ya; y < yb; y += 2) {
+            const int odd = y + 1 < yb ? 1 : 0;
+            const unsigned f1 = odd ? f + t.step : f;
+            const unsigned t0 = p.sc.texAtlasCol[t.texel + (f >> t.shift)], t1 = p.sc.texAtlasCol[t.texel + (f1 >> t.shift)];
+            f += 2u * t.step;
+            frame[(unsigned)(y * GD_SW + x)] = gd_smem[GD_OFF_COLORMAP + (y >= tailA ? cmT : cmN) + t0];
+            frame[(unsigned)((y + odd) * GD_SW + x)] = gd_smem[GD_OFF_COLORMAP + (y + odd >= tailA ? cmT : cmN) + t1];
           }
         }
       }
@@ -1163,6 +1231,9 @@ __device__ __forceinline__ void gd_walk(const GdParams &p, const GdScene &sc, co
   }
   eventCount[x] = nEvents < GD_MAX_EVENTS ? nEvents : GD_MAX_EVENTS;
   if (nEvents > GD_MAX_EVENTS) atomicOr(p.status, GD_STATUS_EVENT_OVERFLOW);
+  const bool open = top < bottom || top < 0;
+  if (open) gd_claimed_rows(sh, x, top, bottom);
+  return open;
 }
 
 #endif
