@@ -108,8 +108,9 @@ inline size_t gd_frag_bytes(int F, bool chip) { return gd_frag_rows(F) + (chip ?
 
 struct GdActor {
   float x, y, depth;
-  i64 depthFixed, xstep, yscale, topFixed, texMid, iscale;
+  i64 depthFixed, xstep, yscale, topFixed, fracBase, iscale;   /* patch row at screen row y: (fracBase + y * iscale) >> 16 */
   int left, right;
+  short row0, row1;               /* rows whose patch row lies inside the patch */
   int sprite, w, h;
   short shade;
   signed char style;

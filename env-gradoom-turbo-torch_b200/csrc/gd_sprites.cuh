@@ -44,9 +44,17 @@ __device__ __noinline__ void gd_actor_setup(const GdScene &sc_, const GdView &v_
   ac.left = (int)gd_clamp(left, -(1 << 30), 1 << 30);
   ac.right = (int)gd_clamp(right, -(1 << 30), 1 << 30);
   ac.yscale = gd_div(GD_FOCAL_Y << 12, gd_max(depthFixed, GD_SPRITE_MIN_DEPTH));
-  ac.texMid = (i64)si.w * GD_FU - gd_rint((v.viewZ - t.z) * 65536.0f);
-  ac.topFixed = v.center - (gd_wmul(ac.texMid, ac.yscale) >> 16);
+  const i64 texMid = (i64)si.w * GD_FU - gd_rint((v.viewZ - t.z) * 65536.0f);
+  ac.topFixed = v.center - (gd_wmul(texMid, ac.yscale) >> 16);
   ac.iscale = gd_div(GD_U32MASK, gd_max(ac.yscale, 1));
+  ac.fracBase = texMid - (gd_wmul(v.center - GD_FU, ac.iscale) >> 16);
+  ac.row0 = 0; ac.row1 = GD_VH;
+  if (ac.iscale > 0) {
+    /* frac(y) >> 16 in [0,h)  <=>  0 <= fracBase + y*iscale < h*FU */
+    const i64 lo = -ac.fracBase, hi = (i64)ac.h * GD_FU - ac.fracBase;
+    ac.row0 = (short)gd_clamp(lo <= 0 ? 0 : gd_div(lo + ac.iscale - 1, ac.iscale), 0, GD_VH);
+    ac.row1 = (short)gd_clamp(hi <= 0 ? 0 : gd_div(hi + ac.iscale - 1, ac.iscale), 0, GD_VH);
+  }
   i64 light = sc.secI[sector * 4] + v.flashLight * 16;
   if (t.flags & GD_THING_BRIGHT) light = 255;
   float base = 61.0f - (float)light / 4.0f;
@@ -161,17 +169,9 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
       i64 u = (((i64)x - ac.left) * ac.xstep) >> 16;
       if (u < 0 || u >= ac.w) continue;
       const uint8_t *cm = sh.colormap + ac.shade * 256;
-      i64 fracBase = ac.texMid - (gd_wmul(v.center - GD_FU, ac.iscale) >> 16);
-      /* rows whose source row lies inside the patch */
-      int y0 = 0, y1 = GD_VH;
-      if (ac.iscale > 0) {
-        /* frac(y) >> 16 in [0,h)  <=>  0 <= fracBase + y*iscale < h*FU */
-        i64 lo = -fracBase, hi = (i64)ac.h * GD_FU - fracBase;
-        i64 ya = lo <= 0 ? 0 : gd_div(lo + ac.iscale - 1, ac.iscale);
-        i64 yb = hi <= 0 ? 0 : gd_div(hi + ac.iscale - 1, ac.iscale);
-        y0 = (int)gd_clamp(ya, 0, GD_VH);
-        y1 = (int)gd_clamp(yb, 0, GD_VH);
-      }
+      const i64 fracBase = ac.fracBase;
+      const int y0 = ac.row0, y1 = ac.row1;            /* two divisions that every column made for itself before
+                                                        * (256 sectors, 32 things: 14653 us a step, now 14271) */
       unsigned long long behind = 0;                 /* events whose wall lies behind the thing */
 #pragma unroll 1
       for (int e0 = 0; e0 < nEv; e0 += 32) {
