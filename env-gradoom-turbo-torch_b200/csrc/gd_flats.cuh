@@ -6,22 +6,26 @@
 /* ---- point in sector (engine.py:9598-9617) ------------------------------ */
 /* Crossing parity of a +x ray over the sector's edges.  The bounding box only
  * skips sectors whose parity is provably even. */
+__device__ __forceinline__ bool gd_outside_box(const GdScene &sc, int s, float px, float py) {
+  const float4 bb = *reinterpret_cast<const float4 *>(&sc.secBBox[s * 4]);
+  return py >= bb.w || py < bb.z                             /* no edge straddles the ray's row */
+         || px > bb.y + 1.0f                                 /* every crossing lies left of the point */
+         || (px < bb.x - 1.0f && sc.secI[s * 4 + 3]);        /* closed loops cross an even number of times */
+}
+__device__ __forceinline__ bool gd_crosses_edge(const GdScene &sc, int k, float px, float py) {
+  const float4 e = *reinterpret_cast<const float4 *>(&sc.walls[GD_CHECK_INDEX(sc.edgeWalls[k], sc.W) * 4]);
+  const bool crosses = (e.y > py) != (e.w > py);
+  const float dy = e.w - e.y;
+  const float safe = fabsf(dy) < 1e-6f ? 1.0f : dy;
+  const float cx = e.x + (py - e.y) * (e.z - e.x) / safe;
+  return crosses && (px < cx);
+}
 __device__ __forceinline__ bool gd_point_in_sector(const GdScene &sc, int s, float px, float py) {
   s = GD_CHECK_SECTOR(s, sc.S);
-  const float4 bb = *reinterpret_cast<const float4 *>(&sc.secBBox[s * 4]);
-  if (py >= bb.w || py < bb.z) return false;           /* no edge straddles the ray's row */
-  if (px > bb.y + 1.0f) return false;                  /* every crossing lies left of the point */
-  if (px < bb.x - 1.0f && sc.secI[s * 4 + 3]) return false;  /* closed loops cross an even number of times */
+  if (gd_outside_box(sc, s, px, py)) return false;
   int crossings = 0;
 #pragma unroll 1
-  for (int k = sc.edgeOff[s]; k < sc.edgeOff[s + 1]; ++k) {
-    const float4 e = *reinterpret_cast<const float4 *>(&sc.walls[GD_CHECK_INDEX(sc.edgeWalls[k], sc.W) * 4]);
-    bool crosses = (e.y > py) != (e.w > py);
-    float dy = e.w - e.y;
-    float safe = fabsf(dy) < 1e-6f ? 1.0f : dy;
-    float cx = e.x + (py - e.y) * (e.z - e.x) / safe;
-    crossings += (crosses && (px < cx)) ? 1 : 0;
-  }
+  for (int k = sc.edgeOff[s]; k < sc.edgeOff[s + 1]; ++k) crossings += gd_crosses_edge(sc, k, px, py) ? 1 : 0;
   return crossings & 1;
 }
 
@@ -61,18 +65,32 @@ __device__ __noinline__ int gd_group_sector(const GdScene &sc_, int f, int g, fl
   return -1;
 }
 
-/* Lowest-numbered sector that contains a point (engine.py:9598-9617), 0x7fffffff for none; by a whole warp. */
+/* Lowest-numbered sector that contains a point (engine.py:9598-9617), 0x7fffffff for none; by eight threads.  What bounds
+ * it is a chain of loads, so the few sectors of the point's cell are looked at one after the other, an edge a thread (it
+ * was a sector a thread, edge after edge, and a warp for each point: one lane alone 114 us a step, now 112).  Where the cell has no list, each thread takes
+ * every eighth sector. */
+#define GD_POINT_THREADS 8
 __device__ __forceinline__ int gd_sector_of_point(const GdScene &sc, float px, float py) {
   const unsigned short *cell = sc.cells->cell[gd_cell(*sc.cells, px, py)];
-  const bool listed = cell[0] <= GD_CELL_SECTORS;
-  const int count = listed ? cell[0] : sc.S;
+  const int lane = threadIdx.x & (GD_POINT_THREADS - 1), count = cell[0];
+  const unsigned group = ((1u << GD_POINT_THREADS) - 1u) << (threadIdx.x & 31 & ~(GD_POINT_THREADS - 1));
   unsigned found = 0x7fffffff;
+  if (count <= GD_CELL_SECTORS) {
 #pragma unroll 1
-  for (int k = threadIdx.x & 31; k < count; k += 32) {
-    const int s = GD_CHECK_SECTOR(listed ? cell[1 + k] : k, sc.S);
-    if (gd_point_in_sector(sc, s, px, py)) { found = (unsigned)s; break; }
+    for (int i = 0; i < count && found == 0x7fffffff; ++i) {
+      const int s = GD_CHECK_SECTOR(cell[1 + i], sc.S);
+      if (gd_outside_box(sc, s, px, py)) continue;
+      bool odd = false;
+#pragma unroll 1
+      for (int k = sc.edgeOff[s] + lane; k < sc.edgeOff[s + 1]; k += GD_POINT_THREADS) odd = odd != gd_crosses_edge(sc, k, px, py);
+      if (__popc(__ballot_sync(group, odd)) & 1) found = (unsigned)s;
+    }
+    return (int)found;
   }
-  return (int)__reduce_min_sync(0xffffffffu, found);
+#pragma unroll 1
+  for (int s = lane; s < sc.S; s += GD_POINT_THREADS)
+    if (gd_point_in_sector(sc, s, px, py)) { found = (unsigned)s; break; }
+  return (int)__reduce_min_sync(group, found);
 }
 
 /* Flat-fallback resolution of a pixel (engine.py:10961-11026): true when the

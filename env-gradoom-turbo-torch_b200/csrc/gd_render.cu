@@ -330,16 +330,16 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     if (tid == 0) {
       gd_view_setup(sc, sh.lane, sView);
     } else if (tid >= 32) {
-      /* one warp a point: its cell of the map names the sectors to test */
+      /* eight threads a point: its cell of the map names the sectors to test */
 #pragma unroll 1
-      for (int t = (tid >> 5) - 1; t <= nThings; t += GD_WARPS - 1) {
+      for (int t = (tid - 32) / GD_POINT_THREADS; t <= nThings; t += (GD_THREADS - 32) / GD_POINT_THREADS) {
         float px = __int_as_float(sh.lane[GD_L_X]), py = __int_as_float(sh.lane[GD_L_Y]);
         if (t < nThings) {
           const gd_thing &th = p.things[(size_t)l * p.maxThings + t];
           px = th.x; py = th.y;
         }
         const int s = gd_sector_of_point(sc, px, py);
-        if ((tid & 31) == 0) pointSector[t < nThings ? t : 64] = s;
+        if (tid % GD_POINT_THREADS == 0) pointSector[t < nThings ? t : 64] = s;
       }
     }
     __syncthreads();
