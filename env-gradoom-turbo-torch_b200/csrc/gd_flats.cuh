@@ -275,28 +275,150 @@ __device__ __noinline__ GdFlatProbe gd_flat_probe(const GdScene &sc_, const GdVi
   return out;
 }
 
+/* Repairs, for the `c` listed columns, rows minY .. maxY: `vsec` gets the vertically repaired sector of every such pixel,
+ * and `anchors` a bit per pixel telling whether it anchors horizontal spans.  First every pixel is probed, a pixel a
+ * thread; then the columns that are unresolved at maxY have the nearest resolved row below it looked for, of its
+ * orientation, by the more threads a column the fewer columns are left without one; then a thread a column carries the
+ * nearest resolved row upwards. */
+#define GD_FLAT_UNRESOLVED 0xFFFFu
+__device__ __noinline__ void gd_flat_sweep(const GdScene &sc_, const GdView &v_, const GdShared &sh_, const GdFlatBounds &b, int currentSector,
+                                           unsigned short *vsec, int c, int minY, int maxY) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  const GdView &v = *gd_as_shared(&v_);
+  const GdShared &sh = *gd_as_shared(&sh_);
+  const int tid = threadIdx.x;
+  unsigned *first = (unsigned *)(gd_smem + GD_OFF_AUX2);             /* row << 16 | sector */
+  const short *list = (const short *)(gd_smem + GD_OFF_FLAT_LIST);
+  short *pending = (short *)(gd_smem + GD_OFF_FLAT_LIST) + GD_SW, *others = pending + GD_SW;
+  int *count = (int *)(gd_smem + GD_OFF_MISC) + 13;
+  const int flipRow = gd_clamp((int)floorf(gd_flat_ray(sc, v, 0).center) + 1, 0, GD_VH);   /* first floor row */
+  const int limit = maxY < flipRow ? flipRow : GD_VH;
+  if (tid == 0) *count = 0;
+#pragma unroll 1
+  for (int i = tid; i < (maxY - minY + 1) * GD_WARPS; i += GD_THREADS) sh.anchors[minY * GD_WARPS + i] = 0u;
+#pragma unroll 1
+  for (int i = tid; i < (maxY - minY + 1) * c; i += GD_THREADS) {
+    const int x = list[i % c], y = minY + i / c;
+    const GdFlatProbe q = gd_flat_probe(sc, v, gd_flat_ray(sc, v, x), b, y, currentSector);
+    vsec[y * GD_SW + x] = (unsigned short)(q.unresolved ? GD_FLAT_UNRESOLVED : (unsigned)q.sector);
+  }
+  __threadfence_block();
+  __syncthreads();
+  if (tid < c) {
+    first[tid] = 0xffffffffu;
+    if (vsec[maxY * GD_SW + list[tid]] == GD_FLAT_UNRESOLVED) pending[atomicAdd(count, 1)] = (short)tid;
+  }
+  __syncthreads();
+  int n = *count;
+  __syncthreads();
+#pragma unroll 1
+  for (int y = maxY + 1; n > 0 && y < limit;) {
+    const int k = GD_THREADS / n, i = tid / k;                       /* rows of a column looked at at once */
+    if (tid == 0) *count = 0;
+    __syncthreads();
+    if (i < n && y + tid % k < limit) {
+      const int row = y + tid % k;
+      const GdFlatProbe q = gd_flat_probe(sc, v, gd_flat_ray(sc, v, list[pending[i]]), b, row, currentSector);
+      if (!q.unresolved) atomicMin(&first[pending[i]], ((unsigned)row << 16) | (unsigned)q.sector);
+    }
+    __syncthreads();
+    if (tid < n && first[pending[tid]] == 0xffffffffu) others[atomicAdd(count, 1)] = pending[tid];
+    __syncthreads();
+    n = *count;
+    y += k;
+    short *swap = pending; pending = others; others = swap;
+    __syncthreads();
+  }
+  if (tid < c) {
+    const int x = list[tid];
+    bool haveBelow = first[tid] != 0xffffffffu, belowFloor = (int)(first[tid] >> 16) >= flipRow;
+    int belowSector = (int)(first[tid] & 0xFFFFu);
+#pragma unroll 1
+    for (int y = maxY; y >= minY; --y) {
+      const unsigned own = vsec[y * GD_SW + x];
+      const bool isFloor = y >= flipRow;
+      bool anchor = true;
+      int repaired = (int)own;
+      if (own != GD_FLAT_UNRESOLVED) {
+        haveBelow = true; belowFloor = isFloor; belowSector = repaired;
+      } else {
+        const bool spans = haveBelow && belowFloor == isFloor;
+        repaired = spans ? belowSector : currentSector;
+        anchor = spans && belowSector != currentSector;
+      }
+      vsec[y * GD_SW + x] = (unsigned short)repaired;
+      if (anchor) atomicOr(&sh.anchors[y * GD_WARPS + (x >> 5)], 1u << (x & 31));
+    }
+  }
+  __threadfence_block();
+  __syncthreads();
+}
+
+/* Draws the queued pixels that are left: each with its own repaired sector, or with the one its nearest anchors left and
+ * right agree on.  Only columns up to `window` from a pixel's own have been repaired: one whose anchors may lie
+ * farther away stays in the queue, and misc[12] tells. */
+__device__ __noinline__ void gd_flat_repaired(const GdScene &sc_, const GdView &v_, const GdShared &sh_, const unsigned short *vsec, int *queue,
+                                              int count, int window) {
+  const GdScene &sc = *gd_as_shared(&sc_);
+  const GdView &v = *gd_as_shared(&v_);
+  const GdShared &sh = *gd_as_shared(&sh_);
+#pragma unroll 1
+  for (int i = threadIdx.x; i < count; i += GD_THREADS) {
+    if (queue[i] < 0) continue;
+    const int px = queue[i] & 0xFFFF, py = queue[i] >> 16;
+    int sector = vsec[py * GD_SW + px];
+    /* nearest anchor at or left of px, at or right of px */
+    int left = -1, right = -1;
+#pragma unroll 1
+    for (int w = 0; w < GD_WARPS; ++w) {
+      unsigned bits = sh.anchors[py * GD_WARPS + w];
+      int base = w * 32;
+      if (base <= px) {
+        unsigned lo = px - base >= 31 ? bits : (bits & ((2u << (px - base)) - 1u));
+        if (lo) left = base + 31 - __clz(lo);
+      }
+      if (base + 31 >= px && right < 0) {
+        unsigned hi = px - base <= 0 ? bits : (bits & ~((1u << (px - base)) - 1u));
+        if (hi) right = base + __ffs(hi) - 1;
+      }
+    }
+    const bool sure = px - left <= window && (right >= 0 ? right : GD_SW) - px <= window;   /* no anchor up to the edge counts too */
+    if (!sure) { sh.misc[12] = 1; continue; }
+    if (left >= 0 && right >= 0) {
+      int sl = vsec[py * GD_SW + left], sr = vsec[py * GD_SW + right];
+      if (sl == sr) sector = sl;
+    }
+    const bool isFloor = ((float)py - gd_flat_ray(sc, v, px).center) > 0;
+    GdPlaneSpan p;
+    gd_plane_setup(sc, sh.planeTab, sector, isFloor, px, p);
+    sh.frame[py * GD_SW + px] = (uint8_t)gd_plane_pixel(sc, p, v.center, py);
+    atomicOr(&sh.masks[(py >> 5) * GD_SW + px], 1u << (py & 31));
+    queue[i] = -1;
+  }
+}
+
 /* Pass over the queued pixels.
  *   A  one thread per queued pixel probes it; a resolved pixel is drawn at
  *      once and leaves the queue.
- *   B  only when unresolved pixels remain, once per lane: over the rows of
- *      every pixel that is still unclaimed, one thread per column first looks
- *      below the last of those rows for the nearest resolved row, then sweeps
- *      the rows bottom-up carrying the nearest resolved row below.  It writes
- *      the vertically repaired sector of every pixel of those rows to `vsec`
- *      and one bit per pixel telling whether it anchors horizontal spans.
- *   C  one thread per remaining queued pixel: its own repaired sector, or the
- *      one its nearest anchors left and right agree on. */
+ *   B  Only when unresolved pixels remain: the columns near theirs are repaired in their rows, which as a rule says what
+ *      they are.  Unresolved pixels are few and lie in a column or two where two lines meet, near the horizon, and repairing
+ *      all 320 columns, down to the first resolved row in each, took up to 1.2 million of a lane's cycles.
+ *   C  Pixels whose anchors lie farther away, or too many columns: all columns are repaired, once per lane, in the rows
+ *      of every pixel that is still unclaimed. */
+#define GD_FLAT_WINDOW 8
 __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdShared &sh_, int currentSector,
                                  unsigned short *vsec, bool &sweepDone) {
   const GdScene &sc = *gd_as_shared(&sc_);
   const GdView &v = *gd_as_shared(&v_);
   const GdShared &sh = *gd_as_shared(&sh_);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int count = min(sh.misc[1], GD_FALLBACK_MAX);
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int queued = sh.misc[1], count = min(queued, GD_FALLBACK_MAX);
   int *queue = (int *)sh.hitD;
-  unsigned *anchors = sh.anchors;                    /* [row][GD_WARPS] column bits */
   unsigned *owned = sh.masks;                        /* drawn pixels are marked as claimed */
-  if (tid == 0) { sh.misc[2] = GD_VH; sh.misc[3] = -1; sh.misc[11] = 0; }
+  unsigned *columns = sh.ownerMask;                  /* with unresolved pixels; 16 words on: to be repaired */
+  short *list = (short *)(gd_smem + GD_OFF_FLAT_LIST);
+  if (tid == 0) { sh.misc[2] = GD_VH; sh.misc[3] = -1; sh.misc[11] = 0; sh.misc[12] = 0; }
+  if (tid < GD_WARPS) columns[tid] = 0u;
   if (warp == 0) gd_flat_bounds_setup(sc, v, sh.misc);
   __syncthreads();
   const GdFlatBounds b = gd_flat_bounds_load(sh.misc);
@@ -313,11 +435,44 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
       queue[i] = -1;
     } else {
       sh.misc[11] = 1;
+      atomicMin(&sh.misc[2], py); atomicMax(&sh.misc[3], py);
+      atomicOr(&columns[px >> 5], 1u << (px & 31));
     }
   }
   __syncthreads();
   if (sh.misc[11] == 0) return;                       /* block-uniform: nothing unresolved */
   if (!sweepDone) {
+    if (queued <= GD_FALLBACK_MAX) {
+      if (tid < GD_WARPS) {
+        const unsigned a = columns[tid], l = tid > 0 ? columns[tid - 1] : 0u, r = tid < GD_WARPS - 1 ? columns[tid + 1] : 0u;
+        unsigned near = a;
+#pragma unroll 1
+        for (int s = 1; s <= GD_FLAT_WINDOW; ++s) near |= (a << s) | (l >> (32 - s)) | (a >> s) | (r << (32 - s));
+        columns[16 + tid] = near;
+      }
+      __syncthreads();
+      int c = 0, rank = 0;
+#pragma unroll 1
+      for (int w = 0; w < GD_WARPS; ++w) {
+        const unsigned near = columns[16 + w];
+        if (w < warp) rank += __popc(near);
+        else if (w == warp) rank += __popc(near & ((1u << (tid & 31)) - 1u));
+        c += __popc(near);
+      }
+      if (c <= GD_SW / 2) {                           /* block-uniform */
+        if ((columns[16 + warp] >> (tid & 31)) & 1u) list[rank] = (short)tid;
+        const int minY = sh.misc[2], maxY = sh.misc[3];
+        __syncthreads();
+        gd_flat_sweep(sc, v, sh, b, currentSector, vsec, c, minY, maxY);
+        gd_flat_repaired(sc, v, sh, vsec, queue, count, GD_FLAT_WINDOW);
+        __syncthreads();
+        if (sh.misc[12] == 0) return;                 /* block-uniform */
+      }
+    }
+    __syncthreads();
+    if (tid == 0) { sh.misc[2] = GD_VH; sh.misc[3] = -1; }
+    list[tid] = (short)tid;
+    __syncthreads();
     {
       const unsigned *own = owned + tid;
       int lo = GD_VH, hi = -1;
@@ -330,70 +485,10 @@ __device__ void gd_fallback_pass(const GdScene &sc_, const GdView &v_, const GdS
     }
     __syncthreads();
     const int minY = sh.misc[2], maxY = sh.misc[3];
-    const GdFlatRay r = gd_flat_ray(sc, v, tid);
-    const int flipRow = gd_clamp((int)floorf(r.center) + 1, 0, GD_VH);   /* first floor row */
-    /* nearest resolved row below maxY, of maxY's orientation */
-    bool haveBelow = false, belowFloor = false;
-    int belowSector = 0;
-    const int limit = maxY < flipRow ? flipRow : GD_VH;
-#pragma unroll 1
-    for (int y = maxY + 1; y < limit; ++y) {
-      GdFlatProbe q = gd_flat_probe(sc, v, r, b, y, currentSector);
-      if (!q.unresolved) { haveBelow = true; belowFloor = q.isFloor; belowSector = q.sector; break; }
-    }
-    __syncwarp();
-#pragma unroll 1
-    for (int y = maxY; y >= minY; --y) {
-      GdFlatProbe q = gd_flat_probe(sc, v, r, b, y, currentSector);
-      bool anchor;
-      int repaired;
-      if (!q.unresolved) {
-        anchor = true;
-        repaired = q.sector;
-        haveBelow = true; belowFloor = q.isFloor; belowSector = q.sector;
-      } else {
-        bool spans = haveBelow && belowFloor == q.isFloor;
-        repaired = spans ? belowSector : currentSector;
-        anchor = spans && belowSector != currentSector;
-      }
-      vsec[y * GD_SW + tid] = (unsigned short)repaired;
-      unsigned m = __ballot_sync(0xffffffffu, anchor);
-      if (lane == 0) anchors[y * GD_WARPS + warp] = m;
-    }
+    gd_flat_sweep(sc, v, sh, b, currentSector, vsec, GD_SW, minY, maxY);
     sweepDone = true;
-    __threadfence_block();
-    __syncthreads();
   }
-#pragma unroll 1
-  for (int i = tid; i < count; i += GD_THREADS) {
-    if (queue[i] < 0) continue;
-    const int px = queue[i] & 0xFFFF, py = queue[i] >> 16;
-    int sector = vsec[py * GD_SW + px];
-    /* nearest anchor at or left of px, at or right of px */
-    int left = -1, right = -1;
-#pragma unroll 1
-    for (int w = 0; w < GD_WARPS; ++w) {
-      unsigned bits = anchors[py * GD_WARPS + w];
-      int base = w * 32;
-      if (base <= px) {
-        unsigned lo = px - base >= 31 ? bits : (bits & ((2u << (px - base)) - 1u));
-        if (lo) left = base + 31 - __clz(lo);
-      }
-      if (base + 31 >= px && right < 0) {
-        unsigned hi = px - base <= 0 ? bits : (bits & ~((1u << (px - base)) - 1u));
-        if (hi) right = base + __ffs(hi) - 1;
-      }
-    }
-    if (left >= 0 && right >= 0) {
-      int sl = vsec[py * GD_SW + left], sr = vsec[py * GD_SW + right];
-      if (sl == sr) sector = sl;
-    }
-    const bool isFloor = ((float)py - gd_flat_ray(sc, v, px).center) > 0;
-    GdPlaneSpan p;
-    gd_plane_setup(sc, sh.planeTab, sector, isFloor, px, p);
-    sh.frame[py * GD_SW + px] = (uint8_t)gd_plane_pixel(sc, p, v.center, py);
-    atomicOr(&owned[(py >> 5) * GD_SW + px], 1u << (py & 31));
-  }
+  gd_flat_repaired(sc, v, sh, vsec, queue, count, GD_SW);
   __syncthreads();
 }
 

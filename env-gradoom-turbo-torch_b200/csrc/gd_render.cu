@@ -142,6 +142,8 @@ struct GdActor {
 #define GD_AUX_BYTES (8 * 320 * 4)
 #define GD_OFF_AUX2 (GD_OFF_AUX + GD_AUX_BYTES)            /* 4,096: sectors of points, status-bar list, sprite columns, chip spans */
 #define GD_AUX2_BYTES 4096
+#define GD_OFF_FLAT_LIST (GD_OFF_AUX2 + GD_SW * 4)         /* flat fallback, behind a word a column: three lists of columns */
+static_assert(GD_SW * 4 + 3 * GD_SW * 2 <= GD_AUX2_BYTES, "the lists");
 #define GD_OFF_HOT (GD_OFF_AUX2 + GD_AUX2_BYTES)           /* W wall records */
 /* the resize, when all before it is done: its sums from the masks on, the result behind them */
 #define GD_OFF_RESULT ((GD_OFF_MASKS + 7 * GD_SW * 8 + 15) / 16 * 16)
