@@ -185,6 +185,12 @@ struct __align__(8) GdWall {
   int tx[2], ty[2];                   /* view coordinates in stored endpoint order */
 };
 
+/* A segment's ends in view coordinates (20.12), and the screen columns they project to. */
+struct GdEnds {
+  i64 tx0, ty0, tx1, ty1, column0, column1;
+  bool front;                         /* the viewer is on its front side */
+};
+
 /* What the column walk reads of a wall of the lane being drawn, kept in shared memory: the ray test's
  * lane-dependent operands, the owned columns and the sectors on its two sides.  A wall outside the
  * frustum has dn = 0 and an empty span, so no column ray ever meets it. */
@@ -203,7 +209,7 @@ struct __align__(16) GdHot {
 #define GD_HOT_NEIGHBOUR (1u << 23)   /* another line between the same two sectors shares an endpoint */
 #define GD_HOT_BRIDGE0 (1u << 24)     /* one-sided lines that may own the columns past its start, past its end */
 #define GD_HOT_BRIDGE1 (1u << 25)
-#define GD_HOT_STATIC (GD_HOT_SPLIT | GD_HOT_NEIGHBOUR | GD_HOT_BRIDGE0 | GD_HOT_BRIDGE1)
+#define GD_HOT_STATIC (GD_HOT_ONESIDED | GD_HOT_SPLIT | GD_HOT_NEIGHBOUR | GD_HOT_BRIDGE0 | GD_HOT_BRIDGE1)
 
 /* Everything of a crossing that depends on the wall and the side it is seen from alone; built by every
  * launch.  The flags assume that the sectors of the crossing are the wall's own two. */

@@ -35,74 +35,45 @@ __device__ __forceinline__ void gd_ray(const GdView &v, int x, float &rx, float 
   ry = v.fsin - v.fcos * c;
 }
 
-/* FWallCoords (engine.py:10791-10869) */
-__device__ void gd_fwall_coords(i64 tx1, i64 ty1, i64 tx2, i64 ty2, i64 &sl, i64 &sr, i64 &dl, i64 &dr) {
-  const i64 cf = 160 * GD_FU;
-  i64 sty1 = ty1 == 0 ? 1 : ty1, sty2 = ty2 == 0 ? 1 : ty2;
-  i64 lp = (cf + gd_div(tx1 * cf, sty1)) >> 16;
-  lp += (tx1 >= 0);
-  if (tx1 >= 0) lp = gd_min(lp, GD_SW);
-  i64 rp = (cf + gd_div(tx2 * cf, sty2)) >> 16;
-  rp += (tx2 >= 0);
-  if (tx2 >= 0) rp = gd_min(rp, GD_SW);
-  i64 lden = tx1 - tx2 - ty2 + ty1, rden = ty2 - ty1 - tx2 + tx1;
-  i64 slden = lden == 0 ? 1 : lden, srden = rden == 0 ? 1 : rden;
-  bool lin = tx1 >= -ty1, rin = tx2 <= ty2;
-  i64 screenL = lin ? lp : 0, screenR = rin ? rp : GD_SW;
-  i64 depthL = lin ? ty1 : ty1 + gd_div((ty2 - ty1) * (tx1 + ty1), slden);
-  i64 depthR = rin ? ty2 : ty1 + gd_div((ty2 - ty1) * (tx1 - ty1), srden);
-  bool invL = (lin ? ((tx1 > ty1) || (ty1 == 0)) : ((tx2 < -ty2) || (lden == 0))) || (depthL < 32);
-  bool invR = (rin ? ((tx2 < -ty2) || (ty2 == 0)) : ((tx1 > ty1) || (rden == 0))) || (depthR < 32);
-  bool inv = invL || invR || (screenR <= screenL);
-  if (inv) screenR = screenL;
-  sl = screenL; sr = screenR; dl = depthL; dr = depthR;
-}
-
-/* wallscan light for one endpoint order (engine.py:11217-11291) */
-__device__ void gd_wall_visibility(i64 tx1, i64 ty1, i64 tx2, i64 ty2, i64 &visL, i64 &visStep, i64 &visSl) {
-  const i64 cf = 160 * GD_FU;
-  i64 sty1 = ty1 == 0 ? 1 : ty1, sty2 = ty2 == 0 ? 1 : ty2;
-  i64 lp = ((cf + gd_div(tx1 * cf, sty1)) >> 16) + (tx1 >= 0);
-  i64 rp = ((cf + gd_div(tx2 * cf, sty2)) >> 16) + (tx2 >= 0);
-  i64 lden = tx1 - tx2 - ty2 + ty1, rden = ty2 - ty1 - tx2 + tx1;
-  i64 slden = lden == 0 ? 1 : lden, srden = rden == 0 ? 1 : rden;
-  bool lin = tx1 >= -ty1, rin = tx2 <= ty2;
-  i64 wsl = lin ? lp : 0, wsr = rin ? rp : GD_SW;
-  i64 wdl = lin ? ty1 : ty1 + gd_div((ty2 - ty1) * (tx1 + ty1), slden);
-  i64 wdr = rin ? ty2 : ty1 + gd_div((ty2 - ty1) * (tx1 - ty1), srden);
-  i64 ll = gd_div(GD_WALL_VIS << 12, gd_max(wdl, 1));
-  i64 lr = gd_div(GD_WALL_VIS << 12, gd_max(wdr, 1));
-  visStep = gd_div(lr - ll, gd_max(wsr - wsl, 1));
-  visL = ll;
-  visSl = wsl;
-}
-
-/* View coordinates, FWallCoords and wallscan light of a segment given by its 16.16 endpoints
- * (engine.py:10747-10869, 11207-11302). */
-__device__ __noinline__ void gd_project_fixed(const GdView &v, const i64 fx[2], const i64 fy[2], GdWall &out) {
-  i64 tx[2], ty[2];
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    i64 rx = fx[e] - v.vx, ry = fy[e] - v.vy;
-    tx[e] = (rx * v.vsin - ry * v.vcos) >> 20;
-    ty[e] = (rx * v.vcos + ry * v.vsin) >> 20;
-    out.tx[e] = (int)tx[e];
-    out.ty[e] = (int)ty[e];
-  }
-  i64 wvx = fx[1] - fx[0], wvy = fy[1] - fy[0];
-  i64 fsx = v.vx - fx[0], fsy = v.vy - fy[0];
-  bool ff = (wvx * fsy - wvy * fsx) < 0;
-  int a = ff ? 0 : 1, b = ff ? 1 : 0;
-  i64 sl, sr, dl, dr;
-  gd_fwall_coords(tx[a], ty[a], tx[b], ty[b], sl, sr, dl, dr);
-  out.sl = sl; out.sr = sr; out.dl = dl; out.dr = dr;
-  i64 ax = tx[0], ay = ty[0], bx = tx[1], by = ty[1];
+/* View coordinates of a segment's 16.16 endpoints, and the screen column that each projects to (engine.py:10747-10790).
+ * Two divisions serve everything below: FWallCoords and the light of either side start from these columns. */
+__device__ __forceinline__ void gd_project_ends(const GdView &v, const i64 fx[2], const i64 fy[2], GdEnds &e) {
 #pragma unroll 1
-  for (int side = 0; side < 2; ++side) {
-    gd_wall_visibility(ax, ay, bx, by, out.visL[side], out.visStep[side], out.visSl[side]);
-    const i64 x = ax, y = ay;
-    ax = bx; ay = by; bx = x; by = y;
+  for (int k = 0; k < 2; ++k) {
+    const i64 rx = (k ? fx[1] : fx[0]) - v.vx, ry = (k ? fy[1] : fy[0]) - v.vy;
+    const i64 tx = (rx * v.vsin - ry * v.vcos) >> 20, ty = (rx * v.vcos + ry * v.vsin) >> 20;
+    const i64 cf = 160 * GD_FU;
+    const i64 column = ((cf + gd_div(tx * cf, ty == 0 ? 1 : ty)) >> 16) + (tx >= 0);
+    if (k) { e.tx1 = tx; e.ty1 = ty; e.column1 = column; } else { e.tx0 = tx; e.ty0 = ty; e.column0 = column; }
   }
+  const i64 wvx = fx[1] - fx[0], wvy = fy[1] - fy[0];
+  const i64 fsx = v.vx - fx[0], fsy = v.vy - fy[0];
+  e.front = (wvx * fsy - wvy * fsx) < 0;
+}
+
+/* The segment taken in its stored order (side 0) or the other way round (side 1): wallscan light of that side
+ * (engine.py:11217-11291), and FWallCoords (10791-10869) of the side that faces the viewer. */
+__device__ __noinline__ void gd_project_side(const GdEnds &e, int side, GdWall &out) {
+  const i64 tx1 = side ? e.tx1 : e.tx0, ty1 = side ? e.ty1 : e.ty0, tx2 = side ? e.tx0 : e.tx1, ty2 = side ? e.ty0 : e.ty1;
+  const i64 lp = side ? e.column1 : e.column0, rp = side ? e.column0 : e.column1;
+  const i64 lden = tx1 - tx2 - ty2 + ty1, rden = ty2 - ty1 - tx2 + tx1;
+  const bool lin = tx1 >= -ty1, rin = tx2 <= ty2;
+  const i64 wsl = lin ? lp : 0, wsr = rin ? rp : GD_SW;
+  i64 depthL = ty1, depthR = ty2;
+  if (!lin) depthL = ty1 + gd_div((ty2 - ty1) * (tx1 + ty1), lden == 0 ? 1 : lden);
+  if (!rin) depthR = ty1 + gd_div((ty2 - ty1) * (tx1 - ty1), rden == 0 ? 1 : rden);
+  const i64 ll = gd_div(GD_WALL_VIS << 12, gd_max(depthL, 1));
+  const i64 lr = gd_div(GD_WALL_VIS << 12, gd_max(depthR, 1));
+  out.visStep[side] = gd_div(lr - ll, gd_max(wsr - wsl, 1));
+  out.visL[side] = ll;
+  out.visSl[side] = wsl;
+  if (e.front != (side == 0)) return;
+  const i64 screenL = lin && tx1 >= 0 ? gd_min(wsl, GD_SW) : wsl;
+  i64 screenR = rin && tx2 >= 0 ? gd_min(wsr, GD_SW) : wsr;
+  const bool invL = (lin ? ((tx1 > ty1) || (ty1 == 0)) : ((tx2 < -ty2) || (lden == 0))) || (depthL < 32);
+  const bool invR = (rin ? ((tx2 < -ty2) || (ty2 == 0)) : ((tx1 > ty1) || (rden == 0))) || (depthR < 32);
+  if (invL || invR || (screenR <= screenL)) screenR = screenL;
+  out.sl = screenL; out.sr = screenR; out.dl = depthL; out.dr = depthR;
 }
 
 /* Crossing record of side i & 1 of wall i >> 1.  Texture indices are passed on as they are (the checked build tests
@@ -142,33 +113,6 @@ __device__ __forceinline__ void gd_side_setup(const GdScene &sc, int i, GdSide &
   out = o;
 }
 
-/* Project wall w of the map for this lane (engine.py:10747-10869, 11207-11302,
- * 11359-11427), and the lane-dependent operands of its column-ray test.  The
- * ray-owned span is completed by gd_wall_spans below. */
-__device__ __forceinline__ void gd_project_wall(const GdScene &sc, const GdView &v, int w, GdWall &out, GdHot &hot) {
-  const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
-  const i64 fx[2] = {gd_rint(wl.x * 65536.0f), gd_rint(wl.z * 65536.0f)};
-  const i64 fy[2] = {gd_rint(wl.y * 65536.0f), gd_rint(wl.w * 65536.0f)};
-  gd_project_fixed(v, fx, fy, out);
-  const bool oneSided = gd_wsec(sc, w * 2 + 1) < 0;
-  const float segx = wl.z - wl.x, segy = wl.w - wl.y;
-  const float vfsx = v.x - wl.x, vfsy = v.y - wl.y;
-  const bool front = (segx * vfsy - segy * vfsx) < 0;
-  hot.segx = segx; hot.segy = segy;
-  hot.offx = wl.x - v.x; hot.offy = wl.y - v.y;
-  hot.dn = hot.offx * segy - hot.offy * segx;
-  const unsigned sl = (unsigned)(gd_clamp(out.sl, -1, GD_SW + 1) + 1), sr = (unsigned)(gd_clamp(out.sr, -1, GD_SW + 1) + 1);
-  hot.bits = sl | (sr << 10) | (oneSided ? GD_HOT_ONESIDED : 0u) | (front ? GD_HOT_FRONT : 0u) | (hot.bits & GD_HOT_STATIC);
-}
-
-/* One piece of a line a node builder split (engine.py:11478-11500): projected like a line, from its
- * own fixed-point endpoints.  Only its FWallCoords and its wallscan light are ever read. */
-__device__ __forceinline__ void gd_project_fragment(const GdScene &sc, const GdView &v, int f, GdWall &out) {
-  const int4 q = *reinterpret_cast<const int4 *>(&sc.fragFixed[f * 4]);
-  const i64 fx[2] = {q.x, q.z}, fy[2] = {q.y, q.w};
-  gd_project_fixed(v, fx, fy, out);
-}
-
 /* Does the column ray (rx, ry) cross the wall (engine.py:11317-11331)?  The
  * comparisons of the rounded quotients dn / den and an / den with 0 and 1 depend
  * only on signs and magnitudes: both numerators are differences of products of
@@ -182,6 +126,79 @@ __device__ __forceinline__ bool gd_ray_geo(const GdHot &h, float rx, float ry) {
   const bool positive = (h.dn != 0.0f) && ((h.dn < 0) == (safe < 0));
   const bool alongOk = (an == 0.0f) || (((an < 0) == (safe < 0)) && fabsf(an) <= fabsf(safe));
   return !(fabsf(den) < 1e-6f) && positive && alongOk;
+}
+
+/* First and last column whose ray crosses a wall, as a span word, found at the projections of its ends.
+ * A ray's cross product with an endpoint is linear in the column, with a slope of its depth / 160.  With both ends
+ * at least 8 units deep and no coordinate above 16384 the rounding of the test moves a crossing's edge by less than
+ * half a column, and that of the projections below by less than a tenth: every column more than one inside the
+ * projected ends gives the same answer, and every one more than one outside is not crossed.  So the four columns
+ * around either end decide.  A wall that does not qualify gets GD_SPAN_SWEEP: all columns are tried. */
+#define GD_SPAN_SWEEP 0xFFFEFFFEu
+__device__ __forceinline__ unsigned gd_crossed_columns(const GdView &v, const GdHot &h) {
+  const float bx = h.offx + h.segx, by = h.offy + h.segy;
+  const float size = fmaxf(fmaxf(fabsf(h.offx), fabsf(h.offy)), fmaxf(fabsf(bx), fabsf(by)));
+  const float da = h.offx * v.fcos + h.offy * v.fsin, db = bx * v.fcos + by * v.fsin;
+  if (!(size <= 16384.0f && fminf(da, db) >= 8.0f)) return GD_SPAN_SWEEP;
+  const float ca = 160.0f + 160.0f * ((h.offx * v.fsin - h.offy * v.fcos) / da);
+  const float cb = 160.0f + 160.0f * ((bx * v.fsin - by * v.fcos) / db);
+  const float low = floorf(fminf(ca, cb)) - 1.0f, high = ceilf(fmaxf(ca, cb)) + 1.0f;
+  if (high < 0.0f || low > (float)(GD_SW - 1)) return 0xFFFFu;
+  const int lo = (int)fmaxf(low, 0.0f), hi = (int)fminf(high, (float)(GD_SW - 1));
+  int first = -1, last = -1;
+#pragma unroll 1
+  for (int k = 0; k < 8; ++k) {
+    const int x = min(max(k < 4 ? lo + k : hi - 7 + k, lo), hi);
+    float rx, ry;
+    gd_ray(v, x, rx, ry);
+    if (!gd_ray_geo(h, rx, ry)) continue;
+    if (first < 0) first = x;
+    last = max(last, x);
+  }
+  return ((unsigned)first & 0xFFFFu) | ((unsigned)(last + 1) << 16);
+}
+
+/* One half of the projection of wall w for this lane (engine.py:10747-10869, 11207-11302, 11359-11427), by a
+ * thread of its own: side 0, the lane-dependent operands of the column-ray test and the ends' columns, or side 1 and the
+ * columns whose rays cross the wall.  What bounds it is the latency of one thread's divisions: one after the other, for
+ * both sides, the ends and the light terms more than once, they were twenty, and span tables and things went before them
+ * (one lane alone 112 us a step, now 109; 4096 lanes 3036 and 2998). */
+__device__ __noinline__ void gd_project_wall(const GdScene &sc, const GdView &v, int w, int side, GdWall &out, GdHot &hot, int2 &columns) {
+  const float4 wl = *reinterpret_cast<const float4 *>(&sc.walls[w * 4]);
+  const i64 fx[2] = {gd_rint(wl.x * 65536.0f), gd_rint(wl.z * 65536.0f)};
+  const i64 fy[2] = {gd_rint(wl.y * 65536.0f), gd_rint(wl.w * 65536.0f)};
+  GdEnds e;
+  gd_project_ends(v, fx, fy, e);
+  gd_project_side(e, side, out);
+  GdHot mine;
+  mine.segx = wl.z - wl.x; mine.segy = wl.w - wl.y;
+  mine.offx = wl.x - v.x; mine.offy = wl.y - v.y;
+  mine.dn = mine.offx * mine.segy - mine.offy * mine.segx;
+  if (e.front == (side == 0)) {
+    const float vfsx = v.x - wl.x, vfsy = v.y - wl.y;
+    const bool front = (mine.segx * vfsy - mine.segy * vfsx) < 0;
+    const unsigned sl = (unsigned)(gd_clamp(out.sl, -1, GD_SW + 1) + 1), sr = (unsigned)(gd_clamp(out.sr, -1, GD_SW + 1) + 1);
+    hot.bits = sl | (sr << 10) | (front ? GD_HOT_FRONT : 0u) | (hot.bits & GD_HOT_STATIC);
+  }
+  if (side == 0) {
+    hot.segx = mine.segx; hot.segy = mine.segy; hot.offx = mine.offx; hot.offy = mine.offy; hot.dn = mine.dn;
+    out.tx[0] = (int)e.tx0; out.tx[1] = (int)e.tx1;
+    out.ty[0] = (int)e.ty0; out.ty[1] = (int)e.ty1;
+    columns = make_int2((int)gd_clamp(e.column0, -1, GD_SW + 1), (int)gd_clamp(e.column1, -1, GD_SW + 1));
+  } else {
+    hot.span = gd_crossed_columns(v, mine);
+  }
+}
+
+/* One piece of a line a node builder split (engine.py:11478-11500): projected like a line, from its
+ * own fixed-point endpoints.  Only its FWallCoords and its wallscan light are ever read. */
+__device__ __forceinline__ void gd_project_fragment(const GdScene &sc, const GdView &v, int f, GdWall &out) {
+  const int4 q = *reinterpret_cast<const int4 *>(&sc.fragFixed[f * 4]);
+  const i64 fx[2] = {q.x, q.z}, fy[2] = {q.y, q.w};
+  GdEnds e;
+  gd_project_ends(v, fx, fy, e);
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) gd_project_side(e, side, out);
 }
 
 /* Does the ray meet the wall's line in front of the viewer (the `positive` of engine.py:11317-11331)? */
@@ -614,49 +631,11 @@ __device__ __forceinline__ bool gd_wall_in_frustum(const float4 wl, const GdView
   return true;
 }
 
-/* First and last column whose ray crosses a wall, as a span word, found at the projections of its ends.
- * A ray's cross product with an endpoint is linear in the column, with a slope of its depth / 160.  With both ends
- * at least 8 units deep and no coordinate above 16384 the rounding of the test moves a crossing's edge by less than
- * half a column, and that of the projections below by less than a tenth: every column more than one inside the
- * projected ends gives the same answer, and every one more than one outside is not crossed.  So the four columns
- * around either end decide.  A wall that does not qualify gets GD_SPAN_SWEEP: all columns are tried. */
-#define GD_SPAN_SWEEP 0xFFFEFFFEu
-__device__ __forceinline__ unsigned gd_crossed_columns(const GdView &v, const GdHot &h) {
-  const float bx = h.offx + h.segx, by = h.offy + h.segy;
-  const float size = fmaxf(fmaxf(fabsf(h.offx), fabsf(h.offy)), fmaxf(fabsf(bx), fabsf(by)));
-  const float da = h.offx * v.fcos + h.offy * v.fsin, db = bx * v.fcos + by * v.fsin;
-  if (!(size <= 16384.0f && fminf(da, db) >= 8.0f)) return GD_SPAN_SWEEP;
-  const float ca = 160.0f + 160.0f * ((h.offx * v.fsin - h.offy * v.fcos) / da);
-  const float cb = 160.0f + 160.0f * ((bx * v.fsin - by * v.fcos) / db);
-  const float low = floorf(fminf(ca, cb)) - 1.0f, high = ceilf(fmaxf(ca, cb)) + 1.0f;
-  if (high < 0.0f || low > (float)(GD_SW - 1)) return 0xFFFFu;
-  const int lo = (int)fmaxf(low, 0.0f), hi = (int)fminf(high, (float)(GD_SW - 1));
-  int first = -1, last = -1;
-#pragma unroll 1
-  for (int k = 0; k < 8; ++k) {
-    const int x = min(max(k < 4 ? lo + k : hi - 7 + k, lo), hi);
-    float rx, ry;
-    gd_ray(v, x, rx, ry);
-    if (!gd_ray_geo(h, rx, ry)) continue;
-    if (first < 0) first = x;
-    last = max(last, x);
-  }
-  return ((unsigned)first & 0xFFFFu) | ((unsigned)(last + 1) << 16);
-}
-
 /* Lists the walls that a column ray may cross, and with them wall 0 and the first blocking wall, which the
- * rules fall back to; projects them; finds their ray-owned spans.  Every other wall gets the record no ray
- * meets.  The list stays in aux until the walk begins. */
-__device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShared &sh_) {
-  const GdScene &sc = *gd_as_shared(&sc_);
-  const GdView &v = *gd_as_shared(&v_);
-  const GdShared &sh = *gd_as_shared(&sh_);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  GdWall *walls = sh.walls;
+ * rules fall back to.  Every other wall gets the record no ray meets.  The list stays in aux until the walk begins. */
+__device__ __forceinline__ void gd_wall_list(const GdScene &sc, const GdView &v) {
   short *list = (short *)(gd_smem + GD_OFF_AUX);
   int *listed = (int *)(gd_smem + GD_OFF_MISC) + 2;
-  if (threadIdx.x == 0) *listed = 0;
-  __syncthreads();
   const int block0 = GD_CHECK_INDEX(sc.blocking[0], sc.W);
 #pragma unroll 1
   for (int w = threadIdx.x; w < sc.W; w += GD_THREADS) {
@@ -668,15 +647,16 @@ __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShar
       gd_hot(w).span = 0xFFFFu;
     }
   }
-  __syncthreads();
-  const int n = *listed;
-#pragma unroll 1
-  for (int i = threadIdx.x; i < n; i += GD_THREADS) {
-    const int w = list[i];
-    gd_project_wall(sc, v, w, walls[w], gd_hot(w));
-    gd_hot(w).span = gd_crossed_columns(v, gd_hot(w));
-  }
-  __syncthreads();
+}
+
+/* The ray-owned spans of the listed walls, which are projected; `prep` still holds the columns of their ends. */
+__device__ __forceinline__ void gd_wall_spans(const GdView &v_, const GdShared &sh_, const float4 *prep) {
+  const GdView &v = *gd_as_shared(&v_);
+  const GdShared &sh = *gd_as_shared(&sh_);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const GdWall *walls = sh.walls;
+  const short *list = (const short *)(gd_smem + GD_OFF_AUX);
+  const int n = ((const int *)(gd_smem + GD_OFF_MISC))[2];
 #pragma unroll 1
   for (int i = warp; i < n; i += GD_WARPS) {
     const int w = list[i];
@@ -700,33 +680,30 @@ __device__ void gd_wall_spans(const GdScene &sc_, const GdView &v_, const GdShar
   for (int i = threadIdx.x; i < n; i += GD_THREADS) {
     const int w = list[i];
     const GdWall &wv = walls[w];
+    const int2 ends = *reinterpret_cast<const int2 *>(&prep[w]);
+    const int column[2] = {ends.x, ends.y};
     GdHot &hot = gd_hot(w);
     const int first = (short)(hot.span & 0xFFFFu), end = (int)(hot.span >> 16);
     bool hasColumns = first >= 0;
-    i64 isl = hasColumns ? first : 0;
-    i64 isr = hasColumns ? end : GD_SW;
-    const i64 cf = 160 * GD_FU;
-    i64 ecol[2];
+    int isl = hasColumns ? first : 0;
+    int isr = hasColumns ? end : GD_SW;
     bool evis[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      i64 ty = wv.ty[e], tx = wv.tx[e];
-      i64 sty = ty == 0 ? 1 : ty;
-      i64 pf = cf + gd_div(tx * cf, sty);
-      ecol[e] = (pf >> 16) + (tx >= 0);
-      evis[e] = ty > 0 && tx >= -ty && tx <= ty && ecol[e] >= 0 && ecol[e] <= GD_SW;
+      const int ty = wv.ty[e], tx = wv.tx[e];
+      evis[e] = ty > 0 && tx >= -ty && tx <= ty && column[e] >= 0 && column[e] <= GD_SW;
     }
     bool fff = (hot.bits & GD_HOT_FRONT) != 0;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       bool visible = evis[e] && hasColumns;
       bool ownsLeft = fff ? (e == 0) : (e == 1);
-      if (visible && ownsLeft) isl = ecol[e];
-      if (visible && !ownsLeft) isr = ecol[e];
+      if (visible && ownsLeft) isl = column[e];
+      if (visible && !ownsLeft) isr = column[e];
     }
     if (evis[0] && evis[1]) {
-      isl = ecol[fff ? 0 : 1];
-      isr = ecol[fff ? 1 : 0];
+      isl = column[fff ? 0 : 1];
+      isr = column[fff ? 1 : 0];
       hasColumns = isr > isl;
     }
     hasColumns = hasColumns && (wv.sr > wv.sl);

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     }
     if (tid < GD_LANE_WORDS) sh.lane[tid] = p.lanes[(size_t)l * GD_LANE_WORDS + tid];
     if (tid < GD_OWNER_WORDS) sh.ownerMask[tid] = 0;
-    if (tid == 0) sh.misc[1] = 0;
+    if (tid == 0) sh.misc[1] = sh.misc[2] = 0;
     /* sector of every thing and of the player (slot 64): lowest index that
      * contains the point (engine.py:9598-9617), found by warps 1 to 9
      * while thread 0 sets up the view */
@@ -363,18 +363,31 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
         const unsigned sl = (unsigned)gd_clamp(q.sl, 0, GD_SW), sr = (unsigned)gd_clamp(q.sr, 0, GD_SW);
         ((unsigned *)(gd_smem + p.offFrags))[f] = q.sr > q.sl ? sl | (sr << 16) : 0u;
       }
-#pragma unroll 1
-    for (int idx = GD_THREADS - 1 - tid; idx < sc.S * 2; idx += GD_THREADS)   /* the threads the things leave idle */
-      gd_plane_entry_setup(sc, v, idx >> 1, (idx & 1) != 0, sh.planeTab[idx], planes[idx]);
-#pragma unroll 1
-    for (int a = tid; a < nThings; a += GD_THREADS) {
-      int sector = pointSector[a] == 0x7fffffff ? 0 : pointSector[a];
-      gd_actor_setup(sc, v, p.things[(size_t)l * p.maxThings + a], sector, sh.actors[a]);
-    }
+    gd_wall_list(sc, v);
     if (tid == GD_THREADS - 1) sh.misc[0] = pointSector[64] == 0x7fffffff ? 0 : pointSector[64];
-    gd_wall_spans(sc, v, sh);
+    __syncthreads();
+    /* the setups of the lane's walls (a thread a side), span tables and things, side by side: what bounds each is the
+     * latency of its divisions */
     const short *frustumList = (const short *)(gd_smem + GD_OFF_AUX);
     const int frustumListed = sh.misc[2];
+    {
+      /* whole warps of one kind, the longest chains first */
+      const int wallTask = (nThings + 31) & ~31, planeTask = (wallTask + frustumListed * 2 + 31) & ~31;
+#pragma unroll 1
+      for (int task = tid; task < planeTask + sc.S * 2; task += GD_THREADS) {
+        if (task < nThings) {
+          gd_actor_setup(sc, v, p.things[(size_t)l * p.maxThings + task], pointSector[task] == 0x7fffffff ? 0 : pointSector[task], sh.actors[task]);
+        } else if (task >= planeTask) {
+          const int idx = task - planeTask;
+          gd_plane_entry_setup(sc, v, idx >> 1, (idx & 1) != 0, sh.planeTab[idx], planes[idx]);
+        } else if (task >= wallTask && task < wallTask + frustumListed * 2) {
+          const int i = task - wallTask, side = i >= frustumListed, w = frustumList[i - (side ? frustumListed : 0)];
+          gd_project_wall(sc, v, w, side, sh.walls[w], gd_hot(w), *reinterpret_cast<int2 *>(&prep[w]));
+        }
+      }
+    }
+    __syncthreads();
+    gd_wall_spans(v, sh, prep);
     __syncthreads();
     /* row projections, light and column operands of the listed walls (the walk selects no other wall) and of the
      * fragments in view */
