@@ -73,23 +73,25 @@ extern "C" const char *gd_error_string(int code) {
  * kernel's static shared memory, so renderers of different scenes can live side
  * by side.  Returns that limit, or -1. */
 typedef void (*gd_kernel_fn)(const GdParams);
-/* the instantiation that draws a scene: with or without the code for split lines, tables on chip or in scratch */
-static gd_kernel_fn gd_kernel_for(const gd_renderer *r) {
-  if (r->base.sc.F > 0) return r->chip ? gd_render_kernel<true, true> : gd_render_kernel<true, false>;
-  return r->chip ? gd_render_kernel<false, true> : gd_render_kernel<false, false>;
+/* the instantiations: without or with the code for split lines; tables in scratch or on chip; all kinds of launches or the
+ * plain ones */
+static const gd_kernel_fn gd_kernels[8] = {
+    gd_render_kernel<false, false, false>, gd_render_kernel<false, false, true>, gd_render_kernel<false, true, false>,
+    gd_render_kernel<false, true, true>, gd_render_kernel<true, false, false>, gd_render_kernel<true, false, true>,
+    gd_render_kernel<true, true, false>, gd_render_kernel<true, true, true>};
+static gd_kernel_fn gd_kernel_for(const gd_renderer *r, bool plain) {
+  return gd_kernels[(r->base.sc.F > 0 ? 4 : 0) + (r->chip ? 2 : 0) + (plain ? 1 : 0)];
 }
 
 static int gd_raise_shared_limit(int maxOptin) {
   int limit = maxOptin;
-  const gd_kernel_fn kernels[4] = {gd_render_kernel<false, false>, gd_render_kernel<true, false>, gd_render_kernel<false, true>,
-                                   gd_render_kernel<true, true>};
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < 8; ++k) {
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, kernels[k]) != cudaSuccess) return -1;
+    if (cudaFuncGetAttributes(&fa, gd_kernels[k]) != cudaSuccess) return -1;
     if (maxOptin - (int)fa.sharedSizeBytes < limit) limit = maxOptin - (int)fa.sharedSizeBytes;
   }
-  for (int k = 0; k < 4; ++k)
-    if (cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) return -1;
+  for (int k = 0; k < 8; ++k)
+    if (cudaFuncSetAttribute(gd_kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) return -1;
   return limit;
 }
 
@@ -211,12 +213,13 @@ extern "C" int gd_renderer_create(const void *blob_header_host, const void *blob
   } else if ((size_t)limit < r->smemBytes || (size_t)sc.W * 2 > GD_AUX_BYTES) {
     rc = GD_ERR_SHARED;
   } else {
-    int perSm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, gd_kernel_for(r), GD_THREADS, r->smemBytes) != cudaSuccess ||
-        perSm < 1)
+    int perSm = 0, perSmPlain = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, gd_kernel_for(r, false), GD_THREADS, r->smemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSmPlain, gd_kernel_for(r, true), GD_THREADS, r->smemBytes) != cudaSuccess ||
+        perSm < 1 || perSmPlain < 1)
       rc = GD_ERR_CUDA;
     else
-      r->ctas = sms * perSm;  /* one persistent CTA per resident slot */
+      r->ctas = sms * (perSm < perSmPlain ? perSm : perSmPlain);  /* one persistent CTA per resident slot */
   }
   if (sc.F > 0) r->fragBytes = gd_frag_bytes(sc.F, r->chip);
   if (rc == GD_OK && sc.F > 0 && gd_fits_static(sc)) {
@@ -295,14 +298,24 @@ extern "C" size_t gd_renderer_shared_bytes_view(const gd_renderer *r) { return r
 
 static int gd_draw(const gd_renderer *r, const GdParams &p, int grid, void *stream) {
   if (!r->chip) gd_side_setup_kernel<<<(p.sc.W * 2 + 127) / 128, 128, 0, (cudaStream_t)stream>>>(p.sc, p.sides);
-  gd_kernel_for(r)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
+  gd_kernel_for(r, !(p.flags & GD_F_STEP_RESET))<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
+}
+
+/* gd_render_step_reset: the old frames of the lanes that are reset, before the resets' frames take their place */
+__global__ void gd_final_frames_kernel(const uint8_t *mask, const uint4 *stack, uint4 *finalStack) {
+  const int frame = GD_OBS * GD_OBS / 16;
+  if (!mask[blockIdx.x]) return;
+  stack += (size_t)blockIdx.x * GD_STACK * frame;
+  finalStack += (size_t)blockIdx.x * GD_STACK * frame;
+  for (int i = threadIdx.x; i < (GD_STACK - 1) * frame; i += blockDim.x) finalStack[i] = stack[frame + i];
 }
 
 static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing *things, int n, int flags,
                      uint8_t *stack, const uint8_t *reset_mask, uint8_t *obs_out, uint8_t *indexed_out,
                      uint8_t *rgb_out, void *scratch, size_t scratch_bytes, int *status, void *stream,
-                     int ring_head = 0) {
+                     int ring_head = 0, const int32_t *reset_lanes = nullptr, const gd_thing *reset_things = nullptr,
+                     uint8_t *final_stack = nullptr) {
   if (!r || !lanes || !scratch || !status) return GD_ERR_NULL;
   if (r->maxThings > 0 && !things) return GD_ERR_NULL;
   if (n < 0) return GD_ERR_SIZE;
@@ -312,8 +325,10 @@ static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing 
   if (current != r->device) return GD_ERR_DEVICE;   /* the launch goes to the current device */
   if (scratch_bytes < gd_renderer_scratch_bytes(r)) return GD_ERR_SCRATCH;
   uintptr_t align = (uintptr_t)lanes | (uintptr_t)things | (uintptr_t)stack | (uintptr_t)obs_out |
-                    (uintptr_t)indexed_out | (uintptr_t)rgb_out | (uintptr_t)scratch;
+                    (uintptr_t)indexed_out | (uintptr_t)rgb_out | (uintptr_t)scratch | (uintptr_t)reset_lanes |
+                    (uintptr_t)reset_things | (uintptr_t)final_stack;
   if (align & 15) return GD_ERR_ALIGN;
+  if ((flags & GD_F_STEP_RESET) && n > 0x3FFFFFFF) return GD_ERR_SIZE;
   GdParams p = r->base;
   p.lanes = lanes; p.things = things; p.n = n; p.flags = flags;
   p.stack = stack; p.ringHead = ring_head; p.resetMask = reset_mask; p.obsOut = obs_out; p.indexedOut = indexed_out; p.rgbOut = rgb_out;
@@ -321,7 +336,13 @@ static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing 
   p.sides = (GdSide *)(p.scratch + r->sidesOffset);
   p.frags = p.scratch + gd_scratch_per_cta(r->base.sc.W, r->base.sc.S);
   p.decals = r->decals; p.decalSlots = r->decalSlots; p.decalScratch = r->decalScratch;
-  return gd_draw(r, p, n < r->ctas ? n : r->ctas, stream);
+  p.resetLanes = reset_lanes; p.resetThings = reset_things; p.finalStack = final_stack;
+  int frames = n;
+  if (flags & GD_F_STEP_RESET) {
+    frames = 2 * n;
+    gd_final_frames_kernel<<<n, 256, 0, (cudaStream_t)stream>>>(reset_mask, (const uint4 *)stack, (uint4 *)final_stack);
+  }
+  return gd_draw(r, p, frames < r->ctas ? frames : r->ctas, stream);
 }
 
 extern "C" int gd_render_step(const gd_renderer *r, const int32_t *lanes, const void *things, int n, int mask_hud,
@@ -362,6 +383,17 @@ extern "C" int gd_render_reset(const gd_renderer *r, const int32_t *lanes, const
   int flags = GD_F_STACK_FILL | (mask_hud ? GD_F_MASK_HUD : GD_F_DRAW_HUD);
   return gd_launch(r, lanes, (const gd_thing *)things, n, flags, stack, reset_mask, nullptr, nullptr, nullptr, scratch,
                    scratch_bytes, status, stream);
+}
+
+extern "C" int gd_render_step_reset(const gd_renderer *r, const int32_t *lanes, const void *things, const int32_t *reset_lanes,
+                                    const void *reset_things, int n, int mask_hud, const uint8_t *reset_mask, uint8_t *stack,
+                                    uint8_t *final_stack, void *scratch, size_t scratch_bytes, int *status, void *stream) {
+  if (r && n == 0) return GD_OK;   /* an empty batch needs no buffers */
+  if (!r || !stack || !final_stack || !reset_mask || !reset_lanes) return GD_ERR_NULL;
+  if (r->maxThings > 0 && !reset_things) return GD_ERR_NULL;
+  int flags = GD_F_STEP_RESET | (mask_hud ? GD_F_MASK_HUD : GD_F_DRAW_HUD);
+  return gd_launch(r, lanes, (const gd_thing *)things, n, flags, stack, reset_mask, nullptr, nullptr, nullptr, scratch,
+                   scratch_bytes, status, stream, 0, reset_lanes, (const gd_thing *)reset_things, final_stack);
 }
 
 extern "C" int gd_render_frames(const gd_renderer *r, const int32_t *lanes, const void *things, int n, int mask_hud,

@@ -50,6 +50,7 @@
 #define GD_F_STACK_FILL 8   /* write all four slots of lanes whose mask byte is set */
 #define GD_F_WRITE_OBS 16   /* write plain (n,84,84) observations to obsOut */
 #define GD_F_STACK_RING 32  /* the stack is a mirrored ring of eight slots per lane (see gd_render_step_ring) */
+#define GD_F_STEP_RESET 64  /* a step of every lane and a reset of the masked ones (see gd_render_step_reset) */
 
 struct GdParams {
   GdScene sc;
@@ -61,6 +62,9 @@ struct GdParams {
   uint8_t *stack;            /* n x 4 x 84 x 84, or n x 8 x 84 x 84 with GD_F_STACK_RING */
   int ringHead;              /* GD_F_STACK_RING: slot 0..3 that takes the new frame (and slot + 4) */
   const uint8_t *resetMask;  /* n, for GD_F_STACK_FILL */
+  const int32_t *resetLanes; /* GD_F_STEP_RESET: the records that the resets are drawn from ... */
+  const gd_thing *resetThings;
+  uint8_t *finalStack;       /* ... and the stacks as the step left them */
   uint8_t *obsOut;           /* n x 84 x 84, optional */
   uint8_t *indexedOut;       /* n x 240 x 320, optional */
   uint8_t *rgbOut;           /* n x 240 x 320 x 3, optional */
@@ -192,8 +196,9 @@ __device__ __forceinline__ int gd_vertex(const GdScene &sc, int w, int slot) { r
 /* ---- the kernel ----------------------------------------------------------- */
 
 /* kSplit: the scene carries projection fragments of split lines.  kChip: the walk's tables fit in shared memory
- * beside a second CTA. */
-template <bool kSplit, bool kChip>
+ * beside a second CTA.  kPlain: every task is one frame of a lane (the code for the other launches costs a step of 4096
+ * lanes 2 % and more, which only the calls that want it should pay). */
+template <bool kSplit, bool kChip, bool kPlain>
 __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_constant__ GdParams p) {
   /* The scene descriptor, the shared-memory map and the lane's view are read by
    * the phases around the walk through references; keeping them in shared memory (one copy
@@ -284,12 +289,16 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     __syncthreads();
     if (tid == 0) nextLane = (int)atomicAdd(&queue[0], 1u);
     __syncthreads();
-    const int l = nextLane;
-    if (l >= p.n) break;
-    if (p.flags & GD_F_STACK_FILL) {
-      if (p.resetMask && !p.resetMask[l]) continue;  /* uniform across the CTA */
-    }
-    if (tid < GD_LANE_WORDS) sh.lane[tid] = p.lanes[(size_t)l * GD_LANE_WORDS + tid];
+    /* a launch that steps and resets has both frames in one queue, the resets' first: as a launch of their own they
+     * waited for the slowest lane of the step (256 environment lanes 584 us a call, now 511; 1024 lanes 1227 and 1042) */
+    int l = nextLane;
+    const bool both = !kPlain && (p.flags & GD_F_STEP_RESET) != 0;
+    if (l >= (both ? 2 * p.n : p.n)) break;
+    const bool fill = both ? l < p.n : (p.flags & GD_F_STACK_FILL) != 0;
+    if (both && !fill) l -= p.n;
+    if (fill && p.resetMask && !p.resetMask[l]) continue;  /* uniform across the CTA */
+    const gd_thing *things = (both && fill ? p.resetThings : p.things) + (size_t)l * p.maxThings;
+    if (tid < GD_LANE_WORDS) sh.lane[tid] = (both && fill ? p.resetLanes : p.lanes)[(size_t)l * GD_LANE_WORDS + tid];
     if (tid < GD_OWNER_WORDS) sh.ownerMask[tid] = 0;
     if (tid == 0) sh.misc[1] = sh.misc[2] = 0;
     /* sector of every thing and of the player (slot 64): lowest index that
@@ -337,7 +346,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       for (int t = (tid - 32) / GD_POINT_THREADS; t <= nThings; t += (GD_THREADS - 32) / GD_POINT_THREADS) {
         float px = __int_as_float(sh.lane[GD_L_X]), py = __int_as_float(sh.lane[GD_L_Y]);
         if (t < nThings) {
-          const gd_thing &th = p.things[(size_t)l * p.maxThings + t];
+          const gd_thing &th = things[t];
           px = th.x; py = th.y;
         }
         const int s = gd_sector_of_point(sc, px, py);
@@ -376,7 +385,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
 #pragma unroll 1
       for (int task = tid; task < planeTask + sc.S * 2; task += GD_THREADS) {
         if (task < nThings) {
-          gd_actor_setup(sc, v, p.things[(size_t)l * p.maxThings + task], pointSector[task] == 0x7fffffff ? 0 : pointSector[task], sh.actors[task]);
+          gd_actor_setup(sc, v, things[task], pointSector[task] == 0x7fffffff ? 0 : pointSector[task], sh.actors[task]);
         } else if (task >= planeTask) {
           const int idx = task - planeTask;
           gd_plane_entry_setup(sc, v, idx >> 1, (idx & 1) != 0, sh.planeTab[idx], planes[idx]);
@@ -541,11 +550,27 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
         }
       } else if (p.stack) {
         uint4 *s0 = (uint4 *)(p.stack + (size_t)l * GD_STACK * GD_OBS * GD_OBS);
-        if (p.flags & GD_F_STACK_FILL) {
+        if (fill) {
 #pragma unroll 1
           for (int i = tid; i < vecs; i += GD_THREADS) {
             uint4 val = src[i];
             s0[i] = val; s0[vecs + i] = val; s0[2 * vecs + i] = val; s0[3 * vecs + i] = val;
+          }
+        } else if (both) {
+          /* the stack rolls, and what it becomes is copied out; a lane that is reset keeps only the copy, whose
+           * three old frames are there already */
+          uint4 *f0 = (uint4 *)(p.finalStack + (size_t)l * GD_STACK * GD_OBS * GD_OBS);
+          const bool ends = p.resetMask[l] != 0;
+#pragma unroll 1
+          for (int i = tid; i < vecs; i += GD_THREADS) {
+            const uint4 val = src[i];
+            f0[3 * vecs + i] = val;
+            if (ends) continue;
+            const uint4 a = s0[vecs + i], b = s0[2 * vecs + i], c = s0[3 * vecs + i];
+            f0[i] = s0[i] = a;
+            f0[vecs + i] = s0[vecs + i] = b;
+            f0[2 * vecs + i] = s0[2 * vecs + i] = c;
+            s0[3 * vecs + i] = val;
           }
         } else if (p.flags & GD_F_STACK_ROLL) {
 #pragma unroll 1

@@ -514,7 +514,48 @@ class GraDoomVecEnv:
         actions, self._pending_actions = self._pending_actions, None
         return self.step(actions)
 
+    def _one_launch(self, seeds) -> bool:
+        """May the step's frames and the restarted lanes' be drawn by one launch?  The lanes are then reset before the
+        step's frames are drawn, from a copy of their records.  That is the same for the built-in producer, whose reset
+        touches nothing but its own buffers; other producers, environments with rules of their own for a step or a
+        reset, rings, chips, and seeds that will be refused take the two calls one after the other."""
+
+        from .stepper import LaneStepper
+
+        producer = self._producer
+        if type(producer) is not LaneStepper or producer.renderer is not self._renderer or self.stack_policy != "roll" \
+                or self._renderer._decals is not None or self.closed:
+            return False
+        for owner, kind, rules in ((self, GraDoomVecEnv, ("step_device", "reset_device")),
+                                   (producer, LaneStepper, ("step", "reset", "render_inputs"))):
+            for rule in rules:
+                if getattr(getattr(owner, rule), "__func__", None) is not getattr(kind, rule):
+                    return False
+        return isinstance(seeds, torch.Tensor) and seeds.device == self.device and seeds.shape == (self.num_envs,) \
+            and seeds.dtype in _ACTION_DTYPES
+
+    def _step_and_reset_at_once(self, actions, reset_seeds) -> DeviceAutoResetTransition:
+        indices = require_device_tensor(actions, "actions", device=self.device, shape=(self.num_envs,),
+                                        dtypes=_ACTION_DTYPES).to(torch.int64)
+        rewards, terminated, truncated = self._producer.step(self._action_matrix[indices])
+        done = terminated | truncated
+        lanes, things = self._producer.render_inputs()
+        final_lanes, final_things = lanes.clone(), things.clone()
+        final_signals = self._producer.signal_buffer.clone()
+        self._producer.reset(done, reset_seeds.to(torch.int64))
+        lanes, things = self._producer.render_inputs()
+        final_frames = torch.empty_like(self._frames)
+        self._renderer.step_reset(final_lanes, final_things, lanes, things, done, self._frames, final_frames,
+                                  mask_hud=self.mask_hud)
+        self._initialized |= done
+        final_observations = final_frames if self.obs_layout == "chw" else final_frames.permute(0, 2, 3, 1)
+        return DeviceAutoResetTransition(self._device_observations(), rewards, terminated, truncated,
+                                         self._producer.signal_buffer, self._info_history, final_observations,
+                                         final_signals, self._info_history.clone())
+
     def step_and_reset_device(self, actions: torch.Tensor, reset_seeds: torch.Tensor) -> DeviceAutoResetTransition:
+        if self._one_launch(reset_seeds):
+            return self._step_and_reset_at_once(actions, reset_seeds)
         t = self.step_device(actions)
         final_observations = t.observations.clone()
         final_signals = t.signals.clone()

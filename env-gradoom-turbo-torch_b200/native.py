@@ -26,7 +26,7 @@ STATUS_BAD_STATE = 16
 
 EXPORTS = (
     "gd_error_string", "gd_renderer_create", "gd_renderer_destroy", "gd_renderer_scratch_bytes",
-    "gd_renderer_ctas", "gd_renderer_shared_bytes", "gd_renderer_shared_bytes_view", "gd_render_step", "gd_render_reset", "gd_render_frames",
+    "gd_renderer_ctas", "gd_renderer_shared_bytes", "gd_renderer_shared_bytes_view", "gd_render_step", "gd_render_reset", "gd_render_step_reset", "gd_render_frames",
     "gd_render_step_frames", "gd_render_step_host", "gd_render_step_ring", "gd_render_reset_ring", "gd_static_scratch_bytes", "gd_static_max_walls", "gd_render_step_static",
     "gd_pack_state_scratch_bytes", "gd_pack_state", "gd_player_tics", "gd_stepper_step", "gd_stepper_reset", "gd_renderer_bind_decals", "gd_probe_libm",
 )
@@ -67,6 +67,8 @@ def load(checked: bool = False) -> ctypes.CDLL:
         lib.gd_render_step.argtypes = [vp, vp, vp, ci, ci, vp, vp, sz, vp, vp]
         lib.gd_render_reset.restype = ci
         lib.gd_render_reset.argtypes = [vp, vp, vp, ci, ci, vp, vp, vp, sz, vp, vp]
+        lib.gd_render_step_reset.restype = ci
+        lib.gd_render_step_reset.argtypes = [vp, vp, vp, vp, vp, ci, ci, vp, vp, vp, vp, sz, vp, vp]
         lib.gd_render_frames.restype = ci
         lib.gd_render_frames.argtypes = [vp, vp, vp, ci, ci, ci, vp, vp, vp, vp, sz, vp, vp]
         lib.gd_render_step_frames.restype = ci
@@ -327,6 +329,24 @@ class Renderer:
                                         self.scratch_bytes, self.status.data_ptr(), self._stream()),
                "gd_render_reset")
         self.launches += 1
+
+    def step_reset(self, lanes, things, reset_lanes, reset_things, reset_mask, stack, final_stack, mask_hud=True):
+        """``step`` with ``lanes`` / ``things``, a copy of the stack to ``final_stack``, then ``reset`` of the lanes of
+        ``reset_mask`` (a bool tensor on the device) with ``reset_lanes`` / ``reset_things``, as one drawing launch."""
+
+        n = self._inputs(lanes, things)
+        if self._inputs(reset_lanes, reset_things) != n:
+            raise ValueError("the step's and the reset's records must be of the same lanes")
+        self._check_stack(stack, n)
+        self._check_stack(final_stack, n)
+        if reset_mask.dtype != torch.bool or tuple(reset_mask.shape) != (n,) or reset_mask.device != self.device:
+            raise TypeError("reset_mask must be a bool (N,) tensor on the renderer's device")
+        mask = reset_mask.contiguous()
+        _check(self.lib.gd_render_step_reset(self.handle, lanes.data_ptr(), things.data_ptr(), reset_lanes.data_ptr(),
+                                             reset_things.data_ptr(), n, int(mask_hud), mask.data_ptr(), stack.data_ptr(),
+                                             final_stack.data_ptr(), self.scratch.data_ptr(), self.scratch_bytes,
+                                             self.status.data_ptr(), self._stream()), "gd_render_step_reset")
+        self.launches += 2
 
     def frames(self, lanes, things, *, obs=False, indexed=False, rgb=False, mask_hud=True, include_hud=True):
         n = self._inputs(lanes, things)

@@ -133,6 +133,17 @@ int gd_render_reset(const gd_renderer *r, const int32_t *lanes, const void *thin
                     void *stream);
 
 /*
+ * A step of every lane and a reset of the lanes whose `reset_mask` byte is nonzero, in one launch of the drawing
+ * kernel: what gd_render_step with `lanes` / `things` does, then a copy of the whole stack to `final_stack` (n x 4 x
+ * 84 x 84 u8), then gd_render_reset with `reset_lanes` / `reset_things` (all n records; those of the masked lanes are
+ * read).  `final_stack` must not overlap the stack.  A bound decal ring belongs to both frames of its lane.
+ * Replaces: the step, the copy and the reset of step_and_reset_device (src/gradoom/env.py:998-1031).
+ */
+int gd_render_step_reset(const gd_renderer *r, const int32_t *lanes, const void *things, const int32_t *reset_lanes,
+                         const void *reset_things, int n, int mask_hud, const uint8_t *reset_mask, uint8_t *stack,
+                         uint8_t *final_stack, void *scratch, size_t scratch_bytes, int *status, void *stream);
+
+/*
  * gd_render_step / gd_render_reset on a mirrored ring instead of the reference's
  * oldest-first stack, for callers that accept a strided view: `ring` is
  * n x 8 x 84 x 84 u8, the new frame goes to slots `head` and `head + 4`
