@@ -296,9 +296,17 @@ extern "C" int gd_renderer_ctas(const gd_renderer *r) { return r ? r->ctas : 0; 
 extern "C" size_t gd_renderer_shared_bytes(const gd_renderer *r) { return r ? r->smemBytes : 0; }
 extern "C" size_t gd_renderer_shared_bytes_view(const gd_renderer *r) { return r ? r->smemBytes : 0; }
 
-static int gd_draw(const gd_renderer *r, const GdParams &p, int grid, void *stream) {
+/* `frames` frames by up to `ctas` CTAs.  When they are so few that three of four CTAs would idle, a lane is drawn by
+ * four of them, each a slice of its columns: what a lane waits for is its slowest warp, and then its sprites, unclaimed
+ * pixels and resize, which a slice has a quarter of.  (64 sectors, 12 things, us a step without and with slices: 1 lane 112 and
+ * 92, 16 lanes 322 and 297, 74 lanes 323 and 314.  Halves of a lane for the next 74 lanes do not pay for setting each
+ * lane up twice: 100 lanes 324 and 327, 148 lanes 326 and 351.) */
+static int gd_draw(const gd_renderer *r, GdParams &p, int frames, int ctas, bool slices, void *stream) {
+  p.sliceShift = slices && frames * 4LL <= ctas ? 2 : 0;
+  const long long tasks = ((long long)((p.flags & GD_F_STEP_RESET) ? 2 : 1) * frames) << p.sliceShift;
+  const int grid = tasks < ctas ? (int)tasks : ctas;
   if (!r->chip) gd_side_setup_kernel<<<(p.sc.W * 2 + 127) / 128, 128, 0, (cudaStream_t)stream>>>(p.sc, p.sides);
-  gd_kernel_for(r, !(p.flags & GD_F_STEP_RESET))<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
+  gd_kernel_for(r, !(p.flags & GD_F_STEP_RESET) && p.sliceShift == 0)<<<grid, GD_THREADS, r->smemBytes, (cudaStream_t)stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
 
@@ -315,7 +323,7 @@ static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing 
                      uint8_t *stack, const uint8_t *reset_mask, uint8_t *obs_out, uint8_t *indexed_out,
                      uint8_t *rgb_out, void *scratch, size_t scratch_bytes, int *status, void *stream,
                      int ring_head = 0, const int32_t *reset_lanes = nullptr, const gd_thing *reset_things = nullptr,
-                     uint8_t *final_stack = nullptr) {
+                     uint8_t *final_stack = nullptr, bool slices = true) {
   if (!r || !lanes || !scratch || !status) return GD_ERR_NULL;
   if (r->maxThings > 0 && !things) return GD_ERR_NULL;
   if (n < 0) return GD_ERR_SIZE;
@@ -337,12 +345,10 @@ static int gd_launch(const gd_renderer *r, const int32_t *lanes, const gd_thing 
   p.frags = p.scratch + gd_scratch_per_cta(r->base.sc.W, r->base.sc.S);
   p.decals = r->decals; p.decalSlots = r->decalSlots; p.decalScratch = r->decalScratch;
   p.resetLanes = reset_lanes; p.resetThings = reset_things; p.finalStack = final_stack;
-  int frames = n;
   if (flags & GD_F_STEP_RESET) {
-    frames = 2 * n;
     gd_final_frames_kernel<<<n, 256, 0, (cudaStream_t)stream>>>(reset_mask, (const uint4 *)stack, (uint4 *)final_stack);
   }
-  return gd_draw(r, p, frames < r->ctas ? frames : r->ctas, stream);
+  return gd_draw(r, p, n, r->ctas, slices, stream);
 }
 
 extern "C" int gd_render_step(const gd_renderer *r, const int32_t *lanes, const void *things, int n, int mask_hud,
@@ -455,7 +461,8 @@ extern "C" int gd_render_step_host(const gd_renderer *r, const int32_t *lanes_ho
         attr.devicePointer != nullptr && (((uintptr_t)attr.devicePointer) & 15) == 0) {
       int flags = GD_F_STACK_ROLL | (mask_hud ? GD_F_MASK_HUD : GD_F_DRAW_HUD);
       return gd_launch(r, lanes_dev, (const gd_thing *)things_dev, n, flags, stack, nullptr,
-                       (uint8_t *)attr.devicePointer, nullptr, nullptr, scratch, scratch_bytes, status, stream);
+                       (uint8_t *)attr.devicePointer, nullptr, nullptr, scratch, scratch_bytes, status, stream, 0, nullptr, nullptr,
+                       nullptr, false);    /* whole frames: a slice's would cross the bus in runs of 21 bytes */
     }
     cudaGetLastError();
   }
@@ -556,9 +563,7 @@ extern "C" int gd_render_step_static(const gd_renderer *r, const int32_t *lanes,
   p.queueOffset = GD_STATIC_QUEUE;
   p.sides = (GdSide *)(scratch + GD_STATIC_SIDES);
   p.decals = r->decals; p.decalSlots = r->decalSlots; p.decalScratch = r->decalScratch;
-  int grid = n < r->ctas ? n : r->ctas;
-  if (grid > GD_STATIC_MAX_CTAS) grid = GD_STATIC_MAX_CTAS;
-  return gd_draw(r, p, grid, stream);
+  return gd_draw(r, p, n, r->ctas < GD_STATIC_MAX_CTAS ? r->ctas : GD_STATIC_MAX_CTAS, true, stream);
 }
 
 /* ---- diagnostic: the device's float32 libm on caller-given arguments -------------------- */

@@ -131,8 +131,9 @@ __device__ __noinline__ void gd_decals(const GdScene &sc_, const GdView &v_, con
   const bool haveMasked = sc.M > 0 && isfinite(sh.maskedDist[x]);
   const int maskedA = haveMasked ? (int)(sh.maskedInfo[x] & 255u) : 0, maskedB = haveMasked ? (int)((sh.maskedInfo[x] >> 8) & 255u) : 0;
   const float maskedDepth = haveMasked ? sh.maskedDist[x] : GD_INF;
+  const int chips = x >= sh.misc[14] && x < sh.misc[15] ? n : 0;
 #pragma unroll 1
-  for (int k = 0; k < n; ++k) {
+  for (int k = 0; k < chips; ++k) {
     const unsigned span = spans[k];
     if (x < (int)(span & 0xFFFFu) || x >= (int)(span >> 16)) continue;
     const GdDecalProj &d = proj[ranked[k]];

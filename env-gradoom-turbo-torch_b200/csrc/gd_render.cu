@@ -65,6 +65,7 @@ struct GdParams {
   const int32_t *resetLanes; /* GD_F_STEP_RESET: the records that the resets are drawn from ... */
   const gd_thing *resetThings;
   uint8_t *finalStack;       /* ... and the stacks as the step left them */
+  int sliceShift;            /* a lane is drawn by 1 << sliceShift CTAs, each a slice of its columns */
   uint8_t *obsOut;           /* n x 84 x 84, optional */
   uint8_t *indexedOut;       /* n x 240 x 320, optional */
   uint8_t *rgbOut;           /* n x 240 x 320 x 3, optional */
@@ -291,7 +292,8 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     __syncthreads();
     /* a launch that steps and resets has both frames in one queue, the resets' first: as a launch of their own they
      * waited for the slowest lane of the step (256 environment lanes 584 us a call, now 511; 1024 lanes 1227 and 1042) */
-    int l = nextLane;
+    const int sliceShift = kPlain ? 0 : p.sliceShift;
+    int l = nextLane >> sliceShift;
     const bool both = !kPlain && (p.flags & GD_F_STEP_RESET) != 0;
     if (l >= (both ? 2 * p.n : p.n)) break;
     const bool fill = both ? l < p.n : (p.flags & GD_F_STACK_FILL) != 0;
@@ -300,7 +302,11 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     const gd_thing *things = (both && fill ? p.resetThings : p.things) + (size_t)l * p.maxThings;
     if (tid < GD_LANE_WORDS) sh.lane[tid] = (both && fill ? p.resetLanes : p.lanes)[(size_t)l * GD_LANE_WORDS + tid];
     if (tid < GD_OWNER_WORDS) sh.ownerMask[tid] = 0;
-    if (tid == 0) sh.misc[1] = sh.misc[2] = 0;
+    if (tid == 0) {
+      sh.misc[1] = sh.misc[2] = 0;
+      sh.misc[14] = GD_SW * (nextLane & ((1 << sliceShift) - 1)) >> sliceShift;     /* the slice's columns */
+      sh.misc[15] = sh.misc[14] + (GD_SW >> sliceShift);
+    }
     /* sector of every thing and of the player (slot 64): lowest index that
      * contains the point (engine.py:9598-9617), found by warps 1 to 9
      * while thread 0 sets up the view */
@@ -438,10 +444,11 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     }
     gd_mark_afterlife_columns(sc, sh);
     if (p.flags & GD_F_DRAW_HUD) gd_hud_list(sc, sh.lane, (int4 *)sh.hitA);   /* the sectors of points have been read */
-    ((unsigned long long *)(gd_smem + GD_OFF_CAND))[tid] = gd_sprite_candidates(sc, v, sh, nThings, frustumList, frustumListed);
+    const bool mine = kPlain || (tid >= sh.misc[14] && tid < sh.misc[15]);
+    ((unsigned long long *)(gd_smem + GD_OFF_CAND))[tid] = !mine ? 0ull : gd_sprite_candidates(sc, v, sh, nThings, frustumList, frustumListed);
     __syncthreads();
-    const bool open = gd_walk<kSplit, kChip>(p, sc, v, sh, frame, tables, events, eventCount, rowproj, sh.misc[0]);
-    if (p.flags & GD_F_DRAW_HUD) gd_hud_column(sc, (const int4 *)sh.hitA, frame + GD_VH * GD_SW);
+    const bool open = gd_walk<kSplit, kChip>(p, sc, v, sh, frame, tables, events, eventCount, rowproj, sh.misc[0], mine);
+    if (mine && (p.flags & GD_F_DRAW_HUD)) gd_hud_column(sc, (const int4 *)sh.hitA, frame + GD_VH * GD_SW);
     __syncthreads();
     /* Rows no seg ever claimed show the per-pixel flat fallback.  They are
      * queued (the first aux area is free once every column has finished its walk)
@@ -473,7 +480,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       __syncthreads();
     }
     if (sc.M > 0) {
-      gd_masked_pass<kSplit>(sc, v, sh);
+      if (mine) gd_masked_pass<kSplit>(sc, v, sh);
       __syncthreads();
     }
 #ifndef GD_NO_DECALS
@@ -483,7 +490,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
 #endif
     gd_sprites(sc, v, sh, events, eventCount, nThings);
     __syncthreads();
-    gd_weapon(sc, sh.lane, sh.frame);
+    gd_weapon(sc, sh, sh.lane, sh.frame);
     __syncthreads();
     const bool wantFull = p.indexedOut != nullptr || p.rgbOut != nullptr;
     if (wantFull && !(p.flags & GD_F_DRAW_HUD)) {
@@ -491,10 +498,15 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       for (int i = tid; i < GD_HUD_H * GD_SW / 4; i += GD_THREADS) ((unsigned *)(sh.frame + GD_VH * GD_SW))[i] = 0;
       __syncthreads();
     }
+    const int x0 = kPlain ? 0 : sh.misc[14], wide = GD_SW / 16 >> sliceShift;       /* the slice, in groups of sixteen columns */
     if (p.indexedOut) {
       uint4 *dst = (uint4 *)(p.indexedOut + (size_t)l * GD_SCREEN_H * GD_SW);
       const uint4 *src = (const uint4 *)sh.frame;
-      for (int i = tid; i < GD_SCREEN_H * GD_SW / 16; i += GD_THREADS) dst[i] = src[i];
+#pragma unroll 1
+      for (int i = tid; i < GD_SCREEN_H * wide; i += GD_THREADS) {
+        const int q = i / wide * (GD_SW / 16) + x0 / 16 + i % wide;
+        dst[q] = src[q];
+      }
     }
     if (p.rgbOut) {
       /* sixteen pixels (one 16-byte load) become three 16-byte stores (a word at a time: 43 of a lane's 442 thousand
@@ -503,7 +515,8 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
       const uint4 *src = (const uint4 *)sh.frame;
       const unsigned *pal32 = (const unsigned *)(gd_smem + GD_OFF_PAL32);
 #pragma unroll 1
-      for (int q = tid; q < GD_SCREEN_H * GD_SW / 16; q += GD_THREADS) {
+      for (int i = tid; i < GD_SCREEN_H * wide; i += GD_THREADS) {
+        const int q = i / wide * (GD_SW / 16) + x0 / 16 + i % wide;
         const uint4 four = src[q];
         const unsigned idx[4] = {four.x, four.y, four.z, four.w};
         unsigned out[12];
@@ -521,70 +534,24 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     }
     if (p.stack || p.obsOut) {
       int srcRows = (p.flags & GD_F_MASK_HUD) ? GD_VH : GD_SCREEN_H;
-      gd_resize(sh.frame, srcRows, sh.obs);
+      gd_resize<kPlain>(sh.frame, srcRows, sh.obs, x0, sliceShift);
       __syncthreads();
-      const uint4 *src = (const uint4 *)sh.obs;
-      const int vecs = GD_OBS * GD_OBS / 16;  /* 441 */
-      if (p.obsOut) {
-        uint4 *dst = (uint4 *)(p.obsOut + (size_t)l * GD_OBS * GD_OBS);
-#pragma unroll 1
-        for (int i = tid; i < vecs; i += GD_THREADS) dst[i] = src[i];
-      }
+      const size_t frameBytes = GD_OBS * GD_OBS;
+      uint8_t *newest = p.obsOut ? p.obsOut + (size_t)l * frameBytes : nullptr, *stack = nullptr, *final = nullptr;
+      int mode = GD_PUT_NONE;
       if (p.stack && (p.flags & GD_F_STACK_RING)) {
-        /* mirrored ring: no old slot is read or moved */
-        uint4 *s0 = (uint4 *)(p.stack + (size_t)l * 2 * GD_STACK * GD_OBS * GD_OBS);
-        if (p.flags & GD_F_STACK_FILL) {
-#pragma unroll 1
-          for (int i = tid; i < vecs; i += GD_THREADS) {
-            uint4 val = src[i];
-#pragma unroll
-            for (int k = 0; k < 2 * GD_STACK; ++k) s0[k * vecs + i] = val;
-          }
-        } else {
-#pragma unroll 1
-          for (int i = tid; i < vecs; i += GD_THREADS) {
-            uint4 val = src[i];
-            s0[p.ringHead * vecs + i] = val;
-            s0[(p.ringHead + GD_STACK) * vecs + i] = val;
-          }
-        }
+        stack = p.stack + (size_t)l * 2 * GD_STACK * frameBytes;
+        mode = fill ? GD_PUT_ALL8 : GD_PUT_RING;
       } else if (p.stack) {
-        uint4 *s0 = (uint4 *)(p.stack + (size_t)l * GD_STACK * GD_OBS * GD_OBS);
-        if (fill) {
-#pragma unroll 1
-          for (int i = tid; i < vecs; i += GD_THREADS) {
-            uint4 val = src[i];
-            s0[i] = val; s0[vecs + i] = val; s0[2 * vecs + i] = val; s0[3 * vecs + i] = val;
-          }
-        } else if (both) {
-          /* the stack rolls, and what it becomes is copied out; a lane that is reset keeps only the copy, whose
-           * three old frames are there already */
-          uint4 *f0 = (uint4 *)(p.finalStack + (size_t)l * GD_STACK * GD_OBS * GD_OBS);
-          const bool ends = p.resetMask[l] != 0;
-#pragma unroll 1
-          for (int i = tid; i < vecs; i += GD_THREADS) {
-            const uint4 val = src[i];
-            f0[3 * vecs + i] = val;
-            if (ends) continue;
-            const uint4 a = s0[vecs + i], b = s0[2 * vecs + i], c = s0[3 * vecs + i];
-            f0[i] = s0[i] = a;
-            f0[vecs + i] = s0[vecs + i] = b;
-            f0[2 * vecs + i] = s0[2 * vecs + i] = c;
-            s0[3 * vecs + i] = val;
-          }
-        } else if (p.flags & GD_F_STACK_ROLL) {
-#pragma unroll 1
-          for (int i = tid; i < vecs; i += GD_THREADS) {
-            s0[i] = s0[vecs + i];
-            s0[vecs + i] = s0[2 * vecs + i];
-            s0[2 * vecs + i] = s0[3 * vecs + i];
-            s0[3 * vecs + i] = src[i];
-          }
-        } else {
-#pragma unroll 1
-          for (int i = tid; i < vecs; i += GD_THREADS) s0[3 * vecs + i] = src[i];
+        stack = p.stack + (size_t)l * GD_STACK * frameBytes;
+        mode = fill ? GD_PUT_ALL : ((p.flags & GD_F_STACK_ROLL) ? GD_PUT_ROLL : GD_PUT_LAST);
+        if (both && !fill) {
+          final = p.finalStack + (size_t)l * GD_STACK * frameBytes;
+          mode = p.resetMask[l] ? GD_PUT_FINAL_LAST : GD_PUT_ROLL_FINAL;
         }
       }
+      if (kPlain || sliceShift == 0) gd_put_frame<uint4>(sh.obs, stack, final, newest, mode, p.ringHead, 0, 0);
+      else gd_put_frame<uint8_t>(sh.obs, stack, final, newest, mode, p.ringHead, x0 * GD_OBS / GD_SW, GD_OBS >> sliceShift);
     }
   }
   if (tid == 0) {

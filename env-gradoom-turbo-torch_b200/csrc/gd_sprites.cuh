@@ -238,8 +238,9 @@ __device__ void gd_sprites(const GdScene &sc_, const GdView &v_, const GdShared 
 
 /* ---- phase: weapon (engine.py:14994-15121) ------------------------------ */
 #define GD_WEAPON_ROWS 4
-__device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, uint8_t *frame, int id, i64 hoff, i64 voff) {
+__device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, const GdShared &sh_, uint8_t *frame, int id, i64 hoff, i64 voff) {
   const GdScene &sc = *gd_as_shared(&sc_);
+  const GdShared &sh = *gd_as_shared(&sh_);
 #ifdef GD_CHECKED
   if (id >= sc.Q || id < -1) { if (threadIdx.x == 0) atomicOr(gdCheckedStatus, GD_STATUS_BAD_INDEX); }
 #endif
@@ -262,7 +263,7 @@ __device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, uint8_t *frame,
 #pragma unroll 1
   for (int sx = threadIdx.x & 31; sx < w; sx += 32) {
     const i64 xx = screenLeft + sx;
-    if (xx < 0 || xx >= GD_SW) continue;
+    if (xx < sh.misc[14] || xx >= sh.misc[15]) continue;
     const int cx = min(sx, sc.wpnW - 1);
 #pragma unroll 1
     for (int y = y0 + (threadIdx.x >> 5); y < y1; y += GD_WARPS * GD_WEAPON_ROWS) {
@@ -284,7 +285,7 @@ __device__ __noinline__ void gd_weapon_patch(const GdScene &sc_, uint8_t *frame,
   }
 }
 
-__device__ void gd_weapon(const GdScene &sc_, const int32_t *lane, uint8_t *frame) {
+__device__ void gd_weapon(const GdScene &sc_, const GdShared &sh, const int32_t *lane, uint8_t *frame) {
   const GdScene &sc = *gd_as_shared(&sc_);
   if (!sc.wpnAvailable) return;
   if (lane[GD_L_FLAGS] & 1) return;
@@ -305,9 +306,9 @@ __device__ void gd_weapon(const GdScene &sc_, const int32_t *lane, uint8_t *fram
   i64 boby = (bob * sc.fineSine[bobAngle & 4095]) >> 16;
   if (!ready) { bobx = 0; boby = 0; }
   i64 voff = verticalTics * 6 * GD_FU + boby;
-  gd_weapon_patch(sc, frame, frameId, bobx, voff);
+  gd_weapon_patch(sc, sh, frame, frameId, bobx, voff);
   __syncthreads();
-  if (flashId >= 0) gd_weapon_patch(sc, frame, flashId, bobx, voff);
+  if (flashId >= 0) gd_weapon_patch(sc, sh, frame, flashId, bobx, voff);
 }
 
 /* ---- phase: status bar (engine.py:15158-15267) --------------------------- */

@@ -824,8 +824,8 @@ __device__ void gd_mark_afterlife_columns(const GdScene &sc, const GdShared &sh)
 }
 
 /* ---- phase: per-column portal walk (engine.py:11561-13371) -------------- */
-/* Thread x walks column x front to back; true: the column's mask tells which of its rows are claimed, else all
- * are.  Nearly every crossing is plain: nothing is carried over from the one
+/* Thread x walks column x front to back; true: it is one of the slice's, and its mask tells which of its
+ * rows are claimed; else all are.  Nearly every crossing is plain: nothing is carried over from the one
  * before, and the nearest wall of the current sector is both crossed by the column's ray and owned by its
  * projected span.  None of the ownership rules can then change the outcome: the owner rules ask for a selected
  * wall that is not projected here (engine.py:11589-11730, 11905-12164), the endpoint rules for one that is not
@@ -905,7 +905,7 @@ __device__ __noinline__ uint3 gd_rows_outside(const GdView &v_, const GdWall &wv
 
 template <bool kSplit, bool kChip>
 __device__ __forceinline__ bool gd_walk(const GdParams &p, const GdScene &sc, const GdView &v, const GdShared &sh, uint8_t *frame,
-                                        uint8_t *tables, GdEvent *events, int *eventCount, const GdRowProj *rowproj, int startSector) {
+                                        uint8_t *tables, GdEvent *events, int *eventCount, const GdRowProj *rowproj, int startSector, bool mine) {
   const int x = threadIdx.x;
   const int quadBase = x & 28;
   const unsigned quad = 15u << quadBase;
@@ -935,7 +935,7 @@ __device__ __forceinline__ bool gd_walk(const GdParams &p, const GdScene &sc, co
   GdCross o;
   int cur = startSector, ceilClip = 0, floorClip = GD_VH;
   float prev = 0.0f;
-  bool pend = false, settled = false;
+  bool pend = false, settled = !mine;
   bool pendEnd = false;             /* all that is pending is that the last crossing met a wall's end only */
   const unsigned *columns = (const unsigned *)(gd_smem + GD_OFF_OWNER) + (x >> 5);
   const bool spanStarts = (columns[32] >> (x & 31)) & 1u;         /* some wall's projected span starts here */
@@ -1231,7 +1231,7 @@ __device__ __forceinline__ bool gd_walk(const GdParams &p, const GdScene &sc, co
   }
   eventCount[x] = nEvents < GD_MAX_EVENTS ? nEvents : GD_MAX_EVENTS;
   if (nEvents > GD_MAX_EVENTS) atomicOr(p.status, GD_STATUS_EVENT_OVERFLOW);
-  const bool open = top < bottom || top < 0;
+  const bool open = mine && (top < bottom || top < 0);
   if (open) gd_claimed_rows(sh, x, top, bottom);
   return open;
 }
