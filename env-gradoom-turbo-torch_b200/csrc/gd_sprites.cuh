@@ -402,11 +402,10 @@ __device__ __noinline__ void gd_hud_list(const GdScene &sc_, const int32_t *lane
   entries[t] = make_int4(tx | (ty << 16), cw | (ch << 16), sx | (sy << 16), e.x < 0 ? 0 : e.x);
 }
 
-/* Column threadIdx.x of the status bar; the list is complete. */
-__device__ __noinline__ void gd_hud_column(const GdScene &sc_, const int4 *entries_, uint8_t *canvas) {
+/* Column x of the status bar; the list is complete. */
+__device__ __noinline__ void gd_hud_column(const GdScene &sc_, const int4 *entries_, uint8_t *canvas, int x) {
   const GdScene &sc = *gd_as_shared(&sc_);
   const int4 *entries = gd_as_shared(entries_);
-  const int x = threadIdx.x;
   unsigned long long mine = 0;                         /* entries that cross this column */
 #pragma unroll 1
   for (int k = 0; k < GD_HUD_PATCHES; ++k) {
