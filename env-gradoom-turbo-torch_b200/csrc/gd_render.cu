@@ -2,12 +2,14 @@
  * Fused render-to-observation kernel for sm_100a.
  *
  * One persistent CTA of 320 threads draws one environment lane at a time, two
- * CTAs to an SM:
+ * CTAs to an SM (four of them a lane, each a quarter of its columns, when the
+ * lanes are few):
  *   1. the walls that a column ray may cross are listed and projected once per
  *      lane, and their ray-owned column spans found at the projections of their
  *      ends (by warps that try all 320 rays where an end is too close);
  *   2. thread x then walks column x front to back through the sector portals,
- *      keeping the ceiling / floor clip pair in registers, drawing wall tiers
+ *      keeping the ceiling / floor clip pair and the rows claimed so far in
+ *      registers, drawing wall tiers
  *      and the visplane rows they uncover straight into the palette-indexed
  *      frame (aligned groups of four columns exchange their tier bounds with
  *      warp shuffles);
@@ -32,7 +34,10 @@
  * 0.9 to 5.0 per issue).  With the plain crossings decided apart from the full
  * set of rules and the walk's tables in 16-byte records, two CTAs per SM took
  * 3.99 and 20.2 ms; with a sixth of the code and the full searches of sprite and
- * fallback pixels gone, 3.4 and 15.2 ms.
+ * fallback pixels gone, 3.4 and 15.2 ms; with claims drawn as runs, the repair of
+ * unclaimed pixels kept to the columns near them, and shorter setups, sprites and
+ * resize, 3.0 and 13.5 ms.  Drawing apart from the walk, from lists of runs, took
+ * 15 to 40 % more; more warps with fewer registers 11 % more.
  *
  * The arithmetic restates src/gradoom/engine.py (file:line beside each
  * function) and must stay bit-identical to it; compile with -fmad=false.
@@ -137,7 +142,8 @@ struct GdActor {
                                                               projected span starts here */
 #define GD_OWNER_WORDS 48
 #define GD_OFF_MISC (GD_OFF_OWNER + GD_OWNER_WORDS * 4)                   /* 16 ints: start sector, fallback queue length, its unresolved
-                                                              rows' range, GdFlatBounds */
+                                                              rows' range, GdFlatBounds, counters of the fallback; 14, 15: the slice's
+                                                              columns */
 #define GD_OFF_MASKS (GD_OFF_MISC + 64)                    /* 7 x 320: per-column row bitmasks */
 #define GD_OFF_MASKED_DIST (GD_OFF_MASKS + 7 * 320 * 4)   /* 320: nearest masked drawseg of the column ... */
 #define GD_OFF_MASKED_INFO (GD_OFF_MASKED_DIST + 320 * 4)  /* ... its wall << 16 | ceiling clip << 8 | floor clip; 0xFFFF0000 | .. = none */
@@ -459,7 +465,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_c
     /* Rows no seg ever claimed show the per-pixel flat fallback.  They are
      * queued (the first aux area is free once every column has finished its walk)
      * and resolved; a frame with more such pixels than the queue holds takes
-     * several rounds, each pass marking what it drew as owned. */
+     * several rounds, each pass marking what it drew as claimed. */
     bool sweepDone = false;                          /* CTA-uniform */
     for (;;) {
       const unsigned *claimed = sh.masks + tid;

@@ -111,8 +111,7 @@ __device__ __forceinline__ unsigned gd_plane_pixel_narrow(const GdNarrowSpan &p,
   return gd_smem[GD_OFF_COLORMAP + shade * 256 + texel];
 }
 
-/* The 208-row column masks live in shared memory, one word column per screen
- * column: word k of column x is m[k * GD_SW]. */
+/* A column's mask of 208 rows is one word column in shared memory: word k of column x is m[k * GD_SW]. */
 /* bits of mask word k (rows 32k..32k+31) that lie in rows [a,b) */
 __device__ __forceinline__ unsigned gd_range_word(int k, int a, int b) {
   int lo = max(a - (k << 5), 0), hi = min(b - (k << 5), 32);
