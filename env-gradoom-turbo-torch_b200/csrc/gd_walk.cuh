@@ -1127,6 +1127,9 @@ __device__ __forceinline__ bool gd_walk(const GdParams &p, const GdScene &sc, co
       const bool oneSided = (flags & GD_C_ONE_SIDED) != 0;
       const bool lowRange = !oneSided && (flags & GD_C_LOWER) && clowtop < cbot, upRange = !oneSided && (flags & GD_C_UPPER) && ctop < cupbot;
       if (flags & (GD_C_TIER0 | GD_C_TIER1 | GD_C_TIER2)) {
+        /* the sector beyond has its ceiling below its floor: the rows that both ranges hold are the lower one's, drawn or
+         * not, and take the second shade of either, so neither tier is one run */
+        const bool meet = lowRange && upRange && clowtop < cupbot;
         const i64 repeat = sd.repeat;
         i64 hoff, vstepBase;
         gd_prep_eval(prep[wall], repeat, x, hoff, vstepBase);
@@ -1168,7 +1171,7 @@ __device__ __forceinline__ bool gd_walk(const GdParams &p, const GdScene &sc, co
           t.step = (unsigned)vstep;
           t.texel = ((unsigned)texId * (unsigned)p.sc.texW + u) * (unsigned)p.sc.texH;
           t.shift = 32 - hbits;
-          if (!gd_claim_fits(top, bottom, ya, yb, upper || oneSided)) {
+          if (meet || !gd_claim_fits(top, bottom, ya, yb, upper || oneSided)) {
             const bool otherTail = !upper && !oneSided && upRange && group2 && shadeN != shadeT;
             const unsigned oTailA = otherTail ? (unsigned)max(ctop, gb2) : 0u, oTailB = otherTail ? (unsigned)cupbot : 0u;
             gd_loose_claim(sc, v, sh, x, top < 0 ? -1 : top | (bottom << 8), -1, t,

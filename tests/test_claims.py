@@ -44,3 +44,58 @@ def test_views_from_lines_and_corners(oracle, config, changes):
         assert np.array_equal(obs.cpu().numpy(), want["obs"])
     r.check_status()
     r.close()
+
+
+@pytest.mark.parametrize("lower", ["as packed", "on some lines", "on no line"])
+@pytest.mark.parametrize("config,changes", [
+    ("c1", {"floor_max": 160, "ceil_lo": 96}), ("c2", {"ceil_lo": 96}), ("c1m", {"floor_max": 160, "ceil_lo": 96}),
+    ("c4s", {"rows": 4, "cols": 4, "floor_max": 160, "ceil_lo": 96})])
+def test_tiers_of_a_line_that_share_rows(oracle, config, changes, lower):
+    """Sectors whose ceiling lies below their floor, seen from rooms that reach farther down and up: the line between has
+    an upper and a lower tier in the same rows.  Those are the lower tier's, or nobody's where it has no texture."""
+
+    spec = dataclasses.replace(gdscene.GRID_CONFIGS[config], **changes)
+    sc = gdscene.make_grid_scene(spec)
+    rng = np.random.default_rng(4)
+    if lower != "as packed":
+        bare = rng.random(sc.side_textures.shape[:2]) < (0.5 if lower == "on some lines" else 1.0)
+        sc.side_textures[..., 1][bare] = -1
+    blob = gdscene.pack_scene(sc)
+    sides = []                               # of lines with such a sector beyond: line, side, lowest and highest shared height
+    for wall, pair in enumerate(sc.wall_sectors):
+        for side in range(2):
+            if pair[1] < 0 or pair[0] == pair[1]:
+                continue
+            (floor, ceil), (floor2, ceil2) = sc.sector_heights[pair[side]], sc.sector_heights[pair[1 - side]]
+            if ceil - floor >= 56 and floor < floor2 and ceil > ceil2 and max(floor, ceil2) < min(floor2, ceil):
+                sides.append((wall, side, max(floor, ceil2), min(floor2, ceil)))
+    assert sides
+    n, k = 96, 5
+    lanes, things = stepper.random_lanes(sc, n, k, seed=6)
+    lf, shared = lanes.view(np.float32), 0
+    for lane in range(n):
+        wall, side, low, high = sides[lane % len(sides)]
+        x1, y1, x2, y2 = (float(c) for c in sc.walls[wall])
+        nx, ny = np.array([y2 - y1, x1 - x2]) / np.hypot(x2 - x1, y2 - y1) * (1 if side == 0 else -1)
+        away, along = rng.uniform(24, spec.room - 24), rng.uniform(0.2, 0.8)
+        bam = int((np.arctan2(-ny, -nx) + rng.uniform(-0.4, 0.4)) / (2 * np.pi) * 2 ** 32) % 2 ** 32
+        for place, fixed, word in ((x1 + along * (x2 - x1) + away * nx, gdstate.L_X_FIXED, gdstate.L_X),
+                                   (y1 + along * (y2 - y1) + away * ny, gdstate.L_Y_FIXED, gdstate.L_Y)):
+            lanes[lane, fixed] = round(place * 65536)
+            lf[lane, word] = np.float32(lanes[lane, fixed]) / np.float32(65536)
+        lanes[lane, gdstate.L_ANGLE_BAM] = np.uint32(bam).view(np.int32)
+        lf[lane, gdstate.L_ANGLE] = np.float32(bam) * np.float32(gdstate.BAM_TO_RADIANS)
+        lf[lane, gdstate.L_VIEW_Z] = sc.sector_heights[sc.wall_sectors[wall, side], 0] + stepper.VIEW_HEIGHT
+        rows = np.clip(104 - (np.array([high, low]) - lf[lane, gdstate.L_VIEW_Z]) * 192 / away, 0, 208)
+        shared += bool(rows[1] - rows[0] >= 2)
+    assert shared >= n // 3, shared          # the tiers do meet in the middle of the view
+    r = native.Renderer(blob, DEV, k)
+    for count in (n, 20):                    # whole lanes, and few enough for slices of them
+        part = [np.ascontiguousarray(a[:count]) for a in (lanes, things)]
+        want = oracle.render(blob, *part, mask_hud=True)
+        obs, indexed, _ = r.frames(*(torch.from_numpy(a).to(DEV) for a in part), obs=True, indexed=True, mask_hud=True, include_hud=False)
+        wrong = (indexed.cpu().numpy()[:, :208] != want["indexed"][:, :208]).any(axis=(1, 2))
+        assert not wrong.any(), (np.nonzero(wrong)[0], shared)
+        assert np.array_equal(obs.cpu().numpy(), want["obs"])
+    r.check_status()
+    r.close()
