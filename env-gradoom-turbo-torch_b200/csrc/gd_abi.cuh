@@ -64,6 +64,7 @@ extern "C" const char *gd_error_string(int code) {
     case GD_ERR_SHARED: return "scene needs more shared memory than one SM offers";
     case GD_ERR_STATIC_LIMIT: return "scene or device index exceeds the limits of the built-in scratch array";
     case GD_ERR_DEVICE: return "the renderer's device is not the current CUDA device";
+    case GD_ERR_OVERLAP: return "the stack and the final stack overlap";
     default: return "unknown error";
   }
 }
@@ -397,6 +398,10 @@ extern "C" int gd_render_step_reset(const gd_renderer *r, const int32_t *lanes, 
   if (r && n == 0) return GD_OK;   /* an empty batch needs no buffers */
   if (!r || !stack || !final_stack || !reset_mask || !reset_lanes) return GD_ERR_NULL;
   if (r->maxThings > 0 && !reset_things) return GD_ERR_NULL;
+  if (n < 0) return GD_ERR_SIZE;
+  /* a lane's step and its reset are drawn in any order and at the same time, the one into both stacks */
+  const uintptr_t bytes = (uintptr_t)n * GD_STACK * GD_OBS * GD_OBS, a = (uintptr_t)stack, b = (uintptr_t)final_stack;
+  if ((a < b ? b - a : a - b) < bytes) return GD_ERR_OVERLAP;
   int flags = GD_F_STEP_RESET | (mask_hud ? GD_F_MASK_HUD : GD_F_DRAW_HUD);
   return gd_launch(r, lanes, (const gd_thing *)things, n, flags, stack, reset_mask, nullptr, nullptr, nullptr, scratch,
                    scratch_bytes, status, stream, 0, reset_lanes, (const gd_thing *)reset_things, final_stack);

@@ -42,7 +42,8 @@ enum gd_error {
   GD_ERR_SCRATCH = -7,
   GD_ERR_SHARED = -8,
   GD_ERR_STATIC_LIMIT = -9,
-  GD_ERR_DEVICE = -10
+  GD_ERR_DEVICE = -10,
+  GD_ERR_OVERLAP = -11
 };
 
 /* device status bits */
@@ -136,7 +137,7 @@ int gd_render_reset(const gd_renderer *r, const int32_t *lanes, const void *thin
  * A step of every lane and a reset of the lanes whose `reset_mask` byte is nonzero, in one launch of the drawing
  * kernel: what gd_render_step with `lanes` / `things` does, then a copy of the whole stack to `final_stack` (n x 4 x
  * 84 x 84 u8), then gd_render_reset with `reset_lanes` / `reset_things` (all n records; those of the masked lanes are
- * read).  `final_stack` must not overlap the stack.  A bound decal ring belongs to both frames of its lane.
+ * read).  `final_stack` must not overlap the stack (GD_ERR_OVERLAP).  A bound decal ring belongs to both frames of its lane.
  * Replaces: the step, the copy and the reset of step_and_reset_device (src/gradoom/env.py:998-1031).
  */
 int gd_render_step_reset(const gd_renderer *r, const int32_t *lanes, const void *things, const int32_t *reset_lanes,

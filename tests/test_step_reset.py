@@ -77,3 +77,24 @@ def test_environment_takes_either_route(scenes, options):
     b.close()
     with pytest.raises(RuntimeError):
         a.step_and_reset_device(actions, seeds)
+
+
+def test_final_stack_over_the_stack_is_refused(scenes):
+    sc, blob = scenes("c1")
+    n = 5
+    r = native.Renderer(blob, DEV, 0)
+    part = [torch.from_numpy(a).to(DEV) for a in stepper.random_lanes(sc, n, 0, seed=1)]
+    mask = torch.tensor([True, False, True, False, False], device=DEV)
+    both = torch.full((2 * n, 4, 84, 84), 9, dtype=torch.uint8, device=DEV)
+    for a, b in ((0, 0), (0, 1), (0, n - 1), (n - 1, 0), (n, 1)):
+        with pytest.raises(native.NativeError, match="overlap"):
+            r.step_reset(*part, *part, mask, both[a:a + n], both[b:b + n])
+    assert bool((both == 9).all())
+    for a, b in ((0, n), (n, 0)):            # one behind the other is accepted
+        want = both[a:a + n].clone()
+        r.step(*part, want)
+        final = want.clone()
+        r.reset(*part, mask, want)
+        r.step_reset(*part, *part, mask, both[a:a + n], both[b:b + n])
+        assert torch.equal(both[a:a + n], want) and torch.equal(both[b:b + n], final)
+    r.close()
