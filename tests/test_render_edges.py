@@ -94,3 +94,12 @@ def test_status_bar_numbers(pkg, oracle, scenes):
     for word in range(gdstate.L_AMMO0, gdstate.L_AMMO3 + 1):
         lf[:, word] = np.roll(values, 3 * word)
     _equal(oracle, sc, lanes, things, 0)
+
+
+@pytest.mark.parametrize("config,things,seed,rows", [("c4s", 24, 5, (2, 83, 224, 275)), ("c2", 12, 5, (2, 99, 100))])
+def test_planes_on_both_sides_of_the_horizon(pkg, oracle, scenes, config, things, seed, rows):
+    """Views whose whole columns are one floor or ceiling: its span has rows at the horizon, which need 64 bits."""
+
+    sc, _ = scenes(config)
+    lanes, records = (a[list(rows)] for a in stepper.random_lanes(sc, 300, things, seed=seed))
+    _equal(oracle, sc, np.ascontiguousarray(lanes), np.ascontiguousarray(records), things)
