@@ -103,3 +103,25 @@ def test_planes_on_both_sides_of_the_horizon(pkg, oracle, scenes, config, things
     sc, _ = scenes(config)
     lanes, records = (a[list(rows)] for a in stepper.random_lanes(sc, 300, things, seed=seed))
     _equal(oracle, sc, np.ascontiguousarray(lanes), np.ascontiguousarray(records), things)
+
+
+@pytest.mark.parametrize("config,things,rows", [("c4s", 24, (292,)), ("c2", 12, (95, 113)), ("c2", 12, ())])
+def test_unclaimed_pixels_far_from_their_anchors(pkg, oracle, scenes, config, things, rows):
+    """Unclaimed pixels that the columns near them do not decide, so that all 320 are repaired; without `rows`, viewers
+    outside the map at many headings, of whose columns none to all find a resolved row below."""
+
+    sc, _ = scenes(config)
+    lanes, records = stepper.random_lanes(sc, 300, things, seed=5)
+    lanes, records = (np.ascontiguousarray(a[list(rows)] if rows else a[:16]) for a in (lanes, records))
+    if not rows:
+        _place(lanes, slice(0, 16), np.tile([-20.0, -90.0, 700.0, 1500.0], 4), np.repeat([-15.0, -200.0, 2060.0, 2300.0], 4))
+    _equal(oracle, sc, lanes, records, things)          # slices of a lane
+    blob = gdscene.pack_scene(sc)
+    want = oracle.render(blob, lanes, records, mask_hud=False)["indexed"]
+    renderer = native.Renderer(blob, DEV, things)       # as many copies as are drawn whole
+    copies = renderer.ctas // 4 // len(lanes) + 1
+    many = [torch.from_numpy(np.tile(a, (copies,) + (1,) * (a.ndim - 1))).to(DEV) for a in (lanes, records)]
+    _, indexed, _ = renderer.frames(*many, indexed=True, mask_hud=False)
+    renderer.check_status()
+    assert np.array_equal(indexed.cpu().numpy(), np.tile(want, (copies, 1, 1)))
+    renderer.close()
