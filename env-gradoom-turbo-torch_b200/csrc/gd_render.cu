@@ -21,7 +21,7 @@
  *      four-frame stack; the RGB24 frame is written only when asked for.
  * Only the lane record, the thing records and the stack slots have to cross
  * HBM; the indexed frame, the clip events and the CTA's tables lie in scratch,
- * most of which L2 holds (4096 lanes of the 64-sector map move 415 MB, 202 of them
+ * most of which L2 holds (4096 lanes of the 64-sector map move 435 MB, 202 of them
  * the stack's: 2 % of what HBM moves in that time).
  * Tensor cores are unused: nothing here is a contraction.
  *
@@ -204,7 +204,7 @@ __device__ __forceinline__ int gd_vertex(const GdScene &sc, int w, int slot) { r
 
 /* kSplit: the scene carries projection fragments of split lines.  kChip: the walk's tables fit in shared memory
  * beside a second CTA.  kPlain: every task is one frame of a lane (the code for the other launches costs a step of 4096
- * lanes 2 % and more, which only the calls that want it should pay). */
+ * lanes 4 %, 3015 and 3133 us, and the 256-sector map 3 %, which only the calls that want it should pay). */
 template <bool kSplit, bool kChip, bool kPlain>
 __global__ void __launch_bounds__(GD_THREADS, 2) gd_render_kernel(const __grid_constant__ GdParams p) {
   /* The scene descriptor, the shared-memory map and the lane's view are read by

@@ -522,7 +522,7 @@ class GraDoomVecEnv:
         reset, rings, chips, and seeds that will be refused take the two calls one after the other.
 
         So do more than _ONE_LAUNCH_LANES lanes.  The joined launch saves the time of the slowest restarted lane (0.2
-        to 0.4 ms) and its kernel draws each frame 3 to 5 % slower, which evens out there.  Microseconds a call, two
+        to 0.4 ms) and its kernel draws each frame 3 to 4 % slower, which evens out there.  Microseconds a call, two
         launches / one, with 0.4 % of the lanes restarted: 64 sectors 836 / 724 at 512 lanes, 2012 / 1929 at 2048,
         3449 / 3438 at 4096, 6306 / 6475 at 8192; 256 sectors 1827 / 1567 at 512, 7736 / 7664 at 4096."""
 
