@@ -21,7 +21,7 @@
  *      four-frame stack; the RGB24 frame is written only when asked for.
  * Only the lane record, the thing records and the stack slots have to cross
  * HBM; the indexed frame, the clip events and the CTA's tables lie in scratch,
- * most of which L2 holds (4096 lanes of the 64-sector map move 435 MB, 202 of them
+ * most of which L2 holds (4096 lanes of the 64-sector map move about 437 MB, 202 of them
  * the stack's: 2 % of what HBM moves in that time).
  * Tensor cores are unused: nothing here is a contraction.
  *
